@@ -688,7 +688,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
 
     // ---- gated: delta of this key row, its extremes over the key tile, running gate bound --------
     // (flash_sparse_attn/ops/triton/flash_gated_bwd.py:406-421; keys past the sequence read as zero)
-    float dlt = 0.f, d_max = 0.f, d_min = 0.f, dd_acc = 0.f, gate_max = -INFINITY;
+    float dlt = 0.f, d_max = 0.f, d_min = 0.f, gate_max = -INFINITY;
+    float2 dd_acc = make_float2(0.f, 0.f);  // even / odd query columns
     const bool logsig = p.flags & F_LOGSIGMOID;
     const float lg_thr = p.softmax_thr > 0.f ? log2f(p.softmax_thr) : -INFINITY;  // for the skip thresholds
     if (KIND == KIND_GATED) {
@@ -710,6 +711,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
       d_max = mx;
       d_min = mn;
     }
+    const float dlt_g = logsig ? dlt * 1.4426950408889634f : dlt;
     auto unpack16 = [&](uint32_t v, float& lo, float& hi) {
       if (IS_BF16) {
         lo = __uint_as_float(v << 16);
@@ -825,21 +827,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
       if (KIND == KIND_GATED) {
         // logits = (q.k + g(alpha_q * delta_k)) * scale, g = logsigmoid or identity (flash_gated_bwd.py:81-98)
         const uint4* al4 = reinterpret_cast<const uint4*>(s_alpha + st * 128 + wg * 64);
+        const float2 dl2 = make_float2(dlt_g, dlt_g);  // delta, times log2(e) for the logsigmoid gate
 #pragma unroll
         for (int i = 0; i < 64; i += 8) {
           const uint4 av = al4[i >> 3];
-          float a8[8];
-          unpack16(av.x, a8[0], a8[1]);
-          unpack16(av.y, a8[2], a8[3]);
-          unpack16(av.z, a8[4], a8[5]);
-          unpack16(av.w, a8[6], a8[7]);
+          const uint32_t aw[4] = {av.x, av.y, av.z, av.w};
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float gx = a8[j] * dlt;
-            float gte = gx;
-            if (logsig)
-              gte = log_sigmoid_fast(gx);
-            sr[i + j] = __float_as_uint(__uint_as_float(sr[i + j]) + gte);
+          for (int j = 0; j < 8; j += 2) {
+            float a0, a1;
+            unpack16(aw[j >> 1], a0, a1);
+            const float2 y = mul2(make_float2(a0, a1), dl2);
+            const float2 s2 = make_float2(__uint_as_float(sr[i + j]), __uint_as_float(sr[i + j + 1]));
+            const float2 r = logsig ? add_log_sigmoid2(s2, y) : add2(s2, y);
+            sr[i + j] = __float_as_uint(r.x);
+            sr[i + j + 1] = __float_as_uint(r.y);
           }
         }
       }
@@ -1014,23 +1015,21 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
           // dalpha[q] += sum_k dS g'(alpha_q delta_k) delta_k, ddelta[k] += sum_q dS g'(alpha_q delta_k) alpha_q,
           // g' = sigmoid(-x) for the logsigmoid gate, 1 for the identity (flash_gated_bwd.py:84-88, :152-160)
           const uint4 av = al4[ch];
-          float a8[8], v[8];
-          unpack16(av.x, a8[0], a8[1]);
-          unpack16(av.y, a8[2], a8[3]);
-          unpack16(av.z, a8[4], a8[5]);
-          unpack16(av.w, a8[6], a8[7]);
+          const uint32_t aw[4] = {av.x, av.y, av.z, av.w};
+          const float2 dg2 = make_float2(dlt_g, dlt_g), dl2 = make_float2(dlt, dlt);
+          float v[8];
 #pragma unroll
           for (int j = 0; j < 8; j += 2) {
-            float e0, e1;
+            float a0, a1, e0, e1;
+            unpack16(aw[j >> 1], a0, a1);
             unpack16(o[j >> 1], e0, e1);
-            if (logsig) {
-              e0 *= __fdividef(1.0f, 1.0f + ex2_approx(a8[j] * dlt * 1.4426950408889634f));
-              e1 *= __fdividef(1.0f, 1.0f + ex2_approx(a8[j + 1] * dlt * 1.4426950408889634f));
-            }
-            dd_acc = fmaf(e0, a8[j], dd_acc);
-            dd_acc = fmaf(e1, a8[j + 1], dd_acc);
-            v[j] = e0 * dlt;
-            v[j + 1] = e1 * dlt;
+            const float2 a2 = make_float2(a0, a1);
+            float2 w2 = make_float2(e0, e1);
+            if (logsig) w2 = mul2(w2, sigmoid_neg2(mul2(a2, dg2)));
+            dd_acc = fma2(w2, a2, dd_acc);
+            const float2 v2 = mul2(w2, dl2);
+            v[j] = v2.x;
+            v[j + 1] = v2.y;
           }
           // three butterfly steps fold the 8 columns onto lane bits 4, 3, 2: one column per lane, summed over 8 lanes
           const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
@@ -1147,13 +1146,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
     if (KIND == KIND_GATED && ok) {
       float* tmp = s_lse;  // every load of the ring has been consumed by now
       if (wg == 1) {
-        tmp[row] = dd_acc;
+        tmp[row] = dd_acc.x + dd_acc.y;
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->dd_sync);
       } else {
         ok = mbar_wait(&bars->dd_sync, 0, abort_flag);
         if (ok && row_ok) {
-          const float val = (dd_acc + tmp[row]) * p.softmax_scale;
+          const float val = (dd_acc.x + dd_acc.y + tmp[row]) * p.softmax_scale;
           const long long at = (long long)bk * p.d_sb + (long long)hkv * p.d_sh + off_k + k_idx;
           if (p.flags & F_SPLIT)
             reinterpret_cast<float*>(p.dd_out)[(long long)split * p.dd_ss + at] = val;

@@ -374,6 +374,26 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
   return f2_unpack(rd);
 }
 
+// s + logsigmoid(x) for two values, x given as y = x * log2(e): the arithmetic of log_sigmoid_fast, packed.
+__device__ __forceinline__ float2 add_log_sigmoid2(float2 s, float2 y) {
+  const float2 u = make_float2(ex2_approx(-fabsf(y.x)), ex2_approx(-fabsf(y.y)));
+  float2 q = fma2(u, make_float2(0.0415511145f, 0.0415511145f), make_float2(-0.157838377f, -0.157838377f));
+  q = fma2(q, u, make_float2(0.3065611f, 0.3065611f));
+  q = fma2(q, u, make_float2(-0.497030843f, -0.497030843f));
+  q = fma2(q, u, make_float2(0.999944993f, 0.999944993f));
+  s = fma2(make_float2(fminf(y.x, 0.f), fminf(y.y, 0.f)), make_float2(0.6931471806f, 0.6931471806f), s);
+  return fma2(make_float2(-u.x, -u.y), q, s);
+}
+
+// sigmoid(-x) = 1 / (1 + 2^y) for two values, y = x * log2(e): one reciprocal for both. 2^y is capped at 2^62, so that the
+// product of the two denominators stays finite; a sigmoid below 2^-62 counts as 2^-62.
+__device__ __forceinline__ float2 sigmoid_neg2(float2 y) {
+  const float2 d = add2(make_float2(ex2_approx(fminf(y.x, 62.f)), ex2_approx(fminf(y.y, 62.f))), make_float2(1.f, 1.f));
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d.x * d.y));
+  return mul2(make_float2(r, r), make_float2(d.y, d.x));
+}
+
 template <typename T>
 __device__ __forceinline__ uint32_t pack2(float lo, float hi);
 template <>
