@@ -117,9 +117,15 @@ __device__ __forceinline__ RowPos locate_row(long long item, int heads, int varl
   r.h = (int)(item % heads);
   const long long row = item / heads;
   if (varlen) {
-    // B is small: linear scan over the sequence starts
-    int b = 0;
-    while (b + 1 < B && cu_q[b + 1] <= row) ++b;
+    // the last sequence that starts at or before the row: log2(B) dependent loads where a scan would take up to B
+    int b = 0, last = B - 1;
+    while (b < last) {
+      const int mid = (b + last + 1) >> 1;
+      if (cu_q[mid] <= row)
+        b = mid;
+      else
+        last = mid - 1;
+    }
     r.b = b;
     r.q = (int)(row - cu_q[b]);
     r.tok = row;
