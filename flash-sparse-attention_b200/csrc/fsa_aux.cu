@@ -56,24 +56,39 @@ __global__ void __launch_bounds__(256) combine_kernel(CombineParams p) {
   for (int i = 0; i < VEC; ++i) acc[i] = 0.f;
   const int d0 = lane * VEC;
   const bool active = d0 < p.head_dim;
-  for (int sp = 0; sp < p.num_splits; ++sp) {
-    const float lse_s = lp[(long long)sp * p.lp_ss];
-    const float new_max = fmaxf(lse_s, e_max);
-    const float old_scale = (e_max == -INFINITY) ? 0.f : exp2f(e_max - new_max);
-    const float w = (lse_s == -INFINITY) ? 0.f : exp2f(lse_s - new_max);
-    if (active) {
-      const float* src = op + (long long)sp * p.op_ss + d0;
+  // 32 splits at a time: lane l holds the log-sum-exp of split l, so their maximum and the weights are one warp
+  // reduction and the loads of the partial rows do not depend on one another.
+  for (int s0 = 0; s0 < p.num_splits; s0 += 32) {
+    const int cnt = min(32, p.num_splits - s0);
+    const float lse_l = lane < cnt ? lp[(long long)(s0 + lane) * p.lp_ss] : -INFINITY;
+    float c_max = lse_l;
 #pragma unroll
-      for (int i = 0; i < VEC; i += 4) {
-        const float4 v = *reinterpret_cast<const float4*>(src + i);
-        acc[i] = acc[i] * old_scale + w * v.x;
-        acc[i + 1] = acc[i + 1] * old_scale + w * v.y;
-        acc[i + 2] = acc[i + 2] * old_scale + w * v.z;
-        acc[i + 3] = acc[i + 3] * old_scale + w * v.w;
+    for (int o = 16; o > 0; o >>= 1) c_max = fmaxf(c_max, __shfl_xor_sync(0xffffffffu, c_max, o));
+    const float new_max = fmaxf(c_max, e_max);
+    const float old_scale = (e_max == -INFINITY) ? 0.f : exp2f(e_max - new_max);
+    const float w_l = (lse_l == -INFINITY) ? 0.f : exp2f(lse_l - new_max);
+    float c_sum = w_l;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) c_sum += __shfl_xor_sync(0xffffffffu, c_sum, o);
+    e_sum = e_sum * old_scale + c_sum;
+    e_max = new_max;
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) acc[i] *= old_scale;
+    const float* src = op + (long long)s0 * p.op_ss + d0;
+#pragma unroll 4
+    for (int sp = 0; sp < cnt; ++sp) {
+      const float w = __shfl_sync(0xffffffffu, w_l, sp);
+      if (active) {
+#pragma unroll
+        for (int i = 0; i < VEC; i += 4) {
+          const float4 v = __ldcs(reinterpret_cast<const float4*>(src + (long long)sp * p.op_ss + i));
+          acc[i] += w * v.x;
+          acc[i + 1] += w * v.y;
+          acc[i + 2] += w * v.z;
+          acc[i + 3] += w * v.w;
+        }
       }
     }
-    e_sum = e_sum * old_scale + w;
-    e_max = new_max;
   }
   const float inv = (e_sum == 0.f || e_sum != e_sum) ? 0.f : 1.0f / e_sum;
   if (active) {

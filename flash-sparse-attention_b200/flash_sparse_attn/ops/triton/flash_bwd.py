@@ -19,6 +19,10 @@ from flash_sparse_attn.ops.triton import assert_inputs, quant, utils
 
 TILE_M = 128
 TILE_N = 128
+# for the split rule (utils.balanced_num_splits): a step (one query tile of one head), what a CTA takes besides its
+# steps, and the rate at which the fp32 partials of dK and dV are written and read
+BWD_STEP_US, BWD_CTA_US = 2.8, 10.0
+PARTIAL_BYTES_PER_US = 5.0e6
 _KIND = {"dense": _lib.KIND_DENSE, "sparse": _lib.KIND_SPARSE, "gated": _lib.KIND_GATED}
 
 
@@ -109,15 +113,23 @@ def attn_backward(
         value = _dequantize(value, value_scale, dout.dtype)
 
     if is_split_qo and num_splits is None:
-        # roles of the two sequence axes are swapped with respect to the forward heuristic
-        num_splits = utils.num_splits_heuristic(
-            seqlen_q=seqlen_k, seqlen_k=seqlen_q, num_SMs=utils.device_num_sms(device), TILE_M=TILE_N,
-            TILE_N=TILE_M, is_local=is_local, num_heads_kv=num_heads_kv,
-        )
         # one CTA per (key tile, KV head, batch): when that already oversubscribes the SMs, splitting the
         # query range only adds fp32 partials of dK/dV
-        if batch * num_heads_kv * (-(-seqlen_k // TILE_N)) >= 2 * utils.device_num_sms(device):
+        ctas = batch * num_heads_kv * (-(-seqlen_k // TILE_N))
+        n_sms = utils.device_num_sms(device)
+        if ctas >= 2 * n_sms:
             num_splits = 1
+        elif is_local:
+            # roles of the two sequence axes are swapped with respect to the forward heuristic
+            num_splits = utils.num_splits_heuristic(
+                seqlen_q=seqlen_k, seqlen_k=seqlen_q, num_SMs=n_sms, TILE_M=TILE_N, TILE_N=TILE_M, is_local=True,
+                num_heads_kv=num_heads_kv,
+            )
+        else:
+            rows = total_k if varlen else batch * seqlen_k
+            num_splits = utils.balanced_num_splits(
+                ctas, -(-seqlen_q // TILE_M), BWD_STEP_US * (num_heads_q // num_heads_kv), BWD_CTA_US,
+                rows * num_heads_kv * head_dim * 16 / PARTIAL_BYTES_PER_US, n_sms)
     elif not is_split_qo:
         num_splits = 1
     use_split = bool(is_split_qo) and num_splits > 1

@@ -18,6 +18,10 @@ from flash_sparse_attn.ops.triton import assert_inputs, quant, utils
 
 TILE_M = 128
 TILE_N = 128
+# What the split rule (utils.balanced_num_splits) reckons with, measured at head size 128: a step of a CTA (two query
+# tiles x one key tile), what a CTA takes besides its steps, and the rate at which fp32 partials are written and read.
+FWD_STEP_US, FWD_CTA_US = 1.5, 7.0
+PARTIAL_BYTES_PER_US = 5.0e6
 
 _KIND = {"dense": _lib.KIND_DENSE, "sparse": _lib.KIND_SPARSE, "gated": _lib.KIND_GATED}
 
@@ -128,16 +132,21 @@ def attn_forward(
             query, key, value = (quant.widen_fp8(t, torch.bfloat16) for t in (query, key, value))
 
     if is_split_kv and num_splits is None:
-        num_splits = utils.num_splits_heuristic(
-            seqlen_q=seqlen_q * group_packed, seqlen_k=seqlen_k, num_SMs=utils.device_num_sms(device),
-            TILE_M=TILE_M, TILE_N=TILE_N, is_local=is_local, num_heads_kv=num_heads_kv,
-        )
-        # The reference's rule only looks at the query tiles of ONE (batch, head). When batch x heads
-        # already gives every SM several CTAs, splitting only adds fp32 partial traffic: keep one split.
         m_pairs = -(-seqlen_q * group_packed // (2 * TILE_M))
         ctas = batch * (num_heads_kv if group_packed > 1 else num_heads_q) * m_pairs
-        if ctas >= 2 * utils.device_num_sms(device):
-            num_splits = 1
+        n_sms = utils.device_num_sms(device)
+        if ctas >= 2 * n_sms:
+            num_splits = 1  # every SM has several CTAs as it is
+        elif is_local:
+            # the tiles that a window leaves are not known on the host: the reference's estimate for its default window
+            num_splits = utils.num_splits_heuristic(
+                seqlen_q=seqlen_q * group_packed, seqlen_k=seqlen_k, num_SMs=n_sms, TILE_M=TILE_M, TILE_N=TILE_N,
+                is_local=True, num_heads_kv=num_heads_kv,
+            )
+        else:
+            rows = total_q if varlen else batch * seqlen_q
+            num_splits = utils.balanced_num_splits(ctas, -(-seqlen_k // TILE_N), FWD_STEP_US, FWD_CTA_US,
+                                                   rows * num_heads_q * head_dim * 8 / PARTIAL_BYTES_PER_US, n_sms)
     elif not is_split_kv:
         num_splits = 1
     # a single split is the unsplit kernel (same schedule, no workspace, no combine pass)

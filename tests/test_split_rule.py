@@ -1,0 +1,40 @@
+"""The rule that picks the number of KV / QO splits when the caller leaves it open, and the merge of many splits."""
+
+import pytest
+import torch
+
+from fixtures import assert_close, seeded_qkv
+from flash_sparse_attn.ops.triton import utils
+from oracle import eager
+
+
+def test_balanced_num_splits():
+    f = lambda ctas, steps: utils.balanced_num_splits(ctas, steps, 1.5, 7.0, 0.5, 148)  # noqa: E731
+    assert f(256, 1) == 1 and f(1, 0) == 1
+    assert utils.balanced_num_splits(290, 94, 1.5, 7.0, 50.0, 148) == 1  # the partials would cost more
+    assert f(4, 120) > 4                       # four CTAs would leave the GPU idle
+    for ctas in (1, 8, 100, 147, 149, 295):
+        for steps in (1, 2, 7, 64, 1000):
+            n = f(ctas, steps)
+            assert 1 <= n <= min(max(steps, 1), 64)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("num_splits", [None, 2, 33, 40])  # 32 splits are merged at a time
+@pytest.mark.parametrize("sq,sk", [(70, 5300), (300, 900)])
+def test_split_forward_and_backward(num_splits, sq, sk):
+    import flash_sparse_attn as fsa
+
+    q, k, v = seeded_qkv(sq + sk, 1, sq, sk, 4, 2, 64)
+    ref, lse_ref = eager.forward(q, k, v, None, True, return_lse=True)
+    dout = torch.randn(q.shape, generator=torch.Generator().manual_seed(1)).to(q.dtype)
+    leaves = [t.cuda().requires_grad_(True) for t in (q, k, v)]
+    out, lse = fsa.flash_dense_attn_func(*leaves, is_causal=True, is_split_kv=True, is_split_qo=True,
+                                         num_splits=num_splits, return_lse=True)
+    grads = torch.autograd.grad(out, leaves, dout.cuda())
+    torch.cuda.synchronize()
+    fsa.check_status()
+    assert_close("out", out, ref)
+    assert torch.allclose(lse.cpu(), lse_ref, rtol=0, atol=2e-3)
+    for name, got, want in zip(("dq", "dk", "dv"), grads, eager.backward(q, k, v, dout, None, True)):
+        assert_close(name, got, want)
