@@ -851,13 +851,17 @@ int fsa_decode(const FsaDecArgs* a, void* stream_) {
     p.peer_rank = pe->rank;
     p.peer_block_floats = pe->block_floats;
   }
+  if (!a->partial_only) {
+    p.cluster = fsa::dec_cluster_splits(a->batch, a->heads_kv, a->heads_q, a->head_dim, ns);
+    if (p.cluster > 1) p.flags &= ~(unsigned)fsa::F_SPLIT;
+  }
   mark(a->ev_before, stream);
   p.D = a->head_dim;
   cudaError_t e = fsa::launch_dec(p, a->kind, a->dtype, head_dim_kernel_wide(a->head_dim), stream);
   mark(a->ev_after, stream);
   if (e == cudaErrorInvalidValue) return FSA_ERR_UNSUPPORTED;
   if (e != cudaSuccess) return FSA_ERR_LAUNCH;
-  if (partial && !a->partial_only) {
+  if (partial && !a->partial_only && p.cluster == 0) {
     fsa::CombineParams c;
     memset(&c, 0, sizeof(c));
     c.out_partial = a->out_partial;

@@ -20,6 +20,7 @@
 //   gathered    pos = gather_kv_indices[b, i], negative = masked     (topk_gather_kv.py:5-77)
 //   gathered + paged: the gathered logical position goes through the page table (the reference
 //   rejects this combination, assert_inputs.py:303-305; here it is defined as the composition).
+#include <cooperative_groups.h>
 #include <mma.h>
 #include "fsa_aux.h"
 #include <type_traits>
@@ -47,6 +48,7 @@ struct DecStages {
   static constexpr int value = ES == 1 ? 2 * FSA_DEC_STAGES16 : FSA_DEC_STAGES16;
 };
 constexpr int DWARPS = 4;
+constexpr int MAX_CLUSTER = 8;  // splits that are merged inside a cluster
 
 template <int HD, int ES = 2>
 struct DecSmem {
@@ -171,11 +173,19 @@ __global__ void __launch_bounds__(DWARPS * 32, OCC) dec_kernel(const DecKernelPa
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
 
-  int idx = blockIdx.x;
-  const int hkv = idx % p.Hkv;
-  idx /= p.Hkv;
-  const int b = idx / p.num_splits;
-  const int split = idx - b * p.num_splits;
+  // KV heads fastest; with the splits of a (sequence, KV head) in one cluster the splits are
+  int idx = blockIdx.x, hkv, split, b;
+  if (p.cluster > 1) {
+    split = idx % p.num_splits;
+    idx /= p.num_splits;
+    hkv = idx % p.Hkv;
+    b = idx / p.Hkv;
+  } else {
+    hkv = idx % p.Hkv;
+    idx /= p.Hkv;
+    b = idx / p.num_splits;
+    split = idx - b * p.num_splits;
+  }
   const bool gather = p.flags & F_GATHER, paged = p.flags & F_PAGED, local = p.flags & F_LOCAL;
   // peer exchange: which of the two receive buffers this step uses (the count of exchanges sent so far lives in this
   // rank's region; the last CTA of the grid advances it)
@@ -791,6 +801,7 @@ __global__ void __launch_bounds__(DWARPS * 32, OCC) dec_kernel(const DecKernelPa
     }
     __syncthreads();
     const float* all = reinterpret_cast<const float*>(dsm);
+    float* xo = reinterpret_cast<float*>(dsm) + DWARPS * (16 * HD + 32);  // cluster: merged state of this CTA
     for (int item = tid; item < 16 * (HD / 4); item += DWARPS * 32) {
       const int r = item / (HD / 4), d0 = (item % (HD / 4)) * 4;
       const int row = mt * MROWS + r;
@@ -811,6 +822,14 @@ __global__ void __launch_bounds__(DWARPS * 32, OCC) dec_kernel(const DecKernelPa
         acc.y += ov.y * wgt;
         acc.z += ov.z * wgt;
         acc.w += ov.w * wgt;
+      }
+      if (p.cluster > 1) {  // this split's state for the others of the cluster
+        *reinterpret_cast<float4*>(xo + r * HD + d0) = acc;
+        if (d0 == 0) {
+          xo[16 * HD + r] = m_tot;
+          xo[16 * HD + 16 + r] = l_tot;
+        }
+        continue;
       }
       const bool dead = (l_tot == 0.f) || (l_tot != l_tot);
       const float inv = dead ? 1.f : v_scale / l_tot;
@@ -842,6 +861,49 @@ __global__ void __launch_bounds__(DWARPS * 32, OCC) dec_kernel(const DecKernelPa
           p.lse[(long long)b * p.l_sb + (long long)head * p.l_sh] =
               dead ? -INFINITY : (m_tot * c + log2f(l_tot)) * 0.6931471805599453f;
       }
+    }
+    if (p.cluster > 1) {
+      // ---- merge the splits of the cluster through distributed shared memory: every CTA finishes its share of the rows
+      namespace cg = cooperative_groups;
+      cg::cluster_group cl = cg::this_cluster();
+      cl.sync();
+      for (int item = split * DWARPS * 32 + tid; item < p.G * (HD / 4); item += p.cluster * DWARPS * 32) {
+        const int r = item / (HD / 4), d0 = (item % (HD / 4)) * 4;
+        if (d0 >= p.D) continue;
+        float m_s[MAX_CLUSTER], m_tot = -INFINITY;
+#pragma unroll
+        for (int i = 0; i < MAX_CLUSTER; ++i) {
+          m_s[i] = i < p.cluster ? cl.map_shared_rank(xo, i)[16 * HD + r] : -INFINITY;
+          m_tot = fmaxf(m_tot, m_s[i]);
+        }
+        float l_tot = 0.f;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < MAX_CLUSTER; ++i) {
+          if (i < p.cluster) {
+            const float* src = cl.map_shared_rank(xo, i);
+            const float ls = src[16 * HD + 16 + r];
+            const float4 ov = *reinterpret_cast<const float4*>(src + r * HD + d0);
+            const float wgt = (m_s[i] == -INFINITY || ls == 0.f) ? 0.f : ex2_approx((m_s[i] - m_tot) * c);
+            l_tot += ls * wgt;
+            acc.x += ov.x * wgt;
+            acc.y += ov.y * wgt;
+            acc.z += ov.z * wgt;
+            acc.w += ov.w * wgt;
+          }
+        }
+        const bool dead = (l_tot == 0.f) || (l_tot != l_tot);
+        const float inv = dead ? 1.f : v_scale / l_tot;
+        const int head = hkv * p.G + r;
+        uint2 v;
+        v.x = pack2<TO>(acc.x * inv, acc.y * inv);
+        v.y = pack2<TO>(acc.z * inv, acc.w * inv);
+        *reinterpret_cast<uint2*>(reinterpret_cast<TO*>(p.out) + (long long)b * p.o_sb + (long long)head * p.o_sh + d0) = v;
+        if (d0 == 0)
+          p.lse[(long long)b * p.l_sb + (long long)head * p.l_sh] =
+              dead ? -INFINITY : (m_tot * c + log2f(l_tot)) * 0.6931471805599453f;
+      }
+      cl.sync();  // nobody leaves while another CTA may still read its shared memory
     }
     __syncthreads();
   }
@@ -928,6 +990,22 @@ cudaError_t launch_variant(const DecKernelParams& p, cudaStream_t stream) {
       if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
     }
   }
+  if (p.cluster > 1) {
+    static_assert(HD > 128 || DWARPS * (16 * HD + 32) * 4 + (16 * HD + 32) * 4 <= ring, "the merged state fits behind the warps'");
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid, 1, 1);
+    cfg.blockDim = dim3(DWARPS * 32, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)p.cluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, p);
+  }
   kern<<<(unsigned)grid, DWARPS * 32, smem, stream>>>(p);
   return cudaGetLastError();
 }
@@ -958,6 +1036,14 @@ cudaError_t launch_one(const DecKernelParams& p, cudaStream_t stream) {
 }
 
 }  // namespace
+
+// Splits merged inside a cluster (their number; 0: partials and a second launch). A call whose CTAs are all resident at
+// once is bound by latencies, and the partials' way through memory and the combine launch are several of them. With more
+// CTAs than slots the kernel is bandwidth bound and a cluster, which starts and ends as one, leaves slots idle.
+int dec_cluster_splits(int batch, int heads_kv, int heads_q, int head_dim, int num_splits) {
+  const bool fits = num_splits > 1 && num_splits <= MAX_CLUSTER && head_dim <= 128 && heads_q <= 16 * heads_kv;
+  return fits && (long long)batch * heads_kv * num_splits <= 2ll * device_sm_count() ? num_splits : 0;
+}
 
 cudaError_t launch_dec(const DecKernelParams& p, int kind, int dtype, int head_dim, cudaStream_t stream) {
 #define FSA_DEC_CASE(HD_, T_, DT_)                                               \

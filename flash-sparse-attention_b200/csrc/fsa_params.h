@@ -126,6 +126,7 @@ struct DecKernelParams {
   int peer_world, peer_rank;
   int D;  // real head size (<= the kernel's HD)
   unsigned flags;
+  int cluster;  // > 1: the num_splits CTAs of a (sequence, KV head) are one cluster and merge their results themselves
 };
 
 // Gated forward workspace: float2 (max, min) of alpha per (batch, grid head, 128-row query tile), then float2
