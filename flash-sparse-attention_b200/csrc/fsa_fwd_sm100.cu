@@ -77,7 +77,8 @@ struct FwdBars {
   uint64_t k0_full;     // first K tile
   uint64_t kv_full[2];  // step t (slot t & 1): V(t) and K(t + 1) have landed (two producer arrivals)
   uint64_t kv_empty[2];  // signal c (slot c & 1): K(c) and V(c - 1) have been consumed; c = 0 comes from the prologue
-  uint64_t s_full[2], p_full[2], o_final[2], wg_sync[2];
+  // p_full: P is in TMEM (FP8: its first half), or the tile is skipped; p_rest: FP8, the second half of a kept tile
+  uint64_t s_full[2], p_full[2], p_rest[2], o_final[2], wg_sync[2];
   uint64_t d_full[2], d_empty[2];  // gated: delta ring (stager warp -> softmax warps)
   uint32_t tmem_base;
   int abort_flag;
@@ -163,6 +164,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
   constexpr bool IS_BF16 = (sizeof(T) == 2) && !__is_same(T, __half);
   static_assert(!F8 || HD == 128, "FP8 tiles are one 128-byte swizzle row wide");
   constexpr uint32_t TMEM_S0 = 0, TMEM_O0 = 256;
+  // FP8: P is handed to the MMA issuer in two halves, so that the first MMAs of P V run under the second half of the
+  // exponentials (B2 S6000 causal 570 -> 543 us). With 16-bit inputs, whose P V takes twice as long, the second barrier
+  // costs the issuer more than that gains (S = 16384: 1.91 -> 1.96 ms).
+  constexpr bool HALVES = F8;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -202,6 +207,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
   }
   const int gpack = p.gpack;
   const int m_blocks_here = fsa_cdiv(si.sq * gpack, TM);  // query tiles this sequence really has
+  if (pair * QT >= m_blocks_here) return;  // the grid is laid out for the longest sequence: nothing to do or to write
 
   // Both groups' schedules are needed by every role.
   FsaFwdSched sched[2];
@@ -310,6 +316,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
     for (int q = 0; q < 2; ++q) {
       mbar_init(&bars->s_full[q], 1);
       mbar_init(&bars->p_full[q], 4);  // one arrival per warp of the group
+      mbar_init(&bars->p_rest[q], 4);
       mbar_init(&bars->o_final[q], 1);
       mbar_init(&bars->wg_sync[q], 4);
       mbar_init(&bars->d_full[q], 1);
@@ -479,7 +486,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
                                     : umma_idesc_f16(TM, HD, IS_BF16, false, true);
     const uint32_t sQ = smem_u32(smem + SM::kQ), sK = smem_u32(smem + SM::kK), sV = smem_u32(smem + SM::kV);
     bool ok = !*abort_flag;
-    int cnt[2] = {0, 0};
+    int cnt[2] = {0, 0}, cnt_kept[2] = {0, 0};
     bool o_started[2] = {false, false};
     bool act[2], last[2];
     int n = (KIND == KIND_GATED) ? walk_next(WALK_START, act, -1) : first_tile();
@@ -570,6 +577,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
           if (!skip) {
 #pragma unroll ISSUE_UNROLL
             for (int kk = 0; kk < KK_PV; ++kk) {
+              if (HALVES && kk == KK_PV / 2) {
+                ok = mbar_wait(&bars->p_rest[q], cnt_kept[q] & 1, abort_flag);  // only kept tiles arrive there
+                if (!ok) break;
+                cnt_kept[q]++;
+                tc_fence_after();
+              }
               if (F8)
                 umma_f8_ts_lead(lead, tmem_base + TMEM_O0 + q * 128, tmem_base + TMEM_S0 + q * 128 + kk * 8,
                                 umma_desc_at(bv, kk * 4096), idesc_o, (kk > 0 || o_started[q]) ? 1u : 0u);
@@ -877,12 +890,19 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
           tmem_st8(tS + ch * 8, pk);
         else
           tmem_st16(tS + ch * 16, pk);
+        if (HALVES && ch == 1) {
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          publish_verdict(false);
+          if (lane == 0) mbar_arrive(&bars->p_full[q]);
+        }
       }
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      publish_verdict(false);
-      if (lane == 0) mbar_arrive(&bars->p_full[q]);
+      if (!HALVES) publish_verdict(false);
+      if (lane == 0) mbar_arrive(HALVES ? &bars->p_rest[q] : &bars->p_full[q]);
       l_ref += (sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y);
       if (KIND != KIND_DENSE) lg_l = lg2_approx(l_ref);
       have_o = true;
