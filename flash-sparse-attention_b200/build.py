@@ -1,4 +1,4 @@
-"""Build libfsa_b200.so (sm_100a only) in-tree with nvcc.
+"""Build libfsa_b200.so (sm_100a only) in-tree with nvcc, and the native launcher flash_sparse_attn/_host.so with g++.
 
 Usage: ``python build.py [--force] [--verbose]``. The library has no dependency on libcuda at link
 time (the one driver entry point it needs is resolved at run time), so it loads on machines without
@@ -8,12 +8,15 @@ a GPU; compute calls then fail with an error code.
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libfsa_b200.so")
+HOST_SRC = os.path.join(CSRC, "fsa_host.cpp")
+HOST_LIB = os.path.join(HERE, "flash_sparse_attn", "_host.so")
 
 SOURCES = [
     "fsa_api.cu",
@@ -79,7 +82,31 @@ def _compile(src, force, verbose):
     return obj, log
 
 
+def build_host(force=False):
+    """The native launcher: a CPython extension against the headers of the installed torch. It holds no device code
+    and reaches the kernels through the addresses that the package hands it."""
+    header = os.path.join(HERE, "..", "include", "fsa_b200.h")
+    newest = max(os.path.getmtime(HOST_SRC), os.path.getmtime(header))
+    if not force and os.path.exists(HOST_LIB) and os.path.getmtime(HOST_LIB) >= newest:
+        return HOST_LIB
+    import torch
+
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
+    for inc in (sysconfig.get_paths()["include"], os.path.join(root, "include"),
+                os.path.join(root, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include")):
+        cmd += ["-isystem", inc]
+    cmd += [HOST_SRC, "-o", HOST_LIB, "-L" + os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch",
+            "-ltorch_python"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("g++ failed for fsa_host.cpp:\n" + res.stdout + res.stderr)
+    return HOST_LIB
+
+
 def build(force=False, verbose=False):
+    build_host(force)
     os.makedirs(OBJ, exist_ok=True)
     with ThreadPoolExecutor(max_workers=min(8, len(SOURCES))) as ex:
         results = list(ex.map(lambda s: _compile(s, force, verbose), SOURCES))

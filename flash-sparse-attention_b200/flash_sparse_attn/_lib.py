@@ -355,6 +355,8 @@ def load():
                                 c_int64, c_void_p]
     lib.fsa_quantize_fp8.restype = c_int
     lib.fsa_quantize_fp8.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p]
+    lib.fsa_pack_scales.restype = c_int
+    lib.fsa_pack_scales.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p]
     lib.fsa_fp8_widen.restype = c_int
     lib.fsa_fp8_widen.argtypes = [c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p]
     lib.fsa_topk_indices.restype = c_int
@@ -392,8 +394,34 @@ def load():
     lib.fsa_debug_bwd_schedule.argtypes = [c_int] * 4 + [POINTER(c_int32)] + [c_int] * 6 + [POINTER(c_int32)]
     if lib.fsa_abi_version() != ABI_VERSION:
         raise RuntimeError("libfsa_b200.so ABI version mismatch: rebuild the library")
+    _load_host(lib)
     _lib = lib
     return lib
+
+
+_host = None
+
+
+def _load_host(lib):
+    """The native launcher of the common calls (csrc/fsa_host.cpp); it is built with the library and as required."""
+    global _host
+    try:
+        from flash_sparse_attn import _host as host
+    except ImportError as e:
+        raise RuntimeError("the native launcher flash_sparse_attn/_host.so is missing or does not load: build it with "
+                           "`python build.py` next to csrc/") from e
+    host.init(ctypes.cast(lib.fsa_decode, c_void_p).value, ctypes.cast(lib.fsa_fwd, c_void_p).value)
+    _host = host
+
+
+def native():
+    """The native launcher, or None while a caller has profile events attached (they travel in the argument block
+    that the Python launchers fill)."""
+    if _profile["before"] is not None or _profile["after"] is not None:
+        return None
+    if _host is None:
+        load()
+    return _host
 
 
 def check(code: int, what: str):
@@ -430,6 +458,9 @@ def status_word(device: torch.device) -> torch.Tensor:
     if t is None:
         t = torch.zeros(1, dtype=torch.int32, device=device)
         _status_words[key] = t
+        if key[0] == "cuda":
+            load()
+            _host.set_status(key[1], t, torch.cuda.get_device_properties(key[1]).multi_processor_count)
     return t
 
 
@@ -465,7 +496,7 @@ def workspace(nbytes: int, device, dtype=torch.float32):
     """A caller-owned workspace of `nbytes` bytes (size from fsa_*_workspace_bytes) viewed as `dtype`, or None."""
     if nbytes == 0:
         return None
-    return torch.empty(nbytes // torch.empty((), dtype=dtype).element_size(), dtype=dtype, device=device)
+    return torch.empty(nbytes // dtype.itemsize, dtype=dtype, device=device)
 
 
 def current_stream_ptr(device) -> int:

@@ -88,6 +88,20 @@ def attn_decode(
     if not query.is_cuda:
         raise RuntimeError("flash_sparse_attn (B200 build) only runs on CUDA tensors; there is no CPU path")
     device = query.device
+    if (kind != "gated" and (tile_mn is None or page_table is None) and tile_map is None and not partial_only
+            and workspace is None and threshold_seqlen_k is None and key_range is None and packed_partials is None
+            and gather_count is None and peers is None
+            and (not is_quant or quant.uniform_scales(query_scale, key_scale, value_scale, device))):
+        host = _lib.native()
+        if host is not None:
+            scales = quant.scales_f32(query_scale, key_scale, value_scale, device) if is_quant else None
+            res = host.decode(_KIND[kind], query, key, value, softmax_scale, window_sizes, softmax_threshold, is_local,
+                              num_splits, page_table, gather_kv_indices, seqused_k, cu_seqlens_k, max_seqlen_k, out, lse,
+                              scales)
+            if res is not None:
+                if type(res) is int:
+                    _lib.check(res, f"fsa_decode[{kind}]")
+                return res
     batch, num_heads_q, head_dim = query.shape
     varlen = cu_seqlens_k is not None
     page_size = None

@@ -31,6 +31,23 @@ def _require_cuda(t: torch.Tensor):
         raise RuntimeError("flash_sparse_attn (B200 build) only runs on CUDA tensors; there is no CPU path")
 
 
+def forward_num_splits(batch, seqlen_q, seqlen_k, rows, num_heads_q, num_heads_kv, head_dim, group_packed, is_local,
+                       num_sms):
+    """KV splits of a forward call that leaves their number open."""
+    m_pairs = -(-seqlen_q * group_packed // (2 * TILE_M))
+    ctas = batch * (num_heads_kv if group_packed > 1 else num_heads_q) * m_pairs
+    if ctas >= 2 * num_sms:
+        return 1  # every SM has several CTAs as it is
+    if is_local:
+        # the tiles that a window leaves are not known on the host: the reference's estimate for its default window
+        return utils.num_splits_heuristic(
+            seqlen_q=seqlen_q * group_packed, seqlen_k=seqlen_k, num_SMs=num_sms, TILE_M=TILE_M, TILE_N=TILE_N,
+            is_local=True, num_heads_kv=num_heads_kv,
+        )
+    return utils.balanced_num_splits(ctas, -(-seqlen_k // TILE_N), FWD_STEP_US, FWD_CTA_US,
+                                     rows * num_heads_q * head_dim * 8 / PARTIAL_BYTES_PER_US, num_sms)
+
+
 def attn_forward(
     kind: str,
     query: torch.Tensor,
@@ -102,6 +119,23 @@ def attn_forward(
     group_packed = group if pack_gqa else 1
     if is_local and window_sizes is None:
         window_sizes = utils.window_sizes_heuristic(seqlen_k, num_heads_kv, device)
+    if not is_split_kv:
+        num_splits = 1
+    elif num_splits is None:
+        num_splits = forward_num_splits(batch, seqlen_q, seqlen_k, total_q if varlen else batch * seqlen_q, num_heads_q,
+                                        num_heads_kv, head_dim, group_packed, is_local, utils.device_num_sms(device))
+    if (kind != "gated" and (tile_mn is None or page_table is None) and tile_map is None
+            and (not is_quant or quant.uniform_scales(query_scale, key_scale, value_scale, device))):
+        host = _lib.native()
+        if host is not None:
+            scales = quant.scales_f32(query_scale, key_scale, value_scale, device) if is_quant else None
+            res = host.forward(_KIND[kind], query, key, value, is_causal, softmax_scale, window_sizes, softmax_threshold,
+                               is_local, num_splits, pack_gqa, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k,
+                               page_table, seqused_q, seqused_k, out, lse, scales)
+            if res is not None:
+                if type(res) is int:
+                    _lib.check(res, f"fsa_fwd[{kind}]")
+                return res + (softmax_scale, softmax_threshold, gate_threshold)
 
     if not skip_checks:
         assert_inputs.assert_fwd_inputs(
@@ -131,24 +165,6 @@ def attn_forward(
         if not native:  # other head sizes / mixed formats: widen (exactly) to bf16 and use the 16-bit kernel
             query, key, value = (quant.widen_fp8(t, torch.bfloat16) for t in (query, key, value))
 
-    if is_split_kv and num_splits is None:
-        m_pairs = -(-seqlen_q * group_packed // (2 * TILE_M))
-        ctas = batch * (num_heads_kv if group_packed > 1 else num_heads_q) * m_pairs
-        n_sms = utils.device_num_sms(device)
-        if ctas >= 2 * n_sms:
-            num_splits = 1  # every SM has several CTAs as it is
-        elif is_local:
-            # the tiles that a window leaves are not known on the host: the reference's estimate for its default window
-            num_splits = utils.num_splits_heuristic(
-                seqlen_q=seqlen_q * group_packed, seqlen_k=seqlen_k, num_SMs=n_sms, TILE_M=TILE_M, TILE_N=TILE_N,
-                is_local=True, num_heads_kv=num_heads_kv,
-            )
-        else:
-            rows = total_q if varlen else batch * seqlen_q
-            num_splits = utils.balanced_num_splits(ctas, -(-seqlen_k // TILE_N), FWD_STEP_US, FWD_CTA_US,
-                                                   rows * num_heads_q * head_dim * 8 / PARTIAL_BYTES_PER_US, n_sms)
-    elif not is_split_kv:
-        num_splits = 1
     # a single split is the unsplit kernel (same schedule, no workspace, no combine pass)
     use_split = bool(is_split_kv) and num_splits > 1
 

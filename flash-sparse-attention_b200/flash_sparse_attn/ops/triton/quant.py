@@ -54,9 +54,27 @@ def widen_fp8(x: torch.Tensor, dtype: torch.dtype = torch.bfloat16, scale: Optio
 
 
 def scales_f32(query_scale, key_scale, value_scale, device):
-    """The three per-tensor scales as one fp32 device tensor (what the kernels read)."""
+    """The three per-tensor scales as one fp32 device tensor (what the kernels read). Scales that are tensors of one
+    type on the device are packed by one kernel of the library; anything else takes the general route."""
+    if uniform_scales(query_scale, key_scale, value_scale, device):
+        out = torch.empty(3, dtype=torch.float32, device=device)
+        with torch.cuda.device(device):
+            rc = _lib.load().fsa_pack_scales(query_scale.data_ptr(), key_scale.data_ptr(), value_scale.data_ptr(),
+                                             _lib.dtype_code(query_scale.dtype), out.data_ptr(),
+                                             _lib.current_stream_ptr(device))
+        _lib.check(rc, "fsa_pack_scales")
+        return out
     return torch.stack([torch.as_tensor(t, device=device).reshape(-1)[0].float()
                         for t in (query_scale, key_scale, value_scale)])
+
+
+def uniform_scales(query_scale, key_scale, value_scale, device):
+    """Whether the three scales are one-element tensors of one floating type on `device`."""
+    for t in (query_scale, key_scale, value_scale):
+        if type(t) is not torch.Tensor or t.numel() != 1 or t.device != device or t.dtype != query_scale.dtype:
+            return False
+    return query_scale.dtype in (torch.float32, torch.bfloat16, torch.float16)
+
 
 
 _block_scaled = False

@@ -437,6 +437,12 @@ int fsa_fp8_widen(const void* x_fp8, void* out, const void* scale, int64_t n, in
                   void* stream);
 
 /*
+ * out[0..2] = the one-element per-tensor scales of q, k, v (all of `dtype`: bf16, fp16 or fp32) as fp32: what the
+ * qkv_scale fields above point at.
+ */
+int fsa_pack_scales(const void* q_scale, const void* k_scale, const void* v_scale, int dtype, float* out, void* stream);
+
+/*
  * Top-k position selection in front of the gathered decode: for every row of `scores`
  * [rows, n] (bf16 / fp16 / fp32, `row_stride` elements between rows) the positions of the k largest
  * entries in ascending order, int32 or int64 [rows, k]. Same contract as

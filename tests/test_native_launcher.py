@@ -1,0 +1,151 @@
+"""The native launcher of the common calls against the Python launchers: the same results for every form it takes, and
+None (the Python launcher runs, with its errors) for the others."""
+
+import pytest
+import torch
+
+DEV = "cuda"
+
+
+def test_decode_split_rule_is_the_same():
+    from flash_sparse_attn import _lib
+    from flash_sparse_attn.ops.triton.flash_dec import decode_num_splits
+
+    _lib.load()
+    for batch in (1, 2, 7, 64, 300):
+        for hkv in (1, 2, 8, 40):
+            for keys in (0, 1, 511, 512, 2048, 5000, 131072, 1 << 20):
+                for sms in (1, 100, 148):
+                    assert _lib._host.decode_num_splits(batch, hkv, keys, sms) == decode_num_splits(batch, hkv, keys, sms)
+
+
+def test_refuses_what_it_does_not_know():
+    from flash_sparse_attn import _lib
+
+    _lib.load()
+    q, k = torch.zeros(1, 4, 64, dtype=torch.bfloat16), torch.zeros(1, 8, 2, 64, dtype=torch.bfloat16)
+    args = [0, q, k, k, None, None, None, False, None, None, None, None, None, None, None, None, None]
+    assert _lib._host.decode(*args) is None  # not on a GPU
+    assert _lib._host.decode(*args[:-1]) is None and _lib._host.forward() is None
+    for i, bad in ((1, None), (2, "k"), (0, 1.5), (7, 1), (8, "two"), (8, -1), (8, 1 << 40)):
+        assert _lib._host.decode(*(args[:i] + [bad] + args[i + 1:])) is None
+
+
+def _both(monkeypatch, fn):
+    """fn() through the native launcher (which must take the call) and through the Python one."""
+    from flash_sparse_attn import _lib
+
+    fn()  # registers the device
+    taken = []
+    host = _lib.native()
+
+    class Spy:
+        def __getattr__(self, name):
+            f = getattr(host, name)
+
+            def call(*a):
+                r = f(*a)
+                taken.append(r is not None)
+                return r
+            return call
+
+    monkeypatch.setattr(_lib, "native", lambda: Spy())
+    got = fn()
+    assert taken and all(taken)
+    monkeypatch.setattr(_lib, "native", lambda: None)
+    want = fn()
+    monkeypatch.undo()
+    torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        assert a.dtype == b.dtype and a.shape == b.shape and a.stride() == b.stride() and torch.equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float8_e4m3fn])
+@pytest.mark.parametrize("form", ["plain", "strided", "paged", "gather", "paged_gather", "varlen", "window", "buffers"])
+def test_decode_forms(monkeypatch, dtype, form):
+    import flash_sparse_attn as fsa
+
+    g = torch.Generator(device=DEV).manual_seed(1)
+    f8 = dtype == torch.float8_e4m3fn
+    mk = lambda *s: torch.randn(*s, generator=g, device=DEV).to(dtype)  # noqa: E731
+    b, hq, hkv, d, sk = 3, 16, 4, 128, 1536
+    q, kw = mk(b, hq, d), {}
+    k, v = mk(b, sk, hkv, d), mk(b, sk, hkv, d)
+    fn = fsa.flash_sparse_attn_with_kvcache_func
+    if form == "strided":
+        q, k, v = mk(hq, b, d).transpose(0, 1), mk(b, hkv, sk, d).transpose(1, 2), mk(b, hkv, sk, d).transpose(1, 2)
+    if "paged" in form:
+        k, v = mk(30, 64, hkv, d), mk(30, 64, hkv, d)
+        kw.update(page_table=torch.randperm(30, generator=g, device=DEV).to(torch.int32).reshape(3, 10),
+                  seqused_k=torch.tensor([600, 1, 77], dtype=torch.int32, device=DEV))
+    if "gather" in form:
+        kw.update(gather_kv_indices=torch.randint(-1, 600, (b, 100), generator=g, device=DEV, dtype=torch.int32))
+    if form == "window":
+        kw.update(window_sizes=torch.tensor([[4, 100, 30, 60]] * hkv, dtype=torch.int32, device=DEV), num_splits=3)
+    if form == "buffers":
+        kw.update(out=torch.empty(b, hq, d, device=DEV, dtype=torch.bfloat16 if f8 else dtype),
+                  lse=torch.empty(b, hq, device=DEV))
+    if f8:
+        s = torch.full((1,), 0.5, device=DEV, dtype=torch.bfloat16)
+        kw.update(is_quant=True, query_scale=s, key_scale=s, value_scale=s)
+    if form == "varlen":
+        cu = torch.tensor([0, 700, 700, 1500], dtype=torch.int32, device=DEV)
+        k, v = mk(1500, hkv, d), mk(1500, hkv, d)
+        fn = lambda q, k, v, **a: fsa.flash_sparse_attn_varlen_with_kvcache_func(q, k, v, cu, 800, **a)  # noqa: E731
+    _both(monkeypatch, lambda: tuple(t.clone() for t in fn(q, k, v, return_lse=True, **kw)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float8_e4m3fn])
+@pytest.mark.parametrize("form", ["plain", "pack", "split", "paged", "varlen", "varlen_used", "window", "local", "buffers"])
+def test_forward_forms(monkeypatch, dtype, form):
+    import flash_sparse_attn as fsa
+
+    g = torch.Generator(device=DEV).manual_seed(2)
+    f8 = dtype == torch.float8_e4m3fn
+    mk = lambda *s: torch.randn(*s, generator=g, device=DEV).to(dtype)  # noqa: E731
+    b, s, hq, hkv, d = 2, 333, 8, 2, 128
+    q, k, v, kw = mk(b, s, hq, d), mk(b, s, hkv, d), mk(b, s, hkv, d), dict(is_causal=True)
+    fn = fsa.flash_sparse_attn_func
+    if form == "pack":
+        kw.update(pack_gqa=True)
+    if form == "split":
+        kw.update(num_splits=3)
+    if form == "paged":
+        k, v = mk(8, 128, hkv, d), mk(8, 128, hkv, d)
+        kw.update(page_table=torch.randperm(8, generator=g, device=DEV).to(torch.int32).reshape(2, 4),
+                  seqused_k=torch.tensor([400, 350], dtype=torch.int32, device=DEV), is_split_kv=True)
+    if form == "window":
+        kw.update(window_sizes=torch.tensor([[4, 100, 30, 60]] * hkv, dtype=torch.int32, device=DEV))
+    if form == "local":
+        kw.update(is_local=True)
+    if form == "buffers":
+        kw.update(out=torch.empty(b, s, hq, d, device=DEV, dtype=torch.bfloat16 if f8 else dtype),
+                  lse=torch.empty(b, hq, s, device=DEV))
+    if f8:
+        sc = torch.full((1,), 0.5, device=DEV)
+        kw.update(is_quant=True, query_scale=sc, key_scale=sc, value_scale=sc)
+    if "varlen" in form:
+        cu = torch.tensor([0, 200, 200, 500], dtype=torch.int32, device=DEV)
+        q, k, v = mk(500, hq, d), mk(500, hkv, d), mk(500, hkv, d)
+        if form == "varlen_used":
+            kw.update(seqused_k=torch.tensor([150, 0, 300], dtype=torch.int32, device=DEV))
+        fn = lambda q, k, v, **a: fsa.flash_sparse_attn_varlen_func(q, k, v, cu, cu, 300, 300, **a)  # noqa: E731
+    _both(monkeypatch, lambda: tuple(t.clone() for t in fn(q, k, v, return_lse=True, **kw)))
+
+
+@pytest.mark.gpu
+def test_errors_are_those_of_the_contract():
+    import flash_sparse_attn as fsa
+
+    q, k = (torch.zeros(1, *s, 64, dtype=torch.bfloat16, device=DEV) for s in ((4,), (8, 2)))
+    fsa.flash_dense_attn_with_kvcache_func(q, k, k)
+    with pytest.raises(AssertionError, match="same dtype"):
+        fsa.flash_dense_attn_with_kvcache_func(q, k.half(), k.half())
+    with pytest.raises(AssertionError, match="multiple of 16"):
+        fsa.flash_dense_attn_with_kvcache_func(q[..., :40], k[..., :40], k[..., :40])
+    with pytest.raises(AssertionError, match="int32"):
+        fsa.flash_dense_attn_with_kvcache_func(q, k, k, seqused_k=torch.ones(1, dtype=torch.int64, device=DEV))
+    with pytest.raises(RuntimeError):
+        fsa.flash_dense_attn_with_kvcache_func(q.cpu(), k.cpu(), k.cpu())
