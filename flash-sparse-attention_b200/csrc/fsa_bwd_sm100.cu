@@ -177,25 +177,41 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
 
   // ---- work decode ------------------------------------------------------------------------------
   int idx = blockIdx.x;
-  int n_block;
+  int n_block, bh, split;
   if (p.flags & F_DETERMINISTIC) {
     // key tiles in descending order, slowest index: a CTA only ever waits for CTAs launched before it
     const int per_tile = p.Hkv * p.B * p.num_splits;
     n_block = p.n_tiles_k - 1 - idx / per_tile;
     idx %= per_tile;
+    const int hkv_ = idx % p.Hkv;
+    idx /= p.Hkv;
+    split = idx % p.num_splits;
+    bh = idx / p.num_splits * p.Hkv + hkv_;
   } else {
-    // Key tiles in ascending order, slowest index: under a causal / window mask the first key tiles meet the most
-    // query tiles, so the longest CTAs start first and the short ones fill the tail (512 CTAs on 148 SMs are 3.5
-    // rounds: with the key tile as the fastest index the last round began with the longest CTAs). CTAs that run
-    // side by side still share their Q / dO tiles through L2: neighbouring key tiles of one head are per_tile apart.
-    const int per_tile = p.Hkv * p.B * p.num_splits;
-    n_block = idx / per_tile;
-    idx %= per_tile;
+    // The (sequence, KV head) pairs in bh_groups groups of equal size (to within one); inside a group the key tiles
+    // ascending, slowest index: under a causal / window mask the first key tiles meet the most query tiles, so the longest
+    // CTAs of a group start first and the short ones fill the tail (512 CTAs on 148 SMs are 3.5 rounds: with the
+    // key tile as the fastest index the last round began with the longest CTAs; 0.499 -> 0.448 ms on the window
+    // workload). Groups, because the CTAs that run together have to share their Q, dO and dQ tiles in L2: with sixteen
+    // packed sequences x eight KV heads in one group, one key tile of each pair was on the SMs at a time, and every
+    // step took its 64 KB of Q and dO from DRAM and read and wrote its 64 KB of dQ there (3.09 -> 2.22 ms).
+    const int pairs_all = p.B * p.Hkv, small = pairs_all / p.bh_groups, n_big = pairs_all - small * p.bh_groups;
+    const int per_pair = p.n_tiles_k * p.num_splits;
+    int first = 0, pairs = small + 1;
+    if (idx < n_big * (small + 1) * per_pair) {
+      first = idx / ((small + 1) * per_pair) * (small + 1);
+    } else {
+      pairs = small;
+      const int g = (idx - n_big * (small + 1) * per_pair) / (small * per_pair);
+      first = n_big * (small + 1) + g * small;
+    }
+    idx -= first * per_pair;
+    n_block = idx / (pairs * p.num_splits);
+    idx -= n_block * pairs * p.num_splits;
+    split = idx / pairs;
+    bh = first + idx - split * pairs;
   }
-  const int hkv = idx % p.Hkv;
-  idx /= p.Hkv;
-  const int b = idx / p.num_splits;
-  const int split = idx - b * p.num_splits;
+  const int b = bh / p.Hkv, hkv = bh - b * p.Hkv;
   const int off_q = (p.flags & F_VARLEN_Q) ? p.cu_q[b] : 0;
   const int off_k = (p.flags & F_VARLEN_K) ? p.cu_k[b] : 0;
   const int sq = (p.flags & F_USED_Q) ? p.used_q[b] : ((p.flags & F_VARLEN_Q) ? p.cu_q[b + 1] - off_q : p.sq);

@@ -91,6 +91,7 @@ struct alignas(64) BwdKernelParams {
   int num_splits, n_tiles_k, num_m_blocks, win_stride;
   float scale_log2, softmax_scale, softmax_thr, gate_thr;
   unsigned flags;
+  int bh_groups;  // groups of (sequence, KV head) pairs whose key tiles are launched together
 };
 
 struct DecKernelParams {
