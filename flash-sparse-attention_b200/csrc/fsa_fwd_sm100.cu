@@ -84,7 +84,13 @@ struct FwdBars {
   int abort_flag;
   int skip_flag[2][2];   // [group][parity of the group's tile counter]
   int vote_any[2][2][4]; // [group][parity][warp]: bit0 = some row wants the tile, bit1 = some row votes skip
-  alignas(16) float dl[2][TN + 4];  // gated: delta of the key tile as fp32 (read as float4), then its max and min
+  // What the producer worked out about the tiles, for the MMA issuer: low word the tile index (-1: none), then bit q: group q
+  // takes part in it, bit 2 + q: it is group q's last. Slot 2: the first tile, published with k0_full. Slot t & 1: the
+  // tile after step t (and whether the one of step t is a group's last), published with kv_full.
+  unsigned long long step_info[3];
+  // gated: delta of the key tile as fp32 (read as float4), then as integers the tile index (-1: the end) and the mask mode
+  // of the two groups (-1: the group does not compute the tile)
+  alignas(16) float dl[2][TN + 4];
 };
 
 static_assert(offsetof(FwdBars, dl) % 16 == 0 && sizeof(FwdBars) <= 2048, "FwdBars layout");
@@ -244,9 +250,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
   // ---- gated: which tiles each group really computes ---------------------------------------------
   // The gate bound of a tile (flash_sparse_attn/ops/triton/activations.py:265-299) needs only the extremes of alpha
   // over the query tile and of delta over the key tile - both computed beforehand by gate_ext_kernel - and one
-  // running scalar per query tile. So every role (producer, MMA issuer, delta stager, softmax warps) walks the
-  // tiles with its own copy of that scalar and reaches the same decisions without talking to the others: a tile
-  // that both groups skip is never loaded, multiplied or staged (flash_gated_fwd.py:54-56 runs nothing for it).
+  // running scalar per query tile. The producer and the delta stager walk the tiles with their own copies of that
+  // scalar and reach the same decisions; the producer passes them to the MMA issuer, the stager to the softmax warps. A
+  // tile that both groups skip is never loaded, multiplied or staged (flash_gated_fwd.py:54-56 runs nothing for it).
   // The first tile of a group is never skipped: its running bound starts at -inf, the difference is +inf.
   float gw_amax[2] = {0.f, 0.f}, gw_amin[2] = {0.f, 0.f}, gw_thr[2] = {0.f, 0.f}, gw_run[2] = {-INFINITY, -INFINITY};
   float gw_c = 0.f;
@@ -270,9 +276,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
       gw_thr[q] = log2f(g_thr);
     }
   }
-  // Next tile below n_prev that at least one group computes; keep[q] says which. mark_q >= 0: this thread records
-  // the gate-skipped tiles of group mark_q in the tile map (value 3).
-  auto walk_next = [&](int n_prev, bool* keep, int mark_q) -> int {
+  // Next tile below n_prev that at least one group computes; keep[q] says which. `mark`: this thread records the
+  // gate-skipped tiles in the tile map (value 3).
+  auto walk_next = [&](int n_prev, bool* keep, bool mark) -> int {
     int n = next_tile(n_prev);
     if constexpr (KIND != KIND_GATED) {
       keep[0] = n >= 0 && fsa_fwd_tile_mode(sched[0], n, causal, local) >= 0;
@@ -289,7 +295,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
           const bool skip = (gmc - gw_run[q]) * gw_c < gw_thr[q];
           if (!skip) gw_run[q] = fmaxf(gmc, gw_run[q]);
           keep[q] = !skip;
-          if (skip && mark_q == q && p.tile_map) {
+          if (skip && mark && p.tile_map) {
             const int mb = pair * QT + q;
             p.tile_map[((((long long)si.b * p.hgrid + si.head) * p.num_m_blocks + mb) * p.num_splits + si.split) *
                            p.n_tiles_k + n] = 3;
@@ -394,13 +400,45 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
       };
       int t = 0, seen = 0;
       bool ok = true;
-      bool keep_unused[2];
-      int n = (KIND == KIND_GATED) ? walk_next(WALK_START, keep_unused, -1) : first_tile();
+      // Which tile comes next and who takes part in it is worked out here, ahead of time, and handed to the MMA issuer with
+      // the barrier that it waits on anyway: on windowed schedules the walk took the issuer 925 of the 4250 cycles of
+      // a step, in which the tensor pipe had nothing to do.
+      bool act[2], act_next[2];
+      auto take_part = [&](int n_t, bool* a) {  // not gated: the groups whose schedule has tile n_t
+#pragma unroll
+        for (int q = 0; q < 2; ++q) a[q] = n_t >= 0 && fsa_fwd_tile_mode(sched[q], n_t, causal, local) >= 0;
+      };
+      auto publish = [&](int slot, int n_t, const bool* a, unsigned last) {
+        const unsigned f = (a[0] ? 1u : 0u) | (a[1] ? 2u : 0u) | (last << 2);
+        *reinterpret_cast<volatile unsigned long long*>(&bars->step_info[slot]) =
+            (unsigned long long)(unsigned)n_t | ((unsigned long long)f << 32);
+      };
+      int n;
+      if constexpr (KIND == KIND_GATED) {
+        n = walk_next(WALK_START, act, false);
+      } else {
+        n = first_tile();
+        take_part(n, act);
+      }
+      publish(2, n, act, 0u);
       if (n >= 0) {
         load_kv(&p.map_k, smem + SM::kK, &bars->k0_full, n);
+      } else {
+        mbar_arrive(&bars->k0_full);
+        if (q_valid[0] || q_valid[1]) ok = mbar_wait(&bars->q_full, 0, abort_flag);  // nobody else waits for Q to land
       }
       while (n >= 0 && ok) {
-        const int n_next = (KIND == KIND_GATED) ? walk_next(n, keep_unused, -1) : next_tile(n);
+        int n_next;
+        unsigned last = 0u;  // gated: not known before the next tile's gate is; its output barriers come after the loop
+        if constexpr (KIND == KIND_GATED) {
+          n_next = walk_next(n, act_next, false);
+        } else {
+          n_next = next_tile(n);
+          take_part(n_next, act_next);
+#pragma unroll
+          for (int q = 0; q < 2; ++q)
+            if (act[q] && fsa_fwd_next_tile_below(sched[q], n, local) < 0) last |= 1u << q;
+        }
         // Release signals arrive in order (signal c: K(c) and V(c - 1) consumed). V(t) goes into the slot of
         // V(t - 2) and K(t + 1) into the slot of K(t - 1): both free after signal t - 1.
         auto need_signal = [&](int c) {
@@ -412,6 +450,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
         // V(t) replaces V(t - VSTAGES), K(t + 1) replaces K(t + 1 - KSTAGES): both are free after this signal
         need_signal(t - (KSTAGES < VSTAGES ? KSTAGES : VSTAGES) + 1);
         if (!ok) break;
+        publish(t & 1, n_next, act_next, last);  // the issuer has read the slot's last word: it came before signal t - 1
         // V is prefetched like K, before the softmax groups have voted on the tile: waiting for the vote
         // would put a full load latency between every S tile and its P V product, and in this
         // tensor-bound kernel a V tile that ends up unused only costs an L2 read: on inputs where 82 % of the
@@ -425,56 +464,54 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
         else
           mbar_arrive(&bars->kv_full[t & 1]);  // the barrier counts two arrivals per step
         n = n_next;
+        act[0] = act_next[0];
+        act[1] = act_next[1];
         ++t;
       }
     }
     __syncwarp();
   } else if (warp == 10) {
     // =============================== delta stager (gated only) ================================
-    // delta of every visited key tile as fp32 in a 2-slot ring, with the tile's max / min for the
-    // gate bound (flash_sparse_attn/ops/triton/flash_gated_fwd.py:100-115). Keys past the sequence
+    // delta of every computed key tile as fp32 in a 2-slot ring, with the tile's index and the groups' mask modes, so
+    // that the softmax warps need not walk the schedule (1600 to 2200 cycles a tile on their critical path)
+    // (flash_sparse_attn/ops/triton/flash_gated_fwd.py:100-115). Keys past the sequence
     // read as 0, like the reference's masked load (scheduler.py:1674-1691).
     if (KIND == KIND_GATED) {
       bool ok = !*abort_flag;
       const TO* dbase = reinterpret_cast<const TO*>(p.delta);
       int t = 0;
-      bool keep_unused[2];
-      for (int n = walk_next(WALK_START, keep_unused, -1); n >= 0 && ok; n = walk_next(n, keep_unused, -1), ++t) {
+      bool keep[2];
+      for (int n = walk_next(WALK_START, keep, lane == 0); ok; n = walk_next(n, keep, lane == 0), ++t) {
         const int s = t & 1, use = t >> 1;
         if (use > 0) ok = mbar_wait(&bars->d_empty[s], (use - 1) & 1, abort_flag);
         if (!ok) break;
-        float dv[4];
-        float dmax = -INFINITY, dmin = INFINITY;
+        if (n >= 0) {
+          float dv[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int k = n * TN + lane * 4 + j;
-          float v = 0.f;
-          if (k < si.sk) {
-            long long e;
-            if (p.flags & F_PAGED) {
-              const int page = p.page_table[(long long)si.b * p.pt_stride + k / p.page_size];
-              e = (long long)page * p.d_sb + (long long)si.hkv * p.d_sh + (k % p.page_size);
-            } else {
-              e = (long long)((p.flags & F_VARLEN_K) ? 0 : si.b) * p.d_sb + (long long)si.hkv * p.d_sh + si.off_k + k;
+          for (int j = 0; j < 4; ++j) {
+            const int k = n * TN + lane * 4 + j;
+            float v = 0.f;
+            if (k < si.sk) {
+              long long e;
+              if (p.flags & F_PAGED) {
+                const int page = p.page_table[(long long)si.b * p.pt_stride + k / p.page_size];
+                e = (long long)page * p.d_sb + (long long)si.hkv * p.d_sh + (k % p.page_size);
+              } else {
+                e = (long long)((p.flags & F_VARLEN_K) ? 0 : si.b) * p.d_sb + (long long)si.hkv * p.d_sh + si.off_k + k;
+              }
+              v = float(dbase[e]);
             }
-            v = float(dbase[e]);
+            dv[j] = v;
           }
-          dv[j] = v;
-          dmax = fmaxf(dmax, v);
-          dmin = fminf(dmin, v);
+          *reinterpret_cast<float4*>(&bars->dl[s][lane * 4]) = make_float4(dv[0], dv[1], dv[2], dv[3]);
         }
-#pragma unroll
-        for (int sft = 16; sft > 0; sft >>= 1) {
-          dmax = fmaxf(dmax, __shfl_xor_sync(0xffffffffu, dmax, sft));
-          dmin = fminf(dmin, __shfl_xor_sync(0xffffffffu, dmin, sft));
-        }
-        *reinterpret_cast<float4*>(&bars->dl[s][lane * 4]) = make_float4(dv[0], dv[1], dv[2], dv[3]);
-        if (lane == 0) {
-          bars->dl[s][TN] = dmax;
-          bars->dl[s][TN + 1] = dmin;
-        }
+        if (lane == 0)
+          *reinterpret_cast<int4*>(&bars->dl[s][TN]) =
+              make_int4(n, n >= 0 && keep[0] ? fsa_fwd_tile_mode(sched[0], n, causal, local) : -1,
+                        n >= 0 && keep[1] ? fsa_fwd_tile_mode(sched[1], n, causal, local) : -1, 0);
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->d_full[s]);
+        if (n < 0) break;
       }
     }
   } else if (warp == 9) {
@@ -488,8 +525,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
     bool ok = !*abort_flag;
     int cnt[2] = {0, 0}, cnt_kept[2] = {0, 0};
     bool o_started[2] = {false, false};
-    bool act[2], last[2];
-    int n = (KIND == KIND_GATED) ? walk_next(WALK_START, act, -1) : first_tile();
+    bool act[2] = {false, false}, last[2];
+    int n = -1;
+    auto read_info = [&](int slot, int& n_t, unsigned& f) {
+      const unsigned long long w = *reinterpret_cast<const volatile unsigned long long*>(&bars->step_info[slot]);
+      n_t = (int)(unsigned)w;
+      f = (unsigned)(w >> 32);
+    };
     // Every lane runs the same (warp-uniform) descriptor arithmetic; the MMA and commit instructions carry the
     // one-lane predicate themselves.
     const uint32_t lead = lane == 0 ? 1u : 0u;
@@ -511,47 +553,42 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
       }
       umma_commit_lead(lead, &bars->s_full[q]);
     };
+    if (ok) ok = mbar_wait(&bars->k0_full, 0, abort_flag);
+    if (ok) {
+      unsigned f;
+      read_info(2, n, f);
+      act[0] = f & 1u;
+      act[1] = f & 2u;
+    }
     if (n >= 0 && ok) {
       ok = mbar_wait(&bars->q_full, 0, abort_flag);
-      ok = ok && mbar_wait(&bars->k0_full, 0, abort_flag);
       tc_fence_after();
       if (ok) {
         for (int q = 0; q < 2; ++q)
-          if ((KIND == KIND_GATED) ? act[q] : (fsa_fwd_tile_mode(sched[q], n, causal, local) >= 0)) issue_s(q, 0);
+          if (act[q]) issue_s(q, 0);
         umma_commit_lead(lead, &bars->kv_empty[0]);
       }
     }
     int t = 0;
     // The tensor pipe takes an MMA from a thread about as fast as it executes one: while its MMAs run this warp
     // is blocked in their issue, and whatever it does between a group publishing P and the next MMA is time the
-    // pipe idles. So everything that does not depend on P (the walk over the tiles, who takes part in the next
-    // tile, the K / V arrivals) happens before the wait for P. (One issuer per group was tried: the second
+    // pipe idles. So the producer walks the tiles and says who takes part in the next one, and the K / V arrivals
+    // are handled before the wait for P. (One issuer per group was tried: the second
     // polling warp slows the softmax warps of its scheduler more than the overlap gains.)
-    if (KIND != KIND_GATED) {
-#pragma unroll
-      for (int q = 0; q < 2; ++q) act[q] = n >= 0 && fsa_fwd_tile_mode(sched[q], n, causal, local) >= 0;
-    }
     while (n >= 0 && ok) {
       bool act_next[2];
-      const int n_next = (KIND == KIND_GATED) ? walk_next(n, act_next, -1) : next_tile(n);
       const int vs = t % VSTAGES;
       const int ks_next = (t + 1) % KSTAGES;
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        if (KIND == KIND_GATED) {
-          // whether a later tile of this group survives the gate is not known yet: the output barriers are
-          // committed after the loop instead
-          last[q] = false;
-        } else if (!local) {  // one contiguous range of tiles per group
-          act_next[q] = n_next >= sched[q].n_min && n_next < sched[q].n_max;
-          last[q] = act[q] && n == sched[q].n_min;
-        } else {
-          act_next[q] = n_next >= 0 && fsa_fwd_tile_mode(sched[q], n_next, causal, local) >= 0;
-          last[q] = act[q] && fsa_fwd_next_tile_below(sched[q], n, local) < 0;
-        }
-      }
       ok = mbar_wait(&bars->kv_full[t & 1], (t >> 1) & 1, abort_flag);  // V(t) and K(t + 1)
       if (!ok) break;
+      int n_next;
+      unsigned f;
+      read_info(t & 1, n_next, f);
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        act_next[q] = (f >> q) & 1u;
+        last[q] = (f >> (2 + q)) & 1u;
+      }
       if ((p.flags & F_KV_RAGGED) && (n + 1) * TN > si.sk) {
         // keys past the sequence end carry probability 0 but their V rows may hold
         // anything: clear them so that 0 * garbage cannot produce NaN
@@ -674,32 +711,33 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
         const TO* ab = reinterpret_cast<const TO*>(p.alpha);
         alpha = float(ab[(long long)((p.flags & F_VARLEN_Q) ? 0 : si.b) * p.a_sb + (long long)q_head * p.a_sh +
                          si.off_q + q_idx]);
+        if (p.flags & F_LOGSIGMOID) alpha *= 1.4426950408889634f;
       }
     }
 
     int t_merged = -1;
-    bool keep[2] = {false, false};
-    const int mark_q = (wq == 0 && lane == 0) ? q : -1;  // one thread per group records its gate-skipped tiles
     int n = -1;
-    if (KIND == KIND_GATED)
-      n = walk_next(WALK_START, keep, mark_q);
-    else if (has_work)
-      n = first_tile();
-    for (; n >= 0 && ok; n = (KIND == KIND_GATED) ? walk_next(n, keep, mark_q) : next_tile(n)) {
+    if (KIND != KIND_GATED && has_work) n = first_tile();
+    for (; (KIND == KIND_GATED || n >= 0) && ok; n = (KIND == KIND_GATED) ? n : next_tile(n)) {
       ++t_merged;
-      const int mode = has_work ? fsa_fwd_tile_mode(my, n, causal, local) : -1;
+      int mode;
       const int ds = t_merged & 1;
-      if (KIND == KIND_GATED) {
-        // every tile that reaches this loop was staged by the delta warp (one of the groups computes it)
+      if constexpr (KIND == KIND_GATED) {
+        // every tile that one of the groups computes was staged by the delta warp, with its index and mask modes
         ok = mbar_wait(&bars->d_full[ds], (t_merged >> 1) & 1, abort_flag);
         if (!ok) break;
-        if (!keep[q]) {  // not in this group's schedule, or skipped by its gate: nothing was issued for it
+        const int4 info = *reinterpret_cast<const int4*>(&bars->dl[ds][TN]);
+        n = info.x;
+        if (n < 0) break;
+        mode = q == 0 ? info.y : info.z;
+        if (mode < 0) {  // not in this group's schedule, or skipped by its gate: nothing was issued for it
           __syncwarp();
           if (lane == 0) mbar_arrive(&bars->d_empty[ds]);
           continue;
         }
-      } else if (mode < 0) {
-        continue;
+      } else {
+        mode = has_work ? fsa_fwd_tile_mode(my, n, causal, local) : -1;
+        if (mode < 0) continue;
       }
       ok = mbar_wait(&bars->s_full[q], cnt_s & 1, abort_flag);
       if (!ok) break;
@@ -709,38 +747,87 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
       const int k0 = n * TN;
 
       // ---- scores of this row: TMEM -> registers (warp-collective loads, one wait) ---------------
-      uint32_t sr[TN];
+      // Gated kind: 32 columns at a time, and the gated and masked logits go back to TMEM, from where the exponentials
+      // below read them in pieces again: with the whole row in registers beside the gate's arithmetic the softmax
+      // warps spill (B4 S8192, windows of 512 to 4096: 3.23 -> 2.90 ms together with the packed gate). The other
+      // kinds hold the row: reading it twice costs them 17 % (dense, S = 16384: 1.93 -> 2.27 ms).
+      constexpr bool GATED = KIND == KIND_GATED;
+      uint32_t sr[GATED ? 32 : TN];
+      float p_mul = 1.0f, o_mul = 1.0f;
+      float m_cur;
+      if constexpr (GATED) {
+        TileMask tm = {{0, 0, 0}, {0u, 0u, 0u}};
+        if (mode != FSA_MASK_NONE) tm = make_tile_mask(rm, mode, k0);
+        // NaN: the maximum of a row without any number is NaN (it then takes no part in the vote)
+        float mx[4] = {__int_as_float(0x7fffffff), __int_as_float(0x7fffffff), __int_as_float(0x7fffffff),
+                       __int_as_float(0x7fffffff)};
+        const float2 al2 = make_float2(alpha, alpha);  // times log2(e) for the logsigmoid gate, whose exponential is 2^x
+        const bool logsig = p.flags & F_LOGSIGMOID;
+        // rolled up: unrolled over the row, the gate's code alone is larger than the instruction caches hold beside the
+        // other roles', and its 128 columns took 6700 cycles
+#pragma unroll 1
+        for (int ch = 0; ch < TN / 32; ++ch) {
+          uint32_t r[32];
+          tmem_ld32(tS + ch * 32, r);
+          tmem_ld_wait();
+          // logits = (q.k + g(alpha * delta_j)) * scale, g = logsigmoid or identity
+          // (flash_sparse_attn/ops/triton/flash_gated_fwd.py:104-122, activations.py:245-262)
+          const float4* d4 = reinterpret_cast<const float4*>(&bars->dl[ds][ch * 32]);
+          if (logsig) {
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+              const float4 dd = d4[i >> 2];
+              const float2 ga = add_log_sigmoid2(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])),
+                                                 mul2(al2, make_float2(dd.x, dd.y)));
+              const float2 gb = add_log_sigmoid2(make_float2(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])),
+                                                 mul2(al2, make_float2(dd.z, dd.w)));
+              r[i] = __float_as_uint(ga.x);
+              r[i + 1] = __float_as_uint(ga.y);
+              r[i + 2] = __float_as_uint(gb.x);
+              r[i + 3] = __float_as_uint(gb.y);
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+              const float4 dd = d4[i >> 2];
+              r[i] = __float_as_uint(fmaf(alpha, dd.x, __uint_as_float(r[i])));
+              r[i + 1] = __float_as_uint(fmaf(alpha, dd.y, __uint_as_float(r[i + 1])));
+              r[i + 2] = __float_as_uint(fmaf(alpha, dd.z, __uint_as_float(r[i + 2])));
+              r[i + 3] = __float_as_uint(fmaf(alpha, dd.w, __uint_as_float(r[i + 3])));
+            }
+          }
+          if (mode != FSA_MASK_NONE) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (!tile_col_visible(tm, i)) r[i] = 0xff800000u;  // -inf
+#pragma unroll
+            for (int j = 0; j < 3; ++j) tm.lo[j] -= 32;
+          } else if (!rm.row_ok) {
+            // rows past the query length read as zero scores in fully visible tiles
+#pragma unroll
+            for (int i = 0; i < 32; ++i) r[i] = 0u;
+          }
+          tmem_st32(tS + ch * 32, r);
+#pragma unroll
+          for (int i = 0; i < 32; i += 8) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              mx[j] = max3(mx[j], __uint_as_float(r[i + 2 * j]), __uint_as_float(r[i + 2 * j + 1]));
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->d_empty[ds]);
+        m_cur = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+      } else {
 #pragma unroll
       for (int ch = 0; ch < TN / 32; ++ch) tmem_ld32(tS + ch * 32, &sr[ch * 32]);
       tmem_ld_wait();
-      float p_mul = 1.0f, o_mul = 1.0f;
       if constexpr (F8) {
         if (bscaled) {
           const float ct = c * kbs[n];
 #pragma unroll
           for (int i = 0; i < TN; ++i) sr[i] = __float_as_uint(__uint_as_float(sr[i]) * ct);
         }
-      }
-      if (KIND == KIND_GATED) {
-        // logits = (q.k + g(alpha * delta_j)) * scale, g = logsigmoid or identity
-        // (flash_sparse_attn/ops/triton/flash_gated_fwd.py:104-122, activations.py:245-262)
-        const float4* d4 = reinterpret_cast<const float4*>(&bars->dl[ds][0]);
-        const bool logsig = p.flags & F_LOGSIGMOID;
-#pragma unroll
-        for (int i = 0; i < TN; i += 4) {
-          const float4 dd = d4[i >> 2];
-          const float dv[4] = {dd.x, dd.y, dd.z, dd.w};
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float x = alpha * dv[j];
-            float gte = x;
-            if (logsig)
-              gte = log_sigmoid_fast(x);
-            sr[i + j] = __float_as_uint(__uint_as_float(sr[i + j]) + gte);
-          }
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars->d_empty[ds]);
       }
       if (mode != FSA_MASK_NONE) {
         const TileMask tm = make_tile_mask(rm, mode, k0);
@@ -774,7 +861,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
         for (int i = 2; i < 32; i += 2)
           mx[j] = max3(mx[j], __uint_as_float(sr[j * 32 + i]), __uint_as_float(sr[j * 32 + i + 1]));
       }
-      const float m_cur = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+      m_cur = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+      }
 
       // ---- tile skip vote (flash_sparse_attn/ops/triton/activations.py:129-138) -----------------
       bool skip = false;
@@ -817,6 +905,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
       };
       if (skip) {
         publish_verdict(true);
+        if (GATED) tmem_st_wait();  // the next S tile overwrites these columns
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->p_full[q]);
@@ -862,15 +951,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
       const float neg_mc = -(m_ref * cc);
       const float2 nm2 = make_float2(neg_mc, neg_mc);
       float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-#pragma unroll
+      if (GATED) tmem_st_wait();
+      constexpr int EXP_UNROLL = GATED ? 1 : TN / 32;
+#pragma unroll EXP_UNROLL
       for (int ch = 0; ch < TN / 32; ++ch) {
         uint32_t pk[16];
+        if constexpr (GATED) {
+          tmem_ld32(tS + ch * 32, sr);
+          tmem_ld_wait();
+        }
+        const uint32_t* src = GATED ? sr : &sr[ch * 32];
 #pragma unroll
         for (int i = 0; i < 32; i += 4) {
-          const float2 ta = fma2(make_float2(__uint_as_float(sr[ch * 32 + i]), __uint_as_float(sr[ch * 32 + i + 1])),
-                                 c2, nm2);
-          const float2 tb =
-              fma2(make_float2(__uint_as_float(sr[ch * 32 + i + 2]), __uint_as_float(sr[ch * 32 + i + 3])), c2, nm2);
+          const float2 ta = fma2(make_float2(__uint_as_float(src[i]), __uint_as_float(src[i + 1])), c2, nm2);
+          const float2 tb = fma2(make_float2(__uint_as_float(src[i + 2]), __uint_as_float(src[i + 3])), c2, nm2);
           float2 ea, eb;
           ea.x = ex2_approx(ta.x);
           ea.y = ex2_approx(ta.y);
