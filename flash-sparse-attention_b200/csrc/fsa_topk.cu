@@ -86,18 +86,27 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* warp_tot, u
   return x + before;
 }
 
+constexpr int TK_COPIES = 8;  // copies of the histogram: the lanes of a warp spread over them (see below)
+constexpr int TK_PITCH = 257;  // a bin's copies lie in different banks
+
 // One thread-block cluster per row: CTA `rank` of `csize` owns the slice [rank * chunk, (rank + 1) * chunk) of the
 // row. The histograms of a radix pass are summed over the cluster through distributed shared memory (every CTA
-// reads all of them and walks the bins itself, so all agree without a broadcast); for the compaction every CTA
-// first counts the greater / equal entries of its slice and takes the counts of the slices before it as its base.
-// With 64 rows one CTA per row would leave more than half of a B200's 148 SMs idle.
-template <typename T, typename I>
+// reads all of them and finds the bin itself, so all agree without a broadcast); for the compaction every CTA
+// takes the counts of the slices before it as its base. With 64 rows one CTA per row would leave more than half of
+// a B200's 148 SMs idle.
+// What bounds it is the chain of dependent steps of a pass, not the bytes: so the bin is found by a scan over the 256
+// bins in parallel, a pass costs one cluster barrier (two sets of sums alternate), lanes spread over eight copies of
+// the histogram because scores share their leading bits (a warp's 32 updates would queue on two or three bins), and
+// with NC > 0 a thread keeps its 8 * NC consecutive entries in registers for all passes (NC = 0 reads the slice again in
+// every pass).
+template <typename T, typename I, int NC>
 __global__ void __launch_bounds__(TK_THREADS) topk_kernel(const T* __restrict__ scores, long long row_stride, int n, int k,
                                                           I* __restrict__ out, int csize, int chunk) {
   static_assert(TK_THREADS == 1024, "block_scan assumes 32 warps");
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
-  __shared__ uint32_t hist[256];
+  __shared__ uint32_t copies[TK_COPIES * TK_PITCH];
+  __shared__ uint32_t hist[2][256];
   __shared__ uint32_t warp_tot[TK_THREADS / 32];
   __shared__ uint32_t sel_prefix, sel_remaining;
   __shared__ uint32_t slice_cnt[2];  // greater / equal entries of this CTA's slice
@@ -105,55 +114,119 @@ __global__ void __launch_bounds__(TK_THREADS) topk_kernel(const T* __restrict__ 
   const int row_idx = blockIdx.x / csize;
   const T* row = scores + (long long)row_idx * row_stride;
   I* dst = out + (long long)row_idx * k;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31;
   const bool vec_ok = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
   constexpr int PASSES = KeyOf<T>::kBits / 8;
   constexpr int STEP = TK_THREADS * TK_V;
   const int lo = rank * chunk < n ? rank * chunk : n;
   const int hi = lo + chunk < n ? lo + chunk : n;  // this CTA's slice [lo, hi); chunk is a multiple of TK_V
+  const int mine = lo + tid * (NC * TK_V);         // NC > 0: this thread's first entry
+  uint32_t kc[NC > 0 ? NC * TK_V : 1];
+  if constexpr (NC > 0) {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) load_keys(row, vec_ok, mine + c * TK_V, hi, 0u, kc + c * TK_V);
+  }
+  for (int i = tid; i < TK_COPIES * TK_PITCH; i += TK_THREADS) copies[i] = 0;
+  __syncthreads();
 
   // ---- radix select: after pass d the top 8(d+1) bits of the k-th largest key are known ----------------
   uint32_t prefix = 0, remaining = (uint32_t)k;  // keys above the prefix range so far: k - remaining
   for (int pass = 0; pass < PASSES; ++pass) {
     const int shift = KeyOf<T>::kBits - 8 - 8 * pass;
     const uint32_t mask_hi = pass == 0 ? 0u : (0xffffffffu << (shift + 8));
-    for (int i = tid; i < 256; i += TK_THREADS) hist[i] = 0;
-    __syncthreads();
-    for (int start = lo; start < hi; start += STEP) {
-      const int i0 = start + tid * TK_V;
-      if (i0 < hi) {
-        uint32_t keys[TK_V];
-        load_keys(row, vec_ok, i0, hi, 0u, keys);
+    uint32_t* my_copy = copies + (lane & (TK_COPIES - 1)) * TK_PITCH;
+    auto count = [&](uint32_t key) {
+      if ((key & mask_hi) == prefix) atomicAdd(my_copy + ((key >> shift) & 255u), 1u);
+    };
+    if constexpr (NC > 0) {
 #pragma unroll
-        for (int j = 0; j < TK_V; ++j)
-          if (i0 + j < hi && (keys[j] & mask_hi) == prefix) atomicAdd(&hist[(keys[j] >> shift) & 255u], 1u);
+      for (int j = 0; j < NC * TK_V; ++j)
+        if (mine + j < hi) count(kc[j]);
+    } else {
+      for (int start = lo; start < hi; start += STEP) {
+        const int i0 = start + tid * TK_V;
+        if (i0 < hi) {
+          uint32_t keys[TK_V];
+          load_keys(row, vec_ok, i0, hi, 0u, keys);
+#pragma unroll
+          for (int j = 0; j < TK_V; ++j)
+            if (i0 + j < hi) count(keys[j]);
+        }
       }
     }
-    cluster.sync();  // every CTA's histogram is complete
-    uint32_t total_bin = 0;
-    if (tid < 256)
-      for (int r = 0; r < csize; ++r) total_bin += *cluster.map_shared_rank(&hist[tid], r);
-    cluster.sync();  // all remote reads done: the histograms may be cleared again
-    if (tid < 256) hist[tid] = total_bin;
     __syncthreads();
-    if (tid == 0) {
-      // walk the bins from the top until `remaining` keys are covered
-      uint32_t rem = remaining;
-      int bin = 255;
-      for (; bin > 0; --bin) {
-        if (hist[bin] >= rem) break;
-        rem -= hist[bin];
+    if (tid < 256) {
+      uint32_t sum = 0;
+#pragma unroll
+      for (int r = 0; r < TK_COPIES; ++r) {
+        sum += copies[r * TK_PITCH + tid];
+        copies[r * TK_PITCH + tid] = 0;  // for the next pass
       }
-      sel_prefix = prefix | ((uint32_t)bin << shift);
-      sel_remaining = rem;  // how many keys of this bin (with this prefix) are still needed
+      hist[pass & 1][tid] = sum;
+    }
+    cluster.sync();  // every CTA's sums are there, and everybody has read those of the pass before
+    if (tid < 256) {
+      // thread t takes bin 255 - t: the first bin from the top at which `remaining` keys are covered
+      const int bin = 255 - tid;
+      uint32_t v = 0;
+#pragma unroll
+      for (int r = 0; r < 8; ++r)  // unrolled: the remote reads are in flight together
+        if (r < csize) v += *cluster.map_shared_rank(&hist[pass & 1][bin], r);
+      uint32_t x = v;
+#pragma unroll
+      for (int s = 1; s < 32; s <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, s);
+        if (lane >= s) x += y;
+      }
+      if (lane == 31) warp_tot[tid >> 5] = x;
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      for (int w = 0; w < (tid >> 5); ++w) x += warp_tot[w];
+      if (x >= remaining && x - v < remaining) {
+        sel_prefix = prefix | ((uint32_t)bin << shift);
+        sel_remaining = remaining - (x - v);  // how many keys of this bin (with this prefix) are still needed
+      }
     }
     __syncthreads();
     prefix = sel_prefix;
     remaining = sel_remaining;
-    __syncthreads();
   }
   const uint32_t thr = prefix;         // key of the k-th largest entry
   const uint32_t need_eq = remaining;  // entries equal to it that belong to the selection (lowest positions)
+
+  if constexpr (NC > 0) {
+    // ---- one scan over the slice; positions come out ascending ------------------------------------------
+    // (greater in the low half, equal in the high half: a slice has at most 1024 * 8 * NC <= 32768 entries)
+    uint32_t cnt = 0, total;
+#pragma unroll
+    for (int j = 0; j < NC * TK_V; ++j)
+      if (mine + j < hi) cnt += (kc[j] > thr ? 1u : 0u) | (kc[j] == thr ? 0x10000u : 0u);
+    const uint32_t inc = block_scan(cnt, warp_tot, &total);
+    uint32_t gt_before = (inc & 0xffffu) - (cnt & 0xffffu), eq_before = (inc >> 16) - (cnt >> 16);
+    if (csize > 1) {
+      if (tid == 0) slice_cnt[0] = total;
+      cluster.sync();
+#pragma unroll
+      for (int r = 0; r < 7; ++r) {
+        const uint32_t t = r < rank ? *cluster.map_shared_rank(&slice_cnt[0], r) : 0u;
+        gt_before += t & 0xffffu;
+        eq_before += t >> 16;
+      }
+    }
+    if (cnt != 0u) {
+#pragma unroll
+      for (int j = 0; j < NC * TK_V; ++j) {
+        if (mine + j < hi) {
+          const bool gt = kc[j] > thr, eq = kc[j] == thr;
+          if (gt || (eq && eq_before < need_eq))
+            dst[gt_before + (eq_before < need_eq ? eq_before : need_eq)] = (I)(mine + j);
+          gt_before += gt ? 1u : 0u;
+          eq_before += eq ? 1u : 0u;
+        }
+      }
+    }
+    cluster.sync();  // nobody leaves while another CTA may still read its shared memory
+    return;
+  }
 
   // ---- counts of this slice, bases from the slices before it ------------------------------------------
   uint32_t base_gt = 0, base_eq = 0;  // greater / equal entries before the current step of this CTA
@@ -216,11 +289,12 @@ __global__ void __launch_bounds__(TK_THREADS) topk_kernel(const T* __restrict__ 
 }
 
 // Cluster size: the largest power of two up to 8 that keeps rows * size within the SM count, and leaves a slice
-// of at least one step per CTA.
+// of at least TOPK_MIN_SLICE entries per CTA (below that the exchange costs more than the shorter slice gains).
+constexpr int TOPK_MIN_SLICE = 2048;
 inline int topk_cluster_size(int rows, int n) {
   int c = 1;
   const int sms = device_sm_count();
-  while (c < 8 && rows * (c * 2) <= sms && n / (c * 2) >= TK_THREADS * TK_V) c *= 2;
+  while (c < 8 && rows * (c * 2) <= sms && n / (c * 2) >= TOPK_MIN_SLICE) c *= 2;
   return c;
 }
 
@@ -241,8 +315,14 @@ cudaError_t launch_topk_t(const void* scores, long long row_stride, int rows, in
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, topk_kernel<T, I>, reinterpret_cast<const T*>(scores), row_stride, n, k,
-                            reinterpret_cast<I*>(out), csize, chunk);
+  const T* x = reinterpret_cast<const T*>(scores);
+  I* o = reinterpret_cast<I*>(out);
+  // slices of up to 8192 / 16384 entries stay in registers
+  if (chunk <= TK_THREADS * TK_V)
+    return cudaLaunchKernelEx(&cfg, topk_kernel<T, I, 1>, x, row_stride, n, k, o, csize, chunk);
+  if (chunk <= TK_THREADS * TK_V * 2)
+    return cudaLaunchKernelEx(&cfg, topk_kernel<T, I, 2>, x, row_stride, n, k, o, csize, chunk);
+  return cudaLaunchKernelEx(&cfg, topk_kernel<T, I, 0>, x, row_stride, n, k, o, csize, chunk);
 }
 
 template <typename T>
