@@ -53,7 +53,7 @@ struct BwdSmem {
   static constexpr int kStage = kDS + 32768;   // dQ staging for the TMA reduce-add: 8 warps x 4 KB
   static constexpr int kAux = kStage + 32768;  // lse2[2][128], dpsum[2][128] fp32, alpha[2][128] 16-bit (gated)
   static constexpr int kBar = kAux + 2560;
-  static constexpr int kTotal = kBar + 256;
+  static constexpr int kTotal = kBar + 384;
 };
 
 struct BwdBars {
@@ -63,11 +63,15 @@ struct BwdBars {
   uint64_t stg_full, stg_free;  // dQ staging: compute warps -> drain warp (job posted) and back (buffers read)
   int job[2][4];                // job descriptors {first row, head, query tile, code}, slot = job index & 1
   int dqjob[2][4];              // MMA issuer -> dQ warps: {first row, head, query tile, code} of the dQ tile in TMEM
+  // Step it (slot it & 1), published by the producer with q_full: head of the group, query tile, mask mode, and bit 0: first
+  // step of its head, bit 1: another step follows. One lane walks the steps; the MMA issuer and the compute warps, whose
+  // time a step is made of, read what they need.
+  alignas(16) int step[2][4];
   uint32_t tmem_base;
   int abort_flag;
   unsigned char vote_any[2][8];
 };
-static_assert(sizeof(BwdBars) <= 256, "barrier block too large");
+static_assert(sizeof(BwdBars) <= 384, "barrier block too large");
 
 // Visible query columns of one key row inside query tile [q0, q0 + TM), as up to three half-open
 // intervals of the tile-local index (mask.py:52-102 read along the query axis).
@@ -448,13 +452,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
         // buffer and is reloaded as soon as dV of the previous step has consumed it.
         bool ok = true;
         StepWalk wk = walk_begin();
-        int g = 0, m = 0, mode_unused = 0;
-        bool first_unused = false;
-        for (int it = 0; ok && walk_next(wk, g, m, mode_unused, first_unused, false); ++it) {
+        int g = 0, m = 0, mode = 0, g_n = 0, m_n = 0, mode_n = 0;
+        bool first = false, first_n = false;
+        bool more = walk_next(wk, g_n, m_n, mode_n, first_n, true);  // records the dropped steps in the tile map
+        for (int it = 0; ok && more; ++it) {
+          g = g_n;
+          m = m_n;
+          mode = mode_n;
+          first = first_n;
+          more = walk_next(wk, g_n, m_n, mode_n, first_n, true);
           const int st = it & 1, use = it >> 1;
           const int head = hkv * p.G + g;
           if (use > 0) ok = mbar_wait(&bars->q_empty[st], (use - 1) & 1, abort_flag);
           if (!ok) break;
+          *reinterpret_cast<int4*>(bars->step[st]) = make_int4(g, m, mode, (first ? 1 : 0) | (more ? 2 : 0));
           mbar_arrive_expect_tx(&bars->q_full[st], SM::kTile + 1024 + (KIND == KIND_GATED ? 256 : 0));
           for (int d = 0; d < HD; d += 64)
             tma_load_4d(smem + SM::kQ + st * SM::kTile + (d / 64) * (TM * 128), &p.map_q, &bars->q_full[st], d, head,
@@ -505,10 +516,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
         }
         umma_commit_lead(lead, &bars->s_full);
       };
-      StepWalk wk = walk_begin();
-      int g_nxt = 0, m_nxt = 0, mode_unused = 0;
-      bool first_unused = false;
-      bool has_cur = ok && walk_next(wk, g_nxt, m_nxt, mode_unused, first_unused, false);
+      int g_nxt = 0, m_nxt = 0;
+      bool has_cur;
+      {
+        StepWalk wk = walk_begin();  // whether there is any step
+        int mode_unused = 0;
+        bool first_unused = false;
+        has_cur = ok && walk_next(wk, g_nxt, m_nxt, mode_unused, first_unused, false);
+      }
       const bool det = p.flags & F_DETERMINISTIC;
       int n_jobs = 0;  // dQ tiles (and, deterministic mode, passes) handed to the dQ warps so far
       // descriptor of the dQ tile the next commit on dq_full announces; written well before the MMAs it follows
@@ -531,7 +546,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
       for (int it = 0; has_cur && ok; ++it) {
         const int st = it & 1;
         const int g_cur = g_nxt, m_cur = m_nxt;
-        const bool has_next = walk_next(wk, g_nxt, m_nxt, mode_unused, first_unused, false);
+        const bool has_next = *reinterpret_cast<const volatile int*>(&bars->step[st][3]) & 2;
         // The verdict of the skip vote is read straight from the votes (the compute warps publish them well before
         // the exponentials), so that dP^T is under way while P^T is still being computed.
         bool skip = false;
@@ -583,6 +598,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
           if (!ok) break;
           tc_fence_after();
           issue_st((it + 1) & 1);
+          g_nxt = *reinterpret_cast<const volatile int*>(&bars->step[(it + 1) & 1][0]);
+          m_nxt = *reinterpret_cast<const volatile int*>(&bars->step[(it + 1) & 1][1]);
         }
         if (!skip) {
           ok = mbar_wait(&bars->ds_full, n_live & 1, abort_flag);
@@ -775,12 +792,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
     };
 
     // ---- P step: scores -> probabilities (and the skip vote) ------------------------------------
-    StepWalk wk = walk_begin();
-    const bool mark_steps = cw == 0 && lane == 0;  // one thread records the dropped steps in the tile map
     int m_p = 0, g_p = 0;  // query tile and head (within the group) of the step p_step just handled
-    // returns the skip decision; steps are visited in order: (g, m, mode, first step of its head) from the walk
-    auto p_step = [&](int it, int g, int m, int mode, bool first_of_head) -> bool {
+    bool more = false;     // another step follows it
+    // returns the skip decision; steps are visited in order, as the producer publishes them
+    auto p_step = [&](int it) -> bool {
       const int st = it & 1, par = it & 1;
+      // the step's description and lse2 / dpsum arrive with the Q tile, well before its scores
+      if (!mbar_wait(&bars->q_full[st], (it >> 1) & 1, abort_flag)) {
+        ok = false;
+        return true;
+      }
+      const int4 info = *reinterpret_cast<const int4*>(bars->step[st]);
+      const int g = info.x, m = info.y, mode = info.z;
+      const bool first_of_head = info.w & 1;
+      more = info.w & 2;
       g_p = g;
       m_p = m;
       // skip thresholds of the group's first and last query column: worked out before S is waited for
@@ -794,11 +819,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
         thr_lo = fminf(lg_thr - lg2_approx(vis_last), 0.0f);
       }
       if (!mbar_wait(&bars->s_full, par, abort_flag)) {
-        ok = false;
-        return true;
-      }
-      // lse2 / dpsum arrived with the Q tile; observing the barrier makes them visible here
-      if (!mbar_wait(&bars->q_full[st], (it >> 1) & 1, abort_flag)) {
         ok = false;
         return true;
       }
@@ -1082,12 +1102,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
       if (lane == 0) mbar_arrive(&bars->ds_full);
     };
 
-    int w_g = 0, w_m = 0, w_mode = 0;
-    bool w_first = false;
-    bool has_cur = ok && walk_next(wk, w_g, w_m, w_mode, w_first, mark_steps);
+    bool has_cur;
+    {
+      StepWalk wk = walk_begin();  // whether there is any step
+      int g0 = 0, m0 = 0, mode0 = 0;
+      bool first0 = false;
+      has_cur = ok && walk_next(wk, g0, m0, mode0, first0, false);
+    }
     const bool any_step = has_cur;
     if (has_cur) {
-      skip_cur = p_step(0, w_g, w_m, w_mode, w_first);
+      skip_cur = p_step(0);
       m_cur = m_p;
       g_cur = g_p;
     }
@@ -1097,8 +1121,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
         n_live++;
       }
       bool skip_next = false;
-      const bool has_next = walk_next(wk, w_g, w_m, w_mode, w_first, mark_steps);
-      if (ok && has_next) skip_next = p_step(it + 1, w_g, w_m, w_mode, w_first);
+      const bool has_next = more;
+      if (ok && has_next) skip_next = p_step(it + 1);
       skip_cur = skip_next;
       m_cur = m_p;
       g_cur = g_p;
