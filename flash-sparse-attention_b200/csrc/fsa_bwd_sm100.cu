@@ -786,10 +786,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
       }
       return cm;
     };
-    auto visible = [&](const ColMask& cm, int i) {
-      return (unsigned(i - cm.lo[0]) < cm.len[0]) | (unsigned(i - cm.lo[1]) < cm.len[1]) |
-             (unsigned(i - cm.lo[2]) < cm.len[2]);
-    };
 
     // ---- P step: scores -> probabilities (and the skip vote) ------------------------------------
     int m_p = 0, g_p = 0;  // query tile and head (within the group) of the step p_step just handled
@@ -912,18 +908,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
         }
       }
       if (masked) {
-        const int n_iv = (cm.len[0] != 0u) + (cm.len[1] != 0u) + (cm.len[2] != 0u);
-        if (__all_sync(0xffffffffu, n_iv <= 1)) {  // at most one interval per key row: one compare per entry
-          const int which = cm.len[1] != 0u ? 1 : (cm.len[2] != 0u ? 2 : 0);
-          const int nlo = wg * 64 - (which == 1 ? cm.lo[1] : (which == 2 ? cm.lo[2] : cm.lo[0]));
-          const unsigned len = which == 1 ? cm.len[1] : (which == 2 ? cm.len[2] : cm.len[0]);
 #pragma unroll
-          for (int i = 0; i < 64; ++i)
-            if (unsigned(i + nlo) >= len) x[i] = -INFINITY;
-        } else {
+        for (int h = 0; h < 2; ++h) {  // one test of a bit per entry, whatever the mask is made of
+          const int base = wg * 64 + h * 32;
+          const uint32_t bits = interval_bits(cm.lo[0], cm.len[0], base) | interval_bits(cm.lo[1], cm.len[1], base) |
+                                interval_bits(cm.lo[2], cm.len[2], base);
 #pragma unroll
-          for (int i = 0; i < 64; ++i)
-            if (!visible(cm, wg * 64 + i)) x[i] = -INFINITY;
+          for (int i = 0; i < 32; ++i)
+            if (!(bits & (1u << i))) x[h * 32 + i] = -INFINITY;
         }
       }
       bool skip = false;

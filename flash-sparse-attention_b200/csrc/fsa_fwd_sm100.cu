@@ -146,9 +146,17 @@ __device__ __forceinline__ TileMask make_tile_mask(const RowMask& rm, int mode, 
   }
   return tm;
 }
-__device__ __forceinline__ bool tile_col_visible(const TileMask& tm, int i) {
-  return (unsigned(i - tm.lo[0]) < tm.len[0]) | (unsigned(i - tm.lo[1]) < tm.len[1]) |
-         (unsigned(i - tm.lo[2]) < tm.len[2]);
+// Visible columns [base, base + 32) as bits, and their application: the row's other entries become -inf. One test of a bit
+// per entry whatever the mask is made of; a masked tile's code is met cold (two of nine tiles under a 1024-token window),
+// so its length counts most.
+__device__ __forceinline__ uint32_t tile_bits(const TileMask& tm, int base) {
+  return interval_bits(tm.lo[0], tm.len[0], base) | interval_bits(tm.lo[1], tm.len[1], base) |
+         interval_bits(tm.lo[2], tm.len[2], base);
+}
+__device__ __forceinline__ void mask_cols32(uint32_t* r, uint32_t bits) {
+#pragma unroll
+  for (int i = 0; i < 32; ++i)
+    if (!(bits & (1u << i))) r[i] = 0xff800000u;
 }
 
 // BSCALE: FP8 inputs with one scale per 128-position block (a separate instantiation: as a run-time switch it cost
@@ -749,7 +757,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
       // ---- scores of this row: TMEM -> registers (warp-collective loads, one wait) ---------------
       // Gated kind: 32 columns at a time, and the gated and masked logits go back to TMEM, from where the exponentials
       // below read them in pieces again: with the whole row in registers beside the gate's arithmetic the softmax
-      // warps spill (B4 S8192, windows of 512 to 4096: 3.23 -> 2.90 ms together with the packed gate). The other
+      // warps spill (B4 S8192, windows of 512 to 4096: 3.24 -> 2.90 ms together with the packed gate). The other
       // kinds hold the row: reading it twice costs them 17 % (dense, S = 16384: 1.93 -> 2.27 ms).
       constexpr bool GATED = KIND == KIND_GATED;
       uint32_t sr[GATED ? 32 : TN];
@@ -797,11 +805,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
             }
           }
           if (mode != FSA_MASK_NONE) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (!tile_col_visible(tm, i)) r[i] = 0xff800000u;  // -inf
-#pragma unroll
-            for (int j = 0; j < 3; ++j) tm.lo[j] -= 32;
+            mask_cols32(r, tile_bits(tm, ch * 32));
           } else if (!rm.row_ok) {
             // rows past the query length read as zero scores in fully visible tiles
 #pragma unroll
@@ -831,21 +835,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
       }
       if (mode != FSA_MASK_NONE) {
         const TileMask tm = make_tile_mask(rm, mode, k0);
-        // most masked tiles leave every row one interval (causal diagonal, one window band, key tail):
-        // one compare per entry instead of three
-        const int n_iv = (tm.len[0] != 0u) + (tm.len[1] != 0u) + (tm.len[2] != 0u);
-        if (__all_sync(0xffffffffu, n_iv <= 1)) {
-          const int which = tm.len[1] != 0u ? 1 : (tm.len[2] != 0u ? 2 : 0);
-          const int nlo = -(which == 1 ? tm.lo[1] : (which == 2 ? tm.lo[2] : tm.lo[0]));
-          const unsigned len = which == 1 ? tm.len[1] : (which == 2 ? tm.len[2] : tm.len[0]);
 #pragma unroll
-          for (int i = 0; i < TN; ++i)
-            if (unsigned(i + nlo) >= len) sr[i] = 0xff800000u;  // -inf
-        } else {
-#pragma unroll
-          for (int i = 0; i < TN; ++i)
-            if (!tile_col_visible(tm, i)) sr[i] = 0xff800000u;  // -inf
-        }
+        for (int ch = 0; ch < TN / 32; ++ch) mask_cols32(&sr[ch * 32], tile_bits(tm, ch * 32));
       } else if (!rm.row_ok) {
         // rows past the query length read as zero scores in fully visible tiles
 #pragma unroll

@@ -342,6 +342,18 @@ __device__ __forceinline__ float lg2_approx(float x) {
   return y;
 }
 
+// Bits [a, a + n) of a word, a and n clamped to it: a in 0..32, n >= 0.
+__device__ __forceinline__ uint32_t bit_range(int a, int n) {
+  uint32_t r;
+  asm("bmsk.clamp.b32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(n));
+  return r;
+}
+// The part of the half-open interval [lo, lo + len) that falls on columns [base, base + 32), as bits.
+__device__ __forceinline__ uint32_t interval_bits(int lo, unsigned len, int base) {
+  const int a = max(lo - base, 0), b = min(lo + (int)len - base, 32);
+  return bit_range(a, max(b - a, 0));
+}
+
 // 3-input maximum and packed two-wide fp32 arithmetic (one instruction for two lanes of data).
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
