@@ -846,6 +846,37 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
         gate_skip = (gmc - gate_max) * c < log2f(g_thr);
         if (!gate_skip) gate_max = fmaxf(gmc, gate_max);
       }
+      if constexpr (KIND == KIND_GATED) {
+        // logits = (q.k + g(alpha_q * delta_k)) * scale, g = logsigmoid or identity (flash_gated_bwd.py:81-98). A rolled
+        // loop over 16 columns, through TMEM: unrolled over the row it does not stay in the instruction caches beside
+        // the code of the other roles.
+        const uint4* al4 = reinterpret_cast<const uint4*>(s_alpha + st * 128 + wg * 64);
+        const float2 dl2 = make_float2(dlt_g, dlt_g);  // delta, times log2(e) for the logsigmoid gate
+        const uint32_t tcol = tmem_base + lane_addr + TMEM_S + wg * 64;
+#pragma unroll 1
+        for (int qt = 0; qt < 4; ++qt) {
+          uint32_t r[16];
+          tmem_ld16(tcol + qt * 16, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int c8 = 0; c8 < 2; ++c8) {
+            const uint4 av = al4[qt * 2 + c8];
+            const uint32_t aw[4] = {av.x, av.y, av.z, av.w};
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) {
+              float a0, a1;
+              unpack16(aw[j >> 1], a0, a1);
+              const float2 y = mul2(make_float2(a0, a1), dl2);
+              const float2 s2 = make_float2(__uint_as_float(r[c8 * 8 + j]), __uint_as_float(r[c8 * 8 + j + 1]));
+              const float2 v = logsig ? add_log_sigmoid2(s2, y) : add2(s2, y);
+              r[c8 * 8 + j] = __float_as_uint(v.x);
+              r[c8 * 8 + j + 1] = __float_as_uint(v.y);
+            }
+          }
+          tmem_st16(tcol + qt * 16, r);
+        }
+        tmem_st_wait();
+      }
       uint32_t sr[64];
       tmem_ld32(tmem_base + lane_addr + TMEM_S + wg * 64, &sr[0]);
       tmem_ld32(tmem_base + lane_addr + TMEM_S + wg * 64 + 32, &sr[32]);
@@ -856,26 +887,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
       if (masked) cm = col_mask(mode, m);  // 64-bit interval arithmetic: only for the tiles that need it
       const float4* lse4 = reinterpret_cast<const float4*>(s_lse + st * 128 + wg * 64);
       float x[64];  // log2 of the probabilities
-      if (KIND == KIND_GATED) {
-        // logits = (q.k + g(alpha_q * delta_k)) * scale, g = logsigmoid or identity (flash_gated_bwd.py:81-98)
-        const uint4* al4 = reinterpret_cast<const uint4*>(s_alpha + st * 128 + wg * 64);
-        const float2 dl2 = make_float2(dlt_g, dlt_g);  // delta, times log2(e) for the logsigmoid gate
-#pragma unroll
-        for (int i = 0; i < 64; i += 8) {
-          const uint4 av = al4[i >> 3];
-          const uint32_t aw[4] = {av.x, av.y, av.z, av.w};
-#pragma unroll
-          for (int j = 0; j < 8; j += 2) {
-            float a0, a1;
-            unpack16(aw[j >> 1], a0, a1);
-            const float2 y = mul2(make_float2(a0, a1), dl2);
-            const float2 s2 = make_float2(__uint_as_float(sr[i + j]), __uint_as_float(sr[i + j + 1]));
-            const float2 r = logsig ? add_log_sigmoid2(s2, y) : add2(s2, y);
-            sr[i + j] = __float_as_uint(r.x);
-            sr[i + j + 1] = __float_as_uint(r.y);
-          }
-        }
-      }
       const float2 c2 = make_float2(c, c);
 #pragma unroll
       for (int i = 0; i < 64; i += 4) {
