@@ -60,6 +60,18 @@ __global__ void __launch_bounds__(256) combine_kernel(CombineParams p) {
   // reduction and the loads of the partial rows do not depend on one another.
   for (int s0 = 0; s0 < p.num_splits; s0 += 32) {
     const int cnt = min(32, p.num_splits - s0);
+    const float* src = op + (long long)s0 * p.op_ss + d0;
+    // the rows of eight splits are requested before their weights are known
+    float4 v[8][VEC / 4];
+    auto load8 = [&](int first) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int i = 0; i < VEC / 4; ++i)
+          v[j][i] = (active && first + j < cnt) ? *reinterpret_cast<const float4*>(src + (long long)(first + j) * p.op_ss + 4 * i)
+                                                : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    load8(0);
     const float lse_l = lane < cnt ? lp[(long long)(s0 + lane) * p.lp_ss] : -INFINITY;
     float c_max = lse_l;
 #pragma unroll
@@ -74,18 +86,17 @@ __global__ void __launch_bounds__(256) combine_kernel(CombineParams p) {
     e_max = new_max;
 #pragma unroll
     for (int i = 0; i < VEC; ++i) acc[i] *= old_scale;
-    const float* src = op + (long long)s0 * p.op_ss + d0;
-#pragma unroll 4
-    for (int sp = 0; sp < cnt; ++sp) {
-      const float w = __shfl_sync(0xffffffffu, w_l, sp);
-      if (active) {
+    for (int first = 0; first < cnt; first += 8) {
+      if (first > 0) load8(first);
 #pragma unroll
-        for (int i = 0; i < VEC; i += 4) {
-          const float4 v = __ldcs(reinterpret_cast<const float4*>(src + (long long)sp * p.op_ss + i));
-          acc[i] += w * v.x;
-          acc[i + 1] += w * v.y;
-          acc[i + 2] += w * v.z;
-          acc[i + 3] += w * v.w;
+      for (int j = 0; j < 8; ++j) {
+        const float w = __shfl_sync(0xffffffffu, w_l, first + j);  // past cnt: weight 0 and rows of zeros
+#pragma unroll
+        for (int i = 0; i < VEC / 4; ++i) {
+          acc[4 * i] += w * v[j][i].x;
+          acc[4 * i + 1] += w * v[j][i].y;
+          acc[4 * i + 2] += w * v[j][i].z;
+          acc[4 * i + 3] += w * v[j][i].w;
         }
       }
     }

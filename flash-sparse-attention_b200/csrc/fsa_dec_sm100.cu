@@ -155,7 +155,9 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
 // accumulator takes 32 registers instead of 64, the Q fragments 16 instead of 32, a tile needs 8 + 8 MMAs instead of
 // 16 + 16, and three CTAs fit an SM instead of two. P^T reaches its B-operand layout through movmatrix.
 // OCC: CTAs per SM the kernel is compiled for (the transposed variant exists for 2 and for 3).
-template <int HD, typename T, int KIND, bool TR, int OCC>
+// CL: the splits of a (sequence, KV head) are one cluster and merge their results themselves (an instantiation of its own:
+// as a run-time switch it cost the bandwidth-bound calls, which never take it, 0.5 %).
+template <int HD, typename T, int KIND, bool TR, int OCC, bool CL>
 __global__ void __launch_bounds__(DWARPS * 32, OCC) dec_kernel(const DecKernelParams p) {
   // T: element type of q, k, v. FP8 (e4m3 / e5m2, head size 128) tiles are copied as bytes and widened
   // exactly to fp16 in registers in front of the fp16 mma.sync; a 16-byte chunk of a key row then holds
@@ -175,7 +177,7 @@ __global__ void __launch_bounds__(DWARPS * 32, OCC) dec_kernel(const DecKernelPa
 
   // KV heads fastest; with the splits of a (sequence, KV head) in one cluster the splits are
   int idx = blockIdx.x, hkv, split, b;
-  if (p.cluster > 1) {
+  if (CL) {
     split = idx % p.num_splits;
     idx /= p.num_splits;
     hkv = idx % p.Hkv;
@@ -801,7 +803,7 @@ __global__ void __launch_bounds__(DWARPS * 32, OCC) dec_kernel(const DecKernelPa
     }
     __syncthreads();
     const float* all = reinterpret_cast<const float*>(dsm);
-    float* xo = reinterpret_cast<float*>(dsm) + DWARPS * (16 * HD + 32);  // cluster: merged state of this CTA
+    [[maybe_unused]] float* xo = reinterpret_cast<float*>(dsm) + DWARPS * (16 * HD + 32);  // CL: merged state of this CTA
     for (int item = tid; item < 16 * (HD / 4); item += DWARPS * 32) {
       const int r = item / (HD / 4), d0 = (item % (HD / 4)) * 4;
       const int row = mt * MROWS + r;
@@ -823,7 +825,7 @@ __global__ void __launch_bounds__(DWARPS * 32, OCC) dec_kernel(const DecKernelPa
         acc.z += ov.z * wgt;
         acc.w += ov.w * wgt;
       }
-      if (p.cluster > 1) {  // this split's state for the others of the cluster
+      if (CL) {  // this split's state for the others of the cluster
         *reinterpret_cast<float4*>(xo + r * HD + d0) = acc;
         if (d0 == 0) {
           xo[16 * HD + r] = m_tot;
@@ -862,7 +864,7 @@ __global__ void __launch_bounds__(DWARPS * 32, OCC) dec_kernel(const DecKernelPa
               dead ? -INFINITY : (m_tot * c + log2f(l_tot)) * 0.6931471805599453f;
       }
     }
-    if (p.cluster > 1) {
+    if constexpr (CL) {
       // ---- merge the splits of the cluster through distributed shared memory: every CTA finishes its share of the rows
       namespace cg = cooperative_groups;
       cg::cluster_group cl = cg::this_cluster();
@@ -973,9 +975,9 @@ __global__ void __launch_bounds__(256) dec_gate_ext_kernel(const DecKernelParams
   if (l16 == 0 && item < n_items) reinterpret_cast<float2*>(p.gate_ws)[item] = make_float2(mx, mn);
 }
 
-template <int HD, typename T, int KIND, bool TR, int OCC>
+template <int HD, typename T, int KIND, bool TR, int OCC, bool CL = false>
 cudaError_t launch_variant(const DecKernelParams& p, cudaStream_t stream) {
-  auto kern = dec_kernel<HD, T, KIND, TR, OCC>;
+  auto kern = dec_kernel<HD, T, KIND, TR, OCC, CL>;
   // the variant for two CTAs per SM asks for enough shared memory that a third cannot join
   constexpr int ring = DecSmem<HD, sizeof(T)>::kTotal;
   constexpr int smem = (TR && OCC == 2 && ring < 80 * 1024) ? 80 * 1024 : ring;
@@ -990,8 +992,8 @@ cudaError_t launch_variant(const DecKernelParams& p, cudaStream_t stream) {
       if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
     }
   }
-  if (p.cluster > 1) {
-    static_assert(HD > 128 || DWARPS * (16 * HD + 32) * 4 + (16 * HD + 32) * 4 <= ring, "the merged state fits behind the warps'");
+  if constexpr (CL) {
+    static_assert(HD <= 128 && DWARPS * (16 * HD + 32) * 4 + (16 * HD + 32) * 4 <= ring, "the merged state fits behind the warps'");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid, 1, 1);
     cfg.blockDim = dim3(DWARPS * 32, 1, 1);
@@ -1017,6 +1019,13 @@ cudaError_t launch_one(const DecKernelParams& p, cudaStream_t stream) {
     // eight query rows per pass over the keys; the 128 KB ring leaves one CTA per SM
     return launch_variant<HD, T, KIND, true, 2>(p, stream);
   } else {
+    // splits merged in a cluster: at most two CTAs per SM by the rule of dec_cluster_splits
+    if (p.cluster > 1) {
+      if constexpr (sizeof(T) == 2) {
+        if (p.G <= 8) return launch_variant<HD, T, KIND, true, 2, true>(p, stream);
+      }
+      return launch_variant<HD, T, KIND, false, FSA_DEC_MINBLOCKS, true>(p, stream);
+    }
     if constexpr (sizeof(T) == 2) {
       if (p.G <= 8) {
         // Transposed products (see dec_kernel), at three or at two CTAs per SM. The grid runs in rounds of occ x SMs
