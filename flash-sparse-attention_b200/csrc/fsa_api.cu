@@ -776,6 +776,9 @@ int fsa_decode(const FsaDecArgs* a, void* stream_) {
   if ((a->k_stride_s % 8) || (a->k_stride_h % 8) || (a->k_stride_b % 8) ||
       (reinterpret_cast<uintptr_t>(a->k) & 15) || (reinterpret_cast<uintptr_t>(a->v) & 15))
     return FSA_ERR_INVALID_ARG;  // 16-byte row copies
+  if (!a->partial_only && ((reinterpret_cast<uintptr_t>(a->out) & 3) || (a->batch > 1 && a->o_stride_b % 2) ||
+                           (a->heads_q > 1 && a->o_stride_h % 2)))
+    return FSA_ERR_INVALID_ARG;  // rows are written in pieces of 4 bytes and more
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
 
   fsa::DecKernelParams p;

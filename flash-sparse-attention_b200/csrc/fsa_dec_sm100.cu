@@ -149,6 +149,19 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
   return d;
 }
 
+// Four neighbouring outputs of a row, scaled. A caller's buffer may start its rows at any 4-byte boundary: that is what
+// the combine kernel, which writes the same buffer for other numbers of splits, asks for.
+template <typename TO>
+__device__ __forceinline__ void store_out4(TO* dst, float4 a, float s) {
+  const uint2 v = make_uint2(pack2<TO>(a.x * s, a.y * s), pack2<TO>(a.z * s, a.w * s));
+  if ((reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
+    *reinterpret_cast<uint2*>(dst) = v;
+  } else {
+    reinterpret_cast<uint32_t*>(dst)[0] = v.x;
+    reinterpret_cast<uint32_t*>(dst)[1] = v.y;
+  }
+}
+
 // TR (16-bit inputs, at most 8 query heads per KV head): the products run transposed, S^T = K Q^T and
 // O^T = V^T P^T, so that the 16 keys of a tile fill the M = 16 side of mma.m16n8k16 and the (up to) 8 query rows the
 // N = 8 side. With the rows on M, half of every fragment is padding when a KV head serves 8 query heads: transposed, the
@@ -854,11 +867,7 @@ __global__ void __launch_bounds__(DWARPS * 32, OCC) dec_kernel(const DecKernelPa
           if (d0 == 0) p.lse_partial[l_at] = lv;
         }
       } else {
-        TO* dst = reinterpret_cast<TO*>(p.out) + (long long)b * p.o_sb + (long long)head * p.o_sh + d0;
-        uint2 v;
-        v.x = pack2<TO>(acc.x * inv, acc.y * inv);
-        v.y = pack2<TO>(acc.z * inv, acc.w * inv);
-        *reinterpret_cast<uint2*>(dst) = v;
+        store_out4(reinterpret_cast<TO*>(p.out) + (long long)b * p.o_sb + (long long)head * p.o_sh + d0, acc, inv);
         if (d0 == 0)
           p.lse[(long long)b * p.l_sb + (long long)head * p.l_sh] =
               dead ? -INFINITY : (m_tot * c + log2f(l_tot)) * 0.6931471805599453f;
@@ -897,10 +906,7 @@ __global__ void __launch_bounds__(DWARPS * 32, OCC) dec_kernel(const DecKernelPa
         const bool dead = (l_tot == 0.f) || (l_tot != l_tot);
         const float inv = dead ? 1.f : v_scale / l_tot;
         const int head = hkv * p.G + r;
-        uint2 v;
-        v.x = pack2<TO>(acc.x * inv, acc.y * inv);
-        v.y = pack2<TO>(acc.z * inv, acc.w * inv);
-        *reinterpret_cast<uint2*>(reinterpret_cast<TO*>(p.out) + (long long)b * p.o_sb + (long long)head * p.o_sh + d0) = v;
+        store_out4(reinterpret_cast<TO*>(p.out) + (long long)b * p.o_sb + (long long)head * p.o_sh + d0, acc, inv);
         if (d0 == 0)
           p.lse[(long long)b * p.l_sb + (long long)head * p.l_sh] =
               dead ? -INFINITY : (m_tot * c + log2f(l_tot)) * 0.6931471805599453f;

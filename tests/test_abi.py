@@ -115,3 +115,17 @@ def test_workspace_sizes_from_the_library():
     d.partial_only = 1
     assert lib.fsa_decode_workspace_bytes(ctypes.byref(d), ctypes.byref(dw)) == 0
     assert dw.out_partial == 4 * 5 * 16 * 128 and dw.lse_partial == 4 * 5 * 16
+
+
+def test_decode_refuses_out_rows_on_odd_elements():
+    """Host check in front of the launch (no GPU needed): rows of the result start on 4-byte boundaries."""
+    from flash_sparse_attn import _lib
+
+    lib = _lib.load()
+    a = _lib.FsaDecArgs()
+    a.q = a.k = a.v = a.lse = a.status = 256
+    a.batch, a.heads_q, a.heads_kv, a.head_dim, a.seqlen_k, a.num_splits = 2, 4, 1, 64, 100, 1
+    a.dtype, a.kind = _lib.DT_BF16, _lib.KIND_DENSE
+    for out, stride_b, stride_h in ((258, 256, 64), (256, 257, 64), (256, 256, 65)):
+        a.out, a.o_stride_b, a.o_stride_h = out, stride_b, stride_h
+        assert lib.fsa_decode(ctypes.byref(a), None) == -1

@@ -31,3 +31,18 @@ def test_cluster_merge(num_splits, hq, hkv, d):
     out, lse = fsa.flash_dense_attn_with_kvcache_func(q.cuda(), k.cuda(), v.cuda(), seqused_k=used.cuda(),
                                                       num_splits=num_splits, return_lse=True)
     assert (out[1] == 0).all() and torch.isneginf(lse[1]).all()
+
+
+@pytest.mark.parametrize("num_splits", [1, 2, 8, 9])  # unsplit, cluster merge, partials and combine
+@pytest.mark.parametrize("hq,d", [(4, 64), (12, 128)])
+def test_rows_of_out_on_4_byte_boundaries(num_splits, hq, d):
+    import flash_sparse_attn as fsa
+
+    g = torch.Generator().manual_seed(hq)
+    q, k, v = (torch.randn(*s, generator=g).to(torch.bfloat16).cuda() for s in ((3, hq, d), (3, 333, 1, d), (3, 333, 1, d)))
+    buf = torch.full((3, hq, d + 2), 7.0, dtype=torch.bfloat16, device="cuda")
+    want = fsa.flash_dense_attn_with_kvcache_func(q, k, v, num_splits=num_splits)
+    out = buf[..., 2:]
+    assert out.data_ptr() % 8 == 4 and out.stride(1) % 4 == 2
+    fsa.flash_dense_attn_with_kvcache_func(q, k, v, num_splits=num_splits, out=out)
+    assert torch.equal(out, want) and (buf[..., :2] == 7).all()
