@@ -13,6 +13,11 @@ def test_balanced_num_splits():
     assert f(256, 1) == 1 and f(1, 0) == 1
     assert utils.balanced_num_splits(290, 94, 1.5, 7.0, 50.0, 148) == 1  # the partials would cost more
     assert f(4, 120) > 4                       # four CTAs would leave the GPU idle
+    # unequal sequences: fewer CTAs than SMs whose steps last long are split (three sequences of 300 queries against up to
+    # 12000 keys, 16 heads of 64: 207 us with one split, 132 us with three)
+    assert utils.balanced_num_splits(96, 94, 1.5, 7.0, 1.5, 148) > 1
+    # nearly two CTAs per SM are not (1000 queries against 16000 keys, 64 heads: 668 us, 709 us with two splits)
+    assert utils.balanced_num_splits(256, 126, 1.5, 7.0, 13.1, 148) == 1
     for ctas in (1, 8, 100, 147, 149, 295):
         for steps in (1, 2, 7, 64, 1000):
             n = f(ctas, steps)
