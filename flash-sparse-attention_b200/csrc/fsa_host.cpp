@@ -11,6 +11,7 @@
 
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cmath>
@@ -118,7 +119,7 @@ PyObject* pair(Tensor out, Tensor lse) {
 //        seqused_k, cu_seqlens_k, max_seqlen_k, out, lse, qkv_scale) -> (out, lse), an error code, or None
 PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 17 || !g_decode) return none();
-  try {
+  HANDLE_TH_ERRORS  // torch's own translation: an allocation that fails raises torch.OutOfMemoryError
     Tensor q, k, v, win, table, gather, used, cu, out, lse, scale;
     if (a[1] == Py_None || a[2] == Py_None || a[3] == Py_None) return none();
     if (!opt_tensor(a[1], &q) || !opt_tensor(a[2], &k) || !opt_tensor(a[3], &v) || !opt_tensor(a[5], &win) ||
@@ -224,10 +225,7 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int rc = g_decode(&x, c10::cuda::getCurrentCUDAStream(dev.index()).stream());
     if (rc != FSA_OK) return PyLong_FromLong(rc);
     return pair(std::move(out), std::move(lse));
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
-  }
+  END_HANDLE_TH_ERRORS
 }
 
 // forward(kind, q, k, v, is_causal, softmax_scale, window_sizes, softmax_threshold, is_local, num_splits, pack_gqa,
@@ -235,7 +233,7 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
 //         -> (out, lse), an error code, or None. num_splits: what the launcher settled on (1: unsplit).
 PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 21 || !g_fwd) return none();
-  try {
+  HANDLE_TH_ERRORS  // torch's own translation: an allocation that fails raises torch.OutOfMemoryError
     Tensor q, k, v, win, cu_q, cu_k, table, used_q, used_k, out, lse, scale;
     if (a[1] == Py_None || a[2] == Py_None || a[3] == Py_None) return none();
     if (!opt_tensor(a[1], &q) || !opt_tensor(a[2], &k) || !opt_tensor(a[3], &v) || !opt_tensor(a[6], &win) ||
@@ -356,10 +354,7 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int rc = g_fwd(&x, c10::cuda::getCurrentCUDAStream(dev.index()).stream());
     if (rc != FSA_OK) return PyLong_FromLong(rc);
     return pair(std::move(out), std::move(lse));
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
-  }
+  END_HANDLE_TH_ERRORS
 }
 
 // init(address of fsa_decode, address of fsa_fwd)

@@ -149,3 +149,22 @@ def test_errors_are_those_of_the_contract():
         fsa.flash_dense_attn_with_kvcache_func(q, k, k, seqused_k=torch.ones(1, dtype=torch.int64, device=DEV))
     with pytest.raises(RuntimeError):
         fsa.flash_dense_attn_with_kvcache_func(q.cpu(), k.cpu(), k.cpu())
+
+
+@pytest.mark.gpu
+def test_out_of_memory_keeps_its_type(monkeypatch):
+    # a workspace of terabytes: the allocation is refused by the allocator, on either route with the class callers catch
+    import flash_sparse_attn as fsa
+    from flash_sparse_attn import _lib
+
+    q, k = (torch.zeros(1, *s, 64, dtype=torch.bfloat16, device=DEV) for s in ((64,), (8, 2)))
+    calls = [lambda n: fsa.flash_dense_attn_with_kvcache_func(q, k, k, num_splits=n),
+             lambda n: fsa.flash_dense_attn_func(q[:, None], k, k, is_split_kv=True, num_splits=n)]
+    for call in calls:
+        call(2)
+        with pytest.raises(torch.OutOfMemoryError):
+            call(1 << 30)
+    monkeypatch.setattr(_lib, "native", lambda: None)
+    for call in calls:
+        with pytest.raises(torch.OutOfMemoryError):
+            call(1 << 30)
