@@ -15,6 +15,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cmath>
+#include <optional>
 
 #include "../../include/fsa_b200.h"
 
@@ -27,6 +28,13 @@ at::Tensor* g_status[MAX_DEVICES] = {};  // registered by the package, one int32
 int g_sms[MAX_DEVICES] = {};
 
 using at::Tensor;
+
+// Held around the allocations and the launch: an allocation may wait for the device, a launch for room in the stream's
+// queue, and other Python threads (one of which may have to feed what is waited for) go on meanwhile.
+struct NoGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~NoGil() { PyEval_RestoreThread(state); }
+};
 
 // Optional tensor argument: None -> undefined. Returns false for anything but None or an exact torch.Tensor.
 bool opt_tensor(PyObject* o, Tensor* t) {
@@ -169,6 +177,8 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
     else if (!get_int(a[8], &splits))
       return none();
     splits = std::max<int64_t>(splits, 1);
+    int32_t* const status = ptr<int32_t>(*g_status[dev.index()]);
+    std::optional<NoGil> no_gil(std::in_place);
     if (!out.defined()) out = at::empty(q.sizes(), q.options().dtype(out_type));
     if (!lse.defined()) lse = at::empty({batch, hq}, q.options().dtype(at::kFloat));
 
@@ -189,7 +199,7 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
     x.page_table = ptr<int32_t>(table);
     x.gather_kv_indices = ptr<int32_t>(gather);
     x.window_sizes = ptr<int32_t>(win);
-    x.status = ptr<int32_t>(*g_status[dev.index()]);
+    x.status = status;
     x.q_stride_b = q.stride(0);
     x.q_stride_h = q.stride(1);
     x.k_stride_b = varlen ? 0 : k.stride(0);
@@ -223,6 +233,7 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
     x.softmax_threshold = (float)thr;
     x.qkv_scale = ptr<float>(scale);
     const int rc = g_decode(&x, c10::cuda::getCurrentCUDAStream(dev.index()).stream());
+    no_gil.reset();
     if (rc != FSA_OK) return PyLong_FromLong(rc);
     return pair(std::move(out), std::move(lse));
   END_HANDLE_TH_ERRORS
@@ -292,6 +303,8 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
       return none();
     double sm_scale, thr;
     if (!opt_double(a[5], 1.0 / std::sqrt((double)d), &sm_scale) || !opt_double(a[7], 1.0, &thr)) return none();
+    int32_t* const status = ptr<int32_t>(*g_status[dev.index()]);
+    std::optional<NoGil> no_gil(std::in_place);
     if (!out.defined()) out = at::empty(q.sizes(), q.options().dtype(out_type));
     if (!lse.defined())
       lse = varlen ? at::empty({hq, total_q}, q.options().dtype(at::kFloat))
@@ -316,7 +329,7 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     x.seqused_k = ptr<int32_t>(used_k);
     x.page_table = ptr<int32_t>(table);
     x.window_sizes = ptr<int32_t>(win);
-    x.status = ptr<int32_t>(*g_status[dev.index()]);
+    x.status = status;
     x.q_stride_b = varlen ? 0 : q.stride(0);
     x.q_stride_s = q.stride(-3);
     x.q_stride_h = q.stride(-2);
@@ -352,6 +365,7 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     x.softmax_threshold = (float)thr;
     x.qkv_scale = ptr<float>(scale);
     const int rc = g_fwd(&x, c10::cuda::getCurrentCUDAStream(dev.index()).stream());
+    no_gil.reset();
     if (rc != FSA_OK) return PyLong_FromLong(rc);
     return pair(std::move(out), std::move(lse));
   END_HANDLE_TH_ERRORS

@@ -168,3 +168,25 @@ def test_out_of_memory_keeps_its_type(monkeypatch):
     for call in calls:
         with pytest.raises(torch.OutOfMemoryError):
             call(1 << 30)
+
+
+@pytest.mark.gpu
+def test_gil_is_free_during_the_launch():
+    # the library calls are replaced by CPython's own "does this thread hold the GIL": 0 reads as success, 1 as an error
+    import ctypes
+
+    import flash_sparse_attn as fsa
+    from flash_sparse_attn import _lib
+
+    q, k = (torch.zeros(1, *s, 64, dtype=torch.bfloat16, device=DEV) for s in ((4,), (8, 2)))
+    fsa.flash_dense_attn_with_kvcache_func(q, k, k)  # registers the device
+    host, lib = _lib._host, _lib.load()
+    address = lambda f: ctypes.cast(f, ctypes.c_void_p).value  # noqa: E731
+    host.init(address(ctypes.pythonapi.PyGILState_Check), address(ctypes.pythonapi.PyGILState_Check))
+    try:
+        dec = host.decode(0, q, k, k, None, None, None, False, 2, None, None, None, None, None, None, None, None)
+        fwd = host.forward(0, q[:, None], k, k, False, None, None, None, False, 2, False, None, None, None, None, None, None,
+                           None, None, None, None)
+    finally:
+        host.init(address(lib.fsa_decode), address(lib.fsa_fwd))
+    assert type(dec) is tuple and type(fwd) is tuple
