@@ -859,10 +859,7 @@ int fsa_decode(const FsaDecArgs* a, void* stream_) {
     p.peer_rank = pe->rank;
     p.peer_block_floats = pe->block_floats;
   }
-  if (!a->partial_only) {
-    p.cluster = fsa::dec_cluster_splits(a->batch, a->heads_kv, a->heads_q, a->head_dim, ns);
-    if (p.cluster > 1) p.flags &= ~(unsigned)fsa::F_SPLIT;
-  }
+  if (!a->partial_only) p.cluster = fsa::dec_cluster_splits(a->batch, a->heads_kv, a->heads_q, a->head_dim, ns);
   mark(a->ev_before, stream);
   p.D = a->head_dim;
   cudaError_t e = fsa::launch_dec(p, a->kind, a->dtype, head_dim_kernel_wide(a->head_dim), stream);

@@ -981,8 +981,45 @@ __global__ void __launch_bounds__(256) dec_gate_ext_kernel(const DecKernelParams
   if (l16 == 0 && item < n_items) reinterpret_cast<float2*>(p.gate_ws)[item] = make_float2(mx, mn);
 }
 
+// Whether the clusters of a call find room as well as its CTAs one by one would. A cluster has to fit inside one GPC, and
+// the GPCs of a device differ in size: of 296 slots (two CTAs on each of 148 SMs) clusters of 7 use 259, clusters of 3 279.
+// One cluster more waits for a whole round (decode of 32 / 8 heads of 128, 4000 keys: 40 clusters of 7 took 24.9 us where
+// partials and the combine launch take 15.5, 96 of 3 52.6 against 36.4). A grid that single CTAs spread over the SMs
+// one by one has to find that room, too: 16 clusters of 8 doubled up on some SMs (2048 FP8 keys a CTA: 39.7 against 35.2 us).
+// Where they fit they save 1 to 1.5 us (a fifth of the smallest calls). The runtime's answers are kept per device.
+template <typename Kernel>
+bool clusters_fit(Kernel kern, int clusters, int size, int smem, std::atomic<int> (*cache)[2][MAX_CLUSTER + 1]) {
+  constexpr int LONE_SMEM = 120 * 1024;  // more than half of an SM's shared memory: one CTA per SM
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return false;
+  const bool lone = (long long)clusters * size <= device_sm_count();
+  std::atomic<int>& known = cache[dev][lone][size];
+  int room = known.load(std::memory_order_relaxed) - 1;  // 0: not asked yet
+  if (room < 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)size, 1, 1);
+    cfg.blockDim = dim3(DWARPS * 32, 1, 1);
+    cfg.dynamicSmemBytes = lone ? LONE_SMEM : smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)size;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LONE_SMEM) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&room, kern, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      room = 0;
+    }
+    known.store(room + 1, std::memory_order_relaxed);
+  }
+  return clusters <= room;
+}
+
+// CL: when the clusters do not fit, p.cluster becomes 0 and nothing is launched.
 template <int HD, typename T, int KIND, bool TR, int OCC, bool CL = false>
-cudaError_t launch_variant(const DecKernelParams& p, cudaStream_t stream) {
+cudaError_t launch_variant(DecKernelParams& p, cudaStream_t stream) {
   auto kern = dec_kernel<HD, T, KIND, TR, OCC, CL>;
   // the variant for two CTAs per SM asks for enough shared memory that a third cannot join
   constexpr int ring = DecSmem<HD, sizeof(T)>::kTotal;
@@ -991,6 +1028,14 @@ cudaError_t launch_variant(const DecKernelParams& p, cudaStream_t stream) {
   if (cudaError_t e = smem_opt_in(kern, smem, opted_in); e != cudaSuccess) return e;
   const long long grid = (long long)p.Hkv * p.B * p.num_splits;
   if (grid <= 0) return cudaSuccess;
+  if constexpr (CL) {
+    static_assert(smem <= 120 * 1024, "the opt-in of clusters_fit covers the launch");
+    static std::atomic<int> room[64][2][MAX_CLUSTER + 1];
+    if (!clusters_fit(kern, p.Hkv * p.B, p.cluster, smem, room)) {
+      p.cluster = 0;
+      return cudaSuccess;
+    }
+  }
   if (KIND == KIND_GATED && p.gate_ws) {
     const long long items = (long long)p.B * p.Hkv * p.n_tiles;
     if (items > 0) {
@@ -1019,7 +1064,7 @@ cudaError_t launch_variant(const DecKernelParams& p, cudaStream_t stream) {
 }
 
 template <int HD, typename T, int KIND>
-cudaError_t launch_one(const DecKernelParams& p, cudaStream_t stream) {
+cudaError_t launch_one(DecKernelParams& p, cudaStream_t stream) {
   if constexpr (HD > 128) {
     // head sizes above 128: only the transposed variant (its accumulator still fits the registers: 16 x 4 per lane),
     // eight query rows per pass over the keys; the 128 KB ring leaves one CTA per SM
@@ -1027,10 +1072,13 @@ cudaError_t launch_one(const DecKernelParams& p, cudaStream_t stream) {
   } else {
     // splits merged in a cluster: at most two CTAs per SM by the rule of dec_cluster_splits
     if (p.cluster > 1) {
-      if constexpr (sizeof(T) == 2) {
-        if (p.G <= 8) return launch_variant<HD, T, KIND, true, 2, true>(p, stream);
-      }
-      return launch_variant<HD, T, KIND, false, FSA_DEC_MINBLOCKS, true>(p, stream);
+      cudaError_t e;
+      if constexpr (sizeof(T) == 2)
+        e = p.G <= 8 ? launch_variant<HD, T, KIND, true, 2, true>(p, stream)
+                     : launch_variant<HD, T, KIND, false, FSA_DEC_MINBLOCKS, true>(p, stream);
+      else
+        e = launch_variant<HD, T, KIND, false, FSA_DEC_MINBLOCKS, true>(p, stream);
+      if (e != cudaSuccess || p.cluster > 1) return e;
     }
     if constexpr (sizeof(T) == 2) {
       if (p.G <= 8) {
@@ -1052,15 +1100,16 @@ cudaError_t launch_one(const DecKernelParams& p, cudaStream_t stream) {
 
 }  // namespace
 
-// Splits merged inside a cluster (their number; 0: partials and a second launch). A call whose CTAs are all resident at
-// once is bound by latencies, and the partials' way through memory and the combine launch are several of them. With more
-// CTAs than slots the kernel is bandwidth bound and a cluster, which starts and ends as one, leaves slots idle.
+// Splits that may be merged inside a cluster (their number; 0: partials and a second launch). A call whose CTAs are all
+// resident at once is bound by latencies, and the partials' way through memory and the combine launch are several of
+// them. With more CTAs than slots the kernel is bandwidth bound and a cluster, which starts and ends as one, leaves slots
+// idle. Whether that many clusters are resident is decided at the launch (clusters_fit).
 int dec_cluster_splits(int batch, int heads_kv, int heads_q, int head_dim, int num_splits) {
   const bool fits = num_splits > 1 && num_splits <= MAX_CLUSTER && head_dim <= 128 && heads_q <= 16 * heads_kv;
   return fits && (long long)batch * heads_kv * num_splits <= 2ll * device_sm_count() ? num_splits : 0;
 }
 
-cudaError_t launch_dec(const DecKernelParams& p, int kind, int dtype, int head_dim, cudaStream_t stream) {
+cudaError_t launch_dec(DecKernelParams& p, int kind, int dtype, int head_dim, cudaStream_t stream) {
 #define FSA_DEC_CASE(HD_, T_, DT_)                                               \
   if (head_dim == HD_ && dtype == DT_) {                                         \
     if (kind == KIND_DENSE) return launch_one<HD_, T_, KIND_DENSE>(p, stream);   \

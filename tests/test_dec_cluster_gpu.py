@@ -46,3 +46,45 @@ def test_rows_of_out_on_4_byte_boundaries(num_splits, hq, d):
     assert out.data_ptr() % 8 == 4 and out.stride(1) % 4 == 2
     fsa.flash_dense_attn_with_kvcache_func(q, k, v, num_splits=num_splits, out=out)
     assert torch.equal(out, want) and (buf[..., :2] == 7).all()
+
+
+def _graph_nodes(fn):
+    """Kernels that one call launches: the nodes of a CUDA graph that captured it."""
+    import ctypes
+
+    fn()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        fn()
+    count = ctypes.c_size_t(0)
+    runtime = ctypes.CDLL("libcudart.so.12")
+    assert runtime.cudaGraphGetNodes(ctypes.c_void_p(graph.raw_cuda_graph()), None, ctypes.byref(count)) == 0
+    return count.value
+
+
+# (sequences x KV heads, splits): 42 clusters of 7 and 49 of 6 would need all but two of the 296 slots that 148 SMs have for
+# two CTAs each, and 18 of 8 or 21 of 7 nearly every SM; GPCs, inside which a cluster has to fit, are not of such sizes
+@pytest.mark.parametrize("pairs,splits,launches", [(4, 8, 1), (42, 7, 2), (49, 6, 2), (18, 8, 2), (21, 7, 2)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float8_e4m3fn])
+def test_clusters_only_where_they_are_resident(dtype, pairs, splits, launches):
+    import flash_sparse_attn as fsa
+
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the numbers are those of 148 SMs")
+    g = torch.Generator().manual_seed(pairs)
+    q, k, v = (torch.randn(*s, generator=g).to(torch.bfloat16) for s in ((pairs, 4, 128), (pairs, 200, 1, 128), (pairs, 200, 1, 128)))
+    ref = eager.decode(q, k, v)
+    kw = {}
+    q, k, v = q.cuda(), k.cuda(), v.cuda()
+    if dtype != torch.bfloat16:
+        q, k, v = q.to(dtype), k.to(dtype), v.to(dtype)
+        ref = eager.decode(*(t.cpu().to(torch.bfloat16) for t in (q, k, v)))
+        one = torch.ones(1, device="cuda")
+        kw = dict(is_quant=True, query_scale=one, key_scale=one, value_scale=one)
+    out, lse = torch.empty(pairs, 4, 128, dtype=torch.bfloat16, device="cuda"), torch.empty(pairs, 4, device="cuda")
+    call = lambda: fsa.flash_dense_attn_with_kvcache_func(q, k, v, num_splits=splits, out=out, lse=lse, **kw)  # noqa: E731
+    assert _graph_nodes(call) == launches + (1 if kw else 0)  # FP8: one more packs the scales
+    call()
+    torch.cuda.synchronize()
+    fsa.check_status()
+    assert_close("out", out, ref)
