@@ -10,6 +10,7 @@ reduction over splits. No host synchronisation happens here.
 """
 
 import ctypes
+import functools
 from typing import Optional, Tuple
 
 import torch
@@ -19,10 +20,11 @@ from flash_sparse_attn.ops.triton import assert_inputs, quant, utils
 
 TILE_M = 128
 TILE_N = 128
-# for the split rule (utils.balanced_num_splits): a step (one query tile of one head), what a CTA takes besides its
-# steps, and the rate at which the fp32 partials of dK and dV are written and read
-BWD_STEP_US, BWD_CTA_US = 2.8, 10.0
+# for backward_num_splits, fitted to its 154 calls: a step (one query tile of one head at head size 128), what a CTA takes
+# besides its steps, the launches that a split brings, and the rate at which fp32 partials are written and read
+STEP_US, CTA_US, LAUNCHES_US = 2.4, 6.0, 30.0
 PARTIAL_BYTES_PER_US = 5.0e6
+
 _KIND = {"dense": _lib.KIND_DENSE, "sparse": _lib.KIND_SPARSE, "gated": _lib.KIND_GATED}
 
 
@@ -30,6 +32,44 @@ def _dequantize(x: torch.Tensor, scale: torch.Tensor, dtype: torch.dtype) -> tor
     # saved tensors of a quantised forward are FP8; the backward runs on their de-quantised values in
     # the gradient dtype (flash_sparse_attn/ops/triton/scheduler.py:2133-2148)
     return quant.widen_fp8(x, dtype, scale)
+
+
+@functools.lru_cache(maxsize=4096)
+def backward_num_splits(kind, batch, seqlen_q, seqlen_k, rows_k, num_heads_q, num_heads_kv, head_dim, is_causal, is_local, num_sms):
+    """Query splits of a backward call that leaves their number open (``rows_k``: key rows of the whole batch).
+
+    One CTA serves a key tile of a (sequence, KV head). A grid that oversubscribes the SMs is not split; with windows the
+    reference's estimate is taken, the roles of the two sequence axes swapped. Otherwise the number that minimises the modelled
+    time: the CTAs' steps spread over the SMs (under a causal mask the mean CTA has about half of the longest one's), half of the
+    longest CTA as unevenness when there is more than one round, never less than the longest CTA; every split writes and
+    reads fp32 partials of dK / dV, and the first one brings two more launches. The estimate alone, which looks at the
+    tiles of one (sequence, head), takes 1.14 times the best number's time in the mean over 154 calls (150 to 6000 tokens,
+    2 to 8 KV heads, all kinds), the model 1.02; over 112 calls that it was not fitted to 1.18 and 1.03, over 28 packed ones 1.21
+    and 1.07."""
+    q_tiles, k_tiles = -(-seqlen_q // TILE_M), -(-seqlen_k // TILE_N)
+    ctas = batch * num_heads_kv * k_tiles
+    if ctas >= 2 * num_sms or ctas <= 0:
+        return 1
+    if is_local:
+        return utils.num_splits_heuristic(seqlen_q=seqlen_k, seqlen_k=seqlen_q, num_SMs=num_sms, TILE_M=TILE_N, TILE_N=TILE_M,
+                                          is_local=True, num_heads_kv=num_heads_kv)
+    step = STEP_US * (num_heads_q // num_heads_kv) * (1.8 if kind == "gated" else 1.0) * (0.8 if head_dim <= 64 else 1.0)
+    longest, share = q_tiles, 1.0
+    if is_causal:  # the share of all (query, key) pairs that the mask leaves; the first key tile meets the most query tiles
+        longest = min(q_tiles, k_tiles)
+        share = (seqlen_k - seqlen_q / 2) / seqlen_k if seqlen_k >= seqlen_q else seqlen_k / (2 * seqlen_q)
+    ctas = max(ctas * rows_k / (batch * seqlen_k), 1.0)  # packed: key tiles past the end of a sequence leave at once
+    partials = rows_k * num_heads_kv * head_dim * 16 / PARTIAL_BYTES_PER_US
+    best, best_us = 1, float("inf")
+    for n in range(1, min(longest, 1 + int(4 * num_sms / ctas)) + 1):
+        cta = -(-longest // n) * step + CTA_US
+        mean = q_tiles * share / n * step + CTA_US
+        us = max(cta, ctas * n / num_sms * mean + (0.5 * cta if ctas * n > num_sms else 0.0))
+        if n > 1:
+            us += LAUNCHES_US + n * partials
+        if us < best_us * 0.98:  # a further split has to be worth it
+            best, best_us = n, us
+    return best
 
 
 def attn_backward(
@@ -113,23 +153,8 @@ def attn_backward(
         value = _dequantize(value, value_scale, dout.dtype)
 
     if is_split_qo and num_splits is None:
-        # one CTA per (key tile, KV head, batch): when that already oversubscribes the SMs, splitting the
-        # query range only adds fp32 partials of dK/dV
-        ctas = batch * num_heads_kv * (-(-seqlen_k // TILE_N))
-        n_sms = utils.device_num_sms(device)
-        if ctas >= 2 * n_sms:
-            num_splits = 1
-        elif is_local:
-            # roles of the two sequence axes are swapped with respect to the forward heuristic
-            num_splits = utils.num_splits_heuristic(
-                seqlen_q=seqlen_k, seqlen_k=seqlen_q, num_SMs=n_sms, TILE_M=TILE_N, TILE_N=TILE_M, is_local=True,
-                num_heads_kv=num_heads_kv,
-            )
-        else:
-            rows = total_k if varlen else batch * seqlen_k
-            num_splits = utils.balanced_num_splits(
-                ctas, -(-seqlen_q // TILE_M), BWD_STEP_US * (num_heads_q // num_heads_kv), BWD_CTA_US,
-                rows * num_heads_kv * head_dim * 16 / PARTIAL_BYTES_PER_US, n_sms)
+        num_splits = backward_num_splits(kind, batch, seqlen_q, seqlen_k, total_k if varlen else batch * seqlen_k, num_heads_q,
+                                         num_heads_kv, head_dim, bool(is_causal), bool(is_local), utils.device_num_sms(device))
     elif not is_split_qo:
         num_splits = 1
     use_split = bool(is_split_qo) and num_splits > 1

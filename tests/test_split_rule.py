@@ -5,6 +5,7 @@ import torch
 
 from fixtures import assert_close, seeded_qkv
 from flash_sparse_attn.ops.triton import utils
+from flash_sparse_attn.ops.triton.flash_bwd import backward_num_splits
 from oracle import eager
 
 
@@ -22,6 +23,22 @@ def test_balanced_num_splits():
         for steps in (1, 2, 7, 64, 1000):
             n = f(ctas, steps)
             assert 1 <= n <= min(max(steps, 1), 64)
+
+
+def test_backward_num_splits():
+    f = lambda b, sq, sk, hq, hkv, d=128, kind="dense", causal=True, local=False: backward_num_splits(  # noqa: E731
+        kind, b, sq, sk, b * sk, hq, hkv, d, causal, local, 148)
+    assert f(2, 1318, 1318, 8, 8) == 1           # 176 CTAs: 80 us, eleven splits 233 us
+    assert f(1, 3838, 3838, 32, 4, 64) >= 3    # 120 CTAs, the longest of 30 steps: 602 us, four splits 332 us
+    assert f(2, 2933, 2933, 8, 2) >= 3        # 92 CTAs: 273 us, three splits 155 us
+    assert f(1, 249, 249, 32, 8) == 1            # two query tiles: 84 us, two splits 101 us
+    assert f(4, 8192, 8192, 32, 8) == 1
+    assert f(0, 500, 500, 8, 2) == f(1, 500, 0, 8, 2) == 1
+    assert f(1, 3838, 3838, 32, 4, local=True) == utils.num_splits_heuristic(3838, 3838, 148, 128, 128, True, 4)
+    for sq in (1, 300, 5000):
+        for sk in (1, 300, 5000):
+            for causal in (True, False):
+                assert 1 <= f(1, sq, sk, 8, 2, causal=causal) <= -(-sq // 128)
 
 
 @pytest.mark.gpu
