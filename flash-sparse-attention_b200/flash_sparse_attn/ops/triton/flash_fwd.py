@@ -18,10 +18,6 @@ from flash_sparse_attn.ops.triton import assert_inputs, quant, utils
 
 TILE_M = 128
 TILE_N = 128
-# What the split rule (utils.balanced_num_splits) reckons with, measured at head size 128: a step of a CTA (two query
-# tiles x one key tile), what a CTA takes besides its steps, and the rate at which fp32 partials are written and read.
-FWD_STEP_US, FWD_CTA_US = 1.5, 7.0
-PARTIAL_BYTES_PER_US = 5.0e6
 
 _KIND = {"dense": _lib.KIND_DENSE, "sparse": _lib.KIND_SPARSE, "gated": _lib.KIND_GATED}
 
@@ -31,21 +27,25 @@ def _require_cuda(t: torch.Tensor):
         raise RuntimeError("flash_sparse_attn (B200 build) only runs on CUDA tensors; there is no CPU path")
 
 
-def forward_num_splits(batch, seqlen_q, seqlen_k, rows, num_heads_q, num_heads_kv, head_dim, group_packed, is_local,
+def forward_num_splits(batch, seqlen_q, seqlen_k, num_heads_q, num_heads_kv, head_dim, group_packed, is_local, ragged,
                        num_sms):
-    """KV splits of a forward call that leaves their number open."""
-    m_pairs = -(-seqlen_q * group_packed // (2 * TILE_M))
-    ctas = batch * (num_heads_kv if group_packed > 1 else num_heads_q) * m_pairs
-    if ctas >= 2 * num_sms:
-        return 1  # every SM has several CTAs as it is
-    if is_local:
-        # the tiles that a window leaves are not known on the host: the reference's estimate for its default window
-        return utils.num_splits_heuristic(
-            seqlen_q=seqlen_q * group_packed, seqlen_k=seqlen_k, num_SMs=num_sms, TILE_M=TILE_M, TILE_N=TILE_N,
-            is_local=True, num_heads_kv=num_heads_kv,
-        )
-    return utils.balanced_num_splits(ctas, -(-seqlen_k // TILE_N), FWD_STEP_US, FWD_CTA_US,
-                                     rows * num_heads_q * head_dim * 8 / PARTIAL_BYTES_PER_US, num_sms)
+    """KV splits of a forward call that leaves their number open: the reference's estimate, which fills the SMs with the
+    tiles of ONE (batch, head), but no more than fill them once with those of all (``ragged``, sequences of different
+    lengths: twice, to even them out). Every further split costs a CTA's set-up and fp32 partials.
+
+    Measured on 76 calls (60 to 5000 queries, up to 16000 keys, head sizes 64 to 256, FP8, gated): 2.5 % behind the best
+    explicit number in the mean and 17 % at most (31 further calls: 4 and 14 %, host noise included); the estimate alone
+    takes 1.9 times the best number's time (2.2; four sequences
+    of 500 queries against up to 12000 keys, 32 heads: 37 splits 1072 us, one 365 us)."""
+    ctas_for = lambda rows: batch * (num_heads_kv if group_packed > 1 else num_heads_q) * -(-seqlen_q * group_packed // rows)  # noqa: E731
+    estimate = utils.num_splits_heuristic(
+        seqlen_q=seqlen_q * group_packed, seqlen_k=seqlen_k, num_SMs=num_sms, TILE_M=TILE_M, TILE_N=TILE_N,
+        is_local=is_local, num_heads_kv=num_heads_kv,
+    )
+    if is_local:  # what a window leaves of the tiles is not known here: the estimate for the default window
+        return 1 if ctas_for(2 * TILE_M) >= 2 * num_sms else estimate
+    ctas = ctas_for(2 * TILE_M if head_dim <= 128 else TILE_M)  # a CTA takes two query tiles, one above head size 128
+    return min(estimate, max(1, (2 if ragged else 1) * num_sms // max(ctas, 1)))
 
 
 def attn_forward(
@@ -122,8 +122,9 @@ def attn_forward(
     if not is_split_kv:
         num_splits = 1
     elif num_splits is None:
-        num_splits = forward_num_splits(batch, seqlen_q, seqlen_k, total_q if varlen else batch * seqlen_q, num_heads_q,
-                                        num_heads_kv, head_dim, group_packed, is_local, utils.device_num_sms(device))
+        ragged = batch > 1 and (varlen or seqused_k is not None or seqused_q is not None)
+        num_splits = forward_num_splits(batch, seqlen_q, seqlen_k, num_heads_q, num_heads_kv, head_dim, group_packed, is_local,
+                                        ragged, utils.device_num_sms(device))
     if (kind != "gated" and (tile_mn is None or page_table is None) and tile_map is None
             and (not is_quant or quant.uniform_scales(query_scale, key_scale, value_scale, device))):
         host = _lib.native()

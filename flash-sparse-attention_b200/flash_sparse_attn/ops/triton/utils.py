@@ -94,26 +94,6 @@ def num_splits_heuristic(
     return max(1, min(num_SMs // max(m_blocks, 1), pow2_cap, usable))
 
 
-@functools.lru_cache(maxsize=4096)
-def balanced_num_splits(ctas: int, steps: int, step_us: float, cta_us: float, partial_us: float, num_sms: int) -> int:
-    """Number of splits that minimises the modelled time of a grid of ``ctas * splits`` CTAs, one per SM, each
-    walking ``steps / splits`` tiles of ``step_us``: a CTA costs ``cta_us`` besides its tiles (set-up, the first loads,
-    the epilogue), CTAs beyond the first wave run back to back with about half a CTA of unevenness at the end, and
-    every split writes and reads fp32 partials (``partial_us``, plus one small launch).
-
-    The reference's rule (:func:`num_splits_heuristic`) looks at the tiles of one (batch, head) only and fills the SMs
-    with splits of each; with many heads or sequences that multiplies set-up and partial traffic."""
-    best, best_us = 1, float("inf")
-    for n in range(1, max(1, min(steps, 64)) + 1):
-        cta = _cdiv(steps, n) * step_us + cta_us
-        us = max(cta, ctas * n / num_sms * cta + (0.5 * cta if ctas * n > num_sms else 0.0))
-        if n > 1:
-            us += 4.0 + n * partial_us
-        if us < best_us * 0.98:  # a further split has to be worth it
-            best, best_us = n, us
-    return best
-
-
 @functools.lru_cache(maxsize=16)
 def device_num_sms(device: torch.device) -> int:
     return torch.cuda.get_device_properties(device).multi_processor_count

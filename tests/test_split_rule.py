@@ -6,23 +6,26 @@ import torch
 from fixtures import assert_close, seeded_qkv
 from flash_sparse_attn.ops.triton import utils
 from flash_sparse_attn.ops.triton.flash_bwd import backward_num_splits
+from flash_sparse_attn.ops.triton.flash_fwd import forward_num_splits
 from oracle import eager
 
 
-def test_balanced_num_splits():
-    f = lambda ctas, steps: utils.balanced_num_splits(ctas, steps, 1.5, 7.0, 0.5, 148)  # noqa: E731
-    assert f(256, 1) == 1 and f(1, 0) == 1
-    assert utils.balanced_num_splits(290, 94, 1.5, 7.0, 50.0, 148) == 1  # the partials would cost more
-    assert f(4, 120) > 4                       # four CTAs would leave the GPU idle
-    # unequal sequences: fewer CTAs than SMs whose steps last long are split (three sequences of 300 queries against up to
-    # 12000 keys, 16 heads of 64: 207 us with one split, 132 us with three)
-    assert utils.balanced_num_splits(96, 94, 1.5, 7.0, 1.5, 148) > 1
-    # nearly two CTAs per SM are not (1000 queries against 16000 keys, 64 heads: 668 us, 709 us with two splits)
-    assert utils.balanced_num_splits(256, 126, 1.5, 7.0, 13.1, 148) == 1
-    for ctas in (1, 8, 100, 147, 149, 295):
-        for steps in (1, 2, 7, 64, 1000):
-            n = f(ctas, steps)
-            assert 1 <= n <= min(max(steps, 1), 64)
+def test_forward_num_splits():
+    f = lambda b, sq, sk, hq, d=128, ragged=False, local=False: forward_num_splits(  # noqa: E731
+        b, sq, sk, hq, max(hq // 4, 1), d, 1, local, ragged, 148)
+    assert f(4, 500, 12000, 32, ragged=True) == 1   # 256 CTAs: two rounds already (37 splits: 1072 us, one: 365 us)
+    assert f(3, 300, 12000, 16, 64, ragged=True) == 3   # 96 CTAs of unequal length (one split: 207 us, three: 132 us)
+    assert f(2, 200, 12000, 32, ragged=True) == 4   # 143 us with two splits, 107 us with four
+    assert f(1, 586, 6400, 16) == 3                 # 48 equal CTAs: one round (three splits 70 us, four 87 us)
+    assert f(1, 1112, 1112, 16, 256) == 1           # one query tile a CTA: 144 of them (38 us, two splits 60 us)
+    assert f(1, 100, 500, 2) == 1                   # four key tiles: never split
+    assert f(4, 500, 12000, 32, ragged=True, local=True) == utils.num_splits_heuristic(500, 12000, 148, 128, 128, True, 8)
+    assert f(0, 500, 12000, 32) >= 1                # an empty batch
+    for sq in (1, 130, 2000):
+        for sk in (1, 513, 4000, 16000):
+            for ragged in (False, True):
+                n = f(2, sq, sk, 8, ragged=ragged)
+                assert 1 <= n <= utils.num_splits_heuristic(sq, sk, 148, 128, 128)
 
 
 def test_backward_num_splits():
