@@ -13,6 +13,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/version.h>
 
 #include <cmath>
 #include <optional>
@@ -418,4 +419,13 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, null
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&module); }
+// ABI_VERSION and TORCH_VERSION: what this was compiled against (the argument blocks of the header, ATen's classes).
+PyMODINIT_FUNC PyInit__host(void) {
+  PyObject* m = PyModule_Create(&module);
+  if (m && (PyModule_AddIntConstant(m, "ABI_VERSION", FSA_ABI_VERSION) < 0 ||
+            PyModule_AddStringConstant(m, "TORCH_VERSION", TORCH_VERSION) < 0)) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}

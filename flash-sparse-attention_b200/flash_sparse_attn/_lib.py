@@ -6,7 +6,10 @@ holds ``csrc/``), and every entry point raises on a non-zero status.
 """
 
 import ctypes
+import importlib
 import os
+import re
+import warnings
 from ctypes import POINTER, c_float, c_int, c_int32, c_int64, c_size_t, c_uint32, c_uint8, c_void_p
 
 import torch
@@ -403,23 +406,30 @@ _host = None
 
 
 def _load_host(lib):
-    """The native launcher of the common calls (csrc/fsa_host.cpp); it is built with the library and as required."""
+    """The native launcher of the common calls (csrc/fsa_host.cpp), built with the library. Without one that fits this library
+    and this torch the Python launchers, which are complete, serve every call; that is said once."""
     global _host
     try:
-        from flash_sparse_attn import _host as host
-    except ImportError as e:
-        raise RuntimeError("the native launcher flash_sparse_attn/_host.so is missing or does not load: build it with "
-                           "`python build.py` next to csrc/") from e
-    host.init(ctypes.cast(lib.fsa_decode, c_void_p).value, ctypes.cast(lib.fsa_fwd, c_void_p).value)
+        host = importlib.import_module("flash_sparse_attn._host")
+        built_for = (host.ABI_VERSION, host.TORCH_VERSION)
+        here = (ABI_VERSION, re.match(r"\d+\.\d+\.\d+", torch.__version__).group())
+        if built_for != here:
+            raise ImportError(f"built for {built_for}, not for {here} (ABI version, torch)")
+        host.init(ctypes.cast(lib.fsa_decode, c_void_p).value, ctypes.cast(lib.fsa_fwd, c_void_p).value)
+    except (ImportError, AttributeError) as e:
+        _host = None
+        warnings.warn("flash_sparse_attn/_host.so is missing or does not load; calls go through the slower Python launchers until "
+                      f"`python build.py` (next to csrc/) has built it: {e}", RuntimeWarning)
+        return
     _host = host
 
 
 def native():
-    """The native launcher, or None while a caller has profile events attached (they travel in the argument block
-    that the Python launchers fill)."""
+    """The native launcher, or None when there is none (see _load_host) and while a caller has profile events attached
+    (they travel in the argument block that the Python launchers fill)."""
     if _profile["before"] is not None or _profile["after"] is not None:
         return None
-    if _host is None:
+    if _lib is None:
         load()
     return _host
 
@@ -460,7 +470,8 @@ def status_word(device: torch.device) -> torch.Tensor:
         _status_words[key] = t
         if key[0] == "cuda":
             load()
-            _host.set_status(key[1], t, torch.cuda.get_device_properties(key[1]).multi_processor_count)
+            if _host is not None:
+                _host.set_status(key[1], t, torch.cuda.get_device_properties(key[1]).multi_processor_count)
     return t
 
 

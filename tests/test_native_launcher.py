@@ -31,6 +31,31 @@ def test_refuses_what_it_does_not_know():
         assert _lib._host.decode(*(args[:i] + [bad] + args[i + 1:])) is None
 
 
+@pytest.mark.parametrize("module", ["missing", "other abi", "other torch", "old"])
+def test_package_works_without_it(monkeypatch, module):
+    """A launcher that is missing or built for something else is left out, with one warning; the Python launchers remain."""
+    import sys
+    import types
+
+    from flash_sparse_attn import _lib
+
+    lib = _lib.load()
+    good = _lib._host
+    fake = None if module == "missing" else types.ModuleType("_host")
+    if module.startswith("other"):
+        fake.ABI_VERSION = good.ABI_VERSION + (module == "other abi")
+        fake.TORCH_VERSION = good.TORCH_VERSION if module == "other abi" else "1.0.0"
+    monkeypatch.setitem(sys.modules, "flash_sparse_attn._host", fake)
+    try:
+        with pytest.warns(RuntimeWarning, match="Python launchers"):
+            _lib._load_host(lib)
+        assert _lib.native() is None and _lib.native() is None
+    finally:
+        monkeypatch.undo()
+        _lib._load_host(lib)
+    assert _lib.native() is good
+
+
 def _both(monkeypatch, fn):
     """fn() through the native launcher (which must take the call) and through the Python one."""
     from flash_sparse_attn import _lib
