@@ -84,11 +84,8 @@ def _compile(src, force, verbose):
 
 def build_host(force=False):
     """The native launcher: a CPython extension against the headers of the installed torch. It holds no device code
-    and reaches the kernels through the addresses that the package hands it."""
-    header = os.path.join(HERE, "..", "include", "fsa_b200.h")
-    newest = max(os.path.getmtime(HOST_SRC), os.path.getmtime(header))
-    if not force and os.path.exists(HOST_LIB) and os.path.getmtime(HOST_LIB) >= newest:
-        return HOST_LIB
+    and reaches the kernels through the addresses that the package hands it. Built again when its sources, the compile
+    command, torch or the interpreter changed since (the key file beside the objects says what it was built with)."""
     import torch
 
     root = os.path.dirname(torch.__file__)
@@ -97,16 +94,27 @@ def build_host(force=False):
     for inc in (sysconfig.get_paths()["include"], os.path.join(root, "include"),
                 os.path.join(root, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include")):
         cmd += ["-isystem", inc]
-    cmd += [HOST_SRC, "-o", HOST_LIB, "-L" + os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch",
-            "-ltorch_python"]
-    res = subprocess.run(cmd, capture_output=True, text=True)
+    cmd += [HOST_SRC, "-L" + os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+    key = "\n".join([torch.__version__, sys.version, *cmd])
+    key_file = os.path.join(OBJ, "_host.key")
+    header = os.path.join(HERE, "..", "include", "fsa_b200.h")
+    newest = max(os.path.getmtime(HOST_SRC), os.path.getmtime(header))
+    if not force and os.path.exists(HOST_LIB) and os.path.getmtime(HOST_LIB) >= newest and os.path.exists(key_file):
+        with open(key_file) as f:
+            if f.read() == key:
+                return HOST_LIB
+    part = HOST_LIB + ".part"
+    res = subprocess.run(cmd + ["-o", part], capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError("g++ failed for fsa_host.cpp:\n" + res.stdout + res.stderr)
+    os.replace(part, HOST_LIB)
+    os.makedirs(OBJ, exist_ok=True)
+    with open(key_file, "w") as f:
+        f.write(key)
     return HOST_LIB
 
 
 def build(force=False, verbose=False):
-    build_host(force)
     os.makedirs(OBJ, exist_ok=True)
     with ThreadPoolExecutor(max_workers=min(8, len(SOURCES))) as ex:
         results = list(ex.map(lambda s: _compile(s, force, verbose), SOURCES))
@@ -120,6 +128,7 @@ def build(force=False, verbose=False):
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError("link failed:\n" + res.stdout + res.stderr)
+    build_host(force)  # last: the library needs neither torch nor its headers
     return LIB
 
 
