@@ -9,6 +9,7 @@ import ctypes
 import importlib
 import os
 import re
+import threading
 import warnings
 from ctypes import POINTER, c_float, c_int, c_int32, c_int64, c_size_t, c_uint32, c_uint8, c_void_p
 
@@ -459,6 +460,7 @@ def dtype_code(dt: torch.dtype) -> int:
 
 
 _status_words = {}
+_status_lock = threading.Lock()
 
 
 def status_word(device: torch.device) -> torch.Tensor:
@@ -466,12 +468,14 @@ def status_word(device: torch.device) -> torch.Tensor:
     key = (device.type, device.index if device.index is not None else torch.cuda.current_device())
     t = _status_words.get(key)
     if t is None:
-        t = torch.zeros(1, dtype=torch.int32, device=device)
-        _status_words[key] = t
-        if key[0] == "cuda":
-            load()
-            if _host is not None:
-                _host.set_status(key[1], t, torch.cuda.get_device_properties(key[1]).multi_processor_count)
+        load()
+        with _status_lock:  # two first calls at a time have to end up with one word: check_status reads only that
+            t = _status_words.get(key)
+            if t is None:
+                t = torch.zeros(1, dtype=torch.int32, device=device)
+                if key[0] == "cuda" and _host is not None:
+                    _host.set_status(key[1], t, torch.cuda.get_device_properties(key[1]).multi_processor_count)
+                _status_words[key] = t
     return t
 
 

@@ -56,6 +56,35 @@ def test_package_works_without_it(monkeypatch, module):
     assert _lib.native() is good
 
 
+def test_status_word_is_one_for_all_threads(monkeypatch):
+    """Threads that make a device's first call at the same time share one status word: the native launcher keeps the one it is
+    given first, and check_status reads the one in the table."""
+    import threading
+    import time
+
+    from flash_sparse_attn import _lib
+
+    _lib.load()
+    zeros, seen = torch.zeros, []
+
+    def slow_zeros(*a, **kw):
+        t = zeros(*a, **kw)
+        time.sleep(0.05)
+        return t
+
+    monkeypatch.setattr(torch, "zeros", slow_zeros)
+    device = torch.device("cpu", 7)
+    threads = [threading.Thread(target=lambda: seen.append(_lib.status_word(device))) for _ in range(4)]
+    try:
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert len(seen) == 4 and all(t is seen[0] for t in seen) and _lib._status_words[("cpu", 7)] is seen[0]
+    finally:
+        _lib._status_words.pop(("cpu", 7), None)
+
+
 def _both(monkeypatch, fn):
     """fn() through the native launcher (which must take the call) and through the Python one."""
     from flash_sparse_attn import _lib
