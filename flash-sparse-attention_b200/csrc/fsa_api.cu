@@ -859,7 +859,8 @@ int fsa_decode(const FsaDecArgs* a, void* stream_) {
     p.peer_rank = pe->rank;
     p.peer_block_floats = pe->block_floats;
   }
-  if (!a->partial_only) p.cluster = fsa::dec_cluster_splits(a->batch, a->heads_kv, a->heads_q, a->head_dim, ns);
+  if (!a->partial_only && (a->flags & FSA_F_SCRATCH_PARTIALS))
+    p.cluster = fsa::dec_cluster_splits(a->batch, a->heads_kv, a->heads_q, a->head_dim, ns);
   mark(a->ev_before, stream);
   p.D = a->head_dim;
   cudaError_t e = fsa::launch_dec(p, a->kind, a->dtype, head_dim_kernel_wide(a->head_dim), stream);

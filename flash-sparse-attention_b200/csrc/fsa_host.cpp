@@ -229,7 +229,7 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
     x.num_splits = (int)splits;
     x.kind = (int)kind;
     x.dtype = code;
-    x.flags = (local ? FSA_F_LOCAL : 0) | FSA_F_LOGSIGMOID;
+    x.flags = (local ? FSA_F_LOCAL : 0) | FSA_F_LOGSIGMOID | FSA_F_SCRATCH_PARTIALS;
     x.softmax_scale = (float)sm_scale;
     x.softmax_threshold = (float)thr;
     x.qkv_scale = ptr<float>(scale);

@@ -76,6 +76,7 @@ int fsa_decode_static_scratch(const FsaDecArgs* a, void* stream) {
   FsaDecArgs b;
   memcpy(&b, a, sizeof(b));
   b.num_splits = ns;
+  b.flags |= FSA_F_SCRATCH_PARTIALS;
   b.out_partial = scratch;
   b.lse_partial = scratch + slots * (size_t)a->head_dim;
   return fsa_decode(&b, stream);

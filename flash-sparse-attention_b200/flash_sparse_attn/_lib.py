@@ -30,6 +30,7 @@ F_PACK_GQA = 1 << 3
 F_LOGSIGMOID = 1 << 4
 F_ADAPT_GATE = 1 << 5
 F_DETERMINISTIC = 1 << 6
+F_SCRATCH_PARTIALS = 1 << 7
 
 
 class FsaFwdArgs(ctypes.Structure):

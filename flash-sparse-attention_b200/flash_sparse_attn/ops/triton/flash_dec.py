@@ -184,6 +184,8 @@ def attn_decode(
     a.kind = _KIND[kind]
     a.dtype = _lib.dtype_code(query.dtype)
     a.flags = (_lib.F_LOCAL if is_local else 0) | (_lib.F_LOGSIGMOID if is_logsigmoid_gate else 0)
+    if workspace is None and packed_partials is None:
+        a.flags |= _lib.F_SCRATCH_PARTIALS  # nobody else sees them
     if kind == "gated":
         # alpha [B, Hq]; delta [B, Hkv, Sk] / [Hkv, Tk] / paged [pages, Hkv, page] (positions contiguous)
         alpha, delta = alpha.to(out_dtype).contiguous(), delta.to(out_dtype).contiguous()

@@ -56,7 +56,8 @@ enum {
   FSA_F_PACK_GQA = 1u << 3,   /* rows of one query tile interleave the G heads of a KV head */
   FSA_F_LOGSIGMOID = 1u << 4, /* gated: gate = logsigmoid(alpha*delta), else alpha*delta */
   FSA_F_ADAPT_GATE = 1u << 5,
-  FSA_F_DETERMINISTIC = 1u << 6 /* backward: add the dQ tiles of the key tiles in a fixed order */
+  FSA_F_DETERMINISTIC = 1u << 6, /* backward: add the dQ tiles of the key tiles in a fixed order */
+  FSA_F_SCRATCH_PARTIALS = 1u << 7 /* decode: out_partial / lse_partial are scratch, the caller will not read them */
 };
 
 /*
@@ -246,7 +247,8 @@ int64_t fsa_bwd_padded_rows(int batch, int seqlen_q, int total_q, int is_varlen)
  *   out_partial [num_splits, batch, heads_q, head_dim], lse_partial [num_splits, heads_q, batch] fp32
  *     (base-2 lse): written when num_splits > 1 or when partial_only is set. With partial_only the
  *     call stops after the partials (no combine), for callers that merge partials of several
- *     devices themselves with fsa_combine.
+ *     devices themselves with fsa_combine. With FSA_F_SCRATCH_PARTIALS (and not partial_only) the buffers
+ *     are still needed, but their contents afterwards are unspecified: splits that can merge on the chip do.
  *   head_dim: a multiple of 8 up to 256 with 16-bit inputs (sizes above 128 run eight query heads of a KV head per
  *     pass over the keys), 128 with FP8 inputs. fsa_fwd takes the same sizes, fsa_bwd stops at 128.
  */

@@ -88,3 +88,18 @@ def test_clusters_only_where_they_are_resident(dtype, pairs, splits, launches):
     torch.cuda.synchronize()
     fsa.check_status()
     assert_close("out", out, ref)
+
+
+@pytest.mark.parametrize("num_splits", [2, 8, 9])
+def test_partials_are_written_either_way(num_splits):
+    """The split partials are a documented output of the library's decode call; a caller that brings the buffers may read them."""
+    from flash_sparse_attn.ops.triton.flash_dec import attn_decode
+
+    g = torch.Generator().manual_seed(num_splits)
+    q, k, v = (torch.randn(*s, generator=g).to(torch.bfloat16).cuda() for s in ((2, 6, 96), (2, 150, 3, 96), (2, 150, 3, 96)))
+    used = torch.tensor([150, 20], dtype=torch.int32, device="cuda")  # splits without a key among them
+    want = attn_decode("dense", q, k, v, seqused_k=used, num_splits=num_splits, partial_only=True)
+    got = tuple(torch.full_like(t, float("nan")) for t in want)
+    attn_decode("dense", q, k, v, seqused_k=used, num_splits=num_splits, workspace=got)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
