@@ -244,3 +244,19 @@ def test_gil_is_free_during_the_launch():
     finally:
         host.init(address(lib.fsa_decode), address(lib.fsa_fwd))
     assert type(dec) is tuple and type(fwd) is tuple
+
+
+@pytest.mark.gpu
+def test_scales_of_a_declined_call_are_packed_once(monkeypatch):
+    import flash_sparse_attn as fsa
+    from flash_sparse_attn.ops.triton import quant
+
+    count, pack = [], quant.scales_f32
+    monkeypatch.setattr(quant, "scales_f32", lambda *a: count.append(1) or pack(*a))
+    x = lambda *s: torch.randn(*s, 64, device=DEV).to(torch.float8_e4m3fn)  # noqa: E731  (native FP8 has 128 columns)
+    one = torch.ones(1, device=DEV)
+    kw = dict(is_quant=True, query_scale=one, key_scale=one, value_scale=one)
+    fsa.flash_dense_attn_with_kvcache_func(x(2, 4), x(2, 50, 2), x(2, 50, 2), **kw)
+    assert len(count) == 1
+    fsa.flash_dense_attn_func(x(2, 50, 4), x(2, 50, 2), x(2, 50, 2), **kw)
+    assert len(count) == 2
