@@ -76,6 +76,18 @@ def test_backward_ragged(sq, sk, causal):
         assert_close(name, a, r)
 
 
+@pytest.mark.parametrize("num_splits", [None, 3])  # two groups of 78 and 77 pairs, six of 26 and 25
+def test_backward_groups_of_pairs(num_splits):
+    """155 (sequence, KV head) pairs: their key tiles are launched in groups of pairs, which do not come out even."""
+    fsa = _ops()
+    q, k, v = seeded_qkv(21, 31, 400, 400, 5, 5, 64)
+    do = torch.randn(q.shape, generator=torch.Generator().manual_seed(22)).to(q.dtype)
+    kw = {} if num_splits is None else dict(is_split_qo=True, num_splits=num_splits)
+    got = _run(fsa.flash_dense_attn_func, q, k, v, do, is_causal=True, **kw)
+    for name, a, b in zip(("dq", "dk", "dv"), got, eager.backward(q, k, v, do, None, True)):
+        assert_close(name, a, b)
+
+
 def test_backward_varlen():
     fsa = _ops()
     lens_q, lens_k = [5, 130, 257, 64], [70, 130, 300, 64]

@@ -1,5 +1,5 @@
-"""Decode calls whose splits are merged inside a thread-block cluster (all CTAs resident at once, two to eight splits), at
-the edges of that rule, against the eager oracle."""
+"""Decode calls whose splits are merged inside a thread-block cluster (two to eight splits, as many clusters as are resident
+at once) and through partials and the combine kernel, at the edges of that rule and for every form, against the eager oracle."""
 
 import pytest
 import torch
@@ -103,3 +103,57 @@ def test_partials_are_written_either_way(num_splits):
     attn_decode("dense", q, k, v, seqused_k=used, num_splits=num_splits, workspace=got)
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("num_splits", [3, 9])  # cluster merge; partials and combine
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float8_e4m3fn])
+@pytest.mark.parametrize("form", ["window", "paged", "gather", "paged gather", "varlen", "gated", "gated gather"])
+def test_both_merges_of_every_form(form, dtype, num_splits):
+    import flash_sparse_attn as fsa
+
+    fp8 = dtype != torch.bfloat16
+    g = torch.Generator().manual_seed(len(form) + num_splits)
+    b, sk, hq, hkv, d, page = 2, 320, 6, 2, 128, 32
+    mk = lambda *s: torch.randn(*s, generator=g).to(torch.bfloat16)  # noqa: E731
+    q, k, v, al, de = mk(b, hq, d), mk(b, sk, hkv, d), mk(b, sk, hkv, d), mk(b, hq), mk(b, sk, hkv)
+    if fp8:  # scales of one: the oracle takes the rounded values
+        q, k, v = (t.to(dtype).to(torch.bfloat16) for t in (q, k, v))
+    put = lambda t: t.to(dtype).cuda()  # noqa: E731
+    args, kw, opts = [put(q), put(k), put(v)], {}, {}
+    fn = fsa.flash_sparse_attn_with_kvcache_func
+    kw["softmax_threshold"] = -128.0  # nothing is skipped
+    if form == "window":
+        opts = dict(is_local=True, window_sizes=torch.tensor([[8, 60, 40, 90], [0, 100, 0, 33]], dtype=torch.int32))
+        kw["window_sizes"] = opts["window_sizes"].cuda()
+    if "paged" in form:
+        table = torch.randperm(b * sk // page, generator=g).to(torch.int32)
+        for i, t in ((1, k), (2, v)):
+            pages = torch.empty(b * sk // page, page, hkv, d, dtype=torch.bfloat16)
+            pages[table.long()] = t.reshape(pages.shape)
+            args[i] = put(pages)
+        kw["page_table"] = table.reshape(b, -1).cuda()
+    gate = dict(alpha=al, delta=de) if "gated" in form else {}
+    if gate:
+        fn = fsa.flash_gated_attn_with_kvcache_func
+        args += [al.cuda(), de.cuda()]
+        kw["gate_threshold"] = -128.0
+    if fp8:
+        one = torch.ones(1, device="cuda")
+        kw.update(is_quant=True, query_scale=one, key_scale=one, value_scale=one)
+    if "gather" in form:
+        idx = torch.stack([torch.randperm(sk, generator=g)[:200] for _ in range(b)]).to(torch.int32)
+        idx[:, 3::11] = -1
+        kw["gather_kv_indices"] = idx.cuda()
+        ref = eager.gather_decode(q, k, v, idx, return_lse=True, **gate)
+    elif form == "varlen":
+        cu = torch.tensor([0, 300, 433], dtype=torch.int32)
+        k, v = k.reshape(-1, hkv, d)[:433], v.reshape(-1, hkv, d)[:433]
+        ref = eager.varlen_decode(q, k, v, cu, return_lse=True)
+        fn, args = fsa.flash_sparse_attn_varlen_with_kvcache_func, [put(q), put(k), put(v), cu.cuda(), 300]
+    else:
+        ref = eager.decode(q, k, v, return_lse=True, **opts, **gate)
+    out, lse = fn(*args, num_splits=num_splits, return_lse=True, **kw)
+    torch.cuda.synchronize()
+    fsa.check_status()
+    assert_close(form, out, ref[0], rtol=2.5e-2, atol=2.5e-2)
+    assert torch.allclose(lse.cpu(), ref[1], rtol=0, atol=2e-3)

@@ -19,7 +19,7 @@ def test_decode_split_rule_is_the_same():
                     assert _lib._host.decode_num_splits(batch, hkv, keys, sms) == decode_num_splits(batch, hkv, keys, sms)
 
 
-def test_refuses_what_it_does_not_know():
+def test_refuses_what_is_not_on_a_gpu():
     from flash_sparse_attn import _lib
 
     _lib.load()
@@ -27,8 +27,6 @@ def test_refuses_what_it_does_not_know():
     args = [0, q, k, k, None, None, None, False, None, None, None, None, None, None, None, None, None]
     assert _lib._host.decode(*args) is None  # not on a GPU
     assert _lib._host.decode(*args[:-1]) is None and _lib._host.forward() is None
-    for i, bad in ((1, None), (2, "k"), (0, 1.5), (7, 1), (8, "two"), (8, -1), (8, 1 << 40)):
-        assert _lib._host.decode(*(args[:i] + [bad] + args[i + 1:])) is None
 
 
 @pytest.mark.parametrize("module", ["missing", "other abi", "other torch", "old"])
@@ -187,6 +185,115 @@ def test_forward_forms(monkeypatch, dtype, form):
             kw.update(seqused_k=torch.tensor([150, 0, 300], dtype=torch.int32, device=DEV))
         fn = lambda q, k, v, **a: fsa.flash_sparse_attn_varlen_func(q, k, v, cu, cu, 300, 300, **a)  # noqa: E731
     _both(monkeypatch, lambda: tuple(t.clone() for t in fn(q, k, v, return_lse=True, **kw)))
+
+
+@pytest.mark.gpu
+def test_refuses_one_wrong_argument():
+    """Calls that it takes, and the same ones with one argument replaced, which it leaves to the Python launcher."""
+    import flash_sparse_attn as fsa
+    from flash_sparse_attn import _lib
+
+    bf = lambda *s: torch.zeros(*s, dtype=torch.bfloat16, device=DEV)  # noqa: E731
+    i32 = lambda *s: torch.zeros(*s, dtype=torch.int32, device=DEV)  # noqa: E731
+    q, k = bf(2, 4, 64), bf(2, 32, 2, 64)
+    fsa.flash_dense_attn_with_kvcache_func(q, k, k)  # registers the device
+    host = _lib._host
+
+    def check(fn, base, wrong):
+        assert type(fn(*base)) is tuple, "the base call is not taken"
+        for i, bads in wrong.items():
+            for bad in bads:
+                assert fn(*(base[:i] + [bad] + base[i + 1:])) is None, (i, bad if not torch.is_tensor(bad) else bad.shape)
+        assert fn(*base[:-1]) is None
+        torch.cuda.synchronize()
+
+    ints = lambda *s: [i32(*s).long(), i32(*s).cpu(), i32(*s).float(), "x"]  # noqa: E731  (wrong type, device, kind)
+    window = torch.tensor([[0, 16, 0, 8]] * 2, dtype=torch.int32, device=DEV)
+    out_wrong = lambda *s: [bf(*s).half(), bf(*s).cpu(), bf(*s[:-1], 32), bf(*s[:-1], 128)[..., ::2], "x"]  # noqa: E731
+    lse_wrong = lambda *s: [bf(*s), torch.zeros(*s), torch.zeros(*s, 1, device=DEV), "x"]  # noqa: E731
+    q_wrong = [None, "q", q.cpu(), q.half(), q.float(), bf(2, 3, 64), bf(2, 4, 72), bf(2, 4, 128)[..., ::2], bf(8, 64)]
+    k_wrong = [None, k.half(), bf(3, 32, 2, 64), bf(2, 32, 2, 128)[..., ::2], bf(2, 2, 32, 64).transpose(1, 2), bf(64, 2, 64)]
+    # kind, q, k, v, scale, windows, threshold, local, splits, table, gather, used, cu, max_k, out, lse, fp8 scales
+    base = [0, q, k, k, None, None, None, False, None, None, None, None, None, None, None, None, None]
+    check(host.decode, base, {0: [1.5, None], 1: q_wrong, 2: k_wrong, 4: ["1", [1.0]], 5: [window], 6: ["1"], 7: [1, True],
+                              8: ["two", -1, 1 << 40, 2.0], 10: ints(2, 5) + [i32(3, 5), i32(5), i32(2, 10)[:, ::2]],
+                              11: ints(2) + [i32(1), i32(2, 1)], 12: [i32(3)], 14: out_wrong(2, 4, 64),
+                              15: lse_wrong(2, 4), 16: [torch.ones(3, device=DEV)]})
+    local = base[:5] + [window, None, True] + base[8:]
+    check(host.decode, local, {5: [None, window.long(), window.cpu(), window[:1], i32(2, 3), i32(8)], 7: [False]})
+    paged = base[:2] + [k, k] + base[4:9] + [i32(2, 1)] + base[10:]
+    check(host.decode, paged, {9: ints(2, 1) + [i32(3, 1), i32(2)], 12: [i32(3)]})
+    packed = [0, q, bf(64, 2, 64), bf(64, 2, 64)] + base[4:12] + [i32(3), 32] + base[14:]
+    check(host.decode, packed, {9: [i32(2, 1)], 12: ints(3) + [i32(2), None], 13: [None, "x", -1, 1.0]})
+
+    q, k = bf(2, 32, 4, 64), bf(2, 32, 2, 64)
+    q_wrong = [None, q.cpu(), q.half(), bf(2, 32, 3, 64), bf(2, 32, 4, 128)[..., ::2], bf(2, 4, 32, 64).transpose(1, 2)]
+    # kind, q, k, v, causal, scale, windows, threshold, local, splits, pack, cu_q, cu_k, max_q, max_k, table, used_q, used_k, out,
+    # lse, fp8 scales
+    base = [0, q, k, k, True, None, None, None, False, 1, False, None, None, None, None, None, None, None, None, None, None]
+    check(host.forward, base, {0: [1.5], 1: q_wrong, 2: k_wrong, 4: [1], 5: ["1"], 6: [window], 7: ["1"], 8: [True, 0],
+                               9: [0, -1, None, 2.0], 10: [1], 11: [i32(3)], 12: [i32(3)], 16: ints(2) + [i32(1)],
+                               17: ints(2) + [i32(1)], 18: out_wrong(2, 32, 4, 64), 19: lse_wrong(2, 4, 32),
+                               20: [torch.ones(3, device=DEV)]})
+    packed = [0, bf(64, 4, 64), bf(64, 2, 64), bf(64, 2, 64)] + base[4:9] + [2] + base[10:11] + [i32(3), i32(3), 32, 32] + base[15:]
+    check(host.forward, packed, {11: ints(3) + [None, i32(2)], 12: ints(3) + [None, i32(2)], 13: [None, -1, 1.0], 14: [None, "x"],
+                                 15: [i32(2, 1)], 16: [i32(2)]})  # used_q with splits: its partials want a fill
+
+
+@pytest.mark.gpu
+def test_unused_query_rows_with_splits():
+    """The declined form: packed sequences of which only some query rows are used, over KV splits."""
+    import flash_sparse_attn as fsa
+    from fixtures import assert_close
+    from oracle import eager
+
+    g = torch.Generator().manual_seed(4)
+    mk = lambda *s: torch.randn(*s, generator=g).to(torch.bfloat16)  # noqa: E731
+    q, k, v = mk(400, 4, 64), mk(1500, 2, 64), mk(1500, 2, 64)
+    cu_q, cu_k = torch.tensor([0, 150, 400], dtype=torch.int32), torch.tensor([0, 900, 1500], dtype=torch.int32)
+    used = torch.tensor([100, 250], dtype=torch.int32)
+    out, lse = fsa.flash_dense_attn_varlen_func(q.to(DEV), k.to(DEV), v.to(DEV), cu_q.to(DEV), cu_k.to(DEV), 250, 900,
+                                                is_split_kv=True, num_splits=3, seqused_q=used.to(DEV), return_lse=True)
+    for s in range(2):
+        rows, keys = slice(cu_q[s], cu_q[s] + used[s]), slice(cu_k[s], cu_k[s + 1])
+        ref = eager.forward(q[None, rows], k[None, keys], v[None, keys], None, False)
+        assert_close(f"sequence {s}", out[None, rows], ref)
+    assert torch.isneginf(lse[:, 100:150]).all()  # rows that are not used
+
+
+@pytest.mark.gpu
+def test_threads_and_streams():
+    """Two threads, each with its own stream and inputs, get what one thread gets."""
+    import threading
+
+    import flash_sparse_attn as fsa
+
+    g = torch.Generator(device=DEV).manual_seed(6)
+    mk = lambda *s: torch.randn(*s, generator=g, device=DEV).to(torch.bfloat16)  # noqa: E731
+    jobs = [(mk(2, 8, 64), mk(2, 700, 2, 64), mk(1, 300, 8, 64), mk(1, 300, 2, 64)) for _ in range(2)]
+
+    def run(job):
+        q, k, qf, kf = job
+        return (fsa.flash_dense_attn_with_kvcache_func(q, k, k, num_splits=9),
+                fsa.flash_sparse_attn_func(qf, kf, kf, is_causal=True, is_split_kv=True, num_splits=2))
+
+    want = [run(j) for j in jobs]
+    torch.cuda.synchronize()
+    got = [None, None]
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(20):
+                got[i] = run(jobs[i])
+            torch.cuda.current_stream().synchronize()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for a, b in zip(got, want):
+        assert all(torch.equal(x, y) for x, y in zip(a, b))
 
 
 @pytest.mark.gpu

@@ -27,9 +27,11 @@ def test_static_scratch_decode_matches_regular_entry_point_twice():
     from flash_sparse_attn.ops.triton.flash_dec import attn_decode
 
     assert static_scratch.scratch_bytes() == 16 * 1024 * 1024
-    # two different problems back to back: the second one reuses (and partly overlaps) the bytes the
-    # first one left in the shared workspace
-    for call, (seed, b, sk, hq, hkv, d, ns) in enumerate([(11, 8, 3000, 32, 4, 128, 4), (12, 5, 1777, 16, 2, 64, 3)]):
+    # different problems back to back: each one reuses (and partly overlaps) the bytes that the ones before left in the
+    # shared workspace. The first two merge their splits on the chip; nine and more splits go through the workspace.
+    for call, (seed, b, sk, hq, hkv, d, ns) in enumerate([(11, 8, 3000, 32, 4, 128, 4), (12, 5, 1777, 16, 2, 64, 3),
+                                                             (14, 8, 3000, 32, 4, 128, 16), (15, 5, 1777, 16, 2, 64, 9),
+                                                             (16, 2, 100, 16, 2, 64, 12)]):
         q, k, v = _inputs(seed, b, sk, hq, hkv, d)
         ref_out, ref_lse = attn_decode("sparse", q, k, v, softmax_threshold=1.0, num_splits=ns)
         out = torch.empty_like(q)
