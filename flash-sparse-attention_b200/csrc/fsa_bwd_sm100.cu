@@ -516,14 +516,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
         }
         umma_commit_lead(lead, &bars->s_full);
       };
-      int g_nxt = 0, m_nxt = 0;
-      bool has_cur;
-      {
-        StepWalk wk = walk_begin();  // whether there is any step
-        int mode_unused = 0;
-        bool first_unused = false;
-        has_cur = ok && walk_next(wk, g_nxt, m_nxt, mode_unused, first_unused, false);
-      }
+      // The dense kind at head size 128 walks the steps here as well: nothing else delays its issuer, and what it reads
+      // from the producer's record makes its branches depend on memory (non-causal, S = 4096, 16 / 4 heads: 371 us a call,
+      // 381 with the record; causal 370 and 372). The 64-wide kernel (330 against 361 us) and the other kinds, which have to
+      // drop steps, read the record.
+      constexpr bool OWN_WALK = KIND == KIND_DENSE && HD == 128;
+      int g_nxt = 0, m_nxt = 0, mode_unused = 0;
+      bool first_unused = false;
+      StepWalk wk = walk_begin();
+      bool has_cur = ok && walk_next(wk, g_nxt, m_nxt, mode_unused, first_unused, false);  // whether there is any step
       const bool det = p.flags & F_DETERMINISTIC;
       int n_jobs = 0;  // dQ tiles (and, deterministic mode, passes) handed to the dQ warps so far
       // descriptor of the dQ tile the next commit on dq_full announces; written well before the MMAs it follows
@@ -546,7 +547,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
       for (int it = 0; has_cur && ok; ++it) {
         const int st = it & 1;
         const int g_cur = g_nxt, m_cur = m_nxt;
-        const bool has_next = *reinterpret_cast<const volatile int*>(&bars->step[st][3]) & 2;
+        bool has_next;
+        if constexpr (OWN_WALK)
+          has_next = walk_next(wk, g_nxt, m_nxt, mode_unused, first_unused, false);
+        else
+          has_next = *reinterpret_cast<const volatile int*>(&bars->step[st][3]) & 2;
         // The verdict of the skip vote is read straight from the votes (the compute warps publish them well before
         // the exponentials), so that dP^T is under way while P^T is still being computed.
         bool skip = false;
@@ -598,8 +603,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
           if (!ok) break;
           tc_fence_after();
           issue_st((it + 1) & 1);
-          g_nxt = *reinterpret_cast<const volatile int*>(&bars->step[(it + 1) & 1][0]);
-          m_nxt = *reinterpret_cast<const volatile int*>(&bars->step[(it + 1) & 1][1]);
+          if constexpr (!OWN_WALK) {
+            g_nxt = *reinterpret_cast<const volatile int*>(&bars->step[(it + 1) & 1][0]);
+            m_nxt = *reinterpret_cast<const volatile int*>(&bars->step[(it + 1) & 1][1]);
+          }
         }
         if (!skip) {
           ok = mbar_wait(&bars->ds_full, n_live & 1, abort_flag);
