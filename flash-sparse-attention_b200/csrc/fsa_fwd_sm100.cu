@@ -179,9 +179,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
   static_assert(!F8 || HD == 128, "FP8 tiles are one 128-byte swizzle row wide");
   constexpr uint32_t TMEM_S0 = 0, TMEM_O0 = 256;
   // FP8: P is handed to the MMA issuer in two halves, so that the first MMAs of P V run under the second half of the
-  // exponentials (B2 S6000 causal 570 -> 543 us). With 16-bit inputs, whose P V takes twice as long, the second barrier
+  // exponentials (B2 S6000 causal, a call: 529 -> 510 us). With 16-bit inputs, whose P V takes twice as long, the second barrier
   // costs the issuer more than that gains (S = 16384: 1.91 -> 1.96 ms).
   constexpr bool HALVES = F8;
+  // Who walks the tiles for the MMA issuer: the producer, ahead of time, except above head size 128 (not gated), where one query
+  // tile leaves the issuer time and reading the producer's record costs more than the walk (dense causal S = 8192,
+  // 16 / 4 heads of 192: 501 us, 523 with the record; a 1024-token window 183 and 187).
+  constexpr bool HANDED = KIND == KIND_GATED || HD <= 128;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -411,7 +415,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
       // Which tile comes next and who takes part in it is worked out here, ahead of time, and handed to the MMA issuer with
       // the barrier that it waits on anyway: on windowed schedules the walk took the issuer 925 of the 4250 cycles of
       // a step, in which the tensor pipe had nothing to do.
-      bool act[2], act_next[2];
+      [[maybe_unused]] bool act[2], act_next[2];
       auto take_part = [&](int n_t, bool* a) {  // not gated: the groups whose schedule has tile n_t
 #pragma unroll
         for (int q = 0; q < 2; ++q) a[q] = n_t >= 0 && fsa_fwd_tile_mode(sched[q], n_t, causal, local) >= 0;
@@ -426,9 +430,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
         n = walk_next(WALK_START, act, false);
       } else {
         n = first_tile();
-        take_part(n, act);
+        if constexpr (HANDED) take_part(n, act);
       }
-      publish(2, n, act, 0u);
+      if constexpr (HANDED) publish(2, n, act, 0u);
       if (n >= 0) {
         load_kv(&p.map_k, smem + SM::kK, &bars->k0_full, n);
       } else {
@@ -437,15 +441,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
       }
       while (n >= 0 && ok) {
         int n_next;
-        unsigned last = 0u;  // gated: not known before the next tile's gate is; its output barriers come after the loop
+        [[maybe_unused]] unsigned last = 0u;  // gated: not known before the next gate is; its output barriers follow the loop
         if constexpr (KIND == KIND_GATED) {
           n_next = walk_next(n, act_next, false);
         } else {
           n_next = next_tile(n);
-          take_part(n_next, act_next);
+          if constexpr (HANDED) {
+            take_part(n_next, act_next);
 #pragma unroll
-          for (int q = 0; q < 2; ++q)
-            if (act[q] && fsa_fwd_next_tile_below(sched[q], n, local) < 0) last |= 1u << q;
+            for (int q = 0; q < 2; ++q)
+              if (act[q] && fsa_fwd_next_tile_below(sched[q], n, local) < 0) last |= 1u << q;
+          }
         }
         // Release signals arrive in order (signal c: K(c) and V(c - 1) consumed). V(t) goes into the slot of
         // V(t - 2) and K(t + 1) into the slot of K(t - 1): both free after signal t - 1.
@@ -458,7 +464,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
         // V(t) replaces V(t - VSTAGES), K(t + 1) replaces K(t + 1 - KSTAGES): both are free after this signal
         need_signal(t - (KSTAGES < VSTAGES ? KSTAGES : VSTAGES) + 1);
         if (!ok) break;
-        publish(t & 1, n_next, act_next, last);  // the issuer has read the slot's last word: it came before signal t - 1
+        // the issuer has read the slot's last word: it came before signal t - 1
+        if constexpr (HANDED) publish(t & 1, n_next, act_next, last);
         // V is prefetched like K, before the softmax groups have voted on the tile: waiting for the vote
         // would put a full load latency between every S tile and its P V product, and in this
         // tensor-bound kernel a V tile that ends up unused only costs an L2 read: on inputs where 82 % of the
@@ -472,8 +479,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
         else
           mbar_arrive(&bars->kv_full[t & 1]);  // the barrier counts two arrivals per step
         n = n_next;
-        act[0] = act_next[0];
-        act[1] = act_next[1];
+        if constexpr (HANDED) {
+          act[0] = act_next[0];
+          act[1] = act_next[1];
+        }
         ++t;
       }
     }
@@ -535,7 +544,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
     bool o_started[2] = {false, false};
     bool act[2] = {false, false}, last[2];
     int n = -1;
-    auto read_info = [&](int slot, int& n_t, unsigned& f) {
+    [[maybe_unused]] auto read_info = [&](int slot, int& n_t, unsigned& f) {
       const unsigned long long w = *reinterpret_cast<const volatile unsigned long long*>(&bars->step_info[slot]);
       n_t = (int)(unsigned)w;
       f = (unsigned)(w >> 32);
@@ -561,12 +570,19 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
       }
       umma_commit_lead(lead, &bars->s_full[q]);
     };
+    if constexpr (!HANDED) {
+      n = first_tile();
+#pragma unroll
+      for (int q = 0; q < 2; ++q) act[q] = n >= 0 && fsa_fwd_tile_mode(sched[q], n, causal, local) >= 0;
+    }
     if (ok) ok = mbar_wait(&bars->k0_full, 0, abort_flag);
-    if (ok) {
-      unsigned f;
-      read_info(2, n, f);
-      act[0] = f & 1u;
-      act[1] = f & 2u;
+    if constexpr (HANDED) {
+      if (ok) {
+        unsigned f;
+        read_info(2, n, f);
+        act[0] = f & 1u;
+        act[1] = f & 2u;
+      }
     }
     if (n >= 0 && ok) {
       ok = mbar_wait(&bars->q_full, 0, abort_flag);
@@ -587,15 +603,30 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
       bool act_next[2];
       const int vs = t % VSTAGES;
       const int ks_next = (t + 1) % KSTAGES;
+      int n_next;
+      if constexpr (!HANDED) {
+        n_next = next_tile(n);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          if (!local) {  // one contiguous range of tiles per group
+            act_next[q] = n_next >= sched[q].n_min && n_next < sched[q].n_max;
+            last[q] = act[q] && n == sched[q].n_min;
+          } else {
+            act_next[q] = n_next >= 0 && fsa_fwd_tile_mode(sched[q], n_next, causal, local) >= 0;
+            last[q] = act[q] && fsa_fwd_next_tile_below(sched[q], n, local) < 0;
+          }
+        }
+      }
       ok = mbar_wait(&bars->kv_full[t & 1], (t >> 1) & 1, abort_flag);  // V(t) and K(t + 1)
       if (!ok) break;
-      int n_next;
-      unsigned f;
-      read_info(t & 1, n_next, f);
+      if constexpr (HANDED) {
+        unsigned f;
+        read_info(t & 1, n_next, f);
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        act_next[q] = (f >> q) & 1u;
-        last[q] = (f >> (2 + q)) & 1u;
+        for (int q = 0; q < 2; ++q) {
+          act_next[q] = (f >> q) & 1u;
+          last[q] = (f >> (2 + q)) & 1u;
+        }
       }
       if ((p.flags & F_KV_RAGGED) && (n + 1) * TN > si.sk) {
         // keys past the sequence end carry probability 0 but their V rows may hold
