@@ -996,22 +996,11 @@ bool clusters_fit(Kernel kern, int clusters, int size, int smem, std::atomic<int
   std::atomic<int>& known = cache[dev][lone][size];
   int room = known.load(std::memory_order_relaxed) - 1;  // 0: not asked yet
   if (room < 0) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)size, 1, 1);
-    cfg.blockDim = dim3(DWARPS * 32, 1, 1);
-    cfg.dynamicSmemBytes = lone ? LONE_SMEM : smem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)size;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LONE_SMEM) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&room, kern, &cfg) != cudaSuccess) {
+    room = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LONE_SMEM) == cudaSuccess)
+      room = resident_clusters(kern, size, DWARPS * 32, lone ? LONE_SMEM : smem);
+    else
       (void)cudaGetLastError();
-      room = 0;
-    }
     known.store(room + 1, std::memory_order_relaxed);
   }
   return clusters <= room;

@@ -153,6 +153,29 @@ inline cudaError_t smem_opt_in(Kernel kern, int smem, std::atomic<unsigned long 
   return e;
 }
 
+// Clusters of `size` CTAs that the current device holds at a time; 0 when the runtime does not say. A cluster has to fit inside
+// one GPC, so that is less than the SMs' room for single CTAs divided by the size.
+template <typename Kernel>
+inline int resident_clusters(Kernel kern, int size, int threads, int smem) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)size, 1, 1);
+  cfg.blockDim = dim3((unsigned)threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)size;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+
 // Multiprocessor count of the current device (148 on B200), cached per device ordinal.
 inline int device_sm_count() {
   static std::atomic<int> cache[64];

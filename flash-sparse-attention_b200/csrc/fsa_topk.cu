@@ -288,21 +288,51 @@ __global__ void __launch_bounds__(TK_THREADS) topk_kernel(const T* __restrict__ 
   cluster.sync();  // nobody leaves while another CTA may still read its shared memory
 }
 
-// Cluster size: the largest power of two up to 8 that keeps rows * size within the SM count, and leaves a slice
-// of at least TOPK_MIN_SLICE entries per CTA (below that the exchange costs more than the shorter slice gains).
 constexpr int TOPK_MIN_SLICE = 2048;
-inline int topk_cluster_size(int rows, int n) {
-  int c = 1;
-  const int sms = device_sm_count();
-  while (c < 8 && rows * (c * 2) <= sms && n / (c * 2) >= TOPK_MIN_SLICE) c *= 2;
-  return c;
+
+// Entries of a row that a CTA of a cluster of c takes.
+inline int topk_chunk(int n, int c) { return ((n + c - 1) / c + TK_V - 1) / TK_V * TK_V; }
+
+// Clusters of c CTAs that the device holds with one CTA per SM, asked once per device.
+template <typename Kernel>
+int topk_room(Kernel kern, int c, std::atomic<int>& known) {
+  constexpr int LONE_SMEM = 120 * 1024;  // more than half of an SM's shared memory
+  int fit = known.load(std::memory_order_relaxed) - 1;
+  if (fit < 0) {
+    fit = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LONE_SMEM) == cudaSuccess)
+      fit = resident_clusters(kern, c, TK_THREADS, LONE_SMEM);
+    else
+      (void)cudaGetLastError();
+    known.store(fit + 1, std::memory_order_relaxed);
+  }
+  return fit;
+}
+
+// Cluster size: the largest power of two up to 8 whose clusters all find room at a time with an SM to each CTA, and that leaves
+// a slice of at least TOPK_MIN_SLICE entries per CTA (below that the exchange costs more than the shorter slice gains).
+// rows * size <= SMs does not say that: 16 clusters of eight have no room on 148 SMs (16 rows of 32000 fp32 scores: 25.9 us
+// with them, 13.1 with clusters of four; bf16, whose CTAs share SMs then, 13.9 and 10.2).
+template <typename T, typename I>
+int topk_cluster_size(int rows, int n) {
+  static std::atomic<int> room[64][3][4];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return 1;
+  for (int lg = 3; lg > 0; --lg) {
+    const int c = 1 << lg, chunk = topk_chunk(n, c);
+    if ((long long)rows * c > device_sm_count() || n / c < TOPK_MIN_SLICE) continue;
+    const int nc = chunk <= TK_THREADS * TK_V ? 1 : chunk <= TK_THREADS * TK_V * 2 ? 2 : 0;
+    std::atomic<int>& known = room[dev][nc][lg];
+    const int fit = nc == 1 ? topk_room(topk_kernel<T, I, 1>, c, known)
+                            : nc == 2 ? topk_room(topk_kernel<T, I, 2>, c, known) : topk_room(topk_kernel<T, I, 0>, c, known);
+    if (rows <= fit) return c;
+  }
+  return 1;
 }
 
 template <typename T, typename I>
 cudaError_t launch_topk_t(const void* scores, long long row_stride, int rows, int n, int k, void* out, cudaStream_t stream) {
-  const int csize = topk_cluster_size(rows, n);
-  int chunk = (n + csize - 1) / csize;
-  chunk = (chunk + TK_V - 1) / TK_V * TK_V;
+  const int csize = topk_cluster_size<T, I>(rows, n), chunk = topk_chunk(n, csize);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(rows * csize), 1, 1);
   cfg.blockDim = dim3(TK_THREADS, 1, 1);

@@ -9,7 +9,7 @@ from oracle import topk as oracle_topk
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("rows", [1, 19, 75, 150])  # clusters of 8, 4, 1 and 1 on 148 SMs
+@pytest.mark.parametrize("rows", [1, 16, 19, 34, 75, 150])  # clusters of 8, 4, 4, 2, 1 and 1 on 148 SMs
 @pytest.mark.parametrize("n", [4095, 4096, 8191, 8193, 16385, 70001])
 def test_slices(rows, n):
     from flash_sparse_attn.utils.mask import topk_indices
