@@ -579,8 +579,12 @@ int fsa_bwd(const FsaBwdArgs* a, void* stream_) {
   p.n_tiles_k = cdiv(a->seqlen_k, 128);
   p.num_m_blocks = cdiv(a->seqlen_q, 128);
   // One group while the SMs hold four key tiles of every pair at a time; with more pairs, groups of about two CTAs per
-  // SM, so that the end of a group never waits for its longest CTA. (32 pairs of 64 key tiles: 5.36 ms in one group,
-  // 5.77 ms in groups of 5; 128 pairs of up to 32: 3.09 ms in one, 2.43 ms in groups of 32, 2.22 ms in groups of 10.)
+  // SM, so that what runs together shares its Q, dO and dQ tiles in L2. Both sides timed in turn, time over that of one group, 4
+  // query heads of 128 per KV head, causal, at 16 / 32 / 64 key tiles a pair: 40 pairs 0.97 / 0.98 / 0.92, 64 pairs 0.92 / 0.94 /
+  // 0.85, 128 pairs 0.84 / 0.75 / 0.71; packed sequences of unequal length 0.99 / 0.95 / 0.84, 0.99 / 0.84 / 0.74, 0.84 / 0.77 /
+  // 0.72; gated 1.01 / 1.00 / 0.90 at 40 pairs and 1.01 / 0.95 / 0.88 at 64. Three of 94 points lose 2 % and more: 56 pairs of 24
+  // tiles 1.03, gated 48 pairs of 16 tiles 1.02, packed 80 pairs of 8 tiles 1.06 (238 us). With 32 pairs groups gain 5 % at 64 tiles and lose up to a fourth at
+  // 16, where the end of a group weighs more.
   const int pairs = a->batch * a->heads_kv, sms = fsa::device_sm_count();
   p.bh_groups = 4 * pairs <= sms ? 1 : pairs / (pairs < cdiv(2 * sms, p.n_tiles_k * ns) ? pairs : cdiv(2 * sms, p.n_tiles_k * ns));
   p.win_stride = a->window_stride;
