@@ -176,7 +176,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
   float* s_dps = reinterpret_cast<float*>(smem + SM::kAux + 1024);   // [2][128]
   T* s_alpha = reinterpret_cast<T*>(smem + SM::kAux + 2048);         // [2][128] (gated)
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // (through a shuffle: the roles' branches are then known to be the same for the whole warp)
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const bool causal = p.flags & F_CAUSAL, local = p.flags & F_LOCAL, split_qo = p.flags & F_SPLIT;
 
   // ---- work decode ------------------------------------------------------------------------------
@@ -500,7 +501,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
       // The whole warp runs the (uniform) descriptor arithmetic and every MMA carries the single-lane predicate: a
       // divergent branch around the MMAs would cost more issue time per MMA than the MMA takes to execute. A
       // descriptor is (low word, constant high word); moving inside a tile is an add on the low word.
-      const uint32_t lead = lane == 0 ? 1u : 0u;
+      const uint32_t lead = elect_one();
       const uint32_t k_lo = umma_desc_lo(sK, 16), v_lo = umma_desc_lo(sV, 16), do_lo = umma_desc_lo(sDO, 16),
                      ds_lo = umma_desc_lo(sDS, 16);                                  // K-major operands
       const uint32_t do_mn = umma_desc_lo(sDO, TM * 128), ds_mn = umma_desc_lo(sDS, 128 * 128),

@@ -215,10 +215,23 @@ __device__ __forceinline__ void umma_f8_ss(uint32_t d_tmem, uint64_t adesc, uint
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// 1 in one lane of a converged warp, 0 in the others.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t r;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred e;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, e;\n\t"
+      "}\n"
+      : "=r"(r));
+  return r;
+}
 // Leader-predicated forms: the whole warp runs the (warp-uniform) address arithmetic and the instruction
-// carries the single-lane predicate, instead of a divergent branch around a block of MMAs. Inside a divergent
-// branch every descriptor word has to be moved from a vector to a uniform register right before its use, which
-// costs more issue time per MMA than the MMA takes to execute. `lead` is non-zero in exactly one lane.
+// carries the single-lane predicate, instead of a divergent branch around a block of MMAs. `lead` has to come from
+// elect_one(): with "lane == 0" in its place the issue of one MMA takes 75 to 100 cycles beside two busy warps on the
+// scheduler, with the elected lane no longer than the MMA itself (16 MMAs of 128 x 128 x 16: 1279 and 1024 cycles; 4 of
+// those and 8 of 128 x 64 x 16: 897 and 619).
 #define FSA_UMMA_LEAD(NAME, KIND, AFMT, ATYPE, ACONS)                                                        \
   __device__ __forceinline__ void NAME(uint32_t lead, uint32_t d_tmem, ATYPE a, uint64_t bdesc, uint32_t idesc, \
                                        uint32_t accumulate) {                                                \
