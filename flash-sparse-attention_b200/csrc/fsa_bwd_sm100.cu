@@ -20,13 +20,17 @@
 //   dK  += dS^T Q      (A = dS^T from shared memory, K-major)
 //   dQ   = dS K        (A = dS^T from shared memory, read MN-major)
 //
-// Roles (512 threads, four warpgroups): warps 0-7 compute P^T and dS^T (warps 0-3 own query columns 0-63 of the
-// tile, warps 4-7 columns 64-127; both cover all 128 key lanes), warp 8 producer (TMA), warp 9 MMA issuer, warp 10
+// Roles (768 threads, six warpgroups): warps 0-15 compute P^T and dS^T (four warps a group of 32 query columns of the
+// tile, each group covers all 128 key lanes), warp 16 producer (TMA), warp 17 MMA issuer, warp 18
 // dQ drain (deterministic mode only: takes the turns and issues the TMA reduce-adds of the staged dQ tiles), warp
-// 11 idle (register budgets are set per warpgroup), warps 12-15 dQ read-out: TMEM -> registers -> staging ->
+// 19 idle (register budgets are set per warpgroup), warps 20-23 dQ read-out: TMEM -> registers -> staging ->
 // TMA reduce-add, so that the accumulator block shared by dP^T and dQ is free again a few hundred cycles after
 // the dQ MMAs finish and the compute warps never touch dQ.
-// TMEM columns: [0,128) S^T, then P^T packed into [0,32) and [96,128) | [128,256) dP^T, later dQ |
+// Sixteen compute warps of 32 columns rather than eight of 64: the phases of a step (scores, exponentials, dS) are chains of
+// TMEM loads, shared-memory reads and special functions that two warps a scheduler leave mostly idle (issue slots 26 % used).
+// Measured with the elected MMA lane on both sides: gated B4 S8192 4112 -> 3770 us, 64-wide dense S4096 H16 313 (lane 0) -> 247,
+// packed 2052 -> 2030, window workload 358 -> 354, dense causal S8192 1320 -> 1319 (bound by the dQ path).
+// TMEM columns: [0,128) S^T, then P^T packed into the first 16 of each 32 | [128,256) dP^T, later dQ |
 // [256,384) dV | [384,512) dK.
 #include "fsa_ptx.cuh"
 #include "fsa_params.h"
@@ -40,7 +44,9 @@ namespace {
 
 constexpr int TM = 128;  // query rows per step
 constexpr int TN = 128;  // keys per CTA
-constexpr int NTHREADS = 512;
+constexpr int NTHREADS = 768;
+constexpr int NCW = 16;  // compute warps
+constexpr int W_PROD = NCW, W_MMA = NCW + 1, W_DRAIN = NCW + 2, W_DQ = NCW + 4;
 
 template <int HD>
 struct BwdSmem {
@@ -53,7 +59,7 @@ struct BwdSmem {
   static constexpr int kStage = kDS + 32768;   // dQ staging for the TMA reduce-add: 8 warps x 4 KB
   static constexpr int kAux = kStage + 32768;  // lse2[2][128], dpsum[2][128] fp32, alpha[2][128] 16-bit (gated)
   static constexpr int kBar = kAux + 2560;
-  static constexpr int kTotal = kBar + 384;
+  static constexpr int kTotal = kBar + 512;
 };
 
 struct BwdBars {
@@ -69,9 +75,9 @@ struct BwdBars {
   alignas(16) int step[2][4];
   uint32_t tmem_base;
   int abort_flag;
-  unsigned char vote_any[2][8];
+  alignas(16) unsigned char vote_any[2][NCW];
 };
-static_assert(sizeof(BwdBars) <= 384, "barrier block too large");
+static_assert(sizeof(BwdBars) <= 512, "barrier block too large");
 
 // Visible query columns of one key row inside query tile [q0, q0 + TM), as up to three half-open
 // intervals of the tile-local index (mask.py:52-102 read along the query axis).
@@ -165,7 +171,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
   constexpr int KK_D = HD / 16;   // MMAs over the head dimension (S^T, dP^T)
   constexpr int KK_M = TM / 16;   // MMAs over the query rows (dV, dK)
   constexpr int KK_N = TN / 16;   // MMAs over the keys (dQ)
-  constexpr int HALF = HD / 2;    // output columns per compute group
+  constexpr int PART = HD / 4;    // output columns per compute group
   constexpr bool IS_BF16 = !__is_same(T, __half);
   constexpr uint32_t TMEM_S = 0, TMEM_DP = 128, TMEM_DV = 256, TMEM_DK = 384;
 
@@ -317,22 +323,22 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
       mbar_init(&bars->q_empty[s], 1);
     }
     mbar_init(&bars->s_full, 1);
-    mbar_init(&bars->p_full, 8);
+    mbar_init(&bars->p_full, NCW);
     mbar_init(&bars->dp_full, 1);
-    mbar_init(&bars->ds_full, 8);
+    mbar_init(&bars->ds_full, NCW);
     mbar_init(&bars->dq_full, 1);
     mbar_init(&bars->dq_empty, 4);
     mbar_init(&bars->do_full, 1);
     mbar_init(&bars->do_empty, 1);
-    mbar_init(&bars->vote_sync, 8);
+    mbar_init(&bars->vote_sync, NCW);
     mbar_init(&bars->acc_full, 1);
-    mbar_init(&bars->dd_sync, 4);
+    mbar_init(&bars->dd_sync, 12);
     mbar_init(&bars->stg_full, 4);
     mbar_init(&bars->stg_free, 1);
     bars->abort_flag = (*reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
     mbar_fence_init();
   }
-  if (warp == 8) {
+  if (warp == W_PROD) {
     tmem_alloc(&bars->tmem_base, 512);
     tmem_relinquish();
   }
@@ -343,14 +349,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
   const int bq = (p.flags & F_VARLEN_Q) ? 0 : b;
   const int bk = (p.flags & F_VARLEN_K) ? 0 : b;
 
-  if (warp >= 12) {
+  // Register budget: 768 threads x 80 at launch = 512 x 80 + 128 x 96 + 128 x 64
+  if (warp >= W_DQ) {
     // =============================== dQ read-out ================================================
     // One warp per TMEM lane quadrant (32 query rows). Per dQ tile: 64 columns at a time leave TMEM for registers
     // and go through this warp's two 4 KB staging buffers into TMA reduce-adds; the TMEM block is handed back
     // as soon as the last columns are in registers. The path from an SM to L2 moves about 21 bytes per clock, so
     // the 64 KB of a tile take about as long as the MMAs of a step: these warps pace themselves on the reads of
     // the staging buffers and nobody else waits for them.
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
     const int wq = warp & 3;
     const uint32_t lane_addr = uint32_t(wq * 32) << 16;
     uint8_t* stage = smem + SM::kStage + wq * 8192;
@@ -435,9 +442,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
     }
     if (lane == 0) bulk_wait0();
     __syncwarp();
-  } else if (warp >= 8) {
+  } else if (warp >= W_PROD) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
-    if (warp == 8) {
+    if (warp == W_PROD) {
       // =============================== producer ==============================================
       if (lane == 0 && !*abort_flag) {
         tma_prefetch_desc(&p.map_q);
@@ -484,7 +491,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
         }
       }
       __syncwarp();
-    } else if (warp == 9) {
+    } else if (warp == W_MMA) {
       // =============================== MMA issuer ==============================================
       constexpr uint32_t idesc_s = umma_idesc_f16(TN, TM, IS_BF16, false, false);   // S^T, dP^T: [keys x queries]
       constexpr uint32_t idesc_dv = umma_idesc_f16(TN, HD, IS_BF16, false, true);   // dV: A from TMEM, B = dO MN-major
@@ -559,7 +566,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
         if (KIND != KIND_DENSE) {
           ok = mbar_wait(&bars->vote_sync, it & 1, abort_flag);
           if (!ok) break;
-          const unsigned long long vv = *reinterpret_cast<const volatile unsigned long long*>(&bars->vote_any[it & 1][0]);
+          const volatile unsigned long long* vp = reinterpret_cast<const volatile unsigned long long*>(&bars->vote_any[it & 1][0]);
+          const unsigned long long vv = vp[0] | vp[1];
           const bool any_want = (vv & 0x0101010101010101ull) != 0ull, any_drop = (vv & 0x0202020202020202ull) != 0ull;
           skip = !any_want && any_drop;
         }
@@ -593,7 +601,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
         if (!skip) {
 #pragma unroll ISSUE_UNROLL
           for (int kk = 0; kk < KK_M; ++kk) {
-            const uint32_t a_col = (kk < 4) ? kk * 8 : 96 + (kk - 4) * 8;
+            const uint32_t a_col = (kk >> 1) * 32 + (kk & 1) * 8;
             umma_ts_lead(lead, tmem_base + TMEM_DV, tmem_base + TMEM_S + a_col, umma_desc_at(do_mn, kk * 2048), idesc_dv,
                          (kk > 0 || acc_started) ? 1u : 0u);
           }
@@ -639,7 +647,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
         post_dq_job(0, 0, 2);
         umma_commit_lead(lead, &bars->dq_full);
       }
-    } else if (warp == 10) {
+    } else if (warp == W_DRAIN) {
       // =============================== dQ drain =================================================
       // Deterministic mode only (otherwise every dQ warp issues the reduce-adds of its own buffers, which
       // measured 3 % faster). Jobs arrive in order: a 64-column pair of chunks of a dQ tile staged by the four
@@ -709,9 +717,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
     }
   } else {
     // =============================== compute warps ===========================================
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 176;");
-    const int cw = warp;            // 0..7
-    const int wg = cw >> 2;         // which half of the query columns / output columns
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 80;");
+    const int cw = warp;            // 0..15
+    const int wg = cw >> 2;         // which quarter of the query columns / output columns
     const int wq = cw & 3;          // TMEM lane quadrant
     const int row = wq * 32 + lane; // key row (S^T, dP^T, dV, dK)
     const uint32_t lane_addr = uint32_t(wq * 32) << 16;
@@ -722,7 +730,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
     uint8_t* ds_buf = smem + SM::kDS;
 
     bool ok = !*abort_flag;
-    uint32_t pk[32];  // P^T of the step in flight, packed pairs (this thread's 64 query columns)
+    uint32_t pk[16];  // P^T of the step in flight, packed pairs (this thread's 32 query columns)
     int n_live = 0;
     bool skip_cur = false;
     int m_cur = 0, g_cur = 0;  // query tile / head of the step whose dS is being handled
@@ -814,9 +822,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
       m_p = m;
       // skip thresholds of the group's first and last query column: worked out before S is waited for
       // (log2(clamp(threshold / visible, 0, 1)) = min(log2 threshold - log2 visible, 0); threshold <= 0 gives -inf)
-      const int q_first = m * TM + wg * 64;
+      const int q_first = m * TM + wg * 32;
       const float vis_first = causal ? float(q_first + off + 1) : float(sk);
-      const float vis_last = causal ? float(q_first + 63 + off + 1) : float(sk);
+      const float vis_last = causal ? float(q_first + 31 + off + 1) : float(sk);
       float thr_hi = 0.f, thr_lo = 0.f;
       if (KIND != KIND_DENSE) {
         thr_hi = fminf(lg_thr - lg2_approx(vis_first), 0.0f);
@@ -858,11 +866,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
         // logits = (q.k + g(alpha_q * delta_k)) * scale, g = logsigmoid or identity (flash_gated_bwd.py:81-98). A rolled
         // loop over 16 columns, through TMEM: unrolled over the row it does not stay in the instruction caches beside
         // the code of the other roles.
-        const uint4* al4 = reinterpret_cast<const uint4*>(s_alpha + st * 128 + wg * 64);
+        const uint4* al4 = reinterpret_cast<const uint4*>(s_alpha + st * 128 + wg * 32);
         const float2 dl2 = make_float2(dlt_g, dlt_g);  // delta, times log2(e) for the logsigmoid gate
-        const uint32_t tcol = tmem_base + lane_addr + TMEM_S + wg * 64;
+        const uint32_t tcol = tmem_base + lane_addr + TMEM_S + wg * 32;
 #pragma unroll 1
-        for (int qt = 0; qt < 4; ++qt) {
+        for (int qt = 0; qt < 2; ++qt) {
           uint32_t r[16];
           tmem_ld16(tcol + qt * 16, r);
           tmem_ld_wait();
@@ -885,19 +893,18 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
         }
         tmem_st_wait();
       }
-      uint32_t sr[64];
-      tmem_ld32(tmem_base + lane_addr + TMEM_S + wg * 64, &sr[0]);
-      tmem_ld32(tmem_base + lane_addr + TMEM_S + wg * 64 + 32, &sr[32]);
+      uint32_t sr[32];
+      tmem_ld32(tmem_base + lane_addr + TMEM_S + wg * 32, sr);
       tmem_ld_wait();
       const bool ragged = ((m + 1) * TM > sq) || ((n_block + 1) * TN > sk);
       const bool masked = (mode != FSA_MASK_NONE) || ragged;
       ColMask cm = {{0, 0, 0}, {0u, 0u, 0u}};
       if (masked) cm = col_mask(mode, m);  // 64-bit interval arithmetic: only for the tiles that need it
-      const float4* lse4 = reinterpret_cast<const float4*>(s_lse + st * 128 + wg * 64);
-      float x[64];  // log2 of the probabilities
+      const float4* lse4 = reinterpret_cast<const float4*>(s_lse + st * 128 + wg * 32);
+      float x[32];  // log2 of the probabilities
       const float2 c2 = make_float2(c, c);
 #pragma unroll
-      for (int i = 0; i < 64; i += 4) {
+      for (int i = 0; i < 32; i += 4) {
         const float4 l = lse4[i >> 2];  // minus lse2
         const float2 xa = fma2(make_float2(__uint_as_float(sr[i]), __uint_as_float(sr[i + 1])), c2, make_float2(l.x, l.y));
         const float2 xb =
@@ -920,27 +927,24 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
           oor_want = x_oor - fminf(lg_thr - lg2_approx(vis_oor), 0.0f) >= 0.0f;
         } else if (!row_ok) {
 #pragma unroll
-          for (int i = 0; i < 64; ++i) {
+          for (int i = 0; i < 32; ++i) {
             const float vis_i = causal ? float(q_first + i + off + 1) : float(sk);
             oor_want |= (x[i] - fminf(lg_thr - lg2_approx(vis_i), 0.0f) >= 0.0f);
           }
         }
       }
       if (masked) {
+        const int base = wg * 32;  // one test of a bit per entry, whatever the mask is made of
+        const uint32_t bits = interval_bits(cm.lo[0], cm.len[0], base) | interval_bits(cm.lo[1], cm.len[1], base) |
+                              interval_bits(cm.lo[2], cm.len[2], base);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {  // one test of a bit per entry, whatever the mask is made of
-          const int base = wg * 64 + h * 32;
-          const uint32_t bits = interval_bits(cm.lo[0], cm.len[0], base) | interval_bits(cm.lo[1], cm.len[1], base) |
-                                interval_bits(cm.lo[2], cm.len[2], base);
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (!(bits & (1u << i))) x[h * 32 + i] = -INFINITY;
-        }
+        for (int i = 0; i < 32; ++i)
+          if (!(bits & (1u << i))) x[i] = -INFINITY;
       }
       bool skip = false;
       if (KIND != KIND_DENSE) {
         // skip iff max over the tile of (log2 p - thr_log2[q]) < 0 (flash_sparse_bwd.py:61-79);
-        // thresholds of this group's 64 query columns live two per lane and travel by shuffle
+        // thresholds of this group's 32 query columns live one per lane and travel by shuffle
         // The threshold falls as the query index grows (causal) or is one number (otherwise): the row
         // maximum against the thresholds of the group's first and last column settles most votes at
         // once; only a warp with a lane in between compares entry by entry.
@@ -957,23 +961,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
         const float mx_first = chain16(0);
         bool want = mx_first >= thr_hi, drop = false;
         if (exact_only || !__any_sync(0xffffffffu, want)) {
-          const float mx = fmaxf(fmaxf(mx_first, chain16(1)), fmaxf(chain16(2), chain16(3)));
+          const float mx = fmaxf(mx_first, chain16(1));
           want = mx >= thr_hi;
           drop = mx < thr_lo;
           const bool unsure = exact_only || (!want && !drop);
           // once a lane of this warp is sure that it wants the tile, the lanes in between do not matter any more
           const bool settled = !exact_only && __any_sync(0xffffffffu, want);
           if (!settled && __any_sync(0xffffffffu, unsure)) {
-            const int q_a = q_first + lane, q_b = q_a + 32;
-            const float vis_a = causal ? float(q_a + off + 1) : float(sk);
-            const float vis_b = causal ? float(q_b + off + 1) : float(sk);
-            const float thr_a = fminf(lg_thr - lg2_approx(vis_a), 0.0f);
-            const float thr_b = fminf(lg_thr - lg2_approx(vis_b), 0.0f);
+            const float vis_l = causal ? float(q_first + lane + off + 1) : float(sk);
+            const float thr_l = fminf(lg_thr - lg2_approx(vis_l), 0.0f);
             want = false;
             drop = false;
 #pragma unroll
-            for (int i = 0; i < 64; ++i) {
-              const float t = __shfl_sync(0xffffffffu, i < 32 ? thr_a : thr_b, i & 31);
+            for (int i = 0; i < 32; ++i) {
+              const float t = __shfl_sync(0xffffffffu, thr_l, i);
               const float v = x[i] - t;
               want |= (v >= 0.0f);
               drop |= (v < 0.0f);
@@ -994,15 +995,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
         // A warp with an entry that wants the tile knows the outcome ("keep") and moves on; only warps whose
         // entries all vote "skip" wait for the others. Every warp arrives once per step, and none reaches the vote
         // of the step after next (same slot) before all have arrived here: S of the next step is only issued
-        // after all eight warps published P or the skip.
+        // after all compute warps published P or the skip.
         if (!w_any) {
           if (!mbar_wait(&bars->vote_sync, par, abort_flag)) {
             ok = false;
             return true;
           }
-          int v = 0;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) v |= bars->vote_any[par][i];
+          const uint4 vv = *reinterpret_cast<const uint4*>(&bars->vote_any[par][0]);
+          uint32_t v = vv.x | vv.y | vv.z | vv.w;
+          v |= v >> 16;
+          v |= v >> 8;
           skip = !(v & 1) && (v & 2);
         }
         if (cw == 0 && lane == 0) {
@@ -1015,10 +1017,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
       }
       if (!skip) {
 #pragma unroll
-        for (int i = 0; i < 64; i += 2) pk[i >> 1] = pack2<T>(ex2_approx(x[i]), ex2_approx(x[i + 1]));
-        const uint32_t pcol = (wg == 0) ? 0u : 96u;
-        tmem_st16(tmem_base + lane_addr + TMEM_S + pcol, &pk[0]);
-        tmem_st16(tmem_base + lane_addr + TMEM_S + pcol + 16, &pk[16]);
+        for (int i = 0; i < 32; i += 2) pk[i >> 1] = pack2<T>(ex2_approx(x[i]), ex2_approx(x[i + 1]));
+        tmem_st16(tmem_base + lane_addr + TMEM_S + wg * 32, pk);
         tmem_st_wait();
       }
       tc_fence_before();
@@ -1035,16 +1035,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
         return;
       }
       tc_fence_after();
-      uint32_t dr[64];
-      tmem_ld32(tmem_base + lane_addr + TMEM_DP + wg * 64, &dr[0]);
-      tmem_ld32(tmem_base + lane_addr + TMEM_DP + wg * 64 + 32, &dr[32]);
+      uint32_t dr[32];
+      tmem_ld32(tmem_base + lane_addr + TMEM_DP + wg * 32, dr);
       tmem_ld_wait();
-      const float4* dps4 = reinterpret_cast<const float4*>(s_dps + st * 128 + wg * 64);
-      const uint4* al4 = reinterpret_cast<const uint4*>(s_alpha + st * 128 + wg * 64);
-      uint8_t* slab = ds_buf + wg * (128 * 128);
-      float da_r[8];  // gated: per chunk, one column's dalpha summed over 8 lanes
+      const float4* dps4 = reinterpret_cast<const float4*>(s_dps + st * 128 + wg * 32);
+      const uint4* al4 = reinterpret_cast<const uint4*>(s_alpha + st * 128 + wg * 32);
+      uint8_t* slab = ds_buf + (wg >> 1) * (128 * 128);
+      float da_r[4];  // gated: per chunk, one column's dalpha summed over 8 lanes
 #pragma unroll
-      for (int ch = 0; ch < 8; ++ch) {
+      for (int ch = 0; ch < 4; ++ch) {
         const float4 d0 = dps4[ch * 2], d1 = dps4[ch * 2 + 1];  // minus dpsum
         const float nd[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
         uint32_t o[4];
@@ -1057,7 +1056,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
                                 make_float2(nd[j], nd[j + 1]));
           o[j >> 1] = hmul2<T>(pk[(ch * 8 + j) >> 1], pack2_sat<T>(t.x, t.y));
         }
-        *reinterpret_cast<uint4*>(slab + sw128_offset(row, ch)) = make_uint4(o[0], o[1], o[2], o[3]);
+        *reinterpret_cast<uint4*>(slab + sw128_offset(row, (wg & 1) * 4 + ch)) = make_uint4(o[0], o[1], o[2], o[3]);
         if (KIND == KIND_GATED) {
           // dalpha[q] += sum_k dS g'(alpha_q delta_k) delta_k, ddelta[k] += sum_q dS g'(alpha_q delta_k) alpha_q,
           // g' = sigmoid(-x) for the logsigmoid gate, 1 for the identity (flash_gated_bwd.py:84-88, :152-160)
@@ -1091,21 +1090,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
         }
       }
       if (KIND == KIND_GATED) {
-        // two more steps fold the 8 chunks onto lane bits 1, 0: each lane ends with two complete column sums
+        // two more steps fold the 4 chunks onto lane bits 1, 0: each lane ends with one complete column sum
         const bool b1 = lane & 2, b0 = lane & 1;
-        float u[4], z[2];
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          u[j] = (b1 ? da_r[j + 4] : da_r[j]) + __shfl_xor_sync(0xffffffffu, b1 ? da_r[j] : da_r[j + 4], 2);
+        float u[2];
 #pragma unroll
         for (int j = 0; j < 2; ++j)
-          z[j] = (b0 ? u[j + 2] : u[j]) + __shfl_xor_sync(0xffffffffu, b0 ? u[j] : u[j + 2], 1);
+          u[j] = (b1 ? da_r[j + 2] : da_r[j]) + __shfl_xor_sync(0xffffffffu, b1 ? da_r[j] : da_r[j + 2], 2);
+        const float z = (b0 ? u[1] : u[0]) + __shfl_xor_sync(0xffffffffu, b0 ? u[0] : u[1], 1);
         const int g = g_cur, m = m_cur;
-        const int chunk0 = (b1 ? 4 : 0) + (b0 ? 2 : 0);
+        const int chunk = (b1 ? 2 : 0) + (b0 ? 1 : 0);
         const int cin = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
-        float* dst = p.da_accum + (long long)(hkv * p.G + g) * p.ws_sh + pad_off + (long long)m * TM + wg * 64 + cin;
-        atomicAdd(dst + chunk0 * 8, z[0]);
-        atomicAdd(dst + (chunk0 + 1) * 8, z[1]);
+        atomicAdd(p.da_accum + (long long)(hkv * p.G + g) * p.ws_sh + pad_off + (long long)m * TM + wg * 32 + chunk * 8 + cin, z);
       }
       fence_proxy_async_smem();
       tc_fence_before();
@@ -1156,36 +1151,36 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
           const float mul = which == 0 ? 1.0f : p.softmax_scale;
           void* outp = which == 0 ? p.dv_out : p.dk_out;
           const long long base = (long long)((p.flags & F_VARLEN_K) ? 0 : b) * p.dkv_sb + rowk * p.dkv_sn +
-                                 (long long)hkv * p.dkv_sh + (long long)split * p.dkv_ss + wg * HALF;
+                                 (long long)hkv * p.dkv_sh + (long long)split * p.dkv_ss + wg * PART;
 #pragma unroll
-          for (int ch = 0; ch < HALF / 32; ++ch) {
-            uint32_t r[32];
+          for (int ch = 0; ch < PART / 16; ++ch) {
+            uint32_t r[16];
             if (have) {
-              tmem_ld32(tmem_base + lane_addr + tcol + wg * HALF + ch * 32, r);
+              tmem_ld16(tmem_base + lane_addr + tcol + wg * PART + ch * 16, r);
               tmem_ld_wait();
             } else {
 #pragma unroll
-              for (int i = 0; i < 32; ++i) r[i] = 0u;
+              for (int i = 0; i < 16; ++i) r[i] = 0u;
             }
             if (row_ok) {
               if (p.flags & F_SPLIT) {
-                float* dst = reinterpret_cast<float*>(outp) + base + ch * 32;
+                float* dst = reinterpret_cast<float*>(outp) + base + ch * 16;
 #pragma unroll
-                for (int i = 0; i < 32; i += 4)
-                  if (wg * HALF + ch * 32 + i < p.D)
+                for (int i = 0; i < 16; i += 4)
+                  if (wg * PART + ch * 16 + i < p.D)
                     *reinterpret_cast<float4*>(dst + i) =
                         make_float4(__uint_as_float(r[i]) * mul, __uint_as_float(r[i + 1]) * mul,
                                     __uint_as_float(r[i + 2]) * mul, __uint_as_float(r[i + 3]) * mul);
               } else {
-                T* dst = reinterpret_cast<T*>(outp) + base + ch * 32;
+                T* dst = reinterpret_cast<T*>(outp) + base + ch * 16;
 #pragma unroll
-                for (int i = 0; i < 32; i += 8) {
+                for (int i = 0; i < 16; i += 8) {
                   uint4 v;
                   v.x = pack2<T>(__uint_as_float(r[i]) * mul, __uint_as_float(r[i + 1]) * mul);
                   v.y = pack2<T>(__uint_as_float(r[i + 2]) * mul, __uint_as_float(r[i + 3]) * mul);
                   v.z = pack2<T>(__uint_as_float(r[i + 4]) * mul, __uint_as_float(r[i + 5]) * mul);
                   v.w = pack2<T>(__uint_as_float(r[i + 6]) * mul, __uint_as_float(r[i + 7]) * mul);
-                  if (wg * HALF + ch * 32 + i < p.D) *reinterpret_cast<uint4*>(dst + i) = v;
+                  if (wg * PART + ch * 16 + i < p.D) *reinterpret_cast<uint4*>(dst + i) = v;
                 }
               }
             }
@@ -1193,17 +1188,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
         }
       }
     }
-    // ---- gated epilogue: ddelta of this key row = (columns 0-63) + (columns 64-127), scaled -------------
+    // ---- gated epilogue: ddelta of this key row = the sum over the four column groups, scaled -------------
     if (KIND == KIND_GATED && ok) {
       float* tmp = s_lse;  // every load of the ring has been consumed by now
-      if (wg == 1) {
-        tmp[row] = dd_acc.x + dd_acc.y;
+      if (wg > 0) {
+        tmp[(wg - 1) * 128 + row] = dd_acc.x + dd_acc.y;
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->dd_sync);
       } else {
         ok = mbar_wait(&bars->dd_sync, 0, abort_flag);
         if (ok && row_ok) {
-          const float val = (dd_acc.x + dd_acc.y + tmp[row]) * p.softmax_scale;
+          const float val = ((dd_acc.x + dd_acc.y + tmp[row]) + (tmp[128 + row] + tmp[256 + row])) * p.softmax_scale;
           const long long at = (long long)bk * p.d_sb + (long long)hkv * p.d_sh + off_k + k_idx;
           if (p.flags & F_SPLIT)
             reinterpret_cast<float*>(p.dd_out)[(long long)split * p.dd_ss + at] = val;
@@ -1218,7 +1213,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
   tc_fence_before();
   __syncthreads();
   if (tid == 0 && *abort_flag) atomicExch(p.status, 1);
-  if (warp == 8) {
+  if (warp == W_PROD) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
