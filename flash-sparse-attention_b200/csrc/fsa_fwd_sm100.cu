@@ -192,7 +192,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
   FwdBars* bars = reinterpret_cast<FwdBars*>(smem + SM::kBar);
   volatile int* abort_flag = &bars->abort_flag;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // (through a shuffle: the roles' branches are then known to be the same for the whole warp)
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const bool causal = p.flags & F_CAUSAL, local = p.flags & F_LOCAL, split_kv = p.flags & F_SPLIT;
 
   // ---- work decode: heads fastest (K/V reuse in L2), heavy query tiles first --------------------
@@ -538,20 +539,29 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
                                     : umma_idesc_f16(TM, TN, IS_BF16, false, false);
     constexpr uint32_t idesc_o = F8 ? umma_idesc_f8(TM, HD, F8_FMT, F8_FMT, false, true)
                                     : umma_idesc_f16(TM, HD, IS_BF16, false, true);
+    // What this warp branches on is made the same in all lanes in a way that the compiler sees, so that it keeps the MMAs'
+    // operands in uniform registers; TMEM starts at 0 because all of it is allocated. Sparse causal S = 16384 1859 -> 1830 us,
+    // a 1024-token window (B4 S8192) 1000 -> 970, but the 16-bit dense kind then spills around it (1764 -> 1793) and goes without.
+    constexpr bool UNIFORM = KIND != KIND_DENSE || F8;
+    auto wait_for = [](uint64_t* bar, uint32_t parity, volatile int* abort) {
+      return UNIFORM ? mbar_wait_uniform(bar, parity, abort) : mbar_wait(bar, parity, abort);
+    };
+    const uint32_t tm = UNIFORM ? 0u : tmem_base;
     const uint32_t sQ = smem_u32(smem + SM::kQ), sK = smem_u32(smem + SM::kK), sV = smem_u32(smem + SM::kV);
-    bool ok = !*abort_flag;
+    bool ok = UNIFORM ? (bool)__any_sync(0xffffffffu, !*abort_flag) : !*abort_flag;
     int cnt[2] = {0, 0}, cnt_kept[2] = {0, 0};
     bool o_started[2] = {false, false};
     bool act[2] = {false, false}, last[2];
     int n = -1;
     [[maybe_unused]] auto read_info = [&](int slot, int& n_t, unsigned& f) {
-      const unsigned long long w = *reinterpret_cast<const volatile unsigned long long*>(&bars->step_info[slot]);
+      unsigned long long w = *reinterpret_cast<const volatile unsigned long long*>(&bars->step_info[slot]);
+      if (UNIFORM) w = __shfl_sync(0xffffffffu, w, 0);
       n_t = (int)(unsigned)w;
       f = (unsigned)(w >> 32);
     };
     // Every lane runs the same (warp-uniform) descriptor arithmetic; the MMA and commit instructions carry the
     // one-lane predicate themselves.
-    const uint32_t lead = lane == 0 ? 1u : 0u;
+    const uint32_t lead = elect_one();
     const uint32_t dq_lo = umma_desc_lo(sQ, 16), dk_lo = umma_desc_lo(sK, 16), dv_lo = umma_desc_lo(sV, TN * 128);
     // The MMA loops are unrolled where this warp is the critical resource (dense and sparse kinds: rolled they cost
     // 9-14 %) and stay rolled for the gated kind, whose softmax warps carry the gate arithmetic (5 % faster rolled).
@@ -562,10 +572,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
       for (int kk = 0; kk < KK_QK; ++kk) {
         const uint32_t koff = (kk >> 2) * (TM * 128) + (kk & 3) * 32;
         if (F8)
-          umma_f8_ss_lead(lead, tmem_base + TMEM_S0 + q * 128, umma_desc_at(aq, koff), umma_desc_at(bk, koff), idesc_s,
+          umma_f8_ss_lead(lead, tm + TMEM_S0 + q * 128, umma_desc_at(aq, koff), umma_desc_at(bk, koff), idesc_s,
                           kk > 0);
         else
-          umma_ss_lead(lead, tmem_base + TMEM_S0 + q * 128, umma_desc_at(aq, koff), umma_desc_at(bk, koff), idesc_s,
+          umma_ss_lead(lead, tm + TMEM_S0 + q * 128, umma_desc_at(aq, koff), umma_desc_at(bk, koff), idesc_s,
                        kk > 0);
       }
       umma_commit_lead(lead, &bars->s_full[q]);
@@ -575,7 +585,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
 #pragma unroll
       for (int q = 0; q < 2; ++q) act[q] = n >= 0 && fsa_fwd_tile_mode(sched[q], n, causal, local) >= 0;
     }
-    if (ok) ok = mbar_wait(&bars->k0_full, 0, abort_flag);
+    if (ok) ok = wait_for(&bars->k0_full, 0, abort_flag);
     if constexpr (HANDED) {
       if (ok) {
         unsigned f;
@@ -585,7 +595,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
       }
     }
     if (n >= 0 && ok) {
-      ok = mbar_wait(&bars->q_full, 0, abort_flag);
+      ok = wait_for(&bars->q_full, 0, abort_flag);
       tc_fence_after();
       if (ok) {
         for (int q = 0; q < 2; ++q)
@@ -617,7 +627,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
           }
         }
       }
-      ok = mbar_wait(&bars->kv_full[t & 1], (t >> 1) & 1, abort_flag);  // V(t) and K(t + 1)
+      ok = wait_for(&bars->kv_full[t & 1], (t >> 1) & 1, abort_flag);  // V(t) and K(t + 1)
       if (!ok) break;
       if constexpr (HANDED) {
         unsigned f;
@@ -645,25 +655,26 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
         if (act[q]) {
-          ok = ok && mbar_wait(&bars->p_full[q], cnt[q] & 1, abort_flag);
+          ok = ok && wait_for(&bars->p_full[q], cnt[q] & 1, abort_flag);
           if (!ok) break;
-          const bool skip = (KIND != KIND_DENSE) && bars->skip_flag[q][cnt[q] & 1];
+          const bool skip = (KIND != KIND_DENSE) &&
+                            __any_sync(0xffffffffu, *reinterpret_cast<const volatile int*>(&bars->skip_flag[q][cnt[q] & 1]));
           cnt[q]++;
           tc_fence_after();
           if (!skip) {
 #pragma unroll ISSUE_UNROLL
             for (int kk = 0; kk < KK_PV; ++kk) {
               if (HALVES && kk == KK_PV / 2) {
-                ok = mbar_wait(&bars->p_rest[q], cnt_kept[q] & 1, abort_flag);  // only kept tiles arrive there
+                ok = wait_for(&bars->p_rest[q], cnt_kept[q] & 1, abort_flag);  // only kept tiles arrive there
                 if (!ok) break;
                 cnt_kept[q]++;
                 tc_fence_after();
               }
               if (F8)
-                umma_f8_ts_lead(lead, tmem_base + TMEM_O0 + q * 128, tmem_base + TMEM_S0 + q * 128 + kk * 8,
+                umma_f8_ts_lead(lead, tm + TMEM_O0 + q * 128, tm + TMEM_S0 + q * 128 + kk * 8,
                                 umma_desc_at(bv, kk * 4096), idesc_o, (kk > 0 || o_started[q]) ? 1u : 0u);
               else
-                umma_ts_lead(lead, tmem_base + TMEM_O0 + q * 128, tmem_base + TMEM_S0 + q * 128 + kk * 8,
+                umma_ts_lead(lead, tm + TMEM_O0 + q * 128, tm + TMEM_S0 + q * 128 + kk * 8,
                              umma_desc_at(bv, kk * 2048), idesc_o, (kk > 0 || o_started[q]) ? 1u : 0u);
             }
             o_started[q] = true;
@@ -957,14 +968,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
       // s_full for this tile was committed after the previous P V of this group, so O is at rest
       if (have_o && (__any_sync(0xffffffffu, need) || o_mul != 1.0f)) {
         const float o_scale = scale * o_mul;
-#pragma unroll
-        for (int ch = 0; ch < OCH; ++ch) {
-          uint32_t r[32];
-          tmem_ld32(tO + ch * 32, r);
+        // few columns at a time: with 32 registers here beside the scores, some of those are spilled
+#pragma unroll 1
+        for (int ch = 0; ch < HD / 16; ++ch) {
+          uint32_t r[16];
+          tmem_ld16(tO + ch * 16, r);
           tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * o_scale);
-          tmem_st32(tO + ch * 32, r);
+          for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * o_scale);
+          tmem_st16(tO + ch * 16, r);
         }
       }
 
