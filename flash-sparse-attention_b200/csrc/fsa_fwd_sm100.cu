@@ -72,6 +72,8 @@ struct OutType<__nv_fp8_e5m2> {
   using type = __nv_bfloat16;
 };
 
+constexpr int MAX_RANKED = FSA_FWD_MAX_RANKED;  // (query tile pair, sequence) items that a CTA ranks at most
+
 struct FwdBars {
   uint64_t q_full;
   uint64_t k0_full;     // first K tile
@@ -94,6 +96,7 @@ struct FwdBars {
 };
 
 static_assert(offsetof(FwdBars, dl) % 16 == 0 && sizeof(FwdBars) <= 2048, "FwdBars layout");
+static_assert(sizeof(FwdBars::dl) >= (MAX_RANKED + 1) * sizeof(int), "room for the items' ranks");
 
 struct SeqInfo {
   int b, split, head, hkv;  // head = query head, or kv head when packing GQA rows
@@ -203,10 +206,34 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
     int idx = blockIdx.x;
     si.head = idx % p.hgrid;
     idx /= p.hgrid;
-    const int bs = idx % (p.B * p.num_splits);
-    pair = p.num_pairs - 1 - idx / (p.B * p.num_splits);
-    si.b = bs / p.num_splits;
-    si.split = bs - si.b * p.num_splits;
+    si.split = idx % p.num_splits;
+    int item = idx / p.num_splits;  // (query tile pair, sequence), sequences fastest, last pair first
+    // Sequences of unequal length: the items in the order of their key tiles, most first, so that the longest CTAs are not
+    // among the last to start (four chunks of 500 queries at 2000 to 12 000 keys, 256 CTAs: 366 -> 280 us).
+    // Every CTA ranks the items itself: one thread an item works out its key tiles and counts the items in front of it.
+    if (p.flags & F_LONGEST_FIRST) {
+      int* tiles = reinterpret_cast<int*>(&bars->dl[0][0]);  // [items], then the item of this CTA; not in use yet
+      const int items = p.B * p.num_pairs;
+      int mine = 0;
+      if (tid < items) {
+        const int b = tid % p.B, pr = p.num_pairs - 1 - tid / p.B;
+        const int sq = (p.flags & F_USED_Q) ? p.used_q[b] : ((p.flags & F_VARLEN_Q) ? p.cu_q[b + 1] - p.cu_q[b] : p.sq);
+        const int sk = (p.flags & F_USED_K) ? p.used_k[b] : ((p.flags & F_VARLEN_K) ? p.cu_k[b + 1] - p.cu_k[b] : p.sk);
+        const int end = min((pr + 1) * QT * TM / p.gpack, sq);  // query rows of the pair end here
+        if (pr * QT * TM < sq * p.gpack) mine = 1 + fsa_cdiv(max(causal ? min(end + sk - sq, sk) : sk, 0), TN);
+        tiles[tid] = mine;
+      }
+      __syncthreads();
+      if (tid < items) {
+        int rank = 0;
+        for (int j = 0; j < items; ++j) rank += tiles[j] > mine || (tiles[j] == mine && j < tid);
+        if (rank == item) tiles[MAX_RANKED] = tid;
+      }
+      __syncthreads();
+      item = __shfl_sync(0xffffffffu, tiles[MAX_RANKED], 0);  // known to be uniform: kept out of the threads' registers
+    }
+    si.b = item % p.B;
+    pair = p.num_pairs - 1 - item / p.B;
     si.hkv = (p.flags & F_PACK_GQA) ? si.head : si.head / p.G;
     si.off_q = (p.flags & F_VARLEN_Q) ? p.cu_q[si.b] : 0;
     si.off_k = (p.flags & F_VARLEN_K) ? p.cu_k[si.b] : 0;

@@ -25,7 +25,10 @@ enum : unsigned {
   F_LSE_LOG2 = 1u << 12,   // store lse in base 2 (split partials), else natural log
   F_KV_RAGGED = 1u << 13,  // rows past the key length may hold foreign data: zero V tails in smem
   F_DETERMINISTIC = 1u << 14,  // backward: dQ contributions of the key tiles are added in a fixed order
+  F_LONGEST_FIRST = 1u << 15,  // forward: (query tile pair, sequence) items are started in the order of their key tiles
 };
+
+constexpr int FSA_FWD_MAX_RANKED = 128;  // F_LONGEST_FIRST: items that a CTA ranks at most
 
 enum { KIND_DENSE = 0, KIND_SPARSE = 1, KIND_GATED = 2 };
 enum { DT_BF16 = 0, DT_FP16 = 1, DT_E4M3 = 2, DT_E5M2 = 3, DT_F32 = 4 };
