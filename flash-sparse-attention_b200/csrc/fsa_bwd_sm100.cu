@@ -173,7 +173,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
   constexpr int KK_N = TN / 16;   // MMAs over the keys (dQ)
   constexpr int PART = HD / 4;    // output columns per compute group
   constexpr bool IS_BF16 = !__is_same(T, __half);
-  constexpr uint32_t TMEM_S = 0, TMEM_DP = 128, TMEM_DV = 256, TMEM_DK = 384;
+  // At head size 64 dV and dK leave room for a dQ block of its own; at 128 dQ takes the block of dP^T.
+  constexpr bool OWN_DQ = HD == 64;
+  constexpr uint32_t TMEM_S = 0, TMEM_DP = 128, TMEM_DV = 256, TMEM_DK = 384, TMEM_DQ = OWN_DQ ? 320 : TMEM_DP;
 
   extern __shared__ __align__(1024) uint8_t smem[];
   BwdBars* bars = reinterpret_cast<BwdBars*>(smem + SM::kBar);
@@ -349,7 +351,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
   const int bq = (p.flags & F_VARLEN_Q) ? 0 : b;
   const int bk = (p.flags & F_VARLEN_K) ? 0 : b;
 
-  // Register budget: 768 threads x 80 at launch = 512 x 80 + 128 x 96 + 128 x 64
+  // Register budget: 768 threads x 80 at launch = 512 x 72 + 128 x 144 + 128 x 48 where the dQ warps take a whole 128-wide tile
+  // at once, 512 x 80 + 128 x 96 + 128 x 64 elsewhere (the gated kind's compute warps need their 80: 72 spill 200 bytes).
+  constexpr bool WHOLE_DQ = KIND != KIND_GATED && HD == 128;
   if (warp >= W_DQ) {
     // =============================== dQ read-out ================================================
     // One warp per TMEM lane quadrant (32 query rows). Per dQ tile: 64 columns at a time leave TMEM for registers
@@ -357,13 +361,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
     // as soon as the last columns are in registers. The path from an SM to L2 moves about 21 bytes per clock, so
     // the 64 KB of a tile take about as long as the MMAs of a step: these warps pace themselves on the reads of
     // the staging buffers and nobody else waits for them.
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
+    if constexpr (WHOLE_DQ)
+      asm volatile("setmaxnreg.inc.sync.aligned.u32 144;");
+    else
+      asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
     const int wq = warp & 3;
     const uint32_t lane_addr = uint32_t(wq * 32) << 16;
     uint8_t* stage = smem + SM::kStage + wq * 8192;
     const bool det = p.flags & F_DETERMINISTIC;
     constexpr int NP = HD / 64;  // 64-column pairs of 32-column chunks per dQ tile
-    constexpr uint32_t TMEM_DQ = 128;
     bool ok = !*abort_flag;
     int jobs = 0;  // staging jobs handed to the drain warp so far (deterministic mode; same count in all four warps)
     // wait until the drain warp's TMA reads of the previous job have left the staging buffers
@@ -405,17 +411,25 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
         continue;
       }
       tc_fence_after();
+      // The whole tile at once where the registers are there (WHOLE_DQ): the block is free again one TMEM load after the MMAs. With
+      // 64 columns at a time the second load waits for the first columns' way through shared memory, 1400 cycles in all, and
+      // dP^T of the next step waits with it (dense causal S = 8192, 32 heads: 1351 -> 1269 us, sparse 1367 -> 1333, packed 2072 -> 2047).
+      constexpr int NR = WHOLE_DQ ? HD : 64;  // columns in registers
+      uint32_t r[NR];
+      auto load_cols = [&](int first, bool last) {
 #pragma unroll
-      for (int cp = 0; cp < NP; ++cp) {
-        uint32_t r[64];
-        tmem_ld32(tmem_base + lane_addr + TMEM_DQ + cp * 64, &r[0]);
-        tmem_ld32(tmem_base + lane_addr + TMEM_DQ + cp * 64 + 32, &r[32]);
+        for (int ch = 0; ch < NR / 32; ++ch) tmem_ld32(tmem_base + lane_addr + TMEM_DQ + first + ch * 32, &r[ch * 32]);
         tmem_ld_wait();
-        if (cp == NP - 1) {  // all of this warp's dQ values are in registers: the TMEM block may be overwritten
+        if (last) {  // all of this warp's dQ values are in registers: the TMEM block may be overwritten
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&bars->dq_empty);
         }
+      };
+      if (WHOLE_DQ) load_cols(0, true);
+#pragma unroll
+      for (int cp = 0; cp < NP; ++cp) {
+        if (!WHOLE_DQ) load_cols(cp * 64, cp == NP - 1);
         if (det) {
           stage_wait_free();
           if (!ok) break;
@@ -423,8 +437,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
           if (lane == 0) bulk_wait_read0();  // the engine has read the previous contents of both buffers
           __syncwarp();
         }
-        stage_store(stage, &r[0]);
-        stage_store(stage + 4096, &r[32]);
+        stage_store(stage, &r[WHOLE_DQ ? cp * 64 : 0]);
+        stage_store(stage + 4096, &r[(WHOLE_DQ ? cp * 64 : 0) + 32]);
         fence_proxy_async_smem();
         __syncwarp();
         if (det) {
@@ -443,7 +457,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
     if (lane == 0) bulk_wait0();
     __syncwarp();
   } else if (warp >= W_PROD) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    if constexpr (WHOLE_DQ)
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+    else
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
     if (warp == W_PROD) {
       // =============================== producer ==============================================
       if (lane == 0 && !*abort_flag) {
@@ -574,7 +591,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
         ok = mbar_wait(&bars->do_full, it & 1, abort_flag);  // every phase is observed, skipped step or not
         if (!ok) break;
         tc_fence_after();
-        if (!skip || det) {
+        if ((!OWN_DQ && !skip) || (skip && det)) {
           // the dQ warps have read the previous tile out of the block that dP^T is about to overwrite (and both
           // descriptor slots are free again)
           if (n_jobs > 0) ok = mbar_wait(&bars->dq_empty, (n_jobs - 1) & 1, abort_flag);
@@ -587,7 +604,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
           n_jobs++;
         }
         if (!skip) {
-          post_dq_job(g_cur, m_cur, 0);
+          if (!OWN_DQ) post_dq_job(g_cur, m_cur, 0);
 #pragma unroll ISSUE_UNROLL
           for (int kk = 0; kk < KK_D; ++kk) {
             const uint32_t koff = (kk >> 2) * (128 * 128) + (kk & 3) * 32;
@@ -621,10 +638,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
           ok = mbar_wait(&bars->ds_full, n_live & 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
+          if (OWN_DQ) {  // the previous tile has left the dQ block
+            if (n_jobs > 0) ok = mbar_wait(&bars->dq_empty, (n_jobs - 1) & 1, abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+            post_dq_job(g_cur, m_cur, 0);
+          }
           // dQ first: its tile has to leave TMEM before dP^T of the next step can be issued
 #pragma unroll ISSUE_UNROLL
           for (int kk = 0; kk < KK_N; ++kk)
-            umma_ss_lead(lead, tmem_base + TMEM_DP, umma_desc_at(ds_mn, kk * 2048), umma_desc_at(k_mn, kk * 2048), idesc_dq,
+            umma_ss_lead(lead, tmem_base + TMEM_DQ, umma_desc_at(ds_mn, kk * 2048), umma_desc_at(k_mn, kk * 2048), idesc_dq,
                          kk > 0);
           umma_commit_lead(lead, &bars->dq_full);
           const uint32_t q_mn = q_mn0 + st * Q_STAGE;
@@ -717,7 +740,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
     }
   } else {
     // =============================== compute warps ===========================================
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 80;");
+    if constexpr (WHOLE_DQ)
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    else
+      asm volatile("setmaxnreg.inc.sync.aligned.u32 80;");
     const int cw = warp;            // 0..15
     const int wg = cw >> 2;         // which quarter of the query columns / output columns
     const int wq = cw & 3;          // TMEM lane quadrant
