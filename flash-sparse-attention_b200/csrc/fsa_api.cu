@@ -366,7 +366,8 @@ int fsa_fwd(const FsaFwdArgs* a, void* stream_) {
   if (a->flags & FSA_F_LOGSIGMOID) f |= fsa::F_LOGSIGMOID;
   if (a->flags & FSA_F_ADAPT_GATE) f |= fsa::F_ADAPT_GATE;
   // Lengths that only the device knows may be very unequal: with more CTAs than the GPU holds at a time (one an SM), the longest
-  // go first. Windows make them nearly equal. Ranking costs a CTA about 0.3 us at 128 items, so not beyond those.
+  // go first. Windows make their work nearly equal. A CTA compares every item with
+  // every other one, so there is a limit to the items; the order without ranks (last query tiles first) serves the rest.
   const long long items = (long long)p.B * p.num_pairs;
   if ((varlen_q || varlen_k || a->seqused_q || a->seqused_k) && !(f & fsa::F_LOCAL) && p.B > 1 && items <= fsa::FSA_FWD_MAX_RANKED &&
       items * hgrid * ns > fsa::device_sm_count())

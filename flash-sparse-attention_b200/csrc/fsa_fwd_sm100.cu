@@ -209,7 +209,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
     si.split = idx % p.num_splits;
     int item = idx / p.num_splits;  // (query tile pair, sequence), sequences fastest, last pair first
     // Sequences of unequal length: the items in the order of their key tiles, most first, so that the longest CTAs are not
-    // among the last to start (four chunks of 500 queries at 2000 to 12 000 keys, 256 CTAs: 366 -> 280 us).
+    // among the last to start (four chunks of 500 queries at 2000 to 12 000 keys, 256 CTAs: 366 -> 280 us,
+    // 257 with the elected MMA lane).
     // Every CTA ranks the items itself: one thread an item works out its key tiles and counts the items in front of it.
     if (p.flags & F_LONGEST_FIRST) {
       int* tiles = reinterpret_cast<int*>(&bars->dl[0][0]);  // [items], then the item of this CTA; not in use yet
