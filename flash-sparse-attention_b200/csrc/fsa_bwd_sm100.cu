@@ -551,9 +551,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
       bool has_cur = ok && walk_next(wk, g_nxt, m_nxt, mode_unused, first_unused, false);  // whether there is any step
       const bool det = p.flags & F_DETERMINISTIC;
       int n_jobs = 0;  // dQ tiles (and, deterministic mode, passes) handed to the dQ warps so far
-      // descriptor of the dQ tile the next commit on dq_full announces; written well before the MMAs it follows
+      // descriptor of the dQ tile the next commit on dq_full announces: written by the lane that commits, whose program order
+      // puts it first (nothing says that the elected lane is lane 0)
       auto post_dq_job = [&](int g, int m, int code) {
-        if (lane == 0) {
+        if (lead) {
           asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(smem_u32(bars->dqjob[n_jobs & 1])),
                        "r"((int)(pad_off + (long long)m * TM)), "r"(hkv * p.G + g), "r"(m), "r"(code)
                        : "memory");

@@ -1,0 +1,35 @@
+"""Which lane of the MMA issuer does what. PTX does not say which lane ``elect.sync`` picks, so what one lane writes for a later
+commit to announce has to be written by the lane that commits: only then program order puts the write first. A mistake here is a
+race on shared memory that a GPU run shows by chance at best, so the source is what is looked at."""
+
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "flash-sparse-attention_b200", "csrc")
+
+
+def _code(name):
+    """The file's text without its comments."""
+    with open(os.path.join(CSRC, name)) as f:
+        return re.sub(r"//[^\n]*|/\*.*?\*/", "", f.read(), flags=re.S)
+
+
+def _rest_of_block(text, at):
+    """From `at` to the end of the innermost block around it."""
+    depth = 0
+    for i in range(at, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        if depth < 0:
+            return text[at:i]
+    raise AssertionError("unbalanced braces")
+
+
+@pytest.mark.parametrize("name", ["fsa_fwd_sm100.cu", "fsa_bwd_sm100.cu"])
+def test_issuer_works_through_its_elected_lane(name):
+    text = _code(name)
+    roles = [_rest_of_block(text, m.start()) for m in re.finditer(r"lead\s*=\s*elect_one\(\)", text)]
+    assert roles and all("umma_commit_lead(lead" in r for r in roles)
+    for role in roles:
+        assert not re.search(r"\blane\s*==", role), "a fixed lane does part of the elected lane's work"
