@@ -67,12 +67,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return false;
 }
 
-// The same for a converged warp, with a result that the compiler knows to be the same in all lanes.
+// The same for a converged warp, with a result that the compiler knows to be the same in all lanes. It waits until every lane has
+// seen the phase: a vote orders no memory, so a lane has acquired only what its own test saw. The phase stays until all have,
+// since the next one needs this warp.
 __device__ __forceinline__ bool mbar_wait_uniform(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  if (__any_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   const long long t0 = clock64();
   for (uint32_t i = 0;; ++i) {
-    if (__any_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
     if ((i & 63u) == 63u) {
       if (__any_sync(0xffffffffu, *abort_flag)) return false;
       if (__any_sync(0xffffffffu, clock64() - t0 > FSA_WAIT_CYCLES)) break;

@@ -33,3 +33,11 @@ def test_issuer_works_through_its_elected_lane(name):
     assert roles and all("umma_commit_lead(lead" in r for r in roles)
     for role in roles:
         assert not re.search(r"\blane\s*==", role), "a fixed lane does part of the elected lane's work"
+
+
+def test_a_warp_waits_until_every_lane_has_seen_the_phase():
+    # A lane acquires what a barrier announces by its own test of the phase; a vote carries the news to the other lanes, but orders
+    # no memory for them. "Any lane" would let the elected lane run ahead of its own acquire.
+    votes = [(name, m.group(0)) for name in sorted(os.listdir(CSRC))
+             for m in re.finditer(r"__(any|all|ballot)_sync\([^;]*mbar_\w*wait", _code(name))]
+    assert votes and all(v.startswith("__all_sync") for _, v in votes), votes
