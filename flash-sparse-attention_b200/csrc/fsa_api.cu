@@ -365,12 +365,8 @@ int fsa_fwd(const FsaFwdArgs* a, void* stream_) {
   if (varlen_k || paged || a->seqused_k) f |= fsa::F_KV_RAGGED;
   if (a->flags & FSA_F_LOGSIGMOID) f |= fsa::F_LOGSIGMOID;
   if (a->flags & FSA_F_ADAPT_GATE) f |= fsa::F_ADAPT_GATE;
-  // Lengths that only the device knows may be very unequal: with more CTAs than the GPU holds at a time (one an SM), the longest
-  // go first. Windows make their work nearly equal. A CTA compares every item with
-  // every other one, so there is a limit to the items; the order without ranks (last query tiles first) serves the rest.
-  const long long items = (long long)p.B * p.num_pairs;
-  if ((varlen_q || varlen_k || a->seqused_q || a->seqused_k) && !(f & fsa::F_LOCAL) && p.B > 1 && items <= fsa::FSA_FWD_MAX_RANKED &&
-      items * hgrid * ns > fsa::device_sm_count())
+  if ((varlen_q || varlen_k || a->seqused_q || a->seqused_k) &&
+      fsa_fwd_longest_first(f & fsa::F_CAUSAL, f & fsa::F_LOCAL, p.B, p.num_pairs, ns, hgrid, p.sq, p.sk, fsa::device_sm_count()))
     f |= fsa::F_LONGEST_FIRST;
   p.flags = f;
 

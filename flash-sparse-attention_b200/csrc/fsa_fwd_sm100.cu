@@ -206,15 +206,18 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
     int idx = blockIdx.x;
     si.head = idx % p.hgrid;
     idx /= p.hgrid;
-    si.split = idx % p.num_splits;
-    int item = idx / p.num_splits;  // (query tile pair, sequence), sequences fastest, last pair first
+    const int bs = idx % (p.B * p.num_splits);
+    pair = p.num_pairs - 1 - idx / (p.B * p.num_splits);
+    si.b = bs / p.num_splits;
+    si.split = bs - si.b * p.num_splits;
     // Sequences of unequal length: the items in the order of their key tiles, most first, so that the longest CTAs are not
-    // among the last to start (four chunks of 500 queries at 2000 to 12 000 keys, 256 CTAs: 366 -> 280 us,
-    // 257 with the elected MMA lane).
-    // Every CTA ranks the items itself: one thread an item works out its key tiles and counts the items in front of it.
+    // among the last to start (fsa_fwd_longest_first says when: four chunks of 500 queries at 2000 to 12 000 keys, 256 CTAs, 329 -> 245 us).
+    // Every CTA ranks the items itself: one thread an item works out its key tiles and counts the items in front of it. (What is
+    // decoded above stands unless they are ranked: decoding by way of the item cost CTAs of one key tile 1 %.)
     if (p.flags & F_LONGEST_FIRST) {
       int* tiles = reinterpret_cast<int*>(&bars->dl[0][0]);  // [items], then the item of this CTA; not in use yet
       const int items = p.B * p.num_pairs;
+      int item = idx / p.num_splits;  // (query tile pair, sequence), sequences fastest, last pair first
       int mine = 0;
       if (tid < items) {
         const int b = tid % p.B, pr = p.num_pairs - 1 - tid / p.B;
@@ -232,9 +235,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
       }
       __syncthreads();
       item = __shfl_sync(0xffffffffu, tiles[MAX_RANKED], 0);  // known to be uniform: kept out of the threads' registers
+      si.b = item % p.B;
+      pair = p.num_pairs - 1 - item / p.B;
     }
-    si.b = item % p.B;
-    pair = p.num_pairs - 1 - item / p.B;
     si.hkv = (p.flags & F_PACK_GQA) ? si.head : si.head / p.G;
     si.off_q = (p.flags & F_VARLEN_Q) ? p.cu_q[si.b] : 0;
     si.off_k = (p.flags & F_VARLEN_K) ? p.cu_k[si.b] : 0;

@@ -28,8 +28,6 @@ enum : unsigned {
   F_LONGEST_FIRST = 1u << 15,  // forward: (query tile pair, sequence) items are started in the order of their key tiles
 };
 
-constexpr int FSA_FWD_MAX_RANKED = 128;  // F_LONGEST_FIRST: items that a CTA ranks at most
-
 enum { KIND_DENSE = 0, KIND_SPARSE = 1, KIND_GATED = 2 };
 enum { DT_BF16 = 0, DT_FP16 = 1, DT_E4M3 = 2, DT_E5M2 = 3, DT_F32 = 4 };
 

@@ -16,28 +16,79 @@ def _randn(*shape, seed):
     return torch.randn(*shape, generator=g, device=DEV, dtype=torch.bfloat16)
 
 
-# (lengths, query heads, KV heads): two to 128 items are ranked (a pair of 128-row query tiles of a sequence is an item), 129 are
-# not; ties, empty sequences and lengths at the edges of tiles
+def _cu(lens):
+    return torch.tensor([0] + list(lens), dtype=torch.int32).cumsum(0).to(torch.int32).to(DEV)
+
+
+# (lengths, query heads, KV heads): packed self-attention, at both sides of every limit of the ranking; "ragged" is ranked without
+# the causal mask. Ties, empty sequences and lengths at the edges of tiles
 @pytest.mark.parametrize("lens, hq, hkv", [
     ([1, 700, 0, 256, 257, 511, 512, 30], 16, 4),
     ([300] * 9, 32, 8),
-    ([128 + 7 * i for i in range(64)], 8, 2),    # up to 569 rows: 3 pairs x 64, not ranked
-    ([129 + i for i in range(128)], 4, 2),       # 1 pair x 128: the most that is ranked
-    ([129 + i for i in range(129)], 4, 2),       # one more: not ranked
+    ([128 + 7 * i for i in range(64)], 8, 2),
+    ([129 + i for i in range(128)], 4, 2),
+    ([129 + i for i in range(129)], 4, 2),
 ], ids=["ragged", "equal", "many", "limit", "past_limit"])
 @pytest.mark.parametrize("causal", [True, False])
 def test_packed_batch_equals_its_sequences(lens, hq, hkv, causal):
     total = sum(lens)
     q, k, v = _randn(total, hq, 64, seed=1), _randn(total, hkv, 64, seed=2), _randn(total, hkv, 64, seed=3)
-    cu = torch.tensor([0] + lens, dtype=torch.int32).cumsum(0).to(torch.int32).to(DEV)
+    cu = _cu(lens)
     out = fsa.flash_dense_attn_varlen_func(q, k, v, cu, cu, max(lens), max(lens), is_causal=causal)
     at = 0
-    for n in lens[:12]:
+    for n in lens:
         if n:
             s = slice(at, at + n)
             alone = fsa.flash_dense_attn_func(q[None, s], k[None, s], v[None, s], is_causal=causal)
             assert torch.equal(out[s], alone[0])
         at += n
+    fsa.check_status()
+
+
+Q_LENS = [300, 17, 129, 256, 257, 1, 128, 200]
+K_LENS = [600, 2000, 129, 1300, 700, 1999, 128, 1024]
+
+
+# queries in front of whose own keys others lie, so the causal forms are ranked: every kind, the packed heads, the CTA of one query
+# tile (head sizes above 128), and as many items as a CTA ranks
+@pytest.mark.parametrize("form", ["dense", "sparse", "gated", "fp8", "pack_gqa", "sparse_wide", "gated_wide", "full", "most_items"])
+def test_longer_keys_equal_single_calls(form):
+    q_lens, k_lens, hq, hkv, d = Q_LENS, K_LENS, 16, 4, 64
+    kw = dict(is_causal=form != "full")
+    if form == "most_items":  # 128 sequences of one pair of query tiles each
+        q_lens, k_lens, hq, hkv = [1 + 2 * i for i in range(128)], [1 + 2 * i + (i * 1237) % 3840 for i in range(127)] + [4096], 4, 2
+    kind = "sparse" if form.startswith("sparse") else "gated" if form.startswith("gated") else "dense"
+    if form.endswith("wide"):
+        d = 192
+    kw.update(dict(pack_gqa=True) if form == "pack_gqa" else {})
+    q, k, v = _randn(sum(q_lens), hq, d, seed=1), _randn(sum(k_lens), hkv, d, seed=2), _randn(sum(k_lens), hkv, d, seed=3)
+    if form == "fp8":
+        d = 128
+        q, k, v = ((_randn(sum(n), h, d, seed=i) * 64).to(torch.float8_e4m3fn)
+                   for i, (n, h) in enumerate(((q_lens, hq), (k_lens, hkv), (k_lens, hkv))))
+        scale = torch.full((1,), 1.0 / 64, device=DEV)
+        kw.update(is_quant=True, query_scale=scale, key_scale=scale, value_scale=scale)
+    gate = [_randn(sum(q_lens), hq, seed=4), _randn(sum(k_lens), hkv, seed=5)] if kind == "gated" else []
+    batched, single = (getattr(fsa, f"flash_{kind}_attn_{x}") for x in ("varlen_func", "func"))
+    out = batched(q, k, v, *gate, _cu(q_lens), _cu(k_lens), max(q_lens), max(k_lens), **kw)
+    at_q = at_k = 0
+    for nq, nk in zip(q_lens, k_lens):
+        sq, sk = slice(at_q, at_q + nq), slice(at_k, at_k + nk)
+        alone = single(q[None, sq], k[None, sk], v[None, sk], *([gate[0][None, sq], gate[1][None, sk]] if gate else []), **kw)
+        assert torch.equal(out[sq], alone[0]), (nq, nk)
+        at_q, at_k = at_q + nq, at_k + nk
+    fsa.check_status()
+
+
+def test_used_queries_equal_single_calls():
+    hq, hkv, d, n = 16, 4, 128, len(Q_LENS)
+    q, k, v = (_randn(n, length, h, d, seed=i) for i, (length, h) in enumerate(((300, hq), (2000, hkv), (2000, hkv))))
+    used_q, used_k = (torch.tensor(x, dtype=torch.int32, device=DEV) for x in (Q_LENS, K_LENS))
+    out = fsa.flash_dense_attn_varlen_func(q.flatten(0, 1), k.flatten(0, 1), v.flatten(0, 1), _cu([300] * n), _cu([2000] * n), 300,
+                                           2000, is_causal=True, seqused_q=used_q, seqused_k=used_k).view(n, 300, hq, d)
+    for b, (nq, nk) in enumerate(zip(Q_LENS, K_LENS)):
+        alone = fsa.flash_dense_attn_func(q[b:b + 1, :nq], k[b:b + 1, :nk], v[b:b + 1, :nk], is_causal=True)
+        assert torch.equal(out[b, :nq], alone[0]), (nq, nk)
     fsa.check_status()
 
 
