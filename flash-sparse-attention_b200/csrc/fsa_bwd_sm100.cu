@@ -165,7 +165,8 @@ __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.comm
 __device__ __forceinline__ void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
-template <int HD, typename T, int KIND>
+// WHOLE_DQ: the dQ warps take a whole 128-wide tile out of TMEM at once (launch_bwd says where).
+template <int HD, typename T, int KIND, bool WHOLE_DQ>
 __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant__ BwdKernelParams p) {
   using SM = BwdSmem<HD>;
   constexpr int KK_D = HD / 16;   // MMAs over the head dimension (S^T, dP^T)
@@ -353,7 +354,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
 
   // Register budget: 768 threads x 80 at launch = 512 x 72 + 128 x 144 + 128 x 48 where the dQ warps take a whole 128-wide tile
   // at once, 512 x 80 + 128 x 96 + 128 x 64 elsewhere (the gated kind's compute warps need their 80: 72 spill 200 bytes).
-  constexpr bool WHOLE_DQ = KIND != KIND_GATED && HD == 128;
   if (warp >= W_DQ) {
     // =============================== dQ read-out ================================================
     // One warp per TMEM lane quadrant (32 query rows). Per dQ tile: 64 columns at a time leave TMEM for registers
@@ -1260,9 +1260,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
   }
 }
 
-template <int HD, typename T, int KIND>
+template <int HD, typename T, int KIND, bool WHOLE_DQ>
 cudaError_t launch_one(const BwdKernelParams& p, cudaStream_t stream) {
-  auto kern = bwd_kernel<HD, T, KIND>;
+  auto kern = bwd_kernel<HD, T, KIND, WHOLE_DQ>;
   constexpr int smem = BwdSmem<HD>::kTotal;
   static std::atomic<unsigned long long> opted_in{0};  // one bit per device: the attribute is per device
   if (cudaError_t e = smem_opt_in(kern, smem, opted_in); e != cudaSuccess) return e;
@@ -1272,15 +1272,25 @@ cudaError_t launch_one(const BwdKernelParams& p, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
+// The dense and sparse kinds take a dQ tile at once at head size 128, where it leaves the block that dP^T of the next step waits for. In
+// deterministic mode the turns set the pace, and 64 columns at a time are faster (S = 4096, 16 / 4 heads: dense 544 us at once,
+// 520 in halves, sparse 533 and 503, a 512-token window 107 and 94). A kernel of its own: as a branch it spills 48 bytes more.
+template <int HD, typename T, int KIND>
+cudaError_t launch_kind(const BwdKernelParams& p, cudaStream_t stream) {
+  if constexpr (HD == 128 && KIND != KIND_GATED)
+    if (!(p.flags & F_DETERMINISTIC)) return launch_one<HD, T, KIND, true>(p, stream);
+  return launch_one<HD, T, KIND, false>(p, stream);
+}
+
 }  // namespace
 
 
 cudaError_t launch_bwd(const BwdKernelParams& p, int kind, int dtype, int head_dim, cudaStream_t stream) {
-#define FSA_BWD_CASE(HD_, T_, DT_)                                               \
-  if (head_dim == HD_ && dtype == DT_) {                                         \
-    if (kind == KIND_DENSE) return launch_one<HD_, T_, KIND_DENSE>(p, stream);   \
-    if (kind == KIND_SPARSE) return launch_one<HD_, T_, KIND_SPARSE>(p, stream); \
-    if (kind == KIND_GATED) return launch_one<HD_, T_, KIND_GATED>(p, stream);   \
+#define FSA_BWD_CASE(HD_, T_, DT_)                                                \
+  if (head_dim == HD_ && dtype == DT_) {                                          \
+    if (kind == KIND_DENSE) return launch_kind<HD_, T_, KIND_DENSE>(p, stream);   \
+    if (kind == KIND_SPARSE) return launch_kind<HD_, T_, KIND_SPARSE>(p, stream); \
+    if (kind == KIND_GATED) return launch_kind<HD_, T_, KIND_GATED>(p, stream);   \
   }
   FSA_BWD_CASE(128, __nv_bfloat16, DT_BF16)
   FSA_BWD_CASE(128, __half, DT_FP16)

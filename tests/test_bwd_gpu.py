@@ -232,3 +232,31 @@ def test_deterministic_dq_varlen_and_skipped_tiles():
         # the eager oracle keeps the probability mass that the skipped tiles drop (threshold 1.0: up to
         # 1 / visible_len per row and tile), so the element-wise bound is the skip error, not rounding
         assert_close("det-varlen-" + name, a, r, rtol=5e-2, atol=5e-2, ew_rtol=5e-2, ew_atol=1e-1)
+
+
+@pytest.mark.parametrize("head_dim", [64, 128])  # 64: dQ has a TMEM block of its own, so live and skipped steps wait for it in other places
+@pytest.mark.parametrize("threshold", [1.0, -128.0])
+def test_deterministic_dq_with_and_without_skips(head_dim, threshold):
+    from flash_sparse_attn.ops.triton import flash_bwd, flash_fwd
+
+    fsa = _ops()
+    s, hq, hkv = 1300, 4, 2  # ragged last tiles
+    g = torch.Generator().manual_seed(9)
+    base = torch.randn(1, s, hkv, head_dim, generator=g)
+    q = (base.repeat_interleave(hq // hkv, dim=2) * 4 + torch.randn(1, s, hq, head_dim, generator=g) * 0.3).to(torch.bfloat16).to(DEV)
+    k = (base + torch.randn(1, s, hkv, head_dim, generator=g) * 0.1).to(torch.bfloat16).to(DEV)
+    v, do = (torch.randn(1, s, h, head_dim, generator=g).to(torch.bfloat16).to(DEV) for h in (hkv, hq))
+    kw = dict(is_causal=True, softmax_threshold=threshold)
+    out, lse, *_ = flash_fwd.attn_forward("sparse", q, k, v, **kw)
+    free = flash_bwd.attn_backward("sparse", q, k, v, out, do, lse, deterministic=False, **kw)
+    runs = []
+    for _ in range(2):
+        tmap = torch.zeros(flash_bwd.tile_map_numel(1, s, s, hq), dtype=torch.uint8, device=DEV)
+        runs.append(flash_bwd.attn_backward("sparse", q, k, v, out, do, lse, deterministic=True, tile_map=tmap, **kw))
+    torch.cuda.synchronize()
+    fsa.check_status()
+    assert (tmap == 1).any() and bool((tmap == 2).any()) == (threshold > 0)
+    for name, f, a, b in zip(("dq", "dk", "dv"), free, *runs):
+        assert torch.equal(a, b), name
+        # the same products in another order of fp32 sums, rounded once to 16 bits
+        assert_close(f"det-{head_dim}-{name}", a, f.cpu(), rtol=2**-7, atol=2**-7)
