@@ -1,13 +1,14 @@
 // Micro-benchmark behind the role layout of the backward kernel: how fast does one thread feed the tensor pipe with
 // the 40 tcgen05.mma (128 x 128 x 16, bf16) of one backward step, and what slows it down?
 //
-// One CTA per SM (148), 12 warps. Warp 8 lane 0 issues the MMAs of the step in the operand forms the kernel uses
+// One CTA per SM (148), 12 warps. One lane of warp 8 (lane 0, or the lane that elect.sync picks) issues the MMAs of the step in
+// the operand forms the kernel uses
 // (S^T / dP^T: both operands K-major; dV: A from TMEM, B MN-major; dQ: both MN-major; dK: A K-major, B MN-major),
 // five commits per step, zero-filled operands. Meanwhile other warps run one kind of "noise":
 //   memory kinds run on warps 1-7 and 9-11 (shared-memory stores / loads, TMEM loads, bulk copies into shared
 //   memory, bulk reduce-adds out of it); arithmetic kinds run on warps 0 and 4, the two warps that share the
 //   issuer's scheduler (warp id mod 4).
-// Prints cycles per MMA (64 = the pipe's rate for this shape).
+// Prints cycles per MMA for both lanes (64 = the pipe's rate for this shape).
 //
 // Build and run (sm_100a):
 //   nvcc -gencode arch=compute_100a,code=sm_100a -O3 -std=c++17 --expt-relaxed-constexpr \
@@ -29,6 +30,7 @@ const char* kNames[N_KINDS] = {"none", "st.shared (10 warps)", "ld.shared (10 wa
                                "packed FFMA2, 16 chains", "IMAD, 32 chains", "ex2 (MUFU), 32 chains",
                                "integer add / xor, 32 chains", "float max, 32 chains", "bf16 pack (cvt), 16 chains"};
 
+template <bool ELECTED>
 __global__ void __launch_bounds__(384) probe(int iters, int noise, uint8_t* gbuf, long long* out, int* err) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 6 * KT);
@@ -63,7 +65,7 @@ __global__ void __launch_bounds__(384) probe(int iters, int noise, uint8_t* gbuf
     constexpr uint32_t id_kk = umma_idesc_f16(128, 128, true, false, false);
     constexpr uint32_t id_km = umma_idesc_f16(128, 128, true, false, true);
     constexpr uint32_t id_mm = umma_idesc_f16(128, 128, true, true, true);
-    const uint32_t lead = lane == 0;
+    const uint32_t lead = ELECTED ? elect_one() : uint32_t(lane == 0);
     const uint32_t k_lo = umma_desc_lo(sK, 16), v_lo = umma_desc_lo(sV, 16), do_lo = umma_desc_lo(sDO, 16),
                    ds_lo = umma_desc_lo(sDS, 16), do_mn = umma_desc_lo(sDO, 128 * 128), ds_mn = umma_desc_lo(sDS, 128 * 128),
                    k_mn = umma_desc_lo(sK, 128 * 128), q_lo0 = umma_desc_lo(sQ, 16), q_mn0 = umma_desc_lo(sQ, 128 * 128);
@@ -198,6 +200,22 @@ __global__ void __launch_bounds__(384) probe(int iters, int noise, uint8_t* gbuf
 }
 }  // namespace
 
+// the slowest CTA's cycles per MMA, or -1
+double run(bool elected, int noise, uint8_t* gbuf, long long* out, int* err) {
+  const int iters = 2000;
+  auto kern = elected ? probe<true> : probe<false>;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+  for (int rep = 0; rep < 2; ++rep) {
+    kern<<<148, 384, SMEM>>>(iters, noise, gbuf, out, err);
+    if (cudaDeviceSynchronize() != cudaSuccess) return -1.0;
+  }
+  std::vector<long long> h(148);
+  cudaMemcpy(h.data(), out, 148 * 8, cudaMemcpyDeviceToHost);
+  long long mx = 0;
+  for (auto v : h) mx = v > mx ? v : mx;
+  return double(mx) / (iters * 40.0);
+}
+
 int main() {
   long long* out;
   int* err;
@@ -207,21 +225,14 @@ int main() {
   cudaMalloc(&gbuf, 1024 * 16384);
   cudaMemset(err, 0, 4);
   cudaMemset(gbuf, 0, 1024 * 16384);
-  cudaFuncSetAttribute(probe, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-  const int iters = 2000;
+  printf("%-34s %8s %8s  (cycles per MMA)\n", "noise on the other warps", "lane 0", "elected");
   for (int noise = 0; noise < N_KINDS; ++noise) {
-    for (int rep = 0; rep < 2; ++rep) {
-      probe<<<148, 384, SMEM>>>(iters, noise, gbuf, out, err);
-      if (cudaDeviceSynchronize() != cudaSuccess) {
-        printf("launch failed\n");
-        return 1;
-      }
+    const double lane0 = run(false, noise, gbuf, out, err), elected = run(true, noise, gbuf, out, err);
+    if (lane0 < 0 || elected < 0) {
+      printf("launch failed\n");
+      return 1;
     }
-    std::vector<long long> h(148);
-    cudaMemcpy(h.data(), out, 148 * 8, cudaMemcpyDeviceToHost);
-    long long mx = 0;
-    for (auto v : h) mx = v > mx ? v : mx;
-    printf("%-34s %6.1f cycles per MMA\n", kNames[noise], double(mx) / (iters * 40.0));
+    printf("%-34s %8.1f %8.1f\n", kNames[noise], lane0, elected);
   }
   int herr = 0;
   cudaMemcpy(&herr, err, 4, cudaMemcpyDeviceToHost);

@@ -27,11 +27,13 @@
 // TMA reduce-add, so that the accumulator block shared by dP^T and dQ is free again a few hundred cycles after
 // the dQ MMAs finish and the compute warps never touch dQ.
 // Sixteen compute warps of 32 columns rather than eight of 64: the phases of a step (scores, exponentials, dS) are chains of
-// TMEM loads, shared-memory reads and special functions that two warps a scheduler leave mostly idle (issue slots 26 % used).
+// TMEM loads, shared-memory reads and special functions that two warps a scheduler leave mostly idle (issue slots used on the
+// window workload 30 %, now 43 %).
 // Measured with the elected MMA lane on both sides: gated B4 S8192 4112 -> 3770 us, 64-wide dense S4096 H16 313 (lane 0) -> 247,
-// packed 2052 -> 2030, window workload 358 -> 354, dense causal S8192 1320 -> 1319 (bound by the dQ path).
-// TMEM columns: [0,128) S^T, then P^T packed into the first 16 of each 32 | [128,256) dP^T, later dQ |
-// [256,384) dV | [384,512) dK.
+// packed 2052 -> 2030, window workload 358 -> 354, dense causal S8192 1320 -> 1319 (bound by the dQ path as it
+// was then: with the whole tile read out at once 1269).
+// TMEM columns at head size 128: [0,128) S^T, then P^T packed into the first 16 of each 32 | [128,256) dP^T, later dQ |
+// [256,384) dV | [384,512) dK. At head size 64 dV takes [256,320), dQ a block of its own, [320,384), and dK [384,448).
 #include "fsa_ptx.cuh"
 #include "fsa_params.h"
 #include "fsa_schedule.h"
@@ -56,17 +58,17 @@ struct BwdSmem {
   static constexpr int kQ = kV + kTile;        // 2 stages
   static constexpr int kDO = kQ + 2 * kTile;   // 1 stage: dO lives only from dP^T to dV of its step
   static constexpr int kDS = kDO + kTile;      // dS^T (16-bit, 128 x 128)
-  static constexpr int kStage = kDS + 32768;   // dQ staging for the TMA reduce-add: 8 warps x 4 KB
+  static constexpr int kStage = kDS + 32768;   // dQ staging for the TMA reduce-add: 4 warps x two 4 KB buffers
   static constexpr int kAux = kStage + 32768;  // lse2[2][128], dpsum[2][128] fp32, alpha[2][128] 16-bit (gated)
   static constexpr int kBar = kAux + 2560;
-  static constexpr int kTotal = kBar + 512;
+  static constexpr int kTotal = kBar + 384;
 };
 
 struct BwdBars {
   uint64_t kv_full, q_full[2], q_empty[2], do_full, do_empty;
   uint64_t s_full, p_full, dp_full, ds_full, dq_full, dq_empty, vote_sync, acc_full;
-  uint64_t dd_sync;  // gated: second column group -> first, partial ddelta handed over in shared memory
-  uint64_t stg_full, stg_free;  // dQ staging: compute warps -> drain warp (job posted) and back (buffers read)
+  uint64_t dd_sync;  // gated: the other three column groups -> the first, partial ddelta handed over in shared memory
+  uint64_t stg_full, stg_free;  // dQ staging: dQ warps -> drain warp (job posted) and back (buffers read)
   int job[2][4];                // job descriptors {first row, head, query tile, code}, slot = job index & 1
   int dqjob[2][4];              // MMA issuer -> dQ warps: {first row, head, query tile, code} of the dQ tile in TMEM
   // Step it (slot it & 1), published by the producer with q_full: head of the group, query tile, mask mode, and bit 0: first
@@ -77,7 +79,7 @@ struct BwdBars {
   int abort_flag;
   alignas(16) unsigned char vote_any[2][NCW];
 };
-static_assert(sizeof(BwdBars) <= 512, "barrier block too large");
+static_assert(sizeof(BwdBars) <= 384, "barrier block too large");
 
 // Visible query columns of one key row inside query tile [q0, q0 + TM), as up to three half-open
 // intervals of the tile-local index (mask.py:52-102 read along the query axis).
@@ -356,9 +358,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
   // at once, 512 x 80 + 128 x 96 + 128 x 64 elsewhere (the gated kind's compute warps need their 80: 72 spill 200 bytes).
   if (warp >= W_DQ) {
     // =============================== dQ read-out ================================================
-    // One warp per TMEM lane quadrant (32 query rows). Per dQ tile: 64 columns at a time leave TMEM for registers
-    // and go through this warp's two 4 KB staging buffers into TMA reduce-adds; the TMEM block is handed back
-    // as soon as the last columns are in registers. The path from an SM to L2 moves about 21 bytes per clock, so
+    // One warp per TMEM lane quadrant (32 query rows). A dQ tile leaves TMEM for registers at once (WHOLE_DQ) or 64 columns
+    // at a time, and goes through this warp's two 4 KB staging buffers into TMA reduce-adds, 64 columns at a time; the TMEM
+    // block is handed back as soon as the last columns are in registers. The path from an SM to L2 moves about 21 bytes per clock, so
     // the 64 KB of a tile take about as long as the MMAs of a step: these warps pace themselves on the reads of
     // the staging buffers and nobody else waits for them.
     if constexpr (WHOLE_DQ)
@@ -644,7 +646,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
             tc_fence_after();
             post_dq_job(g_cur, m_cur, 0);
           }
-          // dQ first: its tile has to leave TMEM before dP^T of the next step can be issued
+          // dQ before dK: its way out is the longer one (at head size 128 dP^T of the next step also waits for the block)
 #pragma unroll ISSUE_UNROLL
           for (int kk = 0; kk < KK_N; ++kk)
             umma_ss_lead(lead, tmem_base + TMEM_DQ, umma_desc_at(ds_mn, kk * 2048), umma_desc_at(k_mn, kk * 2048), idesc_dq,

@@ -246,9 +246,9 @@ __device__ __forceinline__ uint32_t elect_one() {
 }
 // Leader-predicated forms: the whole warp runs the (warp-uniform) address arithmetic and the instruction
 // carries the single-lane predicate, instead of a divergent branch around a block of MMAs. `lead` has to come from
-// elect_one(): with "lane == 0" in its place the issue of one MMA takes 75 to 100 cycles beside two busy warps on the
-// scheduler, with the elected lane no longer than the MMA itself (16 MMAs of 128 x 128 x 16: 1279 and 1024 cycles; 4 of
-// those and 8 of 128 x 64 x 16: 897 and 619).
+// elect_one(): with "lane == 0" in its place the issue of a 128 x 128 x 16 MMA takes 68 to 80 cycles, the more the busier the
+// other warps of the scheduler are, with the elected lane 64, as long as the MMA itself
+// (benchmarks/tcgen05_issue_probe.cu).
 #define FSA_UMMA_LEAD(NAME, KIND, AFMT, ATYPE, ACONS)                                                        \
   __device__ __forceinline__ void NAME(uint32_t lead, uint32_t d_tmem, ATYPE a, uint64_t bdesc, uint32_t idesc, \
                                        uint32_t accumulate) {                                                \
