@@ -482,6 +482,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
         int g = 0, m = 0, mode = 0, g_n = 0, m_n = 0, mode_n = 0;
         bool first = false, first_n = false;
         bool more = walk_next(wk, g_n, m_n, mode_n, first_n, true);  // records the dropped steps in the tile map
+        if (!more) mbar_wait(&bars->kv_full, 0, abort_flag);  // no step: nobody else waits for K and V to land
         for (int it = 0; ok && more; ++it) {
           g = g_n;
           m = m_n;

@@ -41,3 +41,12 @@ def test_a_warp_waits_until_every_lane_has_seen_the_phase():
     votes = [(name, m.group(0)) for name in sorted(os.listdir(CSRC))
              for m in re.finditer(r"__(any|all|ballot)_sync\([^;]*mbar_\w*wait", _code(name))]
     assert votes and all(v.startswith("__all_sync") for _, v in votes), votes
+
+
+def test_backward_producer_waits_for_tiles_that_nobody_uses():
+    # a CTA without a step (an empty split, keys that no window reaches) must not leave while its K and V are on their way into
+    # its shared memory: only the issuer of a CTA with steps waits for them otherwise
+    text = _code("fsa_bwd_sm100.cu")
+    producer = _rest_of_block(text, text.index("mbar_arrive_expect_tx(&bars->kv_full"))
+    first_walk = producer[producer.index("bool more = walk_next("):producer.index("for (int it = 0")]
+    assert re.search(r"if \(!more\)\s*mbar_wait\(&bars->kv_full, 0, abort_flag\);", first_walk)
