@@ -77,6 +77,7 @@ struct BwdBars {
   alignas(16) int step[2][4];
   uint32_t tmem_base;
   int abort_flag;
+  int any_step;  // the CTA has a step; written before the block's barrier
   alignas(16) unsigned char vote_any[2][NCW];
 };
 static_assert(sizeof(BwdBars) <= 384, "barrier block too large");
@@ -247,10 +248,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
     w.right = wp[2];
     w.near_ = wp[3];
   }
-  const FsaBwdSched sched = fsa_bwd_schedule(sq, sk, n_block, split, w, p.num_splits, TN, TM, causal, local, split_qo);
-  const SegList segs = make_segments(sched, causal, local);
+  // Two warps walk the steps, the producer's and the issuer's; the others read what those publish (any_step, step). In all of the 24
+  // warps this arithmetic kept the schedulers busy before the first tile: 16 sequences of 512 tokens, 32 / 8 heads, dense 173.3 us,
+  // in two 165.5, CTAs of one step 100.0 and 96.3, window workload 345.7 and 337.6.
+  const bool walks = warp == W_PROD || warp == W_MMA;
+  SegList segs;
+  segs.n = segs.total = 0;
+  if (walks) segs = make_segments(fsa_bwd_schedule(sq, sk, n_block, split, w, p.num_splits, TN, TM, causal, local, split_qo), causal, local);
   const int NT = segs.total;       // query tiles per head
-  const int N_IT = NT * p.G;       // steps of this CTA (before gate-skipped ones are dropped)
 
   // ---- the steps of this CTA, in order: (head of the group, query tile) ------------------------------------
   // Gated kind: the gate bound of a step (flash_sparse_attn/ops/triton/flash_gated_bwd.py:61-79,
@@ -263,7 +268,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
   const bool preskip = (KIND == KIND_GATED) && !(p.flags & F_DETERMINISTIC) && p.gate_ws != nullptr;
   float gw_dmax = 0.f, gw_dmin = 0.f;
   const float2* gw_aext = nullptr;
-  if (preskip) {
+  if (preskip && walks) {
     const float2* ext = reinterpret_cast<const float2*>(p.gate_ws);
     const float2 de = __ldg(ext + (long long)p.B * p.Hq * p.num_m_blocks + ((long long)b * p.Hkv + hkv) * p.n_tiles_k + n_block);
     gw_dmax = de.x;
@@ -342,6 +347,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
     mbar_init(&bars->stg_free, 1);
     bars->abort_flag = (*reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
     mbar_fence_init();
+  }
+  if (warp == W_MMA) {
+    bool any = NT > 0;
+    if constexpr (KIND == KIND_GATED) {
+      StepWalk wk = walk_begin();
+      int g0, m0, mode0;
+      bool first0;
+      any = walk_next(wk, g0, m0, mode0, first0, false);
+    }
+    if (lane == 0) bars->any_step = any;
   }
   if (warp == W_PROD) {
     tmem_alloc(&bars->tmem_base, 512);
@@ -519,8 +534,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
       constexpr uint32_t idesc_dq = umma_idesc_f16(TM, HD, IS_BF16, true, true);    // dQ: A = dS^T MN-major, B = K MN-major
       const uint32_t sK = smem_u32(smem + SM::kK), sV = smem_u32(smem + SM::kV), sQ = smem_u32(smem + SM::kQ),
                      sDO = smem_u32(smem + SM::kDO), sDS = smem_u32(smem + SM::kDS);
-      bool ok = !*abort_flag && N_IT > 0;
-      (void)N_IT;
+      bool ok = !*abort_flag && NT > 0;
       // The MMA loops are unrolled (sparse causal S = 8192: 1324 us rolled, 1286 unrolled) except in the gated kind, whose compute
       // warps carry the gate arithmetic and whose code the schedulers fetch most.
       constexpr int ISSUE_UNROLL = (KIND == KIND_GATED) ? 1 : 8;
@@ -1152,13 +1166,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
       if (lane == 0) mbar_arrive(&bars->ds_full);
     };
 
-    bool has_cur;
-    {
-      StepWalk wk = walk_begin();  // whether there is any step
-      int g0 = 0, m0 = 0, mode0 = 0;
-      bool first0 = false;
-      has_cur = ok && walk_next(wk, g0, m0, mode0, first0, false);
-    }
+    bool has_cur = ok && *reinterpret_cast<const volatile int*>(&bars->any_step);
     const bool any_step = has_cur;
     if (has_cur) {
       skip_cur = p_step(0);
