@@ -1283,13 +1283,19 @@ cudaError_t launch_one(const BwdKernelParams& p, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
-// The dense and sparse kinds take a dQ tile at once at head size 128, where it leaves the block that dP^T of the next step waits for. In
-// deterministic mode the turns set the pace, and 64 columns at a time are faster (S = 4096, 16 / 4 heads: dense 544 us at once,
-// 520 in halves, sparse 533 and 503, a 512-token window 107 and 94). A kernel of its own: as a branch it spills 48 bytes more.
+// The dense and sparse kinds take a dQ tile at once at head size 128, where it leaves the block that dP^T of the next step waits for. Two
+// calls are better off with 64 columns at a time:
+// - deterministic ones, where the turns set the pace (S = 4096, 16 / 4 heads: dense 544 us at once, 520 in halves, sparse 533 and 503,
+//   a 512-token window 107 and 94);
+// - CTAs of at most four steps, which have no next step to speak of (one step, 64 x 128 tokens, 16 heads: 96.3 us at once and 92.1 in
+//   halves; two 57.9 and 56.2; four 65.7 and 63.8; eight 82.3 and 81.8, sparse 82.5 and 83.7; sixteen 113.4 and 115.4).
+// (As a branch in one kernel it spills 48 bytes more.)
 template <int HD, typename T, int KIND>
 cudaError_t launch_kind(const BwdKernelParams& p, cudaStream_t stream) {
-  if constexpr (HD == 128 && KIND != KIND_GATED)
-    if (!(p.flags & F_DETERMINISTIC)) return launch_one<HD, T, KIND, true>(p, stream);
+  if constexpr (HD == 128 && KIND != KIND_GATED) {
+    const long long steps = (long long)p.G * ((p.num_m_blocks + p.num_splits - 1) / p.num_splits);
+    if (!(p.flags & F_DETERMINISTIC) && steps > 4) return launch_one<HD, T, KIND, true>(p, stream);
+  }
   return launch_one<HD, T, KIND, false>(p, stream);
 }
 

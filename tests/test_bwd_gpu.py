@@ -260,3 +260,19 @@ def test_deterministic_dq_with_and_without_skips(head_dim, threshold):
         assert torch.equal(a, b), name
         # the same products in another order of fp32 sums, rounded once to 16 bits
         assert_close(f"det-{head_dim}-{name}", a, f.cpu(), rtol=2**-7, atol=2**-7)
+
+
+@pytest.mark.parametrize("s, group, splits", [(100, 1, 1), (512, 1, 1), (513, 1, 1), (130, 2, 1), (130, 3, 1), (1000, 2, 4), (1000, 2, 3)])
+@pytest.mark.parametrize("kind", ["dense", "sparse"])
+def test_ctas_of_few_steps(kind, s, group, splits):
+    """Up to four steps a CTA dQ tiles are read out in halves, with more at once."""
+    fsa = _ops()
+    hkv, d = 2, 128
+    q, k, v = seeded_qkv(s + group, 1, s, s, hkv * group, hkv, d)
+    do = torch.randn(1, s, hkv * group, d, generator=torch.Generator().manual_seed(s)).to(torch.bfloat16)
+    ref = eager.backward(q, k, v, do, None, True)
+    kw = dict(is_causal=True) | (dict(softmax_threshold=-128.0) if kind == "sparse" else {})
+    kw |= dict(is_split_qo=True, num_splits=splits) if splits > 1 else {}
+    got = _run(getattr(fsa, f"flash_{kind}_attn_func"), q, k, v, do, **kw)
+    for name, a, r in zip(("dq", "dk", "dv"), got, ref):
+        assert_close(f"{kind}-{s}-{group}-{splits}-{name}", a, r)
