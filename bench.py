@@ -62,7 +62,7 @@ NOMINAL_BF16_TFLOPS = 2250.0
 NOMINAL_HBM_GBS = 8000.0
 # DRAM bytes per launch of the backward main kernel on this workload: a constant copied from the ncu capture that
 # profiles/bwd_kernel_c2.txt summarises (dram__bytes_read.sum + dram__bytes_write.sum); NOT measured by this run
-TRAFFIC_BWD_KERNEL_C2 = 679.0e6
+TRAFFIC_BWD_KERNEL_C2 = 640.8e6
 
 
 def workloads():
