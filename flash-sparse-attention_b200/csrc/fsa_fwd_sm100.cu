@@ -8,7 +8,7 @@
 // TILE_M = TILE_N = 128: same tile schedule, same masks, same online-softmax recurrences and the
 // same per-tile skip rule (activations.py:103-166), evaluated independently for each 128-row tile.
 //
-// Roles (384 threads = 3 warpgroups, registers rebalanced with setmaxnreg):
+// Roles (384 threads = 3 warpgroups, registers rebalanced with setmaxnreg; gated: 640 threads, see FwdRoles):
 //   warps 0-3  : softmax group 0 (query tile 0), one thread per query row / TMEM lane
 //   warps 4-7  : softmax group 1 (query tile 1)
 //   warp  8    : producer - TMA loads of Q, K ring, V ring; allocates / frees TMEM
@@ -32,7 +32,17 @@ namespace {
 
 constexpr int TM = 128;  // query rows per softmax group
 constexpr int TN = 128;  // keys per tile
-constexpr int NTHREADS = 384;  // three warpgroups: softmax 0, softmax 1, {producer, MMA, 2 idle}
+// Warps by kind. One softmax thread per query row, four warps a group; the gated kind has two threads a row, 64 key columns
+// each, eight warps a group (up to head size 128): the gate's chains (an exponential, then five dependent multiply-adds) take a warp 15
+// cycles a column where four warps of a scheduler together take 9. B1 S8192, 32 / 8 heads of 128, with the gate worked out ahead of the
+// scores: full 1951 -> 1713 us, causal 984 -> 942, windows of 512 to 4096 (B4) 1741 -> 1708; head size 64 causal 968 -> 921.
+template <int HD, int KIND>
+struct FwdRoles {
+  static constexpr int HALVES = KIND == KIND_GATED && HD <= 128 ? 2 : 1;  // threads per query row
+  static constexpr int GW = 4 * HALVES;                      // softmax warps of a group
+  static constexpr int W_PROD = 2 * GW, W_MMA = W_PROD + 1, W_STAGE = W_PROD + 2;
+  static constexpr int NTHREADS = (W_PROD + 4) * 32;
+};
 // Two K and two V stages. V(t) and K(t + 1) are consumed by the same loop step of the MMA issuer, so they
 // arrive on one barrier and one "consumed" barrier per step releases both: every barrier the issuer touches
 // costs it 130-250 cycles even when it is already complete. (A third V stage, loaded a whole step earlier, did
@@ -48,14 +58,16 @@ struct FwdShape {
   static constexpr int VSTAGES = HD > 128 ? 1 : 2;
 };
 
-template <int HD, int ES = 2>
+template <int HD, int ES, int KIND>
 struct FwdSmem {
   static constexpr int kTileBytes = TM * HD * ES;  // one Q / K / V tile of ES-byte elements
   static constexpr int kQ = 0;
   static constexpr int kK = kQ + FwdShape<HD>::QT * kTileBytes;
   static constexpr int kV = kK + FwdShape<HD>::KSTAGES * kTileBytes;
   static constexpr int kBar = kV + FwdShape<HD>::VSTAGES * kTileBytes;
-  static constexpr int kTotal = kBar + 2048 + 1024;  // barriers/flags/delta ring + alignment slack
+  // (maximum, sum) of a row's halves: [group][half][row] (gated)
+  static constexpr int kXch = kBar + 2048;
+  static constexpr int kTotal = kXch + (FwdRoles<HD, KIND>::HALVES == 2 ? 4096 : 0) + 1024;  // barriers/flags/delta ring + alignment slack
 };
 
 // Output / gate element type that goes with an input element type.
@@ -85,7 +97,8 @@ struct FwdBars {
   uint32_t tmem_base;
   int abort_flag;
   int skip_flag[2][2];   // [group][parity of the group's tile counter]
-  int vote_any[2][2][4]; // [group][parity][warp]: bit0 = some row wants the tile, bit1 = some row votes skip
+  uint64_t pair_sync[2][4];  // two threads a row: the two warps of a lane quadrant have written their halves' (maximum, sum)
+  int vote_any[2][2][8]; // [group][parity][warp]: bit0 = some row wants the tile, bit1 = some row votes skip
   // What the producer worked out about the tiles, for the MMA issuer: low word the tile index (-1: none), then bit q: group q
   // takes part in it, bit 2 + q: it is group q's last. Slot 2: the first tile, published with k0_full. Slot t & 1: the
   // tile after step t (and whether the one of step t is a group's last), published with kv_full.
@@ -165,7 +178,7 @@ __device__ __forceinline__ void mask_cols32(uint32_t* r, uint32_t bits) {
 // BSCALE: FP8 inputs with one scale per 128-position block (a separate instantiation: as a run-time switch it cost
 // the per-tensor FP8 forward 10 %).
 template <int HD, typename T, int KIND, bool BSCALE = false>
-__global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant__ FwdKernelParams p) {
+__global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(const __grid_constant__ FwdKernelParams p) {
   // T is the element type of Q, K, V and of P: bf16 / fp16 (kind::f16) or FP8 e4m3 / e5m2 (kind::f8f6f4,
   // flash_sparse_attn/ops/triton/flash_sparse_fwd.py:49, :84-86 under IS_QUANT). Outputs and the gate
   // vectors are 16-bit (bf16 for FP8 inputs, flash_sparse_fwd.py:634).
@@ -173,10 +186,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
   constexpr bool F8 = ES == 1;
   constexpr int SLAB = 128 / ES;      // elements per 128-byte swizzle row
   using TO = typename OutType<T>::type;
-  using SM = FwdSmem<HD, ES>;
+  using SM = FwdSmem<HD, ES, KIND>;
+  using RO = FwdRoles<HD, KIND>;
   constexpr int KK_QK = HD * ES / 32;  // MMAs per S tile: every MMA consumes 32 bytes of the head dimension
   constexpr int KK_PV = TN * ES / 32;  // MMAs per P V tile: 32 bytes of the key dimension each
-  constexpr int OCH = HD / 32;        // 32-column chunks of an O tile
   constexpr int QT = FwdShape<HD>::QT, KSTAGES = FwdShape<HD>::KSTAGES, VSTAGES = FwdShape<HD>::VSTAGES;
   constexpr bool IS_BF16 = (sizeof(T) == 2) && !__is_same(T, __half);
   static_assert(!F8 || HD == 128, "FP8 tiles are one 128-byte swizzle row wide");
@@ -184,7 +197,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
   // FP8: P is handed to the MMA issuer in two halves, so that the first MMAs of P V run under the second half of the
   // exponentials (B2 S6000 causal, a call: 529 -> 510 us). With 16-bit inputs, whose P V takes twice as long, the second barrier
   // costs the issuer more than that gains (S = 16384: 1.91 -> 1.96 ms).
-  constexpr bool HALVES = F8;
+  constexpr bool HALVES = F8 && RO::HALVES == 1;
   // Who walks the tiles for the MMA issuer: the producer, ahead of time, except above head size 128 (not gated), where one query
   // tile leaves the issuer time and reading the producer's record costs more than the walk (dense causal S = 8192,
   // 16 / 4 heads of 192: 501 us, 523 with the record; a 1024-token window 183 and 187).
@@ -259,7 +272,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
   const int m_blocks_here = fsa_cdiv(si.sq * gpack, TM);  // query tiles this sequence really has
   if (pair * QT >= m_blocks_here) return;  // the grid is laid out for the longest sequence: nothing to do or to write
 
-  // Both groups' schedules are needed by every role.
+  // Both groups' schedules are needed by every role; gated: by those that walk the tiles, the softmax warps read the stager's.
+  const bool walks = KIND != KIND_GATED || warp >= RO::W_PROD;
   FsaFwdSched sched[2];
   bool q_valid[2];
 #pragma unroll
@@ -269,9 +283,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
     // One query position with windows and split-KV: the reference's rounding drops the first, partial tile of
     // the near band (block_info.py:60-64) although its eager ground truth sees those keys; like the decode
     // kernel, this one visits them (the flag only matters for that combination).
-    sched[q] = fsa_fwd_schedule(si.sq, si.sk, mb, si.split, si.w, p.num_splits, TN, TM, causal, local, split_kv,
-                                gpack, /*cover_single_query=*/true);
-    if (!q_valid[q] || fsa_fwd_sched_empty(sched[q])) {
+    if (walks)
+      sched[q] = fsa_fwd_schedule(si.sq, si.sk, mb, si.split, si.w, p.num_splits, TN, TM, causal, local, split_kv,
+                                  gpack, /*cover_single_query=*/true);
+    if (!walks || !q_valid[q] || fsa_fwd_sched_empty(sched[q])) {
       sched[q].n_min = sched[q].n_max = sched[q].n_max_no_mask = 0;
       sched[q].win_min = sched[q].win_max = sched[q].win_min_no_mask = sched[q].win_max_no_mask = 0;
       sched[q].sink_min = sched[q].sink_max = 0;
@@ -301,7 +316,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
   float gw_amax[2] = {0.f, 0.f}, gw_amin[2] = {0.f, 0.f}, gw_thr[2] = {0.f, 0.f}, gw_run[2] = {-INFINITY, -INFINITY};
   float gw_c = 0.f;
   const float2* gw_dext = nullptr;
-  if (KIND == KIND_GATED) {
+  if (KIND == KIND_GATED && walks) {
     gw_c = p.qkv_scale ? p.scale_log2 * p.qkv_scale[0] * p.qkv_scale[1] : p.scale_log2;
     const float2* aext = reinterpret_cast<const float2*>(p.gate_ws);
     gw_dext = aext + (long long)p.B * p.hgrid * p.num_m_blocks + ((long long)si.b * p.Hkv + si.hkv) * p.n_tiles_k;
@@ -365,17 +380,18 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
     }
     for (int q = 0; q < 2; ++q) {
       mbar_init(&bars->s_full[q], 1);
-      mbar_init(&bars->p_full[q], 4);  // one arrival per warp of the group
+      mbar_init(&bars->p_full[q], RO::GW);  // one arrival per warp of the group
       mbar_init(&bars->p_rest[q], 4);
       mbar_init(&bars->o_final[q], 1);
-      mbar_init(&bars->wg_sync[q], 4);
+      mbar_init(&bars->wg_sync[q], RO::GW);
+      for (int w = 0; w < 4; ++w) mbar_init(&bars->pair_sync[q][w], 2);
       mbar_init(&bars->d_full[q], 1);
-      mbar_init(&bars->d_empty[q], 8);
+      mbar_init(&bars->d_empty[q], 2 * RO::GW);
     }
     bars->abort_flag = (*reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
     mbar_fence_init();
   }
-  if (warp == 8) {
+  if (warp == RO::W_PROD) {
     tmem_alloc(&bars->tmem_base, 512);
     tmem_relinquish();
   }
@@ -386,12 +402,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
 
   const int kv_row_coord_b = (p.flags & (F_VARLEN_K | F_PAGED)) ? 0 : si.b;
 
-  // Register budget: the two softmax groups hold a 128-wide fp32 output row per thread and take
-  // the registers the third warpgroup does not need.
-  if (warp >= 8) {
-    // third warpgroup: all four warps release registers at the same instruction
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
-  if (warp == 8) {
+  // Register budget: a softmax thread holds a 128-wide fp32 score row (gated: 32 scores at a time) and takes the registers
+  // that the last warpgroup does not need: 384 x 168 at launch = 256 x 216 + 128 x 72, gated 640 x 96 = 512 x 104 + 128 x 64.
+  if (warp >= RO::W_PROD) {
+    // last warpgroup: all four warps release registers at the same instruction
+    if constexpr (RO::HALVES == 1)
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    else
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+  if (warp == RO::W_PROD) {
     // =============================== producer ================================================
     if (lane == 0 && !*abort_flag) {
       tma_prefetch_desc(&p.map_q);
@@ -522,7 +541,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
       }
     }
     __syncwarp();
-  } else if (warp == 10) {
+  } else if (warp == RO::W_STAGE) {
     // =============================== delta stager (gated only) ================================
     // delta of every computed key tile as fp32 in a 2-slot ring, with the tile's index and the groups' mask modes, so
     // that the softmax warps need not walk the schedule (1600 to 2200 cycles a tile on their critical path)
@@ -566,7 +585,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
         if (n < 0) break;
       }
     }
-  } else if (warp == 9) {
+  } else if (warp == RO::W_MMA) {
     // =============================== MMA issuer ==============================================
     constexpr int F8_FMT = __is_same(T, __nv_fp8_e5m2) ? 1 : 0;
     constexpr uint32_t idesc_s = F8 ? umma_idesc_f8(TM, TN, F8_FMT, F8_FMT, false, false)
@@ -600,6 +619,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
     // The MMA loops are unrolled in the dense and sparse kinds (rolled: sparse causal S = 16384 1830 -> 2006 us, FP8 472 -> 502)
     // and stay rolled in the gated kind, whose softmax warps carry the gate arithmetic.
     constexpr int ISSUE_UNROLL = (KIND == KIND_GATED) ? 1 : 8;
+    auto p_col = [](int kk) {  // where P of the kk-th MMA lies: each thread of a row writes it over the front of its own scores
+      return kk * 8 + (RO::HALVES == 2 && kk >= KK_PV / 2 ? TN / 2 - KK_PV / 2 * 8 : 0);
+    };
     auto issue_s = [&](int q, int ks) {
       const uint32_t aq = dq_lo + ((q * SM::kTileBytes) >> 4), bk = dk_lo + ((ks * SM::kTileBytes) >> 4);
 #pragma unroll ISSUE_UNROLL
@@ -703,10 +725,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
                 tc_fence_after();
               }
               if (F8)
-                umma_f8_ts_lead(lead, tm + TMEM_O0 + q * 128, tm + TMEM_S0 + q * 128 + kk * 8,
+                umma_f8_ts_lead(lead, tm + TMEM_O0 + q * 128, tm + TMEM_S0 + q * 128 + p_col(kk),
                                 umma_desc_at(bv, kk * 4096), idesc_o, (kk > 0 || o_started[q]) ? 1u : 0u);
               else
-                umma_ts_lead(lead, tm + TMEM_O0 + q * 128, tm + TMEM_S0 + q * 128 + kk * 8,
+                umma_ts_lead(lead, tm + TMEM_O0 + q * 128, tm + TMEM_S0 + q * 128 + p_col(kk),
                              umma_desc_at(bv, kk * 2048), idesc_o, (kk > 0 || o_started[q]) ? 1u : 0u);
             }
             o_started[q] = true;
@@ -735,14 +757,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
   }
   } else {
     // =============================== softmax groups ==========================================
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
-    const int q = warp >> 2;        // group / query tile
+    if constexpr (RO::HALVES == 1)
+      asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+    else
+      asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    constexpr int NC = TN / RO::HALVES;                    // key columns of a thread
+    constexpr int OC = HD / RO::HALVES;                    // output columns of a thread
+    const int q = RO::HALVES == 1 ? warp >> 2 : warp >> 3;                           // group / query tile
+    const int half = RO::HALVES == 1 ? 0 : (warp >> 2) & 1;  // which key (and output) columns
     const int wq = warp & 3;        // warp within group == TMEM lane quadrant
     const int row = wq * 32 + lane; // row within the tile
     const int mb = pair * QT + q;
     const uint32_t lane_addr = uint32_t(wq * 32) << 16;
-    const uint32_t tS = tmem_base + lane_addr + TMEM_S0 + q * 128;
-    const uint32_t tO = tmem_base + lane_addr + TMEM_O0 + q * 128;
+    const uint32_t tS = tmem_base + lane_addr + TMEM_S0 + q * 128 + half * NC;
+    const uint32_t tO = tmem_base + lane_addr + TMEM_O0 + q * 128 + half * OC;
 
     const int offs_m = mb * TM + row;
     const int q_idx = offs_m / gpack;
@@ -779,7 +807,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
     float v_run = 0.f;  // block-scaled: running reference of the value scale (uniform over the tile's rows)
     const float v_scale = p.qkv_scale ? p.qkv_scale[2] : p.v_scale;
     float m_ref = -INFINITY;  // reference maximum all stored exponentials are relative to
-    float l_ref = 0.f;        // sum of exp2((s - m_ref) * c)
+    float l_ref = 0.f;        // sum of exp2((s - m_ref) * c) over this thread's columns
     float lg_l = -INFINITY;   // log2(l_ref) for the skip test, refreshed at the end of a tile (off the S -> P path)
     bool have_o = false;      // some P V has been issued for this tile
     int cnt_s = 0;
@@ -821,17 +849,19 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
         mode = has_work ? fsa_fwd_tile_mode(my, n, causal, local) : -1;
         if (mode < 0) continue;
       }
-      ok = mbar_wait(&bars->s_full[q], cnt_s & 1, abort_flag);
-      if (!ok) break;
-      tc_fence_after();
       const int par = cnt_s & 1;
+      if (KIND != KIND_GATED) {
+        ok = mbar_wait(&bars->s_full[q], par, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+      }
       cnt_s++;
       const int k0 = n * TN;
 
       // ---- scores of this row: TMEM -> registers (warp-collective loads, one wait) ---------------
       // Gated kind: 32 columns at a time, and the gated and masked logits go back to TMEM, from where the exponentials
       // below read them in pieces again: with the whole row in registers beside the gate's arithmetic the softmax
-      // warps spill (B4 S8192, windows of 512 to 4096: 3.24 -> 2.90 ms together with the packed gate). The other
+      // warps spill (64 columns in the registers of two threads a row: 200 bytes, 10 % slower). The other
       // kinds hold the row: reading it twice costs them 17 % (dense, S = 16384: 1.93 -> 2.27 ms).
       constexpr bool GATED = KIND == KIND_GATED;
       uint32_t sr[GATED ? 32 : TN];
@@ -848,54 +878,77 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
         // rolled up: unrolled over the row, the gate's code alone is larger than the instruction caches hold beside the
         // other roles', and its 128 columns took 6700 cycles
 #pragma unroll 1
-        for (int ch = 0; ch < TN / 32; ++ch) {
-          uint32_t r[32];
-          tmem_ld32(tS + ch * 32, r);
-          tmem_ld_wait();
-          // logits = (q.k + g(alpha * delta_j)) * scale, g = logsigmoid or identity
-          // (flash_sparse_attn/ops/triton/flash_gated_fwd.py:104-122, activations.py:245-262)
-          const float4* d4 = reinterpret_cast<const float4*>(&bars->dl[ds][ch * 32]);
+        for (int ch = 0; ch < NC / 32; ++ch) {
+          // g(alpha * delta_j), g = logsigmoid or identity (flash_sparse_attn/ops/triton/flash_gated_fwd.py:104-122,
+          // activations.py:245-262): the first 32 columns before the scores are waited for
+          float2 g[16];
+          {
+            float4 dd[8];
+            const float4* d4 = reinterpret_cast<const float4*>(&bars->dl[ds][half * NC + ch * 32]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) dd[i] = d4[i];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              g[2 * i] = mul2(al2, make_float2(dd[i].x, dd[i].y));
+              g[2 * i + 1] = mul2(al2, make_float2(dd[i].z, dd[i].w));
+            }
+          }
           if (logsig) {
 #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              const float4 dd = d4[i >> 2];
-              const float2 ga = add_log_sigmoid2(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])),
-                                                 mul2(al2, make_float2(dd.x, dd.y)));
-              const float2 gb = add_log_sigmoid2(make_float2(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])),
-                                                 mul2(al2, make_float2(dd.z, dd.w)));
-              r[i] = __float_as_uint(ga.x);
-              r[i + 1] = __float_as_uint(ga.y);
-              r[i + 2] = __float_as_uint(gb.x);
-              r[i + 3] = __float_as_uint(gb.y);
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              const float4 dd = d4[i >> 2];
-              r[i] = __float_as_uint(fmaf(alpha, dd.x, __uint_as_float(r[i])));
-              r[i + 1] = __float_as_uint(fmaf(alpha, dd.y, __uint_as_float(r[i + 1])));
-              r[i + 2] = __float_as_uint(fmaf(alpha, dd.z, __uint_as_float(r[i + 2])));
-              r[i + 3] = __float_as_uint(fmaf(alpha, dd.w, __uint_as_float(r[i + 3])));
-            }
+            for (int i = 0; i < 16; ++i) g[i] = log_sigmoid2(g[i]);
           }
-          if (mode != FSA_MASK_NONE) {
-            mask_cols32(r, tile_bits(tm, ch * 32));
-          } else if (!rm.row_ok) {
-            // rows past the query length read as zero scores in fully visible tiles
-#pragma unroll
-            for (int i = 0; i < 32; ++i) r[i] = 0u;
+          if (ch == 0) {
+            ok = mbar_wait(&bars->s_full[q], par, abort_flag);
+            if (!ok) break;
+            tc_fence_after();
           }
-          tmem_st32(tS + ch * 32, r);
+          const uint32_t bits = mode != FSA_MASK_NONE ? tile_bits(tm, half * NC + ch * 32) : 0u;
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) {
+          for (int h = 0; h < 32; h += 16) {
+            uint32_t r[16];
+            tmem_ld16(tS + ch * 32 + h, r);
+            tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-              mx[j] = max3(mx[j], __uint_as_float(r[i + 2 * j]), __uint_as_float(r[i + 2 * j + 1]));
+            for (int i = 0; i < 16; i += 2) {
+              const float2 v = add2(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), g[(h + i) >> 1]);
+              r[i] = __float_as_uint(v.x);
+              r[i + 1] = __float_as_uint(v.y);
+            }
+            if (mode != FSA_MASK_NONE) {
+#pragma unroll
+              for (int i = 0; i < 16; ++i)
+                if (!(bits & (1u << (h + i)))) r[i] = 0xff800000u;
+            } else if (!rm.row_ok) {
+              // rows past the query length read as zero scores in fully visible tiles
+#pragma unroll
+              for (int i = 0; i < 16; ++i) r[i] = 0u;
+            }
+            tmem_st16(tS + ch * 32 + h, r);
+#pragma unroll
+            for (int i = 0; i < 16; i += 8) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                mx[j] = max3(mx[j], __uint_as_float(r[i + 2 * j]), __uint_as_float(r[i + 2 * j + 1]));
+            }
           }
         }
+        if (!ok) break;
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->d_empty[ds]);
         m_cur = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+        // The other half of the row: its maximum, and its sum up to the tile before. (It has read this thread's values of that tile
+        // before it arrived on p_full, without which this tile's scores were not issued.)
+        if constexpr (RO::HALVES == 2) {
+          float2* xch = reinterpret_cast<float2*>(smem + SM::kXch) + q * 256;
+          xch[half * 128 + row] = make_float2(m_cur, l_ref);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->pair_sync[q][wq]);
+          ok = mbar_wait(&bars->pair_sync[q][wq], par, abort_flag);
+          if (!ok) break;
+          const float2 other = xch[(half ^ 1) * 128 + row];
+          m_cur = fmaxf(m_cur, other.x);
+          lg_l = lg2_approx(l_ref + other.y);
+        }
       } else {
 #pragma unroll
       for (int ch = 0; ch < TN / 32; ++ch) tmem_ld32(tS + ch * 32, &sr[ch * 32]);
@@ -939,7 +992,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
         // group-wide exchange through a (bounded) mbarrier rather than bar.sync, so that an
         // aborting pipeline can never leave part of the group parked on a hardware barrier
         if (lane == 0) {
-          bars->vote_any[q][par][wq] = (want ? 1 : 0) | (drop ? 2 : 0);
+          bars->vote_any[q][par][half * 4 + wq] = (want ? 1 : 0) | (drop ? 2 : 0);
           mbar_arrive(&bars->wg_sync[q]);
         }
         // a warp holding a row that wants the tile already knows the outcome ("keep") and moves on;
@@ -949,8 +1002,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
         if (!want) {
           ok = mbar_wait(&bars->wg_sync[q], par, abort_flag);
           if (!ok) break;
-          const int v = bars->vote_any[q][par][0] | bars->vote_any[q][par][1] | bars->vote_any[q][par][2] |
-                        bars->vote_any[q][par][3];
+          int v = 0;
+#pragma unroll
+          for (int w = 0; w < RO::GW; ++w) v |= bars->vote_any[q][par][w];
           // max over rows ignores NaN rows; a tile is skipped iff that max is < 0
           skip = !(v & 1) && (v & 2);
         }
@@ -958,7 +1012,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
       // The verdict goes to the MMA issuer (and to the tile map) right before this thread's arrival on p_full,
       // whose release orders it: for a kept tile that is after the exponentials, not in front of them.
       auto publish_verdict = [&](bool skipped) {
-        if (KIND != KIND_DENSE && wq == 0 && lane == 0) {
+        if (KIND != KIND_DENSE && half == 0 && wq == 0 && lane == 0) {
           bars->skip_flag[q][par] = skipped ? 1 : 0;
           if (p.tile_map) {
             const long long idx =
@@ -1005,7 +1059,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
         // size 64 sixteen (dense causal S = 4096, 8 heads: 57.0 us, 59.2 with 32).
         constexpr int RC = HD == 64 ? 16 : 32;
 #pragma unroll 1
-        for (int ch = 0; ch < HD / RC; ++ch) {
+        for (int ch = 0; ch < OC / RC; ++ch) {
           uint32_t r[RC];
           if constexpr (RC == 32)
             tmem_ld32(tO + ch * RC, r);
@@ -1027,9 +1081,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
       const float2 nm2 = make_float2(neg_mc, neg_mc);
       float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       if (GATED) tmem_st_wait();
-      constexpr int EXP_UNROLL = GATED ? 1 : TN / 32;
+      constexpr int EXP_UNROLL = GATED ? 1 : NC / 32;
 #pragma unroll EXP_UNROLL
-      for (int ch = 0; ch < TN / 32; ++ch) {
+      for (int ch = 0; ch < NC / 32; ++ch) {
         uint32_t pk[16];
         if constexpr (GATED) {
           tmem_ld32(tS + ch * 32, sr);
@@ -1073,7 +1127,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
       if (!HALVES) publish_verdict(false);
       if (lane == 0) mbar_arrive(HALVES ? &bars->p_rest[q] : &bars->p_full[q]);
       l_ref += (sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y);
-      if (KIND != KIND_DENSE) lg_l = lg2_approx(l_ref);
+      if (KIND != KIND_DENSE && RO::HALVES == 1) lg_l = lg2_approx(l_ref);  // two halves: when the other's sum is known
       have_o = true;
     }
 
@@ -1081,6 +1135,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
     if (ok && have_o) {
       ok = mbar_wait(&bars->o_final[q], 0, abort_flag);
       tc_fence_after();
+      if constexpr (RO::HALVES == 2) {  // the row's sum; the last tile's exchange has been read (its p_full came before o_final)
+        float2* xch = reinterpret_cast<float2*>(smem + SM::kXch) + q * 256;
+        xch[half * 128 + row].y = l_ref;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->pair_sync[q][wq]);
+        ok = ok && mbar_wait(&bars->pair_sync[q][wq], cnt_s & 1, abort_flag);
+        const float other = xch[(half ^ 1) * 128 + row].y;
+        l_ref += other;
+      }
     }
     if (ok && q_valid[q]) {
       const bool dead = (l_ref == 0.0f) || (l_ref != l_ref);
@@ -1088,13 +1151,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
       float lse = dead ? -INFINITY : m_ref * cc + log2f(l_ref);
       if (!(p.flags & F_LSE_LOG2)) lse *= 0.6931471805599453f;
       const long long tok = si.off_q + q_idx;
-      if (rm.row_ok)
+      if (rm.row_ok && half == 0)
         p.lse[(long long)((p.flags & F_VARLEN_Q) ? 0 : si.b) * p.l_sb + (long long)q_head * p.l_sh +
               (long long)si.split * p.l_ss + ((p.flags & F_VARLEN_Q) ? tok : q_idx)] = lse;
       const long long obase = (long long)((p.flags & F_VARLEN_Q) ? 0 : si.b) * p.o_sb + tok * p.o_sm +
-                              (long long)q_head * p.o_sh + (long long)si.split * p.o_ss;
+                              (long long)q_head * p.o_sh + (long long)si.split * p.o_ss + half * OC;
 #pragma unroll
-      for (int ch = 0; ch < OCH; ++ch) {
+      for (int ch = 0; ch < OC / 32; ++ch) {
         uint32_t r[32];
         if (have_o) {
           tmem_ld32(tO + ch * 32, r);
@@ -1108,7 +1171,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
             float* dst = reinterpret_cast<float*>(p.out) + obase + ch * 32;
 #pragma unroll
             for (int i = 0; i < 32; i += 4)
-              if (ch * 32 + i < p.D)
+              if (half * OC + ch * 32 + i < p.D)
                 *reinterpret_cast<float4*>(dst + i) =
                     make_float4(__uint_as_float(r[i]) * inv, __uint_as_float(r[i + 1]) * inv,
                                 __uint_as_float(r[i + 2]) * inv, __uint_as_float(r[i + 3]) * inv);
@@ -1121,7 +1184,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
               v.y = pack2<TO>(__uint_as_float(r[i + 2]) * inv, __uint_as_float(r[i + 3]) * inv);
               v.z = pack2<TO>(__uint_as_float(r[i + 4]) * inv, __uint_as_float(r[i + 5]) * inv);
               v.w = pack2<TO>(__uint_as_float(r[i + 6]) * inv, __uint_as_float(r[i + 7]) * inv);
-              if (ch * 32 + i < p.D) *reinterpret_cast<uint4*>(dst + i) = v;
+              if (half * OC + ch * 32 + i < p.D) *reinterpret_cast<uint4*>(dst + i) = v;
             }
           }
         }
@@ -1133,7 +1196,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
   tc_fence_before();
   __syncthreads();
   if (tid == 0 && *abort_flag) atomicExch(p.status, 1);
-  if (warp == 8) {
+  if (warp == RO::W_PROD) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
@@ -1142,12 +1205,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) fwd_kernel(const __grid_constant_
 template <int HD, typename T, int KIND, bool BSCALE = false>
 cudaError_t launch_one(const FwdKernelParams& p, cudaStream_t stream) {
   auto kern = fwd_kernel<HD, T, KIND, BSCALE>;
-  constexpr int smem = FwdSmem<HD, sizeof(T)>::kTotal;
+  constexpr int smem = FwdSmem<HD, sizeof(T), KIND>::kTotal, threads = FwdRoles<HD, KIND>::NTHREADS;
   static std::atomic<unsigned long long> opted_in{0};  // one bit per device: the attribute is per device
   if (cudaError_t e = smem_opt_in(kern, smem, opted_in); e != cudaSuccess) return e;
   const long long grid = (long long)p.num_pairs * p.hgrid * p.B * p.num_splits;
   if (grid <= 0) return cudaSuccess;
-  kern<<<(unsigned)grid, NTHREADS, smem, stream>>>(p);
+  kern<<<(unsigned)grid, threads, smem, stream>>>(p);
   return cudaGetLastError();
 }
 

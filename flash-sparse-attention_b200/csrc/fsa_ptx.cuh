@@ -416,15 +416,25 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
   return f2_unpack(rd);
 }
 
-// s + logsigmoid(x) for two values, x given as y = x * log2(e): the arithmetic of log_sigmoid_fast, packed.
+// logsigmoid(x) for two values, x given as y = x * log2(e): the arithmetic of log_sigmoid_fast, packed. The polynomial carries the
+// minus sign (a packed operation cannot negate an operand).
+__device__ __forceinline__ float2 log_sigmoid2(float2 y) {
+  const float2 u = make_float2(ex2_approx(-fabsf(y.x)), ex2_approx(-fabsf(y.y)));
+  float2 q = fma2(u, make_float2(-0.0415511145f, -0.0415511145f), make_float2(0.157838377f, 0.157838377f));
+  q = fma2(q, u, make_float2(-0.3065611f, -0.3065611f));
+  q = fma2(q, u, make_float2(0.497030843f, 0.497030843f));
+  q = fma2(q, u, make_float2(-0.999944993f, -0.999944993f));
+  return fma2(make_float2(fminf(y.x, 0.f), fminf(y.y, 0.f)), make_float2(0.6931471806f, 0.6931471806f), mul2(q, u));
+}
+// s + logsigmoid(x)
 __device__ __forceinline__ float2 add_log_sigmoid2(float2 s, float2 y) {
   const float2 u = make_float2(ex2_approx(-fabsf(y.x)), ex2_approx(-fabsf(y.y)));
-  float2 q = fma2(u, make_float2(0.0415511145f, 0.0415511145f), make_float2(-0.157838377f, -0.157838377f));
-  q = fma2(q, u, make_float2(0.3065611f, 0.3065611f));
-  q = fma2(q, u, make_float2(-0.497030843f, -0.497030843f));
-  q = fma2(q, u, make_float2(0.999944993f, 0.999944993f));
+  float2 q = fma2(u, make_float2(-0.0415511145f, -0.0415511145f), make_float2(0.157838377f, 0.157838377f));
+  q = fma2(q, u, make_float2(-0.3065611f, -0.3065611f));
+  q = fma2(q, u, make_float2(0.497030843f, 0.497030843f));
+  q = fma2(q, u, make_float2(-0.999944993f, -0.999944993f));
   s = fma2(make_float2(fminf(y.x, 0.f), fminf(y.y, 0.f)), make_float2(0.6931471806f, 0.6931471806f), s);
-  return fma2(make_float2(-u.x, -u.y), q, s);
+  return fma2(u, q, s);
 }
 
 // sigmoid(-x) = 1 / (1 + 2^y) for two values, y = x * log2(e): one reciprocal for both. 2^y is capped at 2^62, so that the
