@@ -114,6 +114,6 @@ int dec_cluster_splits(int batch, int heads_kv, int heads_q, int head_dim, int n
 // p.cluster > 1 asks for the merge inside clusters; it is 0 afterwards when the splits went to the partials instead.
 cudaError_t launch_dec(DecKernelParams& p, int kind, int dtype, int head_dim, cudaStream_t stream);
 cudaError_t launch_combine(const CombineParams& p, int dtype, cudaStream_t stream);
-cudaError_t launch_fwd(const FwdKernelParams& p, int kind, int dtype, int head_dim, cudaStream_t stream);
+cudaError_t launch_fwd(FwdKernelParams& p, int kind, int dtype, int head_dim, cudaStream_t stream);
 
 }  // namespace fsa

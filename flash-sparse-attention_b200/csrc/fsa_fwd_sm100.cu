@@ -21,6 +21,10 @@
 // row that is only moved (and O rescaled in TMEM) when the true running maximum has drifted by
 // more than 2^8 from it: sums and outputs stay exact up to rounding because every term carries the
 // same reference, and the skip rule reads the same in terms of the reference pair (m, l).
+#include <cooperative_groups.h>
+
+#include <type_traits>
+
 #include "fsa_ptx.cuh"
 #include "fsa_params.h"
 #include "fsa_schedule.h"
@@ -58,16 +62,16 @@ struct FwdShape {
   static constexpr int VSTAGES = HD > 128 ? 1 : 2;
 };
 
-template <int HD, int ES, int KIND>
+template <int HD, int ES, int KIND, bool CL>
 struct FwdSmem {
   static constexpr int kTileBytes = TM * HD * ES;  // one Q / K / V tile of ES-byte elements
   static constexpr int kQ = 0;
   static constexpr int kK = kQ + FwdShape<HD>::QT * kTileBytes;
   static constexpr int kV = kK + FwdShape<HD>::KSTAGES * kTileBytes;
   static constexpr int kBar = kV + FwdShape<HD>::VSTAGES * kTileBytes;
-  // (maximum, sum) of a row's halves: [group][half][row] (gated)
+  // (maximum, sum) of rows: of a row's halves, [group][half][row] (gated), or of the rows whose cluster merges, [group][row]
   static constexpr int kXch = kBar + 2048;
-  static constexpr int kTotal = kXch + (FwdRoles<HD, KIND>::HALVES == 2 ? 4096 : 0) + 1024;  // barriers/flags/delta ring + alignment slack
+  static constexpr int kTotal = kXch + (FwdRoles<HD, KIND>::HALVES == 2 || CL ? 4096 : 0) + 1024;  // barriers/flags/delta ring + alignment slack
 };
 
 // Output / gate element type that goes with an input element type.
@@ -83,6 +87,8 @@ template <>
 struct OutType<__nv_fp8_e5m2> {
   using type = __nv_bfloat16;
 };
+
+constexpr int MAX_CLUSTER = 8;  // CTAs that merge at most
 
 constexpr int MAX_RANKED = FSA_FWD_MAX_RANKED;  // (query tile pair, sequence) items that a CTA ranks at most
 
@@ -177,7 +183,8 @@ __device__ __forceinline__ void mask_cols32(uint32_t* r, uint32_t bits) {
 
 // BSCALE: FP8 inputs with one scale per 128-position block (a separate instantiation: as a run-time switch it cost
 // the per-tensor FP8 forward 10 %).
-template <int HD, typename T, int KIND, bool BSCALE = false>
+// CL: the CTAs of a cluster take shares of the key tiles of the same query tiles and merge their outputs (fwd_cluster_size).
+template <int HD, typename T, int KIND, bool BSCALE = false, bool CL = false>
 __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(const __grid_constant__ FwdKernelParams p) {
   // T is the element type of Q, K, V and of P: bf16 / fp16 (kind::f16) or FP8 e4m3 / e5m2 (kind::f8f6f4,
   // flash_sparse_attn/ops/triton/flash_sparse_fwd.py:49, :84-86 under IS_QUANT). Outputs and the gate
@@ -186,7 +193,7 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
   constexpr bool F8 = ES == 1;
   constexpr int SLAB = 128 / ES;      // elements per 128-byte swizzle row
   using TO = typename OutType<T>::type;
-  using SM = FwdSmem<HD, ES, KIND>;
+  using SM = FwdSmem<HD, ES, KIND, CL>;
   using RO = FwdRoles<HD, KIND>;
   constexpr int KK_QK = HD * ES / 32;  // MMAs per S tile: every MMA consumes 32 bytes of the head dimension
   constexpr int KK_PV = TN * ES / 32;  // MMAs per P V tile: 32 bytes of the key dimension each
@@ -216,7 +223,7 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
   SeqInfo si;
   int pair;
   {
-    int idx = blockIdx.x;
+    int idx = CL ? blockIdx.x / p.cluster : blockIdx.x;
     si.head = idx % p.hgrid;
     idx /= p.hgrid;
     const int bs = idx % (p.B * p.num_splits);
@@ -268,6 +275,7 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
       si.w.sink = si.w.left = si.w.right = si.w.near_ = 0;
     }
   }
+  const int share = CL ? blockIdx.x % p.cluster : si.split, shares = CL ? p.cluster : p.num_splits;  // of the key tiles
   const int gpack = p.gpack;
   const int m_blocks_here = fsa_cdiv(si.sq * gpack, TM);  // query tiles this sequence really has
   if (pair * QT >= m_blocks_here) return;  // the grid is laid out for the longest sequence: nothing to do or to write
@@ -284,7 +292,7 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
     // the near band (block_info.py:60-64) although its eager ground truth sees those keys; like the decode
     // kernel, this one visits them (the flag only matters for that combination).
     if (walks)
-      sched[q] = fsa_fwd_schedule(si.sq, si.sk, mb, si.split, si.w, p.num_splits, TN, TM, causal, local, split_kv,
+      sched[q] = fsa_fwd_schedule(si.sq, si.sk, mb, share, si.w, shares, TN, TM, causal, local, split_kv || CL,
                                   gpack, /*cover_single_query=*/true);
     if (!walks || !q_valid[q] || fsa_fwd_sched_empty(sched[q])) {
       sched[q].n_min = sched[q].n_max = sched[q].n_max_no_mask = 0;
@@ -400,6 +408,8 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
 
+  [[maybe_unused]] auto cluster_sync = []() { cooperative_groups::this_cluster().sync(); };
+  [[maybe_unused]] auto peer = [](auto* ptr, int rank) { return cooperative_groups::this_cluster().map_shared_rank(ptr, rank); };
   const int kv_row_coord_b = (p.flags & (F_VARLEN_K | F_PAGED)) ? 0 : si.b;
 
   // Register budget: a softmax thread holds a 128-wide fp32 score row (gated: 32 scores at a time) and takes the registers
@@ -754,6 +764,11 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
       for (int q = 0; q < 2; ++q)
         if (o_started[q]) umma_commit_lead(lead, &bars->o_final[q]);
     }
+  }
+  if constexpr (CL) {  // the softmax warps merge between the two; these have too few registers to take part
+    __syncwarp();
+    cluster_sync();
+    cluster_sync();
   }
   } else {
     // =============================== softmax groups ==========================================
@@ -1145,7 +1160,111 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
         l_ref += other;
       }
     }
-    if (ok && q_valid[q]) {
+    if constexpr (CL) {
+      // ---- merge: this CTA's rows go to its shared memory, over the K and V ring (all MMAs that read it are done), 16-byte pieces
+      // swizzled by the row; then every CTA finishes 256 / cluster of the rows from the shared memory of all. A remote read takes
+      // as long as a step's MMAs, so sixteen are under way at a time. (Pushing the rows to their owner, a row a thread: 32 packets of 16
+      // bytes a store, S = 1024 at head size 64 16.6 us against 14.3.)
+#pragma unroll
+      for (int g = 0; g < 2; ++g)
+        if (ok && !fsa_fwd_sched_empty(sched[g])) ok = mbar_wait(&bars->o_final[g], 0, abort_flag);
+      tc_fence_after();
+      float4* const own = reinterpret_cast<float4*>(smem + SM::kK);        // [256 rows][HD / 4]
+      float2* const own_ml = reinterpret_cast<float2*>(smem + SM::kXch);   // [256]
+      float2* const all_ml = own_ml + 256;                                 // [CTA][row of this CTA's share]
+      float* const weight = &bars->dl[0][0];                               // likewise
+#pragma unroll
+      for (int ch = 0; ch < HD / 32; ++ch) {
+        uint32_t r[32];
+        if (ok && have_o) {
+          tmem_ld32(tO + ch * 32, r);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) r[i] = 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          own[(q * TM + row) * (HD / 4) + ((ch * 8 + i) ^ (row & 7))] =
+              make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]), __uint_as_float(r[4 * i + 2]),
+                          __uint_as_float(r[4 * i + 3]));
+      }
+      own_ml[q * TM + row] = make_float2(m_ref, l_ref);
+      cluster_sync();
+      const int rows = QT * TM / p.cluster;  // of this CTA's share, a power of two
+      // the place of row r of the share in the results, or -1
+      auto place = [&](int r, int* head, long long* tok) {
+        const int at = share * rows + r, mb_r = pair * QT + at / TM, offs = mb_r * TM + at % TM, qi = offs / gpack;
+        *head = (p.flags & F_PACK_GQA) ? si.hkv * p.G + (offs - qi * gpack) : si.head;
+        *tok = qi;
+        return mb_r < m_blocks_here && qi < si.sq && !*abort_flag;
+      };
+      const long long b_at = (p.flags & F_VARLEN_Q) ? 0 : si.b;
+      int head;
+      long long tok;
+      {  // weights: a thread for every (CTA, row)
+        const int r = tid & (rows - 1), from = tid / rows;
+        const float2 e = peer(own_ml, from)[share * rows + r];
+        all_ml[tid] = e;
+        named_bar_sync(1, 256);
+        float m_tot = -INFINITY, l_tot = 0.f;
+        for (int i = 0; i < p.cluster; ++i) m_tot = fmaxf(m_tot, all_ml[i * rows + r].x);
+        for (int i = 0; i < p.cluster; ++i) {
+          const float2 x = all_ml[i * rows + r];
+          if (x.y != 0.f) l_tot = fmaf(x.y, ex2_approx((x.x - m_tot) * cc), l_tot);
+        }
+        const bool dead = (l_tot == 0.0f) || (l_tot != l_tot);
+        weight[tid] = e.y != 0.f ? ex2_approx((e.x - m_tot) * cc) * (dead ? 1.0f : v_scale / l_tot) : 0.f;
+        if (from == 0 && place(r, &head, &tok))
+          p.lse[b_at * p.l_sb + (long long)head * p.l_sh + ((p.flags & F_VARLEN_Q) ? si.off_q + tok : tok)] =
+              dead ? -INFINITY : (m_tot * cc + log2f(l_tot)) * 0.6931471805599453f;
+        named_bar_sync(1, 256);
+      }
+      auto merge = [&](auto size) {
+        constexpr int C = decltype(size)::value, KB = 16 / C, ITEMS = (HD / 4) / C;  // 16-byte pieces of a thread: at a time, in all
+        static_assert(ITEMS % KB == 0, "whole batches");
+        const int d4 = tid % (HD / 4), r0 = tid / (HD / 4);
+        constexpr int RSTEP = 256 / (HD / 4);  // rows that the threads cover together
+#pragma unroll 1
+        for (int k0 = 0; k0 < ITEMS; k0 += KB) {
+          float4 v[C][KB];
+#pragma unroll
+          for (int i = 0; i < C; ++i) {
+            const float4* src = peer(own, i) + share * rows * (HD / 4);
+#pragma unroll
+            for (int k = 0; k < KB; ++k) {
+              const int r = r0 + (k0 + k) * RSTEP;
+              v[i][k] = src[r * (HD / 4) + (d4 ^ (r & 7))];
+            }
+          }
+#pragma unroll
+          for (int k = 0; k < KB; ++k) {
+            const int r = r0 + (k0 + k) * RSTEP;
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < C; ++i) {
+              const float w = weight[i * rows + r];
+              if (w != 0.f) {
+                acc.x = fmaf(v[i][k].x, w, acc.x);
+                acc.y = fmaf(v[i][k].y, w, acc.y);
+                acc.z = fmaf(v[i][k].z, w, acc.z);
+                acc.w = fmaf(v[i][k].w, w, acc.w);
+              }
+            }
+            if (place(r, &head, &tok) && d4 * 4 < p.D)
+              *reinterpret_cast<uint2*>(reinterpret_cast<TO*>(p.out) + b_at * p.o_sb + (si.off_q + tok) * p.o_sm +
+                                        (long long)head * p.o_sh + d4 * 4) = make_uint2(pack2<TO>(acc.x, acc.y), pack2<TO>(acc.z, acc.w));
+          }
+        }
+      };
+      if (p.cluster == 2)
+        merge(std::integral_constant<int, 2>());
+      else if (p.cluster == 4)
+        merge(std::integral_constant<int, 4>());
+      else
+        merge(std::integral_constant<int, 8>());
+      cluster_sync();  // nobody leaves while another CTA may still read its shared memory
+    } else if (ok && q_valid[q]) {
       const bool dead = (l_ref == 0.0f) || (l_ref != l_ref);
       const float inv = dead ? 1.0f : (bscaled ? v_run : v_scale) / l_ref;
       float lse = dead ? -INFINITY : m_ref * cc + log2f(l_ref);
@@ -1202,14 +1321,55 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
   }
 }
 
-template <int HD, typename T, int KIND, bool BSCALE = false>
-cudaError_t launch_one(const FwdKernelParams& p, cudaStream_t stream) {
-  auto kern = fwd_kernel<HD, T, KIND, BSCALE>;
-  constexpr int smem = FwdSmem<HD, sizeof(T), KIND>::kTotal, threads = FwdRoles<HD, KIND>::NTHREADS;
+// CTAs in a cluster, which share the key tiles of the same query tiles (1: none do). A dense call with fewer CTAs than SMs is as
+// long as its longest CTA; its key tiles go to as many CTAs as there are SMs for, at least two tiles to each of the longest, when
+// that saves four tiles: the merge takes as long as two. Causal, 8 / 2 heads, us: S = 500 stays (12.3 at head size 64, 17.1 in clusters
+// of two as first built), 1024 18.0 -> 14.3 and 2000 31.7 -> 24.8, head size 128 21.1 -> 16.8 and 35.4 -> 28.4.
+// (Not the other kinds: whether a tile is skipped depends on the tiles before it. Windows have few tiles. Whole sequences only:
+// queries over longer keys give the same bits alone and in a batch.)
+template <typename Kernel>
+int fwd_cluster_size(Kernel kern, const FwdKernelParams& p, int threads, int smem) {
+  static std::atomic<int> known[64][MAX_CLUSTER + 1];  // clusters that are resident at a time, plus one; 0: not asked yet
+  const long long base = (long long)p.num_pairs * p.hgrid * p.B;
+  int dev = 0;
+  if ((p.flags & (F_SPLIT | F_LOCAL | F_VARLEN_Q | F_VARLEN_K | F_USED_Q | F_USED_K | F_PAGED)) || p.sq != p.sk || p.tile_map || cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return 1;
+  for (int size = MAX_CLUSTER; size > 1; size >>= 1) {
+    if (base * size > device_sm_count() || p.n_tiles_k < 2 * size || p.n_tiles_k - (p.n_tiles_k + size - 1) / size < 4) continue;
+    int room = known[dev][size].load(std::memory_order_relaxed) - 1;
+    if (room < 0) {
+      room = resident_clusters(kern, size, threads, smem);
+      known[dev][size].store(room + 1, std::memory_order_relaxed);
+    }
+    if (base <= room) return size;
+  }
+  return 1;
+}
+
+template <int HD, typename T, int KIND, bool BSCALE = false, bool CL = false>
+cudaError_t launch_one(FwdKernelParams& p, cudaStream_t stream) {
+  auto kern = fwd_kernel<HD, T, KIND, BSCALE, CL>;
+  constexpr int smem = FwdSmem<HD, sizeof(T), KIND, CL>::kTotal, threads = FwdRoles<HD, KIND>::NTHREADS;
   static std::atomic<unsigned long long> opted_in{0};  // one bit per device: the attribute is per device
   if (cudaError_t e = smem_opt_in(kern, smem, opted_in); e != cudaSuccess) return e;
   const long long grid = (long long)p.num_pairs * p.hgrid * p.B * p.num_splits;
   if (grid <= 0) return cudaSuccess;
+  if constexpr (CL) {
+    p.cluster = fwd_cluster_size(kern, p, threads, smem);
+    if (p.cluster == 1) return launch_one<HD, T, KIND>(p, stream);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid * p.cluster, 1, 1);
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)p.cluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, p);
+  }
   kern<<<(unsigned)grid, threads, smem, stream>>>(p);
   return cudaGetLastError();
 }
@@ -1219,7 +1379,7 @@ cudaError_t launch_one(const FwdKernelParams& p, cudaStream_t stream) {
 // kind: KIND_*, dtype: DT_BF16 / DT_FP16, head_dim: 64 or 128. Returns cudaErrorInvalidValue for
 // unsupported combinations.
 
-cudaError_t launch_fwd(const FwdKernelParams& p, int kind, int dtype, int head_dim, cudaStream_t stream) {
+cudaError_t launch_fwd(FwdKernelParams& p, int kind, int dtype, int head_dim, cudaStream_t stream) {
   if (p.k_bscale) {  // block-scaled FP8: dense and sparse kinds at head_dim 128
     if (head_dim != 128 || kind == KIND_GATED) return cudaErrorInvalidValue;
     if (dtype == DT_E4M3)
@@ -1232,7 +1392,8 @@ cudaError_t launch_fwd(const FwdKernelParams& p, int kind, int dtype, int head_d
   }
 #define FSA_FWD_CASE(HD_, T_, DT_)                                                  \
   if (head_dim == HD_ && dtype == DT_) {                                            \
-    if (kind == KIND_DENSE) return launch_one<HD_, T_, KIND_DENSE>(p, stream);      \
+    if (kind == KIND_DENSE)                                                         \
+      return launch_one<HD_, T_, KIND_DENSE, false, (HD_ <= 128 && sizeof(T_) == 2)>(p, stream); \
     if (kind == KIND_SPARSE) return launch_one<HD_, T_, KIND_SPARSE>(p, stream);    \
     if (kind == KIND_GATED) return launch_one<HD_, T_, KIND_GATED>(p, stream);      \
   }

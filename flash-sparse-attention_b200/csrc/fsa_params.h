@@ -59,6 +59,7 @@ struct alignas(64) FwdKernelParams {
   const float* q_bscale;   // block-scaled FP8: [B, Hq, num_m_blocks], [B, Hkv, n_tiles_k] x 2; or all null
   const float* k_bscale;
   const float* v_bscale;
+  int cluster;  // CTAs that share the key tiles of the same query tiles and merge their outputs (set at the launch)
   unsigned flags;
 };
 

@@ -1,0 +1,47 @@
+"""Dense calls of few CTAs, whose key tiles are shared by the CTAs of a cluster: at the sizes where the cluster grows (none, two, four,
+eight CTAs on 148 SMs), with tiles that are not full, shares without a tile, and what keeps a call out of it."""
+
+import pytest
+import torch
+
+from fixtures import assert_close, seeded_qkv
+from oracle import eager
+
+pytestmark = pytest.mark.gpu
+
+
+# causal, 2 query heads to a KV head: 700 tokens 3 pairs of query tiles a head over 6 key tiles, 1000: 4 over 8, 2050: 9 over 17
+@pytest.mark.parametrize("seqlen, hq", [(641, 4), (700, 4), (1000, 2), (1000, 8), (1025, 2), (2050, 4), (2050, 8), (3000, 2)])
+@pytest.mark.parametrize("head_dim", [48, 64, 128])
+@pytest.mark.parametrize("causal", [True, False])
+def test_shares_of_the_keys(seqlen, hq, head_dim, causal):
+    import flash_sparse_attn as fsa
+
+    q, k, v = seeded_qkv(seqlen + hq, 1, seqlen, seqlen, hq, hq // 2, head_dim)
+    q = q * 3  # maxima that differ between the shares
+    ref, lse_ref = eager.forward(q, k, v, None, causal, return_lse=True)
+    out, lse = fsa.flash_dense_attn_func(*(t.cuda() for t in (q, k, v)), is_causal=causal, return_lse=True)
+    torch.cuda.synchronize()
+    fsa.check_status()
+    assert_close("out", out, ref)
+    assert torch.allclose(lse.cpu(), lse_ref, rtol=0, atol=2e-3)
+
+
+def test_packed_heads_infinite_keys_and_a_second_stream():
+    import flash_sparse_attn as fsa
+
+    q, k, v = (t.cuda() for t in seeded_qkv(7, 1, 1000, 1000, 8, 2, 64))
+    k[0, 300:310] = float("inf")  # a share whose scores are not numbers makes the rows that see it so
+    out = fsa.flash_dense_attn_func(q, k, v, is_causal=True)
+    assert torch.isnan(out[0, 310:]).all() and torch.isfinite(out[0, :300]).all()
+    k[0, 300:310] = 0
+    ref = fsa.flash_dense_attn_func(q, k, v, is_causal=True)
+    assert_close("packed", fsa.flash_dense_attn_func(q, k, v, is_causal=True, pack_gqa=True), ref)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        other = fsa.flash_dense_attn_func(q, k, v, is_causal=True)
+    assert torch.equal(fsa.flash_dense_attn_func(q, k, v, is_causal=True), ref)  # the same bits on every run
+    side.synchronize()
+    assert torch.equal(other, ref)
+    fsa.check_status()
