@@ -183,7 +183,6 @@ __global__ void __launch_bounds__(DWARPS * 32, OCC) dec_kernel(const DecKernelPa
   constexpr int CH = HD * ES / 16;  // 16-byte chunks per key row
   constexpr int DSTAGES = DecStages<ES>::value;
   static_assert(!F8 || HD == 128, "FP8 rows are 128 bytes: eight chunks, as the swizzle assumes");
-  static_assert(!(TR && F8), "the transposed products take 16-bit tiles");
   extern __shared__ __align__(128) uint8_t dsm[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
@@ -330,11 +329,17 @@ __global__ void __launch_bounds__(DWARPS * 32, OCC) dec_kernel(const DecKernelPa
     // TR: this lane's two rows are 2t and 2t+1 (columns of S^T); otherwise g and g + 8
     uint32_t qa[HD / 16][TR ? 2 : 4];
     if constexpr (TR) {
-      // B fragments of Q^T: head columns 16 kk + 2t, +1 and 16 kk + 8 + 2t, +1 of query row g
+      // B fragments of Q^T: head columns 16 kk + 2t, +1 and 16 kk + 8 + 2t, +1 of query row g (FP8: 16 kk + 4t .. +3)
       const int qrow = mt * 8 + g;
       const T* q0 = reinterpret_cast<const T*>(p.q) + (long long)b * p.q_sb + (long long)(hkv * p.G + qrow) * p.q_sh;
 #pragma unroll
       for (int kk = 0; kk < HD / 16; ++kk) {
+        if constexpr (F8) {
+          const uint32_t w0 = (qrow < p.G) ? *reinterpret_cast<const uint32_t*>(q0 + kk * 16 + 4 * t) : 0u;
+          qa[kk][0] = fp8x2_to_f16x2<T, 0>(w0);
+          qa[kk][1] = fp8x2_to_f16x2<T, 1>(w0);
+          continue;
+        }
         const bool lo = kk * 16 + 2 * t < p.D, hi = kk * 16 + 8 + 2 * t < p.D;
         qa[kk][0] = (qrow < p.G && lo) ? *reinterpret_cast<const uint32_t*>(q0 + kk * 16 + 2 * t) : 0u;
         qa[kk][1] = (qrow < p.G && hi) ? *reinterpret_cast<const uint32_t*>(q0 + kk * 16 + 8 + 2 * t) : 0u;
@@ -524,13 +529,31 @@ __global__ void __launch_bounds__(DWARPS * 32, OCC) dec_kernel(const DecKernelPa
       if constexpr (TR) {
         // ---- S^T = K Q^T: keys g and g + 8 (rows), query rows 2t and 2t + 1 (columns) --------------------
         float st[4] = {0.f, 0.f, 0.f, 0.f}, st_alt[4] = {0.f, 0.f, 0.f, 0.f};  // two chains of dependent MMAs
+        if constexpr (F8) {
+          // one ldmatrix.x4: two 16-byte chunks = two k-steps of key rows g and g + 8; every register carries the four head
+          // columns 4t .. 4t+3 of its chunk
 #pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-          const int r = (lane & 7) + 8 * ((lane >> 3) & 1);
-          const int ch = 2 * kk + (lane >> 4);
-          uint32_t a[4];
-          ldsm_x4(kt + r * SM::kRow + ((ch ^ (r & 7)) << 4), a[0], a[1], a[2], a[3]);
-          mma16816<TM>((kk & 1) ? st_alt : st, a, qa[kk][0], qa[kk][1]);
+          for (int kk = 0; kk < HD / 16; kk += 2) {
+            const int r = (lane & 7) + 8 * ((lane >> 3) & 1);
+            const int ch = kk + (lane >> 4);
+            uint32_t w[4];
+            ldsm_x4(kt + r * SM::kRow + ((ch ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              const uint32_t a[4] = {fp8x2_to_f16x2<T, 0>(w[2 * i]), fp8x2_to_f16x2<T, 0>(w[2 * i + 1]),
+                                     fp8x2_to_f16x2<T, 1>(w[2 * i]), fp8x2_to_f16x2<T, 1>(w[2 * i + 1])};
+              mma16816<TM>(i ? st_alt : st, a, qa[kk + i][0], qa[kk + i][1]);
+            }
+          }
+        } else {
+#pragma unroll
+          for (int kk = 0; kk < HD / 16; ++kk) {
+            const int r = (lane & 7) + 8 * ((lane >> 3) & 1);
+            const int ch = 2 * kk + (lane >> 4);
+            uint32_t a[4];
+            ldsm_x4(kt + r * SM::kRow + ((ch ^ (r & 7)) << 4), a[0], a[1], a[2], a[3]);
+            mma16816<TM>((kk & 1) ? st_alt : st, a, qa[kk][0], qa[kk][1]);
+          }
         }
 #pragma unroll
         for (int e = 0; e < 4; ++e) st[e] += st_alt[e];
@@ -604,13 +627,31 @@ __global__ void __launch_bounds__(DWARPS * 32, OCC) dec_kernel(const DecKernelPa
             }
           }
           // ---- O^T += V^T P^T: 16 head columns per MMA ------------------------------------------------------
+          if constexpr (F8) {
+            // The transposing ldmatrix moves byte PAIRS: a register holds head columns (2g, 2g+1) of its chunk for keys 2t and
+            // 2t+1. The even ones become row g of the MMA, the odd ones row g + 8.
 #pragma unroll
-          for (int jd = 0; jd < HD / 16; ++jd) {
-            const int r = (lane & 7) + 8 * (lane >> 4);
-            const int ch = 2 * jd + ((lane >> 3) & 1);
-            uint32_t a[4];
-            ldsm_x4_t(vt + r * SM::kRow + ((ch ^ (r & 7)) << 4), a[0], a[1], a[2], a[3]);
-            mma16816<TM>(o[jd], a, pb0, pb1);
+            for (int jd = 0; jd < HD / 16; jd += 2) {
+              const int r = (lane & 7) + 8 * ((lane >> 3) & 1);
+              const int ch = jd + (lane >> 4);
+              uint32_t w[4];  // chunk jd: keys 0-7, keys 8-15; chunk jd+1: keys 0-7, keys 8-15
+              ldsm_x4_t(vt + r * SM::kRow + ((ch ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
+#pragma unroll
+              for (int i = 0; i < 2; ++i) {
+                const uint32_t a[4] = {fp8x2_to_f16x2<T, 2>(w[2 * i]), fp8x2_to_f16x2<T, 3>(w[2 * i]),
+                                       fp8x2_to_f16x2<T, 2>(w[2 * i + 1]), fp8x2_to_f16x2<T, 3>(w[2 * i + 1])};
+                mma16816<TM>(o[jd + i], a, pb0, pb1);
+              }
+            }
+          } else {
+#pragma unroll
+            for (int jd = 0; jd < HD / 16; ++jd) {
+              const int r = (lane & 7) + 8 * (lane >> 4);
+              const int ch = 2 * jd + ((lane >> 3) & 1);
+              uint32_t a[4];
+              ldsm_x4_t(vt + r * SM::kRow + ((ch ^ (r & 7)) << 4), a[0], a[1], a[2], a[3]);
+              mma16816<TM>(o[jd], a, pb0, pb1);
+            }
           }
         }
       } else {
@@ -785,7 +826,13 @@ __global__ void __launch_bounds__(DWARPS * 32, OCC) dec_kernel(const DecKernelPa
     float* mo = reinterpret_cast<float*>(dsm) + warp * (16 * HD + 32);
     float* mm = mo + 16 * HD;
     float* ml = mm + 16;
-    if constexpr (TR) {
+    if constexpr (TR && F8) {
+#pragma unroll
+      for (int jd = 0; jd < HD / 16; ++jd) {
+        *reinterpret_cast<float2*>(mo + (2 * t) * HD + 16 * jd + 2 * g) = make_float2(o[jd][0], o[jd][2]);
+        *reinterpret_cast<float2*>(mo + (2 * t + 1) * HD + 16 * jd + 2 * g) = make_float2(o[jd][1], o[jd][3]);
+      }
+    } else if constexpr (TR) {
 #pragma unroll
       for (int jd = 0; jd < HD / 16; ++jd) {
         mo[(2 * t) * HD + 16 * jd + g] = o[jd][0];
@@ -1061,27 +1108,22 @@ cudaError_t launch_one(DecKernelParams& p, cudaStream_t stream) {
   } else {
     // splits merged in a cluster: at most two CTAs per SM by the rule of dec_cluster_splits
     if (p.cluster > 1) {
-      cudaError_t e;
-      if constexpr (sizeof(T) == 2)
-        e = p.G <= 8 ? launch_variant<HD, T, KIND, true, 2, true>(p, stream)
-                     : launch_variant<HD, T, KIND, false, FSA_DEC_MINBLOCKS, true>(p, stream);
-      else
-        e = launch_variant<HD, T, KIND, false, FSA_DEC_MINBLOCKS, true>(p, stream);
+      const cudaError_t e = p.G <= 8 ? launch_variant<HD, T, KIND, true, 2, true>(p, stream)
+                                     : launch_variant<HD, T, KIND, false, FSA_DEC_MINBLOCKS, true>(p, stream);
       if (e != cudaSuccess || p.cluster > 1) return e;
     }
-    if constexpr (sizeof(T) == 2) {
-      if (p.G <= 8) {
-        // Transposed products (see dec_kernel), at three or at two CTAs per SM. The grid runs in rounds of occ x SMs
-        // CTAs and a CTA takes about occ times longer with occ neighbours (the step is bandwidth bound), so the cost
-        // is rounds x CTAs per SM: 512 CTAs on 148 SMs are two rounds either way and run faster two per SM (92
-        // against 107 us), 440 CTAs are one round of three (82 us).
-        const long long sms = device_sm_count();
-        const long long ctas = (long long)p.Hkv * p.B * p.num_splits;
-        const long long per_sm = (ctas + sms - 1) / sms;
-        auto cost = [&](long long occ) { return ((ctas + occ * sms - 1) / (occ * sms)) * (per_sm < occ ? per_sm : occ); };
-        return cost(3) <= cost(2) ? launch_variant<HD, T, KIND, true, 3>(p, stream)
-                                  : launch_variant<HD, T, KIND, true, 2>(p, stream);
-      }
+    if (p.G <= 8) {
+      // Transposed products (see dec_kernel; FP8 rows, whose keys took twice as many MMAs with the query rows on the M side: 16 sequences x
+      // 1024 gathered keys 17.2 -> 14.9 us, 32 x 8000 keys 99.7 -> 60.1, 64 x 64 000 1826 -> 1641), at three or at two CTAs per SM. The grid runs in rounds of occ x SMs
+      // CTAs and a CTA takes about occ times longer with occ neighbours (the step is bandwidth bound), so the cost
+      // is rounds x CTAs per SM: 512 CTAs on 148 SMs are two rounds either way and run faster two per SM (92
+      // against 107 us), 440 CTAs are one round of three (82 us).
+      const long long sms = device_sm_count();
+      const long long ctas = (long long)p.Hkv * p.B * p.num_splits;
+      const long long per_sm = (ctas + sms - 1) / sms;
+      auto cost = [&](long long occ) { return ((ctas + occ * sms - 1) / (occ * sms)) * (per_sm < occ ? per_sm : occ); };
+      return cost(3) <= cost(2) ? launch_variant<HD, T, KIND, true, 3>(p, stream)
+                                : launch_variant<HD, T, KIND, true, 2>(p, stream);
     }
     return launch_variant<HD, T, KIND, false, FSA_DEC_MINBLOCKS>(p, stream);
   }
