@@ -34,27 +34,26 @@ namespace fsa {
 namespace {
 
 constexpr int DTN = 16;      // keys per warp tile
-// cp.async ring depth per warp: 2 tiles of 16-bit rows, 4 of FP8 rows (same shared memory, twice as many row
-// fetches in flight). Measured on the paged top-k configuration: depth 2 / 3 = 100.6 / 101.9 us in bf16, 103.4 /
-// 106.1 us in FP8; three CTAs per SM (168 registers, depth 2) 120 us.
-#ifndef FSA_DEC_STAGES16
-#define FSA_DEC_STAGES16 2
-#endif
 #ifndef FSA_DEC_MINBLOCKS
 #define FSA_DEC_MINBLOCKS 2
 #endif
-template <int ES>
-struct DecStages {
-  static constexpr int value = ES == 1 ? 2 * FSA_DEC_STAGES16 : FSA_DEC_STAGES16;
-};
 constexpr int DWARPS = 4;
 constexpr int MAX_CLUSTER = 8;  // splits that are merged inside a cluster
 
-template <int HD, int ES = 2>
+// cp.async ring depth per warp: 64 KB a CTA, two tiles of 128 16-bit columns (paged top-k configuration: depth 2 / 3 = 100.6 / 101.9 us),
+// four of FP8 rows. Of 64 16-bit columns four as well where a warp walks many tiles (DEEP: 8 sequences of 32 000 keys, 32 / 8 heads:
+// 118.6 us at two, 106.0 at four), else two: a warp of few tiles is bound by its own instructions, and the first tile is worked on once
+// the ring is full (one sequence of 500 keys: 8.2 us at two, 8.6 at four; of 4000, merged in a cluster, 10.4 and 11.5 at six).
+template <int HD, int ES, bool DEEP>
+struct DecStages {
+  static constexpr int value = ES == 1 || (HD == 64 && DEEP) ? 4 : 2;
+};
+
+template <int HD, int ES, bool DEEP>
 struct DecSmem {
   static constexpr int kRow = HD * ES;                // bytes per key row
   static constexpr int kTile = DTN * kRow;            // one K or V tile
-  static constexpr int kWarp = DecStages<ES>::value * 2 * kTile;   // ring of one warp
+  static constexpr int kWarp = DecStages<HD, ES, DEEP>::value * 2 * kTile;   // ring of one warp
   static constexpr int kMerge = DWARPS * (16 * HD * 4 + 16 * 8);  // O, m, l of every warp
   static constexpr int kTotal = (DWARPS * kWarp > kMerge ? DWARPS * kWarp : kMerge);
 };
@@ -170,7 +169,7 @@ __device__ __forceinline__ void store_out4(TO* dst, float4 a, float s) {
 // OCC: CTAs per SM the kernel is compiled for (the transposed variant exists for 2 and for 3).
 // CL: the splits of a (sequence, KV head) are one cluster and merge their results themselves (an instantiation of its own:
 // as a run-time switch it cost the bandwidth-bound calls, which never take it, 0.5 %).
-template <int HD, typename T, int KIND, bool TR, int OCC, bool CL>
+template <int HD, typename T, int KIND, bool TR, int OCC, bool CL, bool DEEP>
 __global__ void __launch_bounds__(DWARPS * 32, OCC) dec_kernel(const DecKernelParams p) {
   // T: element type of q, k, v. FP8 (e4m3 / e5m2, head size 128) tiles are copied as bytes and widened
   // exactly to fp16 in registers in front of the fp16 mma.sync; a 16-byte chunk of a key row then holds
@@ -179,9 +178,9 @@ __global__ void __launch_bounds__(DWARPS * 32, OCC) dec_kernel(const DecKernelPa
   constexpr bool F8 = ES == 1;
   using TM = typename DecTypes<T>::mma;   // mma.sync operand type
   using TO = typename DecTypes<T>::out;   // outputs, alpha, delta
-  using SM = DecSmem<HD, ES>;
+  using SM = DecSmem<HD, ES, DEEP>;
   constexpr int CH = HD * ES / 16;  // 16-byte chunks per key row
-  constexpr int DSTAGES = DecStages<ES>::value;
+  constexpr int DSTAGES = DecStages<HD, ES, DEEP>::value;
   static_assert(!F8 || HD == 128, "FP8 rows are 128 bytes: eight chunks, as the swizzle assumes");
   extern __shared__ __align__(128) uint8_t dsm[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1054,11 +1053,11 @@ bool clusters_fit(Kernel kern, int clusters, int size, int smem, std::atomic<int
 }
 
 // CL: when the clusters do not fit, p.cluster becomes 0 and nothing is launched.
-template <int HD, typename T, int KIND, bool TR, int OCC, bool CL = false>
+template <int HD, typename T, int KIND, bool TR, int OCC, bool CL = false, bool DEEP = false>
 cudaError_t launch_variant(DecKernelParams& p, cudaStream_t stream) {
-  auto kern = dec_kernel<HD, T, KIND, TR, OCC, CL>;
+  auto kern = dec_kernel<HD, T, KIND, TR, OCC, CL, DEEP>;
   // the variant for two CTAs per SM asks for enough shared memory that a third cannot join
-  constexpr int ring = DecSmem<HD, sizeof(T)>::kTotal;
+  constexpr int ring = DecSmem<HD, sizeof(T), DEEP>::kTotal;
   constexpr int smem = (TR && OCC == 2 && ring < 80 * 1024) ? 80 * 1024 : ring;
   static std::atomic<unsigned long long> opted_in{0};  // one bit per device: the attribute is per device
   if (cudaError_t e = smem_opt_in(kern, smem, opted_in); e != cudaSuccess) return e;
@@ -1122,6 +1121,11 @@ cudaError_t launch_one(DecKernelParams& p, cudaStream_t stream) {
       const long long ctas = (long long)p.Hkv * p.B * p.num_splits;
       const long long per_sm = (ctas + sms - 1) / sms;
       auto cost = [&](long long occ) { return ((ctas + occ * sms - 1) / (occ * sms)) * (per_sm < occ ? per_sm : occ); };
+      if constexpr (HD == 64 && sizeof(T) == 2) {
+        if (p.n_tiles >= 16ll * DWARPS * p.num_splits)  // sixteen tiles a warp (see DecStages)
+          return cost(3) <= cost(2) ? launch_variant<HD, T, KIND, true, 3, false, true>(p, stream)
+                                    : launch_variant<HD, T, KIND, true, 2, false, true>(p, stream);
+      }
       return cost(3) <= cost(2) ? launch_variant<HD, T, KIND, true, 3>(p, stream)
                                 : launch_variant<HD, T, KIND, true, 2>(p, stream);
     }
