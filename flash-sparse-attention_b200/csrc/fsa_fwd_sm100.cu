@@ -97,14 +97,14 @@ struct FwdBars {
   uint64_t k0_full;     // first K tile
   uint64_t kv_full[2];  // step t (slot t & 1): V(t) and K(t + 1) have landed (two producer arrivals)
   uint64_t kv_empty[2];  // signal c (slot c & 1): K(c) and V(c - 1) have been consumed; c = 0 comes from the prologue
-  // p_full: P is in TMEM (FP8: its first half), or the tile is skipped; p_rest: FP8, the second half of a kept tile
+  // p_full: P of a kept tile is in TMEM (FP8: its first half); p_rest: FP8, the second half; wg_sync: every warp of the group has
+  // read the tile's scores and voted (the kinds that skip tiles)
   uint64_t s_full[2], p_full[2], p_rest[2], o_final[2], wg_sync[2];
   uint64_t d_full[2], d_empty[2];  // gated: delta ring (stager warp -> softmax warps)
   uint32_t tmem_base;
   int abort_flag;
-  int skip_flag[2][2];   // [group][parity of the group's tile counter]
   uint64_t pair_sync[2][4];  // two threads a row: the two warps of a lane quadrant have written their halves' (maximum, sum)
-  int vote_any[2][2][8]; // [group][parity][warp]: bit0 = some row wants the tile, bit1 = some row votes skip
+  alignas(16) int vote_any[2][2][8]; // [group][parity][warp]: bit0 = some row wants the tile, bit1 = some row votes skip
   // What the producer worked out about the tiles, for the MMA issuer: low word the tile index (-1: none), then bit q: group q
   // takes part in it, bit 2 + q: it is group q's last. Slot 2: the first tile, published with k0_full. Slot t & 1: the
   // tile after step t (and whether the one of step t is a group's last), published with kv_full.
@@ -719,19 +719,35 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
         if (act[q]) {
-          ok = ok && wait_for(&bars->p_full[q], cnt[q] & 1, abort_flag);
-          if (!ok) break;
-          const bool skip = (KIND != KIND_DENSE) &&
-                            __any_sync(0xffffffffu, *reinterpret_cast<const volatile int*>(&bars->skip_flag[q][cnt[q] & 1]));
+          // A skipped tile is known from the votes, all of which come after their warps have read the scores: the next scores are
+          // issued at once, while the group is still finding out. The votes of a kept tile are there long before its P. (Verdict
+          // passed on by the group: prompts of S = 16384 with concentrated attention, 8 / 2 heads 346 us, with the votes 304, 6000
+          // tokens x 32 heads 225 and 214, without any skips S = 4096 143.0 and 142.0. Looking for P first, after a kept tile: 337, 221, 141.6.)
+          bool skip = false;
+          if (KIND != KIND_DENSE) {
+            ok = wait_for(&bars->wg_sync[q], cnt[q] & 1, abort_flag);
+            if (!ok) break;
+            int votes = 0;
+#pragma unroll
+            for (int w = 0; w < RO::GW; w += 4) {
+              const int4 v4 = *reinterpret_cast<const int4*>(&bars->vote_any[q][cnt[q] & 1][w]);
+              votes |= v4.x | v4.y | v4.z | v4.w;
+            }
+            // the maximum over rows ignores rows that are not numbers; a tile is skipped iff that maximum is < 0
+            skip = __all_sync(0xffffffffu, votes == 2);
+          }
           cnt[q]++;
+          if (!skip) {
+            ok = wait_for(&bars->p_full[q], cnt_kept[q] & 1, abort_flag);
+            if (!ok) break;
+          }
           tc_fence_after();
           if (!skip) {
 #pragma unroll ISSUE_UNROLL
             for (int kk = 0; kk < KK_PV; ++kk) {
               if (HALVES && kk == KK_PV / 2) {
-                ok = wait_for(&bars->p_rest[q], cnt_kept[q] & 1, abort_flag);  // only kept tiles arrive there
+                ok = wait_for(&bars->p_rest[q], cnt_kept[q] & 1, abort_flag);
                 if (!ok) break;
-                cnt_kept[q]++;
                 tc_fence_after();
               }
               if (F8)
@@ -742,6 +758,7 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
                              umma_desc_at(bv, kk * 2048), idesc_o, (kk > 0 || o_started[q]) ? 1u : 0u);
             }
             o_started[q] = true;
+            cnt_kept[q]++;
           }
           // last key tile of this group: tell it when its output is complete
           if (last[q]) umma_commit_lead(lead, &bars->o_final[q]);
@@ -778,7 +795,7 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
       asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
     constexpr int NC = TN / RO::HALVES;                    // key columns of a thread
     constexpr int OC = HD / RO::HALVES;                    // output columns of a thread
-    const int q = RO::HALVES == 1 ? warp >> 2 : warp >> 3;                           // group / query tile
+    const int q = RO::HALVES == 1 ? warp >> 2 : warp >> 3;   // group / query tile (a shift: a signed division costs FP8 1.8 %)
     const int half = RO::HALVES == 1 ? 0 : (warp >> 2) & 1;  // which key (and output) columns
     const int wq = warp & 3;        // warp within group == TMEM lane quadrant
     const int row = wq * 32 + lane; // row within the tile
@@ -952,7 +969,7 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
         if (lane == 0) mbar_arrive(&bars->d_empty[ds]);
         m_cur = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
         // The other half of the row: its maximum, and its sum up to the tile before. (It has read this thread's values of that tile
-        // before it arrived on p_full, without which this tile's scores were not issued.)
+        // before it voted, without which this tile's scores were not issued.)
         if constexpr (RO::HALVES == 2) {
           float2* xch = reinterpret_cast<float2*>(smem + SM::kXch) + q * 256;
           xch[half * 128 + row] = make_float2(m_cur, l_ref);
@@ -1006,6 +1023,9 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
         const unsigned drop = __ballot_sync(0xffffffffu, val < 0.0f);
         // group-wide exchange through a (bounded) mbarrier rather than bar.sync, so that an
         // aborting pipeline can never leave part of the group parked on a hardware barrier
+        // After the last vote the MMA issuer may write the next scores over these.
+        if (GATED) tmem_st_wait();
+        tc_fence_before();
         if (lane == 0) {
           bars->vote_any[q][par][half * 4 + wq] = (want ? 1 : 0) | (drop ? 2 : 0);
           mbar_arrive(&bars->wg_sync[q]);
@@ -1013,7 +1033,7 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
         // a warp holding a row that wants the tile already knows the outcome ("keep") and moves on;
         // only warps whose rows all vote "skip" have to hear from the others. Every warp still
         // arrives once per tile, and none can reach the next tile's vote before all have arrived
-        // here (the next S tile is only issued after all four warps published P or the skip).
+        // here (the next S tile is only issued after all have voted).
         if (!want) {
           ok = mbar_wait(&bars->wg_sync[q], par, abort_flag);
           if (!ok) break;
@@ -1024,25 +1044,12 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
           skip = !(v & 1) && (v & 2);
         }
       }
-      // The verdict goes to the MMA issuer (and to the tile map) right before this thread's arrival on p_full,
-      // whose release orders it: for a kept tile that is after the exponentials, not in front of them.
-      auto publish_verdict = [&](bool skipped) {
-        if (KIND != KIND_DENSE && half == 0 && wq == 0 && lane == 0) {
-          bars->skip_flag[q][par] = skipped ? 1 : 0;
-          if (p.tile_map) {
-            const long long idx =
-                ((((long long)si.b * p.hgrid + si.head) * p.num_m_blocks + mb) * p.num_splits + si.split) *
-                    p.n_tiles_k + n;
-            p.tile_map[idx] = skipped ? 2 : 1;
-          }
-        }
+      auto mark_tile = [&](int what) {
+        if (KIND != KIND_DENSE && half == 0 && wq == 0 && lane == 0 && p.tile_map)
+          p.tile_map[((((long long)si.b * p.hgrid + si.head) * p.num_m_blocks + mb) * p.num_splits + si.split) * p.n_tiles_k + n] = what;
       };
       if (skip) {
-        publish_verdict(true);
-        if (GATED) tmem_st_wait();  // the next S tile overwrites these columns
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars->p_full[q]);
+        mark_tile(2);
         continue;
       }
 
@@ -1095,7 +1102,6 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
       const float neg_mc = -(m_ref * cc);
       const float2 nm2 = make_float2(neg_mc, neg_mc);
       float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-      if (GATED) tmem_st_wait();
       constexpr int EXP_UNROLL = GATED ? 1 : NC / 32;
 #pragma unroll EXP_UNROLL
       for (int ch = 0; ch < NC / 32; ++ch) {
@@ -1132,16 +1138,15 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
           tmem_st_wait();
           tc_fence_before();
           __syncwarp();
-          publish_verdict(false);
           if (lane == 0) mbar_arrive(&bars->p_full[q]);
         }
       }
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (!HALVES) publish_verdict(false);
       if (lane == 0) mbar_arrive(HALVES ? &bars->p_rest[q] : &bars->p_full[q]);
       l_ref += (sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y);
+      mark_tile(1);  // not in front of the exponentials
       if (KIND != KIND_DENSE && RO::HALVES == 1) lg_l = lg2_approx(l_ref);  // two halves: when the other's sum is known
       have_o = true;
     }
@@ -1150,7 +1155,7 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
     if (ok && have_o) {
       ok = mbar_wait(&bars->o_final[q], 0, abort_flag);
       tc_fence_after();
-      if constexpr (RO::HALVES == 2) {  // the row's sum; the last tile's exchange has been read (its p_full came before o_final)
+      if constexpr (RO::HALVES == 2) {  // the row's sum; the last tile's exchange has been read (all votes came before o_final)
         float2* xch = reinterpret_cast<float2*>(smem + SM::kXch) + q * 256;
         xch[half * 128 + row].y = l_ref;
         __syncwarp();
