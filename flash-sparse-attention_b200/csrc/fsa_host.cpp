@@ -24,6 +24,8 @@ namespace {
 
 decltype(&fsa_decode) g_decode = nullptr;
 decltype(&fsa_fwd) g_fwd = nullptr;
+decltype(&fsa_topk_indices) g_topk = nullptr;
+decltype(&fsa_pack_scales) g_pack = nullptr;
 constexpr int MAX_DEVICES = 64;
 at::Tensor* g_status[MAX_DEVICES] = {};  // registered by the package, one int32 word per device, never replaced
 int g_sms[MAX_DEVICES] = {};
@@ -44,6 +46,41 @@ bool opt_tensor(PyObject* o, Tensor* t) {
   *t = THPVariable_Unpack(o);
   return true;
 }
+int dtype_code(at::ScalarType t) {
+  switch (t) {
+    case at::kBFloat16: return FSA_DT_BF16;
+    case at::kHalf: return FSA_DT_FP16;
+    case at::kFloat8_e4m3fn: return FSA_DT_E4M3;
+    case at::kFloat8_e5m2: return FSA_DT_E5M2;
+    default: return -1;
+  }
+}
+// The de-quantisation scales: None, one fp32 tensor of three, or a tuple of three tensors of one element and one type, which a
+// kernel packs.
+struct Scales {
+  Tensor packed, one[3];
+  bool defined() const { return packed.defined() || one[0].defined(); }
+  bool get(PyObject* o) {
+    if (!PyTuple_CheckExact(o)) return opt_tensor(o, &packed);
+    if (PyTuple_GET_SIZE(o) != 3) return false;
+    for (int i = 0; i < 3; ++i)
+      if (PyTuple_GET_ITEM(o, i) == Py_None || !opt_tensor(PyTuple_GET_ITEM(o, i), &one[i])) return false;
+    return true;
+  }
+  int type() const { return one[0].scalar_type() == at::kFloat ? FSA_DT_F32 : dtype_code(one[0].scalar_type()); }
+  bool ok(const at::Device& dev) const {
+    if (packed.defined())
+      return packed.scalar_type() == at::kFloat && packed.numel() == 3 && packed.device() == dev && packed.is_contiguous();
+    for (const Tensor& t : one)
+      if (t.scalar_type() != one[0].scalar_type() || t.numel() != 1 || t.device() != dev) return false;
+    return g_pack && type() >= 0 && type() != FSA_DT_E4M3 && type() != FSA_DT_E5M2;
+  }
+  int pack(cudaStream_t stream) {
+    if (!one[0].defined()) return FSA_OK;
+    packed = at::empty({3}, one[0].options().dtype(at::kFloat));
+    return g_pack(one[0].data_ptr(), one[1].data_ptr(), one[2].data_ptr(), type(), packed.data_ptr<float>(), stream);
+  }
+};
 bool opt_double(PyObject* o, double dflt, double* v) {
   if (o == Py_None) {
     *v = dflt;
@@ -67,15 +104,6 @@ bool get_int(PyObject* o, int64_t* v) {
   return !overflow && *v >= 0 && *v <= INT32_MAX;
 }
 
-int dtype_code(at::ScalarType t) {
-  switch (t) {
-    case at::kBFloat16: return FSA_DT_BF16;
-    case at::kHalf: return FSA_DT_FP16;
-    case at::kFloat8_e4m3fn: return FSA_DT_E4M3;
-    case at::kFloat8_e5m2: return FSA_DT_E5M2;
-    default: return -1;
-  }
-}
 bool is_fp8(int code) { return code == FSA_DT_E4M3 || code == FSA_DT_E5M2; }
 
 // An int32 vector / matrix on the device with unit inner stride (undefined passes).
@@ -90,16 +118,14 @@ T* ptr(const Tensor& t) {
 
 // q, k, v and the scales: one device (the current one), one type the kernels take as it is, a head size they take.
 // Returns the type code or -1.
-int check_qkv(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& scale, int64_t hq, int64_t hkv, int64_t d) {
+int check_qkv(const Tensor& q, const Tensor& k, const Tensor& v, const Scales& scale, int64_t hq, int64_t hkv, int64_t d) {
   if (!q.is_cuda() || k.device() != q.device() || v.device() != q.device()) return -1;
   const int dev = q.device().index();
   if (dev < 0 || dev >= MAX_DEVICES || !g_status[dev] || c10::cuda::current_device() != dev) return -1;
   const int code = dtype_code(q.scalar_type());
   if (code < 0 || k.scalar_type() != q.scalar_type() || v.scalar_type() != q.scalar_type()) return -1;
   if (is_fp8(code) != scale.defined()) return -1;
-  if (scale.defined() && (scale.scalar_type() != at::kFloat || scale.numel() != 3 || scale.device() != q.device() ||
-                          !scale.is_contiguous() || d != 128))
-    return -1;
+  if (scale.defined() && (!scale.ok(q.device()) || d != 128)) return -1;
   if (hkv <= 0 || hq % hkv != 0 || d % 16 != 0 || d <= 0 || d > 256) return -1;
   if (q.stride(-1) != 1 || k.stride(-1) != 1 || k.sizes() != v.sizes() || k.strides() != v.strides()) return -1;
   return code;
@@ -125,15 +151,16 @@ PyObject* pair(Tensor out, Tensor lse) {
 }
 
 // decode(kind, q, k, v, softmax_scale, window_sizes, softmax_threshold, is_local, num_splits, page_table, gather,
-//        seqused_k, cu_seqlens_k, max_seqlen_k, out, lse, qkv_scale) -> (out, lse), an error code, or None
+//        seqused_k, cu_seqlens_k, max_seqlen_k, out, lse, scales) -> (out, lse), an error code, or None
 PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 17 || !g_decode) return none();
   HANDLE_TH_ERRORS  // torch's own translation: an allocation that fails raises torch.OutOfMemoryError
-    Tensor q, k, v, win, table, gather, used, cu, out, lse, scale;
+    Tensor q, k, v, win, table, gather, used, cu, out, lse;
+    Scales scale;
     if (a[1] == Py_None || a[2] == Py_None || a[3] == Py_None) return none();
     if (!opt_tensor(a[1], &q) || !opt_tensor(a[2], &k) || !opt_tensor(a[3], &v) || !opt_tensor(a[5], &win) ||
         !opt_tensor(a[9], &table) || !opt_tensor(a[10], &gather) || !opt_tensor(a[11], &used) ||
-        !opt_tensor(a[12], &cu) || !opt_tensor(a[14], &out) || !opt_tensor(a[15], &lse) || !opt_tensor(a[16], &scale))
+        !opt_tensor(a[12], &cu) || !opt_tensor(a[14], &out) || !opt_tensor(a[15], &lse) || !scale.get(a[16]))
       return none();
     int64_t kind, splits = 0, max_k = 0;
     if (!get_int(a[0], &kind)) return none();
@@ -232,8 +259,10 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
     x.flags = (local ? FSA_F_LOCAL : 0) | FSA_F_LOGSIGMOID | FSA_F_SCRATCH_PARTIALS;
     x.softmax_scale = (float)sm_scale;
     x.softmax_threshold = (float)thr;
-    x.qkv_scale = ptr<float>(scale);
-    const int rc = g_decode(&x, c10::cuda::getCurrentCUDAStream(dev.index()).stream());
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+    int rc = scale.pack(stream);
+    x.qkv_scale = ptr<float>(scale.packed);
+    if (rc == FSA_OK) rc = g_decode(&x, stream);
     no_gil.reset();
     if (rc != FSA_OK) return PyLong_FromLong(rc);
     return pair(std::move(out), std::move(lse));
@@ -241,17 +270,18 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // forward(kind, q, k, v, is_causal, softmax_scale, window_sizes, softmax_threshold, is_local, num_splits, pack_gqa,
-//         cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, page_table, seqused_q, seqused_k, out, lse, qkv_scale)
+//         cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, page_table, seqused_q, seqused_k, out, lse, scales)
 //         -> (out, lse), an error code, or None. num_splits: what the launcher settled on (1: unsplit).
 PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 21 || !g_fwd) return none();
   HANDLE_TH_ERRORS  // torch's own translation: an allocation that fails raises torch.OutOfMemoryError
-    Tensor q, k, v, win, cu_q, cu_k, table, used_q, used_k, out, lse, scale;
+    Tensor q, k, v, win, cu_q, cu_k, table, used_q, used_k, out, lse;
+    Scales scale;
     if (a[1] == Py_None || a[2] == Py_None || a[3] == Py_None) return none();
     if (!opt_tensor(a[1], &q) || !opt_tensor(a[2], &k) || !opt_tensor(a[3], &v) || !opt_tensor(a[6], &win) ||
         !opt_tensor(a[11], &cu_q) || !opt_tensor(a[12], &cu_k) || !opt_tensor(a[15], &table) ||
         !opt_tensor(a[16], &used_q) || !opt_tensor(a[17], &used_k) || !opt_tensor(a[18], &out) ||
-        !opt_tensor(a[19], &lse) || !opt_tensor(a[20], &scale))
+        !opt_tensor(a[19], &lse) || !scale.get(a[20]))
       return none();
     int64_t kind, splits, max_q = 0, max_k = 0;
     if (!get_int(a[0], &kind) || !get_int(a[9], &splits) || splits < 1) return none();
@@ -364,25 +394,59 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
               (pack && hq > hkv ? FSA_F_PACK_GQA : 0) | FSA_F_LOGSIGMOID | FSA_F_ADAPT_GATE;
     x.softmax_scale = (float)sm_scale;
     x.softmax_threshold = (float)thr;
-    x.qkv_scale = ptr<float>(scale);
-    const int rc = g_fwd(&x, c10::cuda::getCurrentCUDAStream(dev.index()).stream());
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+    int rc = scale.pack(stream);
+    x.qkv_scale = ptr<float>(scale.packed);
+    if (rc == FSA_OK) rc = g_fwd(&x, stream);
     no_gil.reset();
     if (rc != FSA_OK) return PyLong_FromLong(rc);
     return pair(std::move(out), std::move(lse));
   END_HANDLE_TH_ERRORS
 }
 
-// init(address of fsa_decode, address of fsa_fwd)
+// topk(scores, k, positions as int64) -> positions, an error code, or None. Scores of 16 or 32 bits whose rows are equally far apart.
+PyObject* topk(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 3 || !g_topk || !THPVariable_CheckExact(a[0]) || !PyBool_Check(a[2])) return none();
+  HANDLE_TH_ERRORS
+    int64_t k;
+    const Tensor x = THPVariable_Unpack(a[0]);
+    if (!get_int(a[1], &k) || !x.is_cuda() || x.dim() < 1) return none();
+    const int dev = x.device().index();
+    if (dev < 0 || dev >= MAX_DEVICES || c10::cuda::current_device() != dev) return none();
+    const int type = x.scalar_type() == at::kFloat ? FSA_DT_F32 : dtype_code(x.scalar_type());
+    const int64_t len = x.size(-1);
+    if (type < 0 || is_fp8(type) || k <= 0 || k > len || len > INT32_MAX || x.numel() == 0) return none();
+    if (!x.is_contiguous() && (x.dim() != 2 || x.stride(1) != 1 || x.stride(0) < len)) return none();
+    const int64_t rows = x.numel() / len, pitch = x.is_contiguous() ? len : x.stride(0);
+    if (rows > INT32_MAX) return none();
+    auto shape = x.sizes().vec();
+    shape.back() = k;
+    const bool wide = a[2] == Py_True;
+    std::optional<NoGil> no_gil(std::in_place);
+    Tensor out = at::empty(shape, x.options().dtype(wide ? at::kLong : at::kInt));
+    const int rc = g_topk(x.data_ptr(), type, (int)rows, (int)len, pitch, (int)k, out.data_ptr(), wide ? 1 : 0,
+                          c10::cuda::getCurrentCUDAStream(dev).stream());
+    no_gil.reset();
+    if (rc != FSA_OK) return PyLong_FromLong(rc);
+    return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+// init(addresses of fsa_decode, fsa_fwd[, fsa_topk_indices, fsa_pack_scales])
 PyObject* init(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  if (n != 2) {
-    PyErr_SetString(PyExc_TypeError, "init takes two addresses");
+  if (n != 2 && n != 4) {
+    PyErr_SetString(PyExc_TypeError, "init takes two or four addresses");
     return nullptr;
   }
-  void* dec = PyLong_AsVoidPtr(a[0]);
-  void* fwd = PyErr_Occurred() ? nullptr : PyLong_AsVoidPtr(a[1]);
+  void* at[4] = {};
+  for (Py_ssize_t i = 0; i < n && !PyErr_Occurred(); ++i) at[i] = PyLong_AsVoidPtr(a[i]);
   if (PyErr_Occurred()) return nullptr;
-  g_decode = reinterpret_cast<decltype(g_decode)>(dec);
-  g_fwd = reinterpret_cast<decltype(g_fwd)>(fwd);
+  if (n == 4) {
+    g_topk = reinterpret_cast<decltype(g_topk)>(at[2]);
+    g_pack = reinterpret_cast<decltype(g_pack)>(at[3]);
+  }
+  g_decode = reinterpret_cast<decltype(g_decode)>(at[0]);
+  g_fwd = reinterpret_cast<decltype(g_fwd)>(at[1]);
   return none();
 }
 
@@ -413,6 +477,7 @@ PyMethodDef methods[] = {
     {"set_status", reinterpret_cast<PyCFunction>(set_status), METH_FASTCALL, nullptr},
     {"decode", reinterpret_cast<PyCFunction>(decode), METH_FASTCALL, nullptr},
     {"forward", reinterpret_cast<PyCFunction>(forward), METH_FASTCALL, nullptr},
+    {"topk", reinterpret_cast<PyCFunction>(topk), METH_FASTCALL, nullptr},
     {"decode_num_splits", reinterpret_cast<PyCFunction>(decode_num_splits), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -417,7 +417,8 @@ def _load_host(lib):
         here = (ABI_VERSION, re.match(r"\d+\.\d+\.\d+", torch.__version__).group())
         if built_for != here:
             raise ImportError(f"built for {built_for}, not for {here} (ABI version, torch)")
-        host.init(ctypes.cast(lib.fsa_decode, c_void_p).value, ctypes.cast(lib.fsa_fwd, c_void_p).value)
+        host.init(ctypes.cast(lib.fsa_decode, c_void_p).value, ctypes.cast(lib.fsa_fwd, c_void_p).value,
+                  ctypes.cast(lib.fsa_topk_indices, c_void_p).value, ctypes.cast(lib.fsa_pack_scales, c_void_p).value)
     except (ImportError, AttributeError) as e:
         _host = None
         warnings.warn("flash_sparse_attn/_host.so is missing or does not load; calls go through the slower Python launchers until "

@@ -88,14 +88,13 @@ def attn_decode(
     if not query.is_cuda:
         raise RuntimeError("flash_sparse_attn (B200 build) only runs on CUDA tensors; there is no CPU path")
     device = query.device
-    scales = None  # packed for the native launcher; kept when it declines the call
     if (kind != "gated" and (tile_mn is None or page_table is None) and tile_map is None and not partial_only
             and workspace is None and threshold_seqlen_k is None and key_range is None and packed_partials is None
             and gather_count is None and peers is None
             and (not is_quant or quant.uniform_scales(query_scale, key_scale, value_scale, device))):
         host = _lib.native()
         if host is not None:
-            scales = quant.scales_f32(query_scale, key_scale, value_scale, device) if is_quant else None
+            scales = (query_scale, key_scale, value_scale) if is_quant else None
             res = host.decode(_KIND[kind], query, key, value, softmax_scale, window_sizes, softmax_threshold, is_local,
                               num_splits, page_table, gather_kv_indices, seqused_k, cu_seqlens_k, max_seqlen_k, out, lse,
                               scales)
@@ -140,7 +139,7 @@ def attn_decode(
     qkv_scale = None
     if is_quant:
         # FP8 query and cache: widened (exactly) to bf16 before the kernel; scales as in the forward
-        qkv_scale = scales if scales is not None else quant.scales_f32(query_scale, key_scale, value_scale, device)
+        qkv_scale = quant.scales_f32(query_scale, key_scale, value_scale, device)
         native = head_dim == 128 and query.dtype == key.dtype == value.dtype
         if not native:  # other head sizes / mixed formats: widen the tensors and run the 16-bit kernel
             query, key, value = (quant.widen_fp8(t, torch.bfloat16) for t in (query, key, value))

@@ -125,12 +125,11 @@ def attn_forward(
         ragged = batch > 1 and (varlen or seqused_k is not None or seqused_q is not None)
         num_splits = forward_num_splits(batch, seqlen_q, seqlen_k, num_heads_q, num_heads_kv, head_dim, group_packed, is_local,
                                         ragged, utils.device_num_sms(device))
-    scales = None  # packed for the native launcher; kept when it declines the call
     if (kind != "gated" and (tile_mn is None or page_table is None) and tile_map is None
             and (not is_quant or quant.uniform_scales(query_scale, key_scale, value_scale, device))):
         host = _lib.native()
         if host is not None:
-            scales = quant.scales_f32(query_scale, key_scale, value_scale, device) if is_quant else None
+            scales = (query_scale, key_scale, value_scale) if is_quant else None
             res = host.forward(_KIND[kind], query, key, value, is_causal, softmax_scale, window_sizes, softmax_threshold,
                                is_local, num_splits, pack_gqa, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k,
                                page_table, seqused_q, seqused_k, out, lse, scales)
@@ -162,7 +161,7 @@ def attn_forward(
     elif is_quant:
         # FP8 inputs: widened (exactly) to bf16 in one pass; the per-tensor scales stay on the device and
         # enter the kernel as in scheduler.py:298-307 (logit scale *= q_scale * k_scale, out *= v_scale)
-        qkv_scale = scales if scales is not None else quant.scales_f32(query_scale, key_scale, value_scale, device)
+        qkv_scale = quant.scales_f32(query_scale, key_scale, value_scale, device)
         native = head_dim == 128 and query.dtype == key.dtype == value.dtype
         if not native:  # other head sizes / mixed formats: widen (exactly) to bf16 and use the 16-bit kernel
             query, key, value = (quant.widen_fp8(t, torch.bfloat16) for t in (query, key, value))

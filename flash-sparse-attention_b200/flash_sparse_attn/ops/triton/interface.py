@@ -54,6 +54,55 @@ def _swap(tile_mn):
     return (tile_mn[1], tile_mn[0]) if tile_mn is not None else None
 
 
+def _forward(kind, varlen, query, key, value, alpha, delta, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, is_causal,
+             softmax_scale, query_scale, key_scale, value_scale, window_sizes, softmax_threshold, gate_threshold,
+             is_logsigmoid_gate, is_adapt_gate, is_local, is_quant, is_split_kv, is_split_qo, pack_gqa, num_splits, page_table,
+             seqused_q, seqused_k, out, lse, is_autotune, tile_mn, skip_checks):
+    """The forward pass: what the call settled on (the backward needs it), out and lse."""
+    single = (max_seqlen_q == 1) if varlen else (query.shape[1] == 1)
+    is_causal, is_local, is_split_kv, is_split_qo = _normalise(
+        single, is_causal, window_sizes, is_local, num_splits, is_split_kv, is_split_qo
+    )
+    query, key, value, query_scale, key_scale, value_scale = _maybe_quantize(
+        is_quant, query, key, value, query_scale, key_scale, value_scale, cu_seqlens_q, cu_seqlens_k,
+        max_seqlen_q, max_seqlen_k, block_ok=(kind != "gated" and not pack_gqa and page_table is None)
+    )
+    if kind == "gated":
+        # kernels read alpha as [.., heads, positions] rows, like the reference's transposed copies
+        alpha = alpha.transpose(-2, -1).contiguous()
+        delta = delta.transpose(-2, -1).contiguous()
+
+    out, lse, softmax_scale, softmax_threshold, gate_threshold = attn_forward(
+        kind, query, key, value, alpha=alpha, delta=delta, cu_seqlens_q=cu_seqlens_q,
+        cu_seqlens_k=cu_seqlens_k, max_seqlen_q=max_seqlen_q, max_seqlen_k=max_seqlen_k, is_causal=is_causal,
+        softmax_scale=softmax_scale, query_scale=query_scale, key_scale=key_scale, value_scale=value_scale,
+        window_sizes=window_sizes, softmax_threshold=softmax_threshold, gate_threshold=gate_threshold,
+        is_logsigmoid_gate=is_logsigmoid_gate, is_adapt_gate=is_adapt_gate, is_local=is_local,
+        is_quant=is_quant, is_split_kv=is_split_kv, pack_gqa=pack_gqa, num_splits=num_splits,
+        page_table=page_table, seqused_q=seqused_q, seqused_k=seqused_k, out=out, lse=lse,
+        is_autotune=is_autotune, tile_mn=tile_mn, skip_checks=skip_checks,
+    )
+    return (query, key, value, alpha, delta, query_scale, key_scale, value_scale, is_causal, is_local, is_split_qo, out, lse,
+            softmax_scale, softmax_threshold, gate_threshold)
+
+
+def _nothing_to_record(*tensors) -> bool:
+    """Whether the autograd Function would only run its forward: plain tensors, none of which a gradient is asked for, and no
+    transform, dual number, trace or compiler that wants to see the Function."""
+    if torch.compiler.is_compiling():
+        return False
+    if torch.is_grad_enabled():
+        for t in tensors:
+            if t is not None and (type(t) is not torch.Tensor or t.requires_grad):
+                return False
+    else:
+        for t in tensors:
+            if t is not None and type(t) is not torch.Tensor:
+                return False
+    return not (torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0
+                or torch._C._get_tracing_state() is not None)
+
+
 class _AttnFunc(torch.autograd.Function):
     """Shared forward/backward for the batched and packed, dense / sparse / gated operators."""
 
@@ -63,30 +112,12 @@ class _AttnFunc(torch.autograd.Function):
                 softmax_threshold, gate_threshold, is_logsigmoid_gate, is_adapt_gate, is_local, is_quant,
                 is_split_kv, is_split_qo, pack_gqa, num_splits, page_table, seqused_q, seqused_k, out, lse,
                 is_autotune, tile_mn, skip_checks, return_lse):
-        single = (max_seqlen_q == 1) if varlen else (query.shape[1] == 1)
-        is_causal, is_local, is_split_kv, is_split_qo = _normalise(
-            single, is_causal, window_sizes, is_local, num_splits, is_split_kv, is_split_qo
-        )
-        query, key, value, query_scale, key_scale, value_scale = _maybe_quantize(
-            is_quant, query, key, value, query_scale, key_scale, value_scale, cu_seqlens_q, cu_seqlens_k,
-            max_seqlen_q, max_seqlen_k, block_ok=(kind != "gated" and not pack_gqa and page_table is None)
-        )
-        if kind == "gated":
-            # kernels read alpha as [.., heads, positions] rows, like the reference's transposed copies
-            alpha = alpha.transpose(-2, -1).contiguous()
-            delta = delta.transpose(-2, -1).contiguous()
-
-        out, lse, softmax_scale, softmax_threshold, gate_threshold = attn_forward(
-            kind, query, key, value, alpha=alpha, delta=delta, cu_seqlens_q=cu_seqlens_q,
-            cu_seqlens_k=cu_seqlens_k, max_seqlen_q=max_seqlen_q, max_seqlen_k=max_seqlen_k, is_causal=is_causal,
-            softmax_scale=softmax_scale, query_scale=query_scale, key_scale=key_scale, value_scale=value_scale,
-            window_sizes=window_sizes, softmax_threshold=softmax_threshold, gate_threshold=gate_threshold,
-            is_logsigmoid_gate=is_logsigmoid_gate, is_adapt_gate=is_adapt_gate, is_local=is_local,
-            is_quant=is_quant, is_split_kv=is_split_kv, pack_gqa=pack_gqa, num_splits=num_splits,
-            page_table=page_table, seqused_q=seqused_q, seqused_k=seqused_k, out=out, lse=lse,
-            is_autotune=is_autotune, tile_mn=tile_mn, skip_checks=skip_checks,
-        )
-
+        (query, key, value, alpha, delta, query_scale, key_scale, value_scale, is_causal, is_local, is_split_qo, out, lse,
+         softmax_scale, softmax_threshold, gate_threshold) = _forward(
+            kind, varlen, query, key, value, alpha, delta, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, is_causal,
+            softmax_scale, query_scale, key_scale, value_scale, window_sizes, softmax_threshold, gate_threshold,
+            is_logsigmoid_gate, is_adapt_gate, is_local, is_quant, is_split_kv, is_split_qo, pack_gqa, num_splits, page_table,
+            seqused_q, seqused_k, out, lse, is_autotune, tile_mn, skip_checks)
         ctx.save_for_backward(query, key, value, alpha, delta, out, lse, cu_seqlens_q, cu_seqlens_k, seqused_q,
                               seqused_k)
         ctx.kind, ctx.varlen = kind, varlen
@@ -143,6 +174,13 @@ def _apply(kind, varlen, query, key, value, alpha, delta, cu_seqlens_q, cu_seqle
      page_table, seqused_q, seqused_k, out, lse) = _contig(
         query, key, value, alpha, delta, cu_seqlens_q, cu_seqlens_k, query_scale, key_scale, value_scale,
         window_sizes, page_table, seqused_q, seqused_k, out, lse)
+    # (a caller's result buffers: the Function hands them back through views of their own)
+    if out is None and lse is None and _nothing_to_record(query, key, value, alpha, delta):
+        res = _forward(kind, varlen, query, key, value, alpha, delta, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k,
+                       is_causal, softmax_scale, query_scale, key_scale, value_scale, window_sizes, softmax_threshold,
+                       gate_threshold, is_logsigmoid_gate, is_adapt_gate, is_local, is_quant, is_split_kv, is_split_qo, pack_gqa,
+                       num_splits, page_table, seqused_q, seqused_k, out, lse, is_autotune, tile_mn, skip_checks)
+        return (res[11], res[12]) if return_lse else res[11]
     return _AttnFunc.apply(kind, varlen, query, key, value, alpha, delta, cu_seqlens_q, cu_seqlens_k, max_seqlen_q,
                            max_seqlen_k, is_causal, softmax_scale, query_scale, key_scale, value_scale, window_sizes,
                            softmax_threshold, gate_threshold, is_logsigmoid_gate, is_adapt_gate, is_local, is_quant,

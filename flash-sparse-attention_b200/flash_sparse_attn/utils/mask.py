@@ -19,6 +19,13 @@ def topk_indices(attention_bias: torch.Tensor, window_size: int, dtype: torch.dt
     if not attention_bias.is_cuda:
         raise RuntimeError("flash_sparse_attn (B200 build) only runs on CUDA tensors; there is no CPU path")
     assert dtype in (torch.int32, torch.int64)
+    host = _lib.native()
+    if host is not None:
+        res = host.topk(attention_bias, window_size, dtype == torch.int64)
+        if res is not None:
+            if type(res) is int:
+                _lib.check(res, "fsa_topk_indices")
+            return res
     x = attention_bias.detach()
     n = x.shape[-1]
     assert 0 < window_size <= n, "window_size must be in [1, key_len]"
