@@ -14,6 +14,7 @@ namespace {
 // _dec_combine_kernel (flash_dec_combine.py:15-153).
 template <typename T, int VEC>
 __global__ void __launch_bounds__(256) combine_kernel(CombineParams p) {
+  after_previous();
   const int lane = threadIdx.x & 31;
   const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   long long buf_off = 0;
@@ -168,6 +169,7 @@ __device__ __forceinline__ RowPos locate_row(long long item, int heads, int varl
 // the sequence count as 0, like the reference's masked loads (scheduler.py:1658-1691).
 template <typename T>
 __global__ void __launch_bounds__(256) gate_ext_kernel(GateExtParams p) {
+  after_previous();
   const int lane = threadIdx.x & 31;
   long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const long long n_alpha = (long long)p.B * p.hgrid * p.num_m_blocks;
@@ -233,6 +235,7 @@ constexpr int PP_ITEMS = 1;  // (row, head) items per lane group in the pre / po
 // flash_sparse_attn/ops/triton/flash_bwd_preprocess.py:170-195.
 template <typename T>
 __global__ void __launch_bounds__(256) bwd_pre_kernel(BwdPreParams p) {
+  after_previous();
   const int lpr = p.head_dim_pad >> 3;  // lanes per row (8 or 16); lanes past the real head size idle
   const int lane = threadIdx.x & 31, sub = lane % lpr;
   const int groups = 32 / lpr;
@@ -294,6 +297,7 @@ __global__ void __launch_bounds__(256) bwd_pre_kernel(BwdPreParams p) {
 // head_dim / 8 lanes per (query row, head). flash_sparse_attn/ops/triton/flash_bwd_postprocess.py:60-148.
 template <typename T>
 __global__ void __launch_bounds__(256) bwd_post_kernel(BwdPostParams p) {
+  after_previous();
   const int lpr = p.head_dim_pad >> 3;
   const int lane = threadIdx.x & 31, sub = lane % lpr;
   const int groups = 32 / lpr;
@@ -340,6 +344,7 @@ __global__ void __launch_bounds__(256) bwd_post_kernel(BwdPostParams p) {
 }
 
 __global__ void __launch_bounds__(128) dq_order_kernel(DqOrderParams p) {
+  after_previous();
   const long long item = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (item >= (long long)p.B * p.Hkv * p.num_m_blocks) return;
   const int m = (int)(item % p.num_m_blocks);
@@ -371,6 +376,7 @@ __global__ void __launch_bounds__(128) dq_order_kernel(DqOrderParams p) {
 
 template <typename T>
 __global__ void __launch_bounds__(256) flat_sum_kernel(FlatSumParams p) {
+  after_previous();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= p.n) return;
   float acc = 0.f;
@@ -381,6 +387,7 @@ __global__ void __launch_bounds__(256) flat_sum_kernel(FlatSumParams p) {
 // One warp per (key row, head): sum the split partials in split order (fixed order, deterministic).
 template <typename T>
 __global__ void __launch_bounds__(256) split_sum_kernel(SplitSumParams p) {
+  after_previous();
   const int lane = threadIdx.x & 31;
   const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (item >= (long long)p.rows * p.heads) return;
@@ -416,10 +423,8 @@ cudaError_t launch_bwd_pre(const BwdPreParams& p, int dtype, cudaStream_t stream
   const int per_block = 8 * (32 / (p.head_dim_pad >> 3)) * PP_ITEMS;
   const unsigned grid = (unsigned)((items + per_block - 1) / per_block);
   if (dtype == DT_BF16)
-    bwd_pre_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(p);
-  else
-    bwd_pre_kernel<__half><<<grid, 256, 0, stream>>>(p);
-  return cudaGetLastError();
+    return launch_early(bwd_pre_kernel<__nv_bfloat16>, grid, 256, 0, stream, 1, p);
+  return launch_early(bwd_pre_kernel<__half>, grid, 256, 0, stream, 1, p);
 }
 
 cudaError_t launch_bwd_post(const BwdPostParams& p, int dtype, cudaStream_t stream) {
@@ -430,10 +435,8 @@ cudaError_t launch_bwd_post(const BwdPostParams& p, int dtype, cudaStream_t stre
   const int per_block = 8 * (32 / (p.head_dim_pad >> 3)) * PP_ITEMS;
   const unsigned grid = (unsigned)((items + per_block - 1) / per_block);
   if (dtype == DT_BF16)
-    bwd_post_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(p);
-  else
-    bwd_post_kernel<__half><<<grid, 256, 0, stream>>>(p);
-  return cudaGetLastError();
+    return launch_early(bwd_post_kernel<__nv_bfloat16>, grid, 256, 0, stream, 1, p);
+  return launch_early(bwd_post_kernel<__half>, grid, 256, 0, stream, 1, p);
 }
 
 cudaError_t launch_gate_ext(const GateExtParams& p, int dtype, cudaStream_t stream) {
@@ -441,27 +444,22 @@ cudaError_t launch_gate_ext(const GateExtParams& p, int dtype, cudaStream_t stre
   if (items <= 0) return cudaSuccess;
   const unsigned grid = (unsigned)((items + 7) / 8);
   if (dtype == DT_FP16)
-    gate_ext_kernel<__half><<<grid, 256, 0, stream>>>(p);
-  else
-    gate_ext_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(p);
-  return cudaGetLastError();
+    return launch_early(gate_ext_kernel<__half>, grid, 256, 0, stream, 1, p);
+  return launch_early(gate_ext_kernel<__nv_bfloat16>, grid, 256, 0, stream, 1, p);
 }
 
 cudaError_t launch_dq_order(const DqOrderParams& p, cudaStream_t stream) {
   const long long items = (long long)p.B * p.Hkv * p.num_m_blocks;
   if (items <= 0) return cudaSuccess;
-  dq_order_kernel<<<(unsigned)((items + 127) / 128), 128, 0, stream>>>(p);
-  return cudaGetLastError();
+  return launch_early(dq_order_kernel, (unsigned)((items + 127) / 128), 128, 0, stream, 1, p);
 }
 
 cudaError_t launch_flat_sum(const FlatSumParams& p, int dtype, cudaStream_t stream) {
   if (p.n <= 0) return cudaSuccess;
   const unsigned grid = (unsigned)((p.n + 255) / 256);
   if (dtype == DT_BF16)
-    flat_sum_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(p);
-  else
-    flat_sum_kernel<__half><<<grid, 256, 0, stream>>>(p);
-  return cudaGetLastError();
+    return launch_early(flat_sum_kernel<__nv_bfloat16>, grid, 256, 0, stream, 1, p);
+  return launch_early(flat_sum_kernel<__half>, grid, 256, 0, stream, 1, p);
 }
 
 cudaError_t launch_split_sum(const SplitSumParams& p, int dtype, cudaStream_t stream) {
@@ -469,10 +467,8 @@ cudaError_t launch_split_sum(const SplitSumParams& p, int dtype, cudaStream_t st
   if (items <= 0) return cudaSuccess;
   const unsigned grid = (unsigned)((items + 7) / 8);
   if (dtype == DT_BF16)
-    split_sum_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(p);
-  else
-    split_sum_kernel<__half><<<grid, 256, 0, stream>>>(p);
-  return cudaGetLastError();
+    return launch_early(split_sum_kernel<__nv_bfloat16>, grid, 256, 0, stream, 1, p);
+  return launch_early(split_sum_kernel<__half>, grid, 256, 0, stream, 1, p);
 }
 
 cudaError_t launch_combine(const CombineParams& p, int dtype, cudaStream_t stream) {
@@ -482,18 +478,11 @@ cudaError_t launch_combine(const CombineParams& p, int dtype, cudaStream_t strea
   const unsigned grid = (unsigned)((items + warps - 1) / warps);
   if (p.head_dim % 4 != 0 || p.head_dim > 256) return cudaErrorInvalidValue;
   // VEC floats per lane, 32 lanes: head_dim <= 128 -> 4, <= 256 -> 8
-  if (p.head_dim <= 128) {
-    if (dtype == DT_BF16)
-      combine_kernel<__nv_bfloat16, 4><<<grid, warps * 32, 0, stream>>>(p);
-    else
-      combine_kernel<__half, 4><<<grid, warps * 32, 0, stream>>>(p);
-  } else {
-    if (dtype == DT_BF16)
-      combine_kernel<__nv_bfloat16, 8><<<grid, warps * 32, 0, stream>>>(p);
-    else
-      combine_kernel<__half, 8><<<grid, warps * 32, 0, stream>>>(p);
-  }
-  return cudaGetLastError();
+  if (p.head_dim <= 128)
+    return dtype == DT_BF16 ? launch_early(combine_kernel<__nv_bfloat16, 4>, grid, warps * 32, 0, stream, 1, p)
+                            : launch_early(combine_kernel<__half, 4>, grid, warps * 32, 0, stream, 1, p);
+  return dtype == DT_BF16 ? launch_early(combine_kernel<__nv_bfloat16, 8>, grid, warps * 32, 0, stream, 1, p)
+                          : launch_early(combine_kernel<__half, 8>, grid, warps * 32, 0, stream, 1, p);
 }
 
 }  // namespace fsa

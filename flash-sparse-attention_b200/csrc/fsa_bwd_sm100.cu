@@ -181,6 +181,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) bwd_kernel(const __grid_constant_
   constexpr bool OWN_DQ = HD == 64;
   constexpr uint32_t TMEM_S = 0, TMEM_DP = 128, TMEM_DV = 256, TMEM_DK = 384, TMEM_DQ = OWN_DQ ? 320 : TMEM_DP;
 
+  after_previous();
   extern __shared__ __align__(1024) uint8_t smem[];
   BwdBars* bars = reinterpret_cast<BwdBars*>(smem + SM::kBar);
   volatile int* abort_flag = &bars->abort_flag;
@@ -1279,8 +1280,7 @@ cudaError_t launch_one(const BwdKernelParams& p, cudaStream_t stream) {
   if (cudaError_t e = smem_opt_in(kern, smem, opted_in); e != cudaSuccess) return e;
   const long long grid = (long long)p.n_tiles_k * p.Hkv * p.B * p.num_splits;
   if (grid <= 0) return cudaSuccess;
-  kern<<<(unsigned)grid, NTHREADS, smem, stream>>>(p);
-  return cudaGetLastError();
+  return launch_early(kern, (unsigned)grid, NTHREADS, smem, stream, 1, p);
 }
 
 // The dense and sparse kinds take a dQ tile at once at head size 128, where it leaves the block that dP^T of the next step waits for. Two

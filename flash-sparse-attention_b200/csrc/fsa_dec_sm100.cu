@@ -182,6 +182,7 @@ __global__ void __launch_bounds__(DWARPS * 32, OCC) dec_kernel(const DecKernelPa
   constexpr int CH = HD * ES / 16;  // 16-byte chunks per key row
   constexpr int DSTAGES = DecStages<HD, ES, DEEP>::value;
   static_assert(!F8 || HD == 128, "FP8 rows are 128 bytes: eight chunks, as the swizzle assumes");
+  after_previous();
   extern __shared__ __align__(128) uint8_t dsm[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
@@ -984,6 +985,7 @@ __global__ void __launch_bounds__(DWARPS * 32, OCC) dec_kernel(const DecKernelPa
 // these before it requests a tile's rows.
 template <typename TO>
 __global__ void __launch_bounds__(256) dec_gate_ext_kernel(const DecKernelParams p) {
+  after_previous();
   const int lane = threadIdx.x & 31, l16 = lane & 15;
   const long long item = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 2 + (lane >> 4);
   const long long n_items = (long long)p.B * p.Hkv * p.n_tiles;
@@ -1074,28 +1076,16 @@ cudaError_t launch_variant(DecKernelParams& p, cudaStream_t stream) {
   if (KIND == KIND_GATED && p.gate_ws) {
     const long long items = (long long)p.B * p.Hkv * p.n_tiles;
     if (items > 0) {
-      dec_gate_ext_kernel<typename DecTypes<T>::out><<<(unsigned)((items + 15) / 16), 256, 0, stream>>>(p);
-      if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
+      if (cudaError_t e = launch_early(dec_gate_ext_kernel<typename DecTypes<T>::out>, (unsigned)((items + 15) / 16), 256, 0, stream, 1, p);
+          e != cudaSuccess)
+        return e;
     }
   }
   if constexpr (CL) {
     static_assert(HD <= 128 && DWARPS * (16 * HD + 32) * 4 + (16 * HD + 32) * 4 <= ring, "the merged state fits behind the warps'");
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid, 1, 1);
-    cfg.blockDim = dim3(DWARPS * 32, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)p.cluster;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, p);
+    return launch_early(kern, (unsigned)grid, DWARPS * 32, smem, stream, p.cluster, p);
   }
-  kern<<<(unsigned)grid, DWARPS * 32, smem, stream>>>(p);
-  return cudaGetLastError();
+  return launch_early(kern, (unsigned)grid, DWARPS * 32, smem, stream, 1, p);
 }
 
 template <int HD, typename T, int KIND>

@@ -210,6 +210,7 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
   // 16 / 4 heads of 192: 501 us, 523 with the record; a 1024-token window 183 and 187).
   constexpr bool HANDED = KIND == KIND_GATED || HD <= 128;
 
+  after_previous();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   FwdBars* bars = reinterpret_cast<FwdBars*>(smem + SM::kBar);
@@ -1361,22 +1362,9 @@ cudaError_t launch_one(FwdKernelParams& p, cudaStream_t stream) {
   if constexpr (CL) {
     p.cluster = fwd_cluster_size(kern, p, threads, smem);
     if (p.cluster == 1) return launch_one<HD, T, KIND>(p, stream);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid * p.cluster, 1, 1);
-    cfg.blockDim = dim3(threads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)p.cluster;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, p);
+    return launch_early(kern, (unsigned)grid * p.cluster, threads, smem, stream, p.cluster, p);
   }
-  kern<<<(unsigned)grid, threads, smem, stream>>>(p);
-  return cudaGetLastError();
+  return launch_early(kern, (unsigned)grid, threads, smem, stream, 1, p);
 }
 
 }  // namespace

@@ -178,6 +178,41 @@ inline int resident_clusters(Kernel kern, int size, int threads, int smem) {
   return n;
 }
 
+// Launch whose blocks may be set up while the kernel in front of it in the stream still runs: the kernel has to begin with
+// after_previous(). `cluster` CTAs form a cluster (1: none). What it saves is 1 to 2 us between two kernels: a decode step of one
+// sequence over and over 12.3 -> 10.4 us, top-k selection, scales and FP8 decode 33.3 -> 29.6, a short prompt 16.4 -> 14.6, a paged
+// batch and its combine 186.9 -> 184.2.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_early(void (*kern)(Params...), unsigned grid, int threads, int smem, cudaStream_t stream, int cluster,
+                                Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid, 1, 1);
+  cfg.blockDim = dim3((unsigned)threads, 1, 1);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
+}
+
+#ifdef __CUDACC__
+// In front of everything that a kernel reads or writes: waits until the kernel in front of it has completed and what it wrote is
+// visible, then lets the kernel behind it be set up; blocks of that one are only started once all of this kernel's have been, so they
+// take no room from them. (The other way round three kernels deep: single calls the same, decode of 4 sequences x 4000 keys
+// 12.7 -> 13.9 us, whose blocks find the SMs unevenly taken.)
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+#endif
+
 // Multiprocessor count of the current device (148 on B200), cached per device ordinal.
 inline int device_sm_count() {
   static std::atomic<int> cache[64];

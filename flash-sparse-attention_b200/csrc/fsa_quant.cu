@@ -228,6 +228,7 @@ int widen_typed(const void* x, void* out, const void* scale, long long n, int fp
 // took up to seven.
 template <typename T>
 __global__ void pack_scales_kernel(const void* q, const void* k, const void* v, float* out) {
+  after_previous();
   const void* src[3] = {q, k, v};
   if (threadIdx.x < 3) out[threadIdx.x] = float(*reinterpret_cast<const T*>(src[threadIdx.x]));
 }
@@ -298,13 +299,14 @@ int fsa_quantize_fp8_blockwise(const FsaBlockQuantArgs* a, void* stream_) {
 int fsa_pack_scales(const void* q_scale, const void* k_scale, const void* v_scale, int dtype, float* out, void* stream_) {
   if (!q_scale || !k_scale || !v_scale || !out) return FSA_ERR_INVALID_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
+  cudaError_t e;
   switch (dtype) {
-    case FSA_DT_BF16: fsa::pack_scales_kernel<__nv_bfloat16><<<1, 32, 0, s>>>(q_scale, k_scale, v_scale, out); break;
-    case FSA_DT_FP16: fsa::pack_scales_kernel<__half><<<1, 32, 0, s>>>(q_scale, k_scale, v_scale, out); break;
-    case FSA_DT_F32: fsa::pack_scales_kernel<float><<<1, 32, 0, s>>>(q_scale, k_scale, v_scale, out); break;
+    case FSA_DT_BF16: e = fsa::launch_early(fsa::pack_scales_kernel<__nv_bfloat16>, 1, 32, 0, s, 1, q_scale, k_scale, v_scale, out); break;
+    case FSA_DT_FP16: e = fsa::launch_early(fsa::pack_scales_kernel<__half>, 1, 32, 0, s, 1, q_scale, k_scale, v_scale, out); break;
+    case FSA_DT_F32: e = fsa::launch_early(fsa::pack_scales_kernel<float>, 1, 32, 0, s, 1, q_scale, k_scale, v_scale, out); break;
     default: return FSA_ERR_UNSUPPORTED;
   }
-  return cudaGetLastError() == cudaSuccess ? FSA_OK : FSA_ERR_LAUNCH;
+  return e == cudaSuccess ? FSA_OK : FSA_ERR_LAUNCH;
 }
 
 int fsa_fp8_widen(const void* x_fp8, void* out, const void* scale, int64_t n, int fp8_dtype, int out_dtype,

@@ -103,6 +103,7 @@ template <typename T, typename I, int NC>
 __global__ void __launch_bounds__(TK_THREADS) topk_kernel(const T* __restrict__ scores, long long row_stride, int n, int k,
                                                           I* __restrict__ out, int csize, int chunk) {
   static_assert(TK_THREADS == 1024, "block_scan assumes 32 warps");
+  after_previous();
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ uint32_t copies[TK_COPIES * TK_PITCH];
@@ -333,26 +334,14 @@ int topk_cluster_size(int rows, int n) {
 template <typename T, typename I>
 cudaError_t launch_topk_t(const void* scores, long long row_stride, int rows, int n, int k, void* out, cudaStream_t stream) {
   const int csize = topk_cluster_size<T, I>(rows, n), chunk = topk_chunk(n, csize);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(rows * csize), 1, 1);
-  cfg.blockDim = dim3(TK_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)csize;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   const T* x = reinterpret_cast<const T*>(scores);
   I* o = reinterpret_cast<I*>(out);
   // slices of up to 8192 / 16384 entries stay in registers
   if (chunk <= TK_THREADS * TK_V)
-    return cudaLaunchKernelEx(&cfg, topk_kernel<T, I, 1>, x, row_stride, n, k, o, csize, chunk);
+    return launch_early(topk_kernel<T, I, 1>, (unsigned)(rows * csize), TK_THREADS, 0, stream, csize, x, row_stride, n, k, o, csize, chunk);
   if (chunk <= TK_THREADS * TK_V * 2)
-    return cudaLaunchKernelEx(&cfg, topk_kernel<T, I, 2>, x, row_stride, n, k, o, csize, chunk);
-  return cudaLaunchKernelEx(&cfg, topk_kernel<T, I, 0>, x, row_stride, n, k, o, csize, chunk);
+    return launch_early(topk_kernel<T, I, 2>, (unsigned)(rows * csize), TK_THREADS, 0, stream, csize, x, row_stride, n, k, o, csize, chunk);
+  return launch_early(topk_kernel<T, I, 0>, (unsigned)(rows * csize), TK_THREADS, 0, stream, csize, x, row_stride, n, k, o, csize, chunk);
 }
 
 template <typename T>

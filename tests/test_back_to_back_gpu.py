@@ -1,0 +1,107 @@
+"""Calls that feed one another without a synchronisation in between: kernels are set up while those in front of them run, so each has
+to wait for what it reads and for what still reads what it writes. Same bits as with a synchronisation after every call, on the
+default stream, on a side stream, between kernels of torch, and from a captured graph."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _chain(state, sync):
+    """Selection, scales and FP8 decode, 16-bit decode in splits, prompt, forward and backward; every output is an input of the next."""
+    import flash_sparse_attn as fsa
+    from flash_sparse_attn.utils.mask import topk_indices
+
+    def done():
+        if sync:
+            torch.cuda.synchronize()
+
+    got = []
+    q, k, v, score, one = (state[n] for n in ("q", "k", "v", "score", "one"))
+    for _ in range(3):
+        idx = topk_indices(score, 256, dtype=torch.int32)
+        done()
+        q8, k8, v8 = ((t * 16).to(torch.float8_e4m3fn) for t in (q[:, -1], k, v))
+        dec = fsa.flash_sparse_attn_with_kvcache_func(q8, k8, v8, gather_kv_indices=idx, is_quant=True, query_scale=one, key_scale=one,
+                                                      value_scale=one)
+        done()
+        dec = fsa.flash_dense_attn_with_kvcache_func(dec, k, v, num_splits=9)
+        done()
+        dec = fsa.flash_dense_attn_with_kvcache_func(dec, k, v, num_splits=3)
+        done()
+        q = q + dec[:, None]
+        out = fsa.flash_dense_attn_func(q, k, v, is_causal=True)
+        done()
+        out = fsa.flash_sparse_attn_func(out, k, v, is_causal=True, is_split_kv=True, num_splits=2)
+        done()
+        gated = fsa.flash_gated_attn_func(out, k, v, out[..., 0], k[..., 0], is_causal=True)
+        done()
+        q = (out + gated) * 0.5
+        score = score + q[:, :1, 0, :1].float().flatten(1)
+        got += [idx, dec, out, gated]
+    return got
+
+
+def _state():
+    g = torch.Generator(device="cuda").manual_seed(3)
+    mk = lambda *s: torch.randn(*s, generator=g, device="cuda", dtype=torch.bfloat16)  # noqa: E731
+    return dict(q=mk(2, 1000, 4, 128), k=mk(2, 1000, 2, 128), v=mk(2, 1000, 2, 128), score=mk(2, 1000).float(),
+                one=torch.full((1,), 1 / 16, device="cuda"))
+
+
+def test_chain_equals_its_calls():
+    import flash_sparse_attn as fsa
+
+    state = _state()
+    want = _chain(state, True)
+    for _ in range(5):
+        for a, b in zip(_chain(state, False), want):
+            assert torch.equal(a, b)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        got = _chain(state, False)
+    torch.cuda.current_stream().wait_stream(side)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = _chain(state, False)
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    fsa.check_status()
+
+
+def test_backward_passes_in_a_row():
+    import flash_sparse_attn as fsa
+
+    s = _state()
+    leaves = [s[n].clone().requires_grad_(True) for n in "qkv"]
+    do = torch.randn_like(leaves[0])
+
+    def grads(sync):
+        got = []
+        x = do
+        for _ in range(3):
+            out = fsa.flash_dense_attn_func(*leaves, is_causal=True, is_split_kv=True, is_split_qo=True, num_splits=2)
+            if sync:
+                torch.cuda.synchronize()
+            got += torch.autograd.grad(out, leaves, x)
+            if sync:
+                torch.cuda.synchronize()
+            x = got[-3] * 0.5  # the next pass starts from this one's dq
+        return got
+
+    fsa.set_deterministic(True)
+    try:
+        want = grads(True)
+        for _ in range(3):
+            for a, b in zip(grads(False), want):
+                assert torch.equal(a, b)
+    finally:
+        fsa.set_deterministic(False)
+    fsa.check_status()
