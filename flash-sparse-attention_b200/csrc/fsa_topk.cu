@@ -289,8 +289,6 @@ __global__ void __launch_bounds__(TK_THREADS) topk_kernel(const T* __restrict__ 
   cluster.sync();  // nobody leaves while another CTA may still read its shared memory
 }
 
-constexpr int TOPK_MIN_SLICE = 2048;
-
 // Entries of a row that a CTA of a cluster of c takes.
 inline int topk_chunk(int n, int c) { return ((n + c - 1) / c + TK_V - 1) / TK_V * TK_V; }
 
@@ -310,8 +308,9 @@ int topk_room(Kernel kern, int c, std::atomic<int>& known) {
   return fit;
 }
 
-// Cluster size: the largest power of two up to 8 whose clusters all find room at a time with an SM to each CTA, and that leaves
-// a slice of at least TOPK_MIN_SLICE entries per CTA (below that the exchange costs more than the shorter slice gains).
+// Cluster size: the smallest power of two up to 8 that brings a slice down to what TK_V entries a thread hold, or the
+// largest below that whose clusters all find room at a time with an SM to each CTA. Smaller slices gain less than the exchange costs
+// (one row of 8000 fp32 scores: two CTAs 10.9 us, one 9.5; 32 of 16 000 bf16: four 10.8, two 9.1).
 // rows * size <= SMs does not say that: 16 clusters of eight have no room on 148 SMs (16 rows of 32000 fp32 scores: 25.9 us
 // with them, 13.1 with clusters of four; bf16, whose CTAs share SMs then, 13.9 and 10.2).
 template <typename T, typename I>
@@ -321,7 +320,7 @@ int topk_cluster_size(int rows, int n) {
   if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return 1;
   for (int lg = 3; lg > 0; --lg) {
     const int c = 1 << lg, chunk = topk_chunk(n, c);
-    if ((long long)rows * c > device_sm_count() || n / c < TOPK_MIN_SLICE) continue;
+    if ((long long)rows * c > device_sm_count() || n <= TK_THREADS * TK_V * (c / 2)) continue;
     const int nc = chunk <= TK_THREADS * TK_V ? 1 : chunk <= TK_THREADS * TK_V * 2 ? 2 : 0;
     std::atomic<int>& known = room[dev][nc][lg];
     const int fit = nc == 1 ? topk_room(topk_kernel<T, I, 1>, c, known)
