@@ -139,10 +139,9 @@ struct RowPos {
   int b, q, h;
   long long tok;
 };
-__device__ __forceinline__ RowPos locate_row(long long item, int heads, int varlen, const int* cu_q, int B, int sq) {
+__device__ __forceinline__ RowPos locate_row(long long row, int h, int varlen, const int* cu_q, int B, int sq) {
   RowPos r;
-  r.h = (int)(item % heads);
-  const long long row = item / heads;
+  r.h = h;
   if (varlen) {
     // the last sequence that starts at or before the row: log2(B) dependent loads where a scan would take up to B
     int b = 0, last = B - 1;
@@ -229,7 +228,9 @@ __global__ void __launch_bounds__(256) gate_ext_kernel(GateExtParams p) {
   if (lane == 0) *reinterpret_cast<float2*>(dst) = make_float2(mx, mn);
 }
 
-constexpr int PP_ITEMS = 1;  // (row, head) items per lane group in the pre / post passes (4 and 8 measured slower: fewer CTAs)
+// Consecutive rows of a head per lane group in the pre / post passes: twice the bytes in flight of one, and the accumulator's rows lie
+// side by side (pre pass, B4 S8192, 32 heads of 128: 200 us with one row, 185 with two, 217 with four; packed 215, 194, 236).
+constexpr int PP_ITEMS = 2;
 
 // head_dim / 8 lanes per (query row, head), 16-byte loads; also clears the row of the fp32 dQ accumulator.
 // flash_sparse_attn/ops/triton/flash_bwd_preprocess.py:170-195.
@@ -239,20 +240,20 @@ __global__ void __launch_bounds__(256) bwd_pre_kernel(BwdPreParams p) {
   const int lpr = p.head_dim_pad >> 3;  // lanes per row (8 or 16); lanes past the real head size idle
   const int lane = threadIdx.x & 31, sub = lane % lpr;
   const int groups = 32 / lpr;
-  const long long first =
-      (((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * groups + lane / lpr) * PP_ITEMS;
+  const long long item = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * groups + lane / lpr;
+  const int head = (int)(item % p.heads);
+  const long long first = item / p.heads * PP_ITEMS;
   const long long rows = p.varlen ? p.total_q : (long long)p.B * p.sq;
-  const long long n_items = rows * p.heads;
   RowPos r[PP_ITEMS];
   uint4 a[PP_ITEMS], g[PP_ITEMS];
   bool live[PP_ITEMS];
 #pragma unroll
   for (int u = 0; u < PP_ITEMS; ++u) {
-    live[u] = first + u < n_items;
+    live[u] = first + u < rows;
     r[u] = RowPos{0, 0, 0, 0};
     a[u] = g[u] = make_uint4(0, 0, 0, 0);
     if (live[u]) {
-      r[u] = locate_row(first + u, p.heads, p.varlen, p.cu_q, p.B, p.sq);
+      r[u] = locate_row(first + u, head, p.varlen, p.cu_q, p.B, p.sq);
       if (sub * 8 < p.head_dim) {
         const T* o = reinterpret_cast<const T*>(p.out) + (p.varlen ? 0 : (long long)r[u].b * p.o_sb) + r[u].tok * p.o_sm +
                      (long long)r[u].h * p.o_sh + sub * 8;
@@ -301,22 +302,22 @@ __global__ void __launch_bounds__(256) bwd_post_kernel(BwdPostParams p) {
   const int lpr = p.head_dim_pad >> 3;
   const int lane = threadIdx.x & 31, sub = lane % lpr;
   const int groups = 32 / lpr;
-  const long long first =
-      (((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * groups + lane / lpr) * PP_ITEMS;
+  const long long item = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * groups + lane / lpr;
+  const int head = (int)(item % p.heads);
+  const long long first = item / p.heads * PP_ITEMS;
   const long long rows = p.varlen ? p.total_q : (long long)p.B * p.sq;
-  const long long n_items = rows * p.heads;
   RowPos r[PP_ITEMS];
   long long wrow[PP_ITEMS];
   float4 v0[PP_ITEMS], v1[PP_ITEMS];
   bool live[PP_ITEMS];
 #pragma unroll
   for (int u = 0; u < PP_ITEMS; ++u) {
-    live[u] = first + u < n_items;
+    live[u] = first + u < rows;
     r[u] = RowPos{0, 0, 0, 0};
     wrow[u] = 0;
     v0[u] = v1[u] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (live[u]) {
-      r[u] = locate_row(first + u, p.heads, p.varlen, p.cu_q, p.B, p.sq);
+      r[u] = locate_row(first + u, head, p.varlen, p.cu_q, p.B, p.sq);
       wrow[u] = (long long)r[u].h * p.ws_sh + padded_row(p.varlen, p.cu_q, r[u].b, p.sq, r[u].q);
       if (sub * 8 < p.head_dim) {
         const float4* src = reinterpret_cast<const float4*>(p.dq_accum + wrow[u] * p.head_dim_pad + sub * 8);
@@ -417,10 +418,10 @@ __global__ void __launch_bounds__(256) split_sum_kernel(SplitSumParams p) {
 
 cudaError_t launch_bwd_pre(const BwdPreParams& p, int dtype, cudaStream_t stream) {
   const long long rows = p.varlen ? p.total_q : (long long)p.B * p.sq;
-  const long long items = rows * p.heads;
+  const long long items = (rows + PP_ITEMS - 1) / PP_ITEMS * p.heads;
   if (items <= 0) return cudaSuccess;
   if (p.head_dim_pad != 64 && p.head_dim_pad != 128) return cudaErrorInvalidValue;
-  const int per_block = 8 * (32 / (p.head_dim_pad >> 3)) * PP_ITEMS;
+  const int per_block = 8 * (32 / (p.head_dim_pad >> 3));
   const unsigned grid = (unsigned)((items + per_block - 1) / per_block);
   if (dtype == DT_BF16)
     return launch_early(bwd_pre_kernel<__nv_bfloat16>, grid, 256, 0, stream, 1, p);
@@ -429,10 +430,10 @@ cudaError_t launch_bwd_pre(const BwdPreParams& p, int dtype, cudaStream_t stream
 
 cudaError_t launch_bwd_post(const BwdPostParams& p, int dtype, cudaStream_t stream) {
   const long long rows = p.varlen ? p.total_q : (long long)p.B * p.sq;
-  const long long items = rows * p.heads;
+  const long long items = (rows + PP_ITEMS - 1) / PP_ITEMS * p.heads;
   if (items <= 0) return cudaSuccess;
   if (p.head_dim_pad != 64 && p.head_dim_pad != 128) return cudaErrorInvalidValue;
-  const int per_block = 8 * (32 / (p.head_dim_pad >> 3)) * PP_ITEMS;
+  const int per_block = 8 * (32 / (p.head_dim_pad >> 3));
   const unsigned grid = (unsigned)((items + per_block - 1) / per_block);
   if (dtype == DT_BF16)
     return launch_early(bwd_post_kernel<__nv_bfloat16>, grid, 256, 0, stream, 1, p);
