@@ -231,11 +231,14 @@ __global__ void __launch_bounds__(256) gate_ext_kernel(GateExtParams p) {
 // Consecutive rows of a head per lane group in the pre / post passes: twice the bytes in flight of one, and the accumulator's rows lie
 // side by side (pre pass, B4 S8192, 32 heads of 128: 200 us with one row, 185 with two, 217 with four; packed 215, 194, 236).
 constexpr int PP_ITEMS = 2;
+// Small blocks: a block leaves when its last warp's loads have come, and fewer warps wait for that (whole backward, 256 threads a block and 128:
+// 16 384 tokens 598.5 -> 594.4 us, B4 S8192 1231.9 -> 1223.7, 2000 tokens 178.2 -> 177.9; a loop over resident blocks instead 606 and 1259).
+constexpr int PP_THREADS = 128;
 
 // head_dim / 8 lanes per (query row, head), 16-byte loads; also clears the row of the fp32 dQ accumulator.
 // flash_sparse_attn/ops/triton/flash_bwd_preprocess.py:170-195.
 template <typename T>
-__global__ void __launch_bounds__(256) bwd_pre_kernel(BwdPreParams p) {
+__global__ void __launch_bounds__(PP_THREADS) bwd_pre_kernel(BwdPreParams p) {
   after_previous();
   const int lpr = p.head_dim_pad >> 3;  // lanes per row (8 or 16); lanes past the real head size idle
   const int lane = threadIdx.x & 31, sub = lane % lpr;
@@ -297,7 +300,7 @@ __global__ void __launch_bounds__(256) bwd_pre_kernel(BwdPreParams p) {
 
 // head_dim / 8 lanes per (query row, head). flash_sparse_attn/ops/triton/flash_bwd_postprocess.py:60-148.
 template <typename T>
-__global__ void __launch_bounds__(256) bwd_post_kernel(BwdPostParams p) {
+__global__ void __launch_bounds__(PP_THREADS) bwd_post_kernel(BwdPostParams p) {
   after_previous();
   const int lpr = p.head_dim_pad >> 3;
   const int lane = threadIdx.x & 31, sub = lane % lpr;
@@ -421,11 +424,11 @@ cudaError_t launch_bwd_pre(const BwdPreParams& p, int dtype, cudaStream_t stream
   const long long items = (rows + PP_ITEMS - 1) / PP_ITEMS * p.heads;
   if (items <= 0) return cudaSuccess;
   if (p.head_dim_pad != 64 && p.head_dim_pad != 128) return cudaErrorInvalidValue;
-  const int per_block = 8 * (32 / (p.head_dim_pad >> 3));
+  const int per_block = PP_THREADS / (p.head_dim_pad >> 3);
   const unsigned grid = (unsigned)((items + per_block - 1) / per_block);
   if (dtype == DT_BF16)
-    return launch_early(bwd_pre_kernel<__nv_bfloat16>, grid, 256, 0, stream, 1, p);
-  return launch_early(bwd_pre_kernel<__half>, grid, 256, 0, stream, 1, p);
+    return launch_early(bwd_pre_kernel<__nv_bfloat16>, grid, PP_THREADS, 0, stream, 1, p);
+  return launch_early(bwd_pre_kernel<__half>, grid, PP_THREADS, 0, stream, 1, p);
 }
 
 cudaError_t launch_bwd_post(const BwdPostParams& p, int dtype, cudaStream_t stream) {
@@ -433,14 +436,14 @@ cudaError_t launch_bwd_post(const BwdPostParams& p, int dtype, cudaStream_t stre
   const long long items = (rows + PP_ITEMS - 1) / PP_ITEMS * p.heads;
   if (items <= 0) return cudaSuccess;
   if (p.head_dim_pad != 64 && p.head_dim_pad != 128) return cudaErrorInvalidValue;
-  const int per_block = 8 * (32 / (p.head_dim_pad >> 3));
+  const int per_block = PP_THREADS / (p.head_dim_pad >> 3);
   const unsigned grid = (unsigned)((items + per_block - 1) / per_block);
   const auto kern = dtype == DT_BF16 ? bwd_post_kernel<__nv_bfloat16> : bwd_post_kernel<__half>;
   // Set up while the main kernel still runs only if it has few blocks: that saves 0.5 to 2 us, but each block then takes longer to start.
-  // Whole backward, early and not: 1024 blocks 98.3 and 100.3 us, 4096 175.1 and 175.6, 8000 251.9 and 252.3, 8192 331.8 and 330.2, 16384
-  // 603.6 and 598.5, 32768 1224.7 and 1213.2.
-  if (grid < 8192) return launch_early(kern, grid, 256, 0, stream, 1, p);
-  kern<<<grid, 256, 0, stream>>>(p);
+  // Whole backward, early and not, with blocks twice as large: 1024 blocks 98.3 and 100.3 us, 4096 175.1 and 175.6, 8000 251.9 and 252.3,
+  // 8192 331.8 and 330.2, 16384 603.6 and 598.5, 32768 1224.7 and 1213.2.
+  if (grid < 16384) return launch_early(kern, grid, PP_THREADS, 0, stream, 1, p);
+  kern<<<grid, PP_THREADS, 0, stream>>>(p);
   return cudaGetLastError();
 }
 

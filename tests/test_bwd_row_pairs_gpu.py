@@ -35,7 +35,7 @@ def test_pairs_of_rows(lens, heads, head_dim):
         assert_close(name, a, b)
 
 
-@pytest.mark.parametrize("batch", [4095, 4096])  # 8190 and 8192 blocks: the pass behind the main kernel starts early or after it
+@pytest.mark.parametrize("batch", [4095, 4096])  # 16 380 and 16 384 blocks: the pass behind the main kernel starts early or after it
 def test_many_blocks(batch):
     import flash_sparse_attn as fsa
 
