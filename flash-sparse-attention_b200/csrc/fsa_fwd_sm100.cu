@@ -1057,7 +1057,11 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
       // ---- move the reference maximum only when it lags by more than 2^8 -------------------------
       float m_cand = fmaxf(m_cur, m_ref);
       if (mode != FSA_MASK_NONE) m_cand = fmaxf(m_cand, -1e6f);
-      const bool need = !((m_cand - m_ref) * cc <= 8.0f);  // also true on the first tile (m_ref = -inf)
+      // A share of the keys may begin with tiles that are not masked (whole sequences begin with the diagonal) and where every score of a
+      // row is -inf. There is no maximum to refer to yet: the exponentials, all zero, are taken as they are. (Not a finite maximum instead:
+      // it would outweigh scores below it in the tiles that follow.)
+      const bool none = CL && m_cand == -INFINITY;
+      const bool need = !none && !((m_cand - m_ref) * cc <= 8.0f);  // also true on the first tile (m_ref = -inf)
       float scale = 1.0f;
       if (need) {
         scale = ex2_approx((m_ref - m_cand) * cc);
@@ -1100,7 +1104,7 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
 
       // ---- P = exp2(S*c - m*c), row sum, publish P (16-bit pairs) over the S columns -----------------
       const float2 c2 = make_float2(cc, cc);
-      const float neg_mc = -(m_ref * cc);
+      const float neg_mc = none ? 0.f : -(m_ref * cc);
       const float2 nm2 = make_float2(neg_mc, neg_mc);
       float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       constexpr int EXP_UNROLL = GATED ? 1 : NC / 32;

@@ -45,3 +45,35 @@ def test_packed_heads_infinite_keys_and_a_second_stream():
     side.synchronize()
     assert torch.equal(other, ref)
     fsa.check_status()
+
+
+# Key tiles that score -inf for every second row, and once for all rows (a product that overflows: masking by an extra column does
+# that). 897 tokens x 8 heads: clusters of four, the next two of two, one head: of eight. Every CTA but the one of the last share begins
+# with tiles that carry no mask
+@pytest.mark.parametrize("seqlen, hq, hkv", [(897, 8, 2), (1024, 16, 4), (2304, 8, 2), (2050, 1, 1)])
+@pytest.mark.parametrize("head_dim", [64, 128])
+@pytest.mark.parametrize("causal", [True, False])
+def test_shares_that_begin_at_minus_infinity(seqlen, hq, hkv, head_dim, causal):
+    import flash_sparse_attn as fsa
+
+    q, k, v = seeded_qkv(seqlen + head_dim, 1, seqlen, seqlen, hq, hkv, head_dim)
+    tiles = seqlen // 128
+    # one tile; two neighbours; the whole of the first share of two; all but the first and the last; every second one
+    for out_tiles in ([3], [1, 2], range(1, tiles // 2), range(1, tiles), range(tiles - 1, 0, -2)):
+        qq, kk = q.clone(), k.clone()
+        qq[..., 5], kk[..., 5] = 0, 0
+        qq[:, ::2, :, 5] = 1e20
+        for t in out_tiles:
+            kk[:, 128 * t:128 * (t + 1), :, 5] = -1e20
+        ref, lse_ref = eager.forward(qq, kk, v, None, causal, return_lse=True)
+        out, lse = fsa.flash_dense_attn_func(*(t.cuda() for t in (qq, kk, v)), is_causal=causal, return_lse=True)
+        assert torch.isfinite(lse_ref).all()  # keys 0 to 127 are there for every row
+        assert_close(f"out {list(out_tiles)}", out, ref)
+        assert torch.allclose(lse.cpu(), lse_ref, rtol=0, atol=2e-3), list(out_tiles)
+    # no key is left to any row: probability zero for every one, as where everything is masked
+    if causal:
+        qq, kk = q.clone(), k.clone()
+        qq[..., 5], kk[..., 5] = 1e20, -1e20
+        out, lse = fsa.flash_dense_attn_func(*(t.cuda() for t in (qq, kk, v)), is_causal=True, return_lse=True)
+        assert (out == 0).all() and torch.isneginf(lse).all()
+    fsa.check_status()
