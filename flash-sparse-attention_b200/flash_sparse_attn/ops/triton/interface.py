@@ -175,7 +175,7 @@ def _apply(kind, varlen, query, key, value, alpha, delta, cu_seqlens_q, cu_seqle
         query, key, value, alpha, delta, cu_seqlens_q, cu_seqlens_k, query_scale, key_scale, value_scale,
         window_sizes, page_table, seqused_q, seqused_k, out, lse)
     # (a caller's result buffers: the Function hands them back through views of their own)
-    if out is None and lse is None and _nothing_to_record(query, key, value, alpha, delta):
+    if out is None and lse is None and _nothing_to_record(query, key, value, alpha, delta, query_scale, key_scale, value_scale):
         res = _forward(kind, varlen, query, key, value, alpha, delta, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k,
                        is_causal, softmax_scale, query_scale, key_scale, value_scale, window_sizes, softmax_threshold,
                        gate_threshold, is_logsigmoid_gate, is_adapt_gate, is_local, is_quant, is_split_kv, is_split_qo, pack_gqa,

@@ -24,6 +24,27 @@ def test_what_the_function_has_to_see():
     assert seen == [False, False, False]
 
 
+@pytest.mark.parametrize("asked", ["query", "key", "value", "query_scale", "key_scale", "value_scale", None])
+def test_every_tensor_that_asks_for_a_gradient_is_recorded(asked, monkeypatch):
+    from flash_sparse_attn.ops.triton import interface
+
+    class Function:
+        apply = staticmethod(lambda *a: "recorded")
+
+    monkeypatch.setattr(interface, "_AttnFunc", Function)
+    monkeypatch.setattr(interface, "_forward", lambda *a: ("not recorded",) * 13)
+    one = {n: torch.ones(1) for n in ("query_scale", "key_scale", "value_scale")}
+    x = {n: torch.zeros(1, 4, 1, 128) for n in ("query", "key", "value")}
+    for t in (x, one):
+        if asked in t:
+            t[asked].requires_grad_(True)
+    want = "not recorded" if asked is None else "recorded"
+    assert interface.flash_dense_attn_func(**x, is_quant=True, **one) == want
+    assert interface.flash_sparse_attn_func(**x, is_quant=True, **one) == want
+    with torch.no_grad():
+        assert interface.flash_dense_attn_func(**x, is_quant=True, **one) == "not recorded"
+
+
 @pytest.mark.gpu
 def test_same_results_and_refusals():
     import flash_sparse_attn as fsa
