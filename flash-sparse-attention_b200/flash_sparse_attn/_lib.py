@@ -419,7 +419,7 @@ def _load_host(lib):
             raise ImportError(f"built for {built_for}, not for {here} (ABI version, torch)")
         host.init(ctypes.cast(lib.fsa_decode, c_void_p).value, ctypes.cast(lib.fsa_fwd, c_void_p).value,
                   ctypes.cast(lib.fsa_topk_indices, c_void_p).value, ctypes.cast(lib.fsa_pack_scales, c_void_p).value)
-    except (ImportError, AttributeError) as e:
+    except (ImportError, AttributeError, TypeError) as e:  # TypeError: a launcher that takes other addresses
         _host = None
         warnings.warn("flash_sparse_attn/_host.so is missing or does not load; calls go through the slower Python launchers until "
                       f"`python build.py` (next to csrc/) has built it: {e}", RuntimeWarning)

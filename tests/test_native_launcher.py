@@ -29,7 +29,7 @@ def test_refuses_what_is_not_on_a_gpu():
     assert _lib._host.decode(*args[:-1]) is None and _lib._host.forward() is None
 
 
-@pytest.mark.parametrize("module", ["missing", "other abi", "other torch", "old"])
+@pytest.mark.parametrize("module", ["missing", "other abi", "other torch", "old", "fewer entry points"])
 def test_package_works_without_it(monkeypatch, module):
     """A launcher that is missing or built for something else is left out, with one warning; the Python launchers remain."""
     import sys
@@ -43,6 +43,12 @@ def test_package_works_without_it(monkeypatch, module):
     if module.startswith("other"):
         fake.ABI_VERSION = good.ABI_VERSION + (module == "other abi")
         fake.TORCH_VERSION = good.TORCH_VERSION if module == "other abi" else "1.0.0"
+    elif module == "fewer entry points":  # built before the launcher took the addresses of top-k and of the packing of scales
+        def init(*addresses):
+            if len(addresses) != 2:
+                raise TypeError("init takes two addresses")
+
+        fake.ABI_VERSION, fake.TORCH_VERSION, fake.init = good.ABI_VERSION, good.TORCH_VERSION, init
     monkeypatch.setitem(sys.modules, "flash_sparse_attn._host", fake)
     try:
         with pytest.warns(RuntimeWarning, match="Python launchers"):
