@@ -199,7 +199,9 @@ inline cudaError_t launch_early(void (*kern)(Params...), unsigned grid, int thre
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = cluster > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
+  if (e != cudaSuccess) (void)cudaGetLastError();  // it is returned here, and not to the next launch that asks for the last error
+  return e;
 }
 
 #ifdef __CUDACC__

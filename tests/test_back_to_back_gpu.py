@@ -105,3 +105,30 @@ def test_backward_passes_in_a_row():
     finally:
         fsa.set_deterministic(False)
     fsa.check_status()
+
+
+def test_a_refused_launch_is_reported_once():
+    # A launch into a capture that something else has spoilt is refused on the host. The call says so, and the next one, whose launch
+    # asks for the last error, knows nothing of it.
+    import ctypes
+
+    from flash_sparse_attn import _lib
+    from flash_sparse_attn.ops.triton import quant
+
+    lib = _lib.load()
+    rt = ctypes.CDLL("libcudart.so.12")  # torch's; the library has a runtime of its own
+    x = torch.ones(64, device="cuda").to(torch.float8_e4m3fn)
+    one, out = torch.ones(1, device="cuda"), torch.empty(3, device="cuda")
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    stream = ctypes.c_void_p(side.cuda_stream)
+    graph = ctypes.c_void_p()
+    assert rt.cudaStreamBeginCapture(stream, 1) == 0  # 1: thread local
+    try:
+        assert rt.cudaStreamSynchronize(stream) != 0  # not allowed in a capture, which is spoilt by it
+        rc = lib.fsa_pack_scales(one.data_ptr(), one.data_ptr(), one.data_ptr(), 4, out.data_ptr(), stream)  # 4: FSA_DT_F32
+    finally:
+        rt.cudaStreamEndCapture(stream, ctypes.byref(graph))
+        rt.cudaGetLastError()
+    assert rc == -3, rc  # FSA_ERR_LAUNCH
+    assert torch.equal(quant.widen_fp8(x).float(), torch.ones(64, device="cuda"))
