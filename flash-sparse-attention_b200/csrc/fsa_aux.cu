@@ -14,7 +14,7 @@ namespace {
 // _dec_combine_kernel (flash_dec_combine.py:15-153).
 template <typename T, int VEC>
 __global__ void __launch_bounds__(256) combine_kernel(CombineParams p) {
-  after_previous();
+  wait_for_previous();
   const int lane = threadIdx.x & 31;
   const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   long long buf_off = 0;
@@ -43,6 +43,7 @@ __global__ void __launch_bounds__(256) combine_kernel(CombineParams p) {
     __syncthreads();
     buf_off = (long long)((step - 1) & 1ull) * p.buf_stride;
   }
+  let_next_be_set_up();
   if (item >= (long long)p.rows * p.heads) return;
   const int h = (int)(item % p.heads);
   const long long row = item / p.heads;

@@ -179,7 +179,7 @@ inline int resident_clusters(Kernel kern, int size, int threads, int smem) {
 }
 
 // Launch whose blocks may be set up while the kernel in front of it in the stream still runs: the kernel has to begin with
-// after_previous(). `cluster` CTAs form a cluster (1: none). What it saves is 1 to 2 us between two kernels: a decode step of one
+// after_previous() or wait_for_previous(). `cluster` CTAs form a cluster (1: none). What it saves is 1 to 2 us between two kernels: a decode step of one
 // sequence over and over 12.3 -> 10.4 us, top-k selection, scales and FP8 decode 33.3 -> 29.6, a short prompt 16.4 -> 14.6, a paged
 // batch and its combine 186.9 -> 184.2.
 template <typename... Params, typename... Args>
@@ -208,10 +208,13 @@ inline cudaError_t launch_early(void (*kern)(Params...), unsigned grid, int thre
 // In front of everything that a kernel reads or writes: waits until the kernel in front of it has completed and what it wrote is
 // visible, then lets the kernel behind it be set up; blocks of that one are only started once all of this kernel's have been, so they
 // take no room from them. (The other way round three kernels deep: single calls the same, decode of 4 sequences x 4000 keys
-// 12.7 -> 13.9 us, whose blocks find the SMs unevenly taken.)
+// 12.7 -> 13.9 us, whose blocks find the SMs unevenly taken.) A kernel that waits for another GPU lets the next one be set up behind
+// that wait only: blocks that wait for this kernel would hold their room on the SMs, which other streams could use, as long.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_be_set_up() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void after_previous() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  wait_for_previous();
+  let_next_be_set_up();
 }
 #endif
 
