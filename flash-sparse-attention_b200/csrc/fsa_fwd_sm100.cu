@@ -88,8 +88,6 @@ struct OutType<__nv_fp8_e5m2> {
   using type = __nv_bfloat16;
 };
 
-constexpr int MAX_CLUSTER = 8;  // CTAs that merge at most
-
 constexpr int MAX_RANKED = FSA_FWD_MAX_RANKED;  // (query tile pair, sequence) items that a CTA ranks at most
 
 struct FwdBars {
@@ -1331,28 +1329,22 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
   }
 }
 
-// CTAs in a cluster, which share the key tiles of the same query tiles (1: none do). A dense call with fewer CTAs than SMs is as
-// long as its longest CTA; its key tiles go to as many CTAs as there are SMs for, at least two tiles to each of the longest, when
-// that saves four tiles: the merge takes as long as two. Causal, 8 / 2 heads, us: S = 500 stays (12.3 at head size 64, 17.1 in clusters
-// of two as first built), 1024 18.0 -> 14.3 and 2000 31.7 -> 24.8, head size 128 21.1 -> 16.8 and 35.4 -> 28.4.
-// (Not the other kinds: whether a tile is skipped depends on the tiles before it. Windows have few tiles. Whole sequences only:
-// queries over longer keys give the same bits alone and in a batch.)
+// Calls whose key tiles may be shared inside clusters (fsa_fwd_cluster_size): whole sequences of equal query and key length. Not the
+// other kinds: whether a tile is skipped depends on the tiles before it. Windows have few tiles. Not calls with lengths of their own,
+// pages or keys in front of the queries: those give the same bits alone and in a batch.
+// `known`: the runtime's answers, per device and for one kernel: resident clusters plus one, 0: not asked yet.
 template <typename Kernel>
-int fwd_cluster_size(Kernel kern, const FwdKernelParams& p, int threads, int smem) {
-  static std::atomic<int> known[64][MAX_CLUSTER + 1];  // clusters that are resident at a time, plus one; 0: not asked yet
-  const long long base = (long long)p.num_pairs * p.hgrid * p.B;
+int fwd_cluster_size(Kernel kern, const FwdKernelParams& p, int threads, int smem, std::atomic<int> (*known)[FSA_FWD_MAX_CLUSTER + 1]) {
   int dev = 0;
   if ((p.flags & (F_SPLIT | F_LOCAL | F_VARLEN_Q | F_VARLEN_K | F_USED_Q | F_USED_K | F_PAGED)) || p.sq != p.sk || p.tile_map || cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return 1;
-  for (int size = MAX_CLUSTER; size > 1; size >>= 1) {
-    if (base * size > device_sm_count() || p.n_tiles_k < 2 * size || p.n_tiles_k - (p.n_tiles_k + size - 1) / size < 4) continue;
+  return fsa_fwd_cluster_size((long long)p.num_pairs * p.hgrid * p.B, p.n_tiles_k, device_sm_count(), [&](int size) {
     int room = known[dev][size].load(std::memory_order_relaxed) - 1;
     if (room < 0) {
       room = resident_clusters(kern, size, threads, smem);
       known[dev][size].store(room + 1, std::memory_order_relaxed);
     }
-    if (base <= room) return size;
-  }
-  return 1;
+    return room;
+  });
 }
 
 template <int HD, typename T, int KIND, bool BSCALE = false, bool CL = false>
@@ -1364,7 +1356,8 @@ cudaError_t launch_one(FwdKernelParams& p, cudaStream_t stream) {
   const long long grid = (long long)p.num_pairs * p.hgrid * p.B * p.num_splits;
   if (grid <= 0) return cudaSuccess;
   if constexpr (CL) {
-    p.cluster = fwd_cluster_size(kern, p, threads, smem);
+    static std::atomic<int> known[64][FSA_FWD_MAX_CLUSTER + 1];
+    p.cluster = fwd_cluster_size(kern, p, threads, smem, known);
     if (p.cluster == 1) return launch_one<HD, T, KIND>(p, stream);
     return launch_early(kern, (unsigned)grid * p.cluster, threads, smem, stream, p.cluster, p);
   }

@@ -64,6 +64,19 @@ FSA_HD bool fsa_fwd_longest_first(bool causal, bool local, long long batch, long
          items * splits <= 4 * tiles;
 }
 
+// Forward, dense whole sequences: CTAs in a cluster, which share the key tiles of the same query tiles (1: none do). A call of `ctas` CTAs,
+// fewer than SMs, is as long as its longest CTA; its `tiles` key tiles go to as many CTAs as there are SMs for, at least two tiles to each
+// of the longest, when that saves four tiles: the merge takes as long as two. room(size): clusters that are resident at a time.
+// Causal, 8 / 2 heads, us: S = 500 stays (12.3 at head size 64, 17.1 in clusters of two as first built), 1024 18.0 -> 14.3 and 2000
+// 31.7 -> 24.8, head size 128 21.1 -> 16.8 and 35.4 -> 28.4.
+enum { FSA_FWD_MAX_CLUSTER = 8 };
+template <typename Room>
+inline int fsa_fwd_cluster_size(long long ctas, int tiles, int sms, Room room) {
+  for (int size = FSA_FWD_MAX_CLUSTER; size > 1; size >>= 1)
+    if (ctas * size <= sms && tiles >= 2 * size && tiles - (tiles + size - 1) / size >= 4 && ctas <= room(size)) return size;
+  return 1;
+}
+
 // Share of `total` blocks owned by split `s` of `ns`: the first total%ns splits get one extra.
 FSA_HD void fsa_split_range(int total, int ns, int s, int* off, int* cnt) {
   const int base = total / ns, extra = total % ns;
