@@ -1331,7 +1331,7 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
 
 // Calls whose key tiles may be shared inside clusters (fsa_fwd_cluster_size): whole sequences of equal query and key length. Not the
 // other kinds: whether a tile is skipped depends on the tiles before it. Windows have few tiles. Not calls with lengths of their own,
-// pages or keys in front of the queries: those give the same bits alone and in a batch.
+// pages or keys in front of the queries: unsplit, those give a sequence the same bits alone as in a batch, at every size.
 // `known`: the runtime's answers, per device and for one kernel: resident clusters plus one, 0: not asked yet.
 template <typename Kernel>
 int fwd_cluster_size(Kernel kern, const FwdKernelParams& p, int threads, int smem, std::atomic<int> (*known)[FSA_FWD_MAX_CLUSTER + 1]) {

@@ -69,6 +69,8 @@ FSA_HD bool fsa_fwd_longest_first(bool causal, bool local, long long batch, long
 // of the longest, when that saves four tiles: the merge takes as long as two. room(size): clusters that are resident at a time.
 // Causal, 8 / 2 heads, us: S = 500 stays (12.3 at head size 64, 17.1 in clusters of two as first built), 1024 18.0 -> 14.3 and 2000
 // 31.7 -> 24.8, head size 128 21.1 -> 16.8 and 35.4 -> 28.4.
+// The size follows from all CTAs of a call, and a share is summed for itself: from 897 tokens on a sequence of such a call may differ in
+// rounding with how many stand beside it, and from the same sequence in a packed call, which keeps one CTA for all its key tiles.
 enum { FSA_FWD_MAX_CLUSTER = 8 };
 template <typename Room>
 inline int fsa_fwd_cluster_size(long long ctas, int tiles, int sms, Room room) {

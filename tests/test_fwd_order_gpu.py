@@ -1,5 +1,8 @@
 """Forward over sequences of unequal length: the CTAs start in the order of their key tiles, worked out on the device. Which
-CTA computes a tile changes nothing about its arithmetic, so a batch has to equal its sequences called one by one, bit for bit."""
+CTA computes a tile changes nothing about its arithmetic, so a batch has to equal its sequences called one by one, bit for bit. That
+holds for calls with lengths of their own, pages or keys in front of the queries at every size, and between those and dense calls over
+whole sequences up to 896 tokens: from 897 on the latter may have their key tiles shared inside a cluster (fsa_fwd_cluster_size), each
+share summed for itself, and equal the others up to the rounding of 16-bit probabilities."""
 
 import pytest
 import torch
@@ -41,6 +44,32 @@ def test_packed_batch_equals_its_sequences(lens, hq, hkv, causal):
             s = slice(at, at + n)
             alone = fsa.flash_dense_attn_func(q[None, s], k[None, s], v[None, s], is_causal=causal)
             assert torch.equal(out[s], alone[0])
+        at += n
+    fsa.check_status()
+
+
+# 896 tokens are the most that no cluster shares; 897, 1000 and 2000 at 8 / 2 heads are shared by four, four and two CTAs, but not
+# when five of them are one dense batch
+@pytest.mark.parametrize("head_dim", [64, 128])
+@pytest.mark.parametrize("causal", [True, False])
+def test_up_to_where_whole_sequences_have_the_bits_of_a_batch(head_dim, causal):
+    lens, hq, hkv = [896, 897, 1000, 2000], 8, 2
+    q, k, v = _randn(sum(lens), hq, head_dim, seed=1), _randn(sum(lens), hkv, head_dim, seed=2), _randn(sum(lens), hkv, head_dim, seed=3)
+    packed = lambda s, n: fsa.flash_dense_attn_varlen_func(q[s], k[s], v[s], _cu(n), _cu(n), max(n), max(n), is_causal=causal)  # noqa: E731
+    out = packed(slice(None), lens)
+    at = 0
+    for n in lens:
+        s = slice(at, at + n)
+        assert torch.equal(out[s], packed(s, [n]))  # packed: at every size
+        alone = fsa.flash_dense_attn_func(q[None, s], k[None, s], v[None, s], is_causal=causal)[0]
+        five = fsa.flash_dense_attn_func(*(t[None, s].repeat(5, 1, 1, 1) for t in (q, k, v)), is_causal=causal)
+        assert all(torch.equal(five[i], out[s]) for i in range(5))
+        if n <= 896:
+            assert torch.equal(alone, out[s])
+        # Each side rounds its probabilities and its results to bf16: four roundings of 2^-9 of a value at most, 2^-9 / sqrt(3) in the
+        # root mean square, independent of one another and, as the values have random signs, over the keys: 2^-9 * sqrt(4 / 3) together.
+        x, y = alone.double(), out[s].double()
+        assert (x - y).norm() <= 2.0 ** -8 * y.norm()
         at += n
     fsa.check_status()
 
