@@ -440,9 +440,9 @@ cudaError_t launch_bwd_post(const BwdPostParams& p, int dtype, cudaStream_t stre
   const int per_block = PP_THREADS / (p.head_dim_pad >> 3);
   const unsigned grid = (unsigned)((items + per_block - 1) / per_block);
   const auto kern = dtype == DT_BF16 ? bwd_post_kernel<__nv_bfloat16> : bwd_post_kernel<__half>;
-  // Set up while the main kernel still runs only if it has few blocks: that saves 0.5 to 2 us, but each block then takes longer to start.
-  // Whole backward, early and not, with blocks twice as large: 1024 blocks 98.3 and 100.3 us, 4096 175.1 and 175.6, 8000 251.9 and 252.3,
-  // 8192 331.8 and 330.2, 16384 603.6 and 598.5, 32768 1224.7 and 1213.2.
+  // Set up while the main kernel still runs only if it has few blocks: that saves 1 to 2 us, but each block then takes longer to start.
+  // Whole backward, early and not, at 128-wide rows: 2048 blocks 98.3 and 99.3 us, 8000 172.0 and 173.6, 12 000 249.8 and 250.3, 16 000 323.6
+  // and 321.5, 16 384 327.7 and 327.1, 24 000 450.4 and 444.9, 65 536 1230 and 1215; 64-wide, 16 384: 400.8 and 402.9.
   if (grid < 16384) return launch_early(kern, grid, PP_THREADS, 0, stream, 1, p);
   kern<<<grid, PP_THREADS, 0, stream>>>(p);
   return cudaGetLastError();

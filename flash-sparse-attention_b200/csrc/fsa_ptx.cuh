@@ -417,7 +417,9 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
 }
 
 // logsigmoid(x) for two values, x given as y = x * log2(e): the arithmetic of log_sigmoid_fast, packed. The polynomial carries the
-// minus sign (a packed operation cannot negate an operand).
+// minus sign (a packed operation cannot negate an operand). The forward adds it to the scores in a rounding of its own where the backward
+// takes add_log_sigmoid2: they differ by an ulp of the logit, and both are off by 4.1e-5 at most and 4.9e-6 in the root mean square, which
+// is the polynomial (two million points of |x| <= 20, scores of deviation 1 to 30).
 __device__ __forceinline__ float2 log_sigmoid2(float2 y) {
   const float2 u = make_float2(ex2_approx(-fabsf(y.x)), ex2_approx(-fabsf(y.y)));
   float2 q = fma2(u, make_float2(-0.0415511145f, -0.0415511145f), make_float2(0.157838377f, 0.157838377f));
