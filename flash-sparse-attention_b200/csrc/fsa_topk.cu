@@ -292,10 +292,14 @@ __global__ void __launch_bounds__(TK_THREADS) topk_kernel(const T* __restrict__ 
 // Entries of a row that a CTA of a cluster of c takes.
 inline int topk_chunk(int n, int c) { return ((n + c - 1) / c + TK_V - 1) / TK_V * TK_V; }
 
+// Shared memory that keeps a second CTA off the SM: more than half of what it has. Clusters are launched with it: set up while a call in
+// front of them still runs, they would double up on the SMs that it leaves free (32 rows of 131 072 bf16 scores over and over, clusters
+// of four: 31.8 us, with an SM to each CTA 25.8, launched behind one another 26.2).
+constexpr int LONE_SMEM = 120 * 1024;
+
 // Clusters of c CTAs that the device holds with one CTA per SM, asked once per device.
 template <typename Kernel>
 int topk_room(Kernel kern, int c, std::atomic<int>& known) {
-  constexpr int LONE_SMEM = 120 * 1024;  // more than half of an SM's shared memory
   int fit = known.load(std::memory_order_relaxed) - 1;
   if (fit < 0) {
     fit = 0;
@@ -335,12 +339,14 @@ cudaError_t launch_topk_t(const void* scores, long long row_stride, int rows, in
   const int csize = topk_cluster_size<T, I>(rows, n), chunk = topk_chunk(n, csize);
   const T* x = reinterpret_cast<const T*>(scores);
   I* o = reinterpret_cast<I*>(out);
+  const int smem = csize > 1 ? LONE_SMEM : 0;  // topk_room has asked for it
+  const auto launch = [&](void (*kern)(const T*, long long, int, int, I*, int, int)) {
+    return launch_early(kern, (unsigned)(rows * csize), TK_THREADS, smem, stream, csize, x, row_stride, n, k, o, csize, chunk);
+  };
   // slices of up to 8192 / 16384 entries stay in registers
-  if (chunk <= TK_THREADS * TK_V)
-    return launch_early(topk_kernel<T, I, 1>, (unsigned)(rows * csize), TK_THREADS, 0, stream, csize, x, row_stride, n, k, o, csize, chunk);
-  if (chunk <= TK_THREADS * TK_V * 2)
-    return launch_early(topk_kernel<T, I, 2>, (unsigned)(rows * csize), TK_THREADS, 0, stream, csize, x, row_stride, n, k, o, csize, chunk);
-  return launch_early(topk_kernel<T, I, 0>, (unsigned)(rows * csize), TK_THREADS, 0, stream, csize, x, row_stride, n, k, o, csize, chunk);
+  if (chunk <= TK_THREADS * TK_V) return launch(topk_kernel<T, I, 1>);
+  if (chunk <= TK_THREADS * TK_V * 2) return launch(topk_kernel<T, I, 2>);
+  return launch(topk_kernel<T, I, 0>);
 }
 
 template <typename T>

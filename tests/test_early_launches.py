@@ -34,14 +34,9 @@ def _kernels():
 
 
 def _early():
-    """Names of the kernels that are launched early."""
-    text = "".join(_code(n) for n in sorted(os.listdir(CSRC)) if n.endswith((".cu", ".h")))
-    calls = re.findall(r"launch_early\(([^,;]*)", text)
-    assert calls
-    names = set(re.findall(r"\b(\w+_kernel)\b", " ".join(calls)))
-    if any(re.fullmatch(r"\s*kern\s*", c) for c in calls):  # auto kern = ...
-        names |= set(re.findall(r"\bkern = [^;]*?(\w+_kernel)", text))
-    return names
+    """Names of the kernels that are launched early: those that no source launches by their name in the plain form."""
+    text = "".join(_code(n) for n in sorted(os.listdir(CSRC)) if n.endswith(".cu"))
+    return set(_kernels()) - set(re.findall(r"\b(\w+_kernel)\s*(?:<[^;(){}]*>)?\s*<<<", text))
 
 
 def test_kernels_that_are_launched_early_wait_before_they_touch_memory():
