@@ -39,6 +39,7 @@ constexpr int DTN = 16;      // keys per warp tile
 #endif
 constexpr int DWARPS = 4;
 constexpr int MAX_CLUSTER = 8;  // splits that are merged inside a cluster
+constexpr int LONE_SMEM = 120 * 1024, PAIR_SMEM = 80 * 1024;  // shared memory that keeps a second, a third CTA off an SM
 
 // cp.async ring depth per warp: 64 KB a CTA, two tiles of 128 16-bit columns (paged top-k configuration: depth 2 / 3 = 100.6 / 101.9 us),
 // four of FP8 rows. Of 64 16-bit columns four as well where a warp walks many tiles (DEEP: 8 sequences of 32 000 keys, 32 / 8 heads:
@@ -1035,23 +1036,19 @@ __global__ void __launch_bounds__(256) dec_gate_ext_kernel(const DecKernelParams
 // partials and the combine launch take 15.5, 96 of 3 52.6 against 36.4). A grid that single CTAs spread over the SMs
 // one by one has to find that room, too: 16 clusters of 8 doubled up on some SMs (2048 FP8 keys a CTA: 39.7 against 35.2 us).
 // Where they fit they save 1 to 1.5 us (a fifth of the smallest calls). The runtime's answers are kept per device.
+// Returns how many are resident at a time, 0 where the call's do not fit.
 template <typename Kernel>
-bool clusters_fit(Kernel kern, int clusters, int size, int smem, std::atomic<int> (*cache)[2][MAX_CLUSTER + 1]) {
-  constexpr int LONE_SMEM = 120 * 1024;  // more than half of an SM's shared memory: one CTA per SM
+int clusters_fit(Kernel kern, int clusters, int size, int smem, std::atomic<int> (*cache)[2][MAX_CLUSTER + 1]) {
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return false;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return 0;
   const bool lone = (long long)clusters * size <= device_sm_count();
   std::atomic<int>& known = cache[dev][lone][size];
   int room = known.load(std::memory_order_relaxed) - 1;  // 0: not asked yet
   if (room < 0) {
-    room = 0;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LONE_SMEM) == cudaSuccess)
-      room = resident_clusters(kern, size, DWARPS * 32, lone ? LONE_SMEM : smem);
-    else
-      (void)cudaGetLastError();
+    room = resident_clusters(kern, size, DWARPS * 32, lone ? LONE_SMEM : smem);
     known.store(room + 1, std::memory_order_relaxed);
   }
-  return clusters <= room;
+  return clusters <= room ? room : 0;
 }
 
 // CL: when the clusters do not fit, p.cluster becomes 0 and nothing is launched.
@@ -1060,19 +1057,23 @@ cudaError_t launch_variant(DecKernelParams& p, cudaStream_t stream) {
   auto kern = dec_kernel<HD, T, KIND, TR, OCC, CL, DEEP>;
   // the variant for two CTAs per SM asks for enough shared memory that a third cannot join
   constexpr int ring = DecSmem<HD, sizeof(T), DEEP>::kTotal;
-  constexpr int smem = (TR && OCC == 2 && ring < 80 * 1024) ? 80 * 1024 : ring;
+  constexpr int smem = (TR && OCC == 2 && ring < PAIR_SMEM) ? PAIR_SMEM : ring;
   static std::atomic<unsigned long long> opted_in{0};  // one bit per device: the attribute is per device
-  if (cudaError_t e = smem_opt_in(kern, smem, opted_in); e != cudaSuccess) return e;
+  if (cudaError_t e = smem_opt_in(kern, smem > LONE_SMEM ? smem : LONE_SMEM, opted_in); e != cudaSuccess) return e;
   const long long grid = (long long)p.Hkv * p.B * p.num_splits;
   if (grid <= 0) return cudaSuccess;
+  int room = 0;
   if constexpr (CL) {
-    static_assert(smem <= 120 * 1024, "the opt-in of clusters_fit covers the launch");
-    static std::atomic<int> room[64][2][MAX_CLUSTER + 1];
-    if (!clusters_fit(kern, p.Hkv * p.B, p.cluster, smem, room)) {
+    static_assert(smem <= LONE_SMEM, "the opt-in covers the launch");
+    static std::atomic<int> rooms[64][2][MAX_CLUSTER + 1];
+    room = clusters_fit(kern, p.Hkv * p.B, p.cluster, smem, rooms);
+    if (room == 0) {
       p.cluster = 0;
       return cudaSuccess;
     }
   }
+  const FsaDecLaunch how = fsa_dec_launch(grid, HD > 128 ? 1 : OCC, CL ? p.cluster : 1, room, p.n_tiles / (DWARPS * p.num_splits), device_sm_count());
+  const int share = how.per_sm == 1 ? LONE_SMEM : how.per_sm == 2 ? PAIR_SMEM : 0;
   if (KIND == KIND_GATED && p.gate_ws) {
     const long long items = (long long)p.B * p.Hkv * p.n_tiles;
     if (items > 0) {
@@ -1083,9 +1084,9 @@ cudaError_t launch_variant(DecKernelParams& p, cudaStream_t stream) {
   }
   if constexpr (CL) {
     static_assert(HD <= 128 && DWARPS * (16 * HD + 32) * 4 + (16 * HD + 32) * 4 <= ring, "the merged state fits behind the warps'");
-    return launch_early(kern, (unsigned)grid, DWARPS * 32, smem, stream, p.cluster, p);
+    return launch_early_if(how.early, kern, (unsigned)grid, DWARPS * 32, smem > share ? smem : share, stream, p.cluster, p);
   }
-  return launch_early(kern, (unsigned)grid, DWARPS * 32, smem, stream, 1, p);
+  return launch_early_if(how.early, kern, (unsigned)grid, DWARPS * 32, smem > share ? smem : share, stream, 1, p);
 }
 
 template <int HD, typename T, int KIND>

@@ -3,6 +3,8 @@
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
+
+#include <utility>
 #include <stdint.h>
 
 #include <atomic>
@@ -179,12 +181,12 @@ inline int resident_clusters(Kernel kern, int size, int threads, int smem) {
 }
 
 // Launch whose blocks may be set up while the kernel in front of it in the stream still runs: the kernel has to begin with
-// after_previous() or wait_for_previous(). `cluster` CTAs form a cluster (1: none). What it saves is 1 to 2 us between two kernels: a decode step of one
-// sequence over and over 12.3 -> 10.4 us, top-k selection, scales and FP8 decode 33.3 -> 29.6, a short prompt 16.4 -> 14.6, a paged
-// batch and its combine 186.9 -> 184.2.
+// after_previous() or wait_for_previous(). `cluster` CTAs form a cluster (1: none). What it saves is 1 to 2 us between two kernels: a
+// decode step of one sequence over and over 12.3 -> 10.4 us, top-k selection, scales and FP8 decode 33.3 -> 29.6, a short prompt
+// 16.4 -> 14.6, a paged batch and its combine 186.9 -> 184.2. `early` false: behind the kernel in front after all.
 template <typename... Params, typename... Args>
-inline cudaError_t launch_early(void (*kern)(Params...), unsigned grid, int threads, int smem, cudaStream_t stream, int cluster,
-                                Args&&... args) {
+inline cudaError_t launch_early_if(bool early, void (*kern)(Params...), unsigned grid, int threads, int smem, cudaStream_t stream, int cluster,
+                                   Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid, 1, 1);
   cfg.blockDim = dim3((unsigned)threads, 1, 1);
@@ -192,7 +194,7 @@ inline cudaError_t launch_early(void (*kern)(Params...), unsigned grid, int thre
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[0].val.programmaticStreamSerializationAllowed = early ? 1 : 0;
   attr[1].id = cudaLaunchAttributeClusterDimension;
   attr[1].val.clusterDim.x = (unsigned)cluster;
   attr[1].val.clusterDim.y = 1;
@@ -202,6 +204,11 @@ inline cudaError_t launch_early(void (*kern)(Params...), unsigned grid, int thre
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
   if (e != cudaSuccess) (void)cudaGetLastError();  // it is returned here, and not to the next launch that asks for the last error
   return e;
+}
+template <typename... Params, typename... Args>
+inline cudaError_t launch_early(void (*kern)(Params...), unsigned grid, int threads, int smem, cudaStream_t stream, int cluster,
+                                Args&&... args) {
+  return launch_early_if(true, kern, grid, threads, smem, stream, cluster, std::forward<Args>(args)...);
 }
 
 #ifdef __CUDACC__

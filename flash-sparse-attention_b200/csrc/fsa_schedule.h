@@ -79,6 +79,28 @@ inline int fsa_fwd_cluster_size(long long ctas, int tiles, int sms, Room room) {
   return 1;
 }
 
+// Decode: whether a call is set up while the kernel in front of it still runs, and how many of its CTAs an SM may hold then (0: as many
+// as find room). `occ`: CTAs that find room on an SM; `cluster`: CTAs of a cluster (1: none), `room`: clusters that are resident at a
+// time; `tiles`: key tiles of a warp. Setting it up early saves 0.3 to 1 us, but the SMs that the kernel in front leaves first would take
+// as many CTAs as fit, and others none. Of calls of one round, us, over and over, one split, 4 KV heads of 128:
+// - fewer to an SM than fit: the share is kept to what an even spread is. 280 CTAs of 300 keys 9.8 early, 9.0 behind one another, 8.9
+//   so; 260 of 2500 keys 54.1, 53.6 and 53.3; 128 in clusters of four 13.6, 13.4 and 13.0; gated, behind the pass over delta, 100 of 1000 keys
+//   36.5, 32.0 and 31.5.
+// - as many as fit: it pays where a call is short (340 CTAs of 300 keys 10.2 early, 10.6 not; of 1000 keys 32.1 and 31.5).
+// - nearly all clusters that are resident: the last ones find no room until the call in front has left (56 clusters of five 15.8 early, 12.6
+//   not; 48 12.3 and 12.7). Pairs always do.
+struct FsaDecLaunch {
+  bool early;
+  int per_sm;
+};
+inline FsaDecLaunch fsa_dec_launch(long long ctas, int occ, int cluster, int room, long long tiles, int sms) {
+  if (occ == 1 || ctas > occ * (long long)sms) return {true, 0};
+  const int per_sm = (int)((ctas + sms - 1) / sms);
+  if (per_sm < occ) return {true, per_sm};
+  if (cluster > 1) return {cluster == 2 || ctas / cluster <= room - room / 16, 0};
+  return {tiles < 12, 0};
+}
+
 // Share of `total` blocks owned by split `s` of `ns`: the first total%ns splits get one extra.
 FSA_HD void fsa_split_range(int total, int ns, int s, int* off, int* cnt) {
   const int base = total / ns, extra = total % ns;
