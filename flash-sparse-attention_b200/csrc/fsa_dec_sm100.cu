@@ -42,8 +42,8 @@ constexpr int MAX_CLUSTER = 8;  // splits that are merged inside a cluster
 constexpr int LONE_SMEM = 120 * 1024, PAIR_SMEM = 80 * 1024;  // shared memory that keeps a second, a third CTA off an SM
 
 // cp.async ring depth per warp: 64 KB a CTA, two tiles of 128 16-bit columns (paged top-k configuration: depth 2 / 3 = 100.6 / 101.9 us),
-// four of FP8 rows. Of 64 16-bit columns four as well where a warp walks many tiles (DEEP: 8 sequences of 32 000 keys, 32 / 8 heads:
-// 118.6 us at two, 106.0 at four), else two: a warp of few tiles is bound by its own instructions, and the first tile is worked on once
+// four of FP8 rows. Of 64 16-bit columns four as well where a warp walks many tiles and an SM has room for more in flight (DEEP,
+// fsa_dec_deep_ring: 8 sequences of 32 000 keys, 32 / 8 heads: 118.6 us at two, 106.0 at four), else two: a warp of few tiles is bound by its own instructions, and the first tile is worked on once
 // the ring is full (one sequence of 500 keys: 8.2 us at two, 8.6 at four; of 4000, merged in a cluster, 10.4 and 11.5 at six).
 template <int HD, int ES, bool DEEP>
 struct DecStages {
@@ -1113,7 +1113,7 @@ cudaError_t launch_one(DecKernelParams& p, cudaStream_t stream) {
       const long long per_sm = (ctas + sms - 1) / sms;
       auto cost = [&](long long occ) { return ((ctas + occ * sms - 1) / (occ * sms)) * (per_sm < occ ? per_sm : occ); };
       if constexpr (HD == 64 && sizeof(T) == 2) {
-        if (p.n_tiles >= 16ll * DWARPS * p.num_splits)  // sixteen tiles a warp (see DecStages)
+        if (fsa_dec_deep_ring(ctas, cost(3) <= cost(2) ? 3 : 2, p.n_tiles / (DWARPS * p.num_splits), (int)sms))
           return cost(3) <= cost(2) ? launch_variant<HD, T, KIND, true, 3, false, true>(p, stream)
                                     : launch_variant<HD, T, KIND, true, 2, false, true>(p, stream);
       }

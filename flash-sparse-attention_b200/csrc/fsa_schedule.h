@@ -101,6 +101,17 @@ inline FsaDecLaunch fsa_dec_launch(long long ctas, int occ, int cluster, int roo
   return {tiles < 12, 0};
 }
 
+// Decode, 64-wide rows of 16 bits: whether a warp's ring holds four tiles instead of two. `tiles`: of a warp; `occ`: CTAs that find room on
+// an SM. Two tiles of 64 columns are half the bytes in flight that two of 128 are, which short walks do not notice (one round, 1100 keys:
+// 200 CTAs 16.3 us at two, 17.0 at four) and three CTAs on nearly every SM make up for: 2500 keys, one round of 444, 300 CTAs 38.8 and 36.5, 360
+// 43.3 and 41.5, 400 43.2 and 45.1, 440 46.5 and 49.1; two rounds, 6000 keys, 800 185 and 181, 840 191 and 201; 592, two rounds
+// of 296 in pairs, 2500 keys, 72.0 and 64.6, 1100 keys 6 % faster.
+inline bool fsa_dec_deep_ring(long long ctas, int occ, long long tiles, int sms) {
+  const long long slots = occ * (long long)sms, rounds = (ctas + slots - 1) / slots;
+  if (tiles < (rounds > 1 ? 16 : 32)) return false;
+  return occ < 3 || (rounds > 1 ? 13 * ctas <= 12 * rounds * slots : 7 * ctas <= 6 * slots);
+}
+
 // Share of `total` blocks owned by split `s` of `ns`: the first total%ns splits get one extra.
 FSA_HD void fsa_split_range(int total, int ns, int s, int* off, int* cnt) {
   const int base = total / ns, extra = total % ns;

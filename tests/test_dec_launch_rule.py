@@ -1,4 +1,5 @@
-"""The rule that sets a decode call up while the kernel in front of it still runs, from the header that the launcher takes it from. (us:
+"""The rules that set a decode call up while the kernel in front of it still runs, and that give a warp of 64-wide rows a deeper ring, from
+the header that the launcher takes them from. (us:
 the same call over and over, one split unless clusters are named, 4 KV heads.)"""
 
 import ctypes
@@ -18,9 +19,12 @@ def rule(tmp_path_factory):
     d = tmp_path_factory.mktemp("rule")
     (d / "rule.cpp").write_text(f'#include "{os.path.abspath(HEADER)}"\n'
                                 'extern "C" int rule(long long c, int occ, int cluster, int room, long long tiles, int sms) {\n'
-                                '  const FsaDecLaunch r = fsa_dec_launch(c, occ, cluster, room, tiles, sms); return r.early ? r.per_sm : -1; }\n')
+                                '  const FsaDecLaunch r = fsa_dec_launch(c, occ, cluster, room, tiles, sms); return r.early ? r.per_sm : -1; }\n'
+                                'extern "C" int deep(long long c, int occ, long long tiles, int sms) {\n'
+                                '  return fsa_dec_deep_ring(c, occ, tiles, sms); }\n')
     subprocess.run(["g++", "-O1", "-shared", "-fPIC", "-std=c++17", "-o", str(d / "rule.so"), str(d / "rule.cpp")], check=True)
-    fn = ctypes.CDLL(str(d / "rule.so")).rule
+    lib = ctypes.CDLL(str(d / "rule.so"))
+    fn = lib.rule
     fn.argtypes = [ctypes.c_longlong, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_longlong, ctypes.c_int]
 
     def call(ctas, occ=3, cluster=1, keys=1000):
@@ -28,6 +32,7 @@ def rule(tmp_path_factory):
         room = (LONE if ctas <= SMS else ROOM).get(cluster, 0)
         return fn(ctas, occ, cluster, room, -(-keys // 16) // 4, SMS)
 
+    call.deep = lambda ctas, occ, keys: bool(lib.deep(ctypes.c_longlong(ctas), occ, ctypes.c_longlong(-(-keys // 16) // 4), SMS))
     return call
 
 
@@ -47,3 +52,15 @@ def test_what_waits(rule):
     assert rule(296, occ=2, cluster=2) == 0 and rule(256, occ=2, cluster=4) == 0
     assert rule(340, keys=300) == 0 and rule(340, keys=1000) == -1    # 10.2 us early, 10.6 not; 32.1 and 31.5
     assert rule(444, keys=768) == -1 and rule(296, occ=2, keys=2500) == -1
+
+
+def test_deep_ring(rule):
+    # thirty-two tiles a warp in one round, sixteen in several (1100 keys: 200 CTAs 16.3 us with two tiles, 17.0 with four)
+    assert rule.deep(128, 3, 2033) and not rule.deep(128, 3, 2032)
+    assert rule.deep(500, 2, 1009) and not rule.deep(500, 2, 1008)
+    # 2500 keys, two tiles and four: 360 CTAs 43.3 and 41.5 us, 400 43.2 and 45.1, 440 46.5 and 49.1
+    assert rule.deep(300, 3, 2500) and rule.deep(360, 3, 2500) and rule.deep(380, 3, 2500)
+    assert not rule.deep(384, 3, 4700) and not rule.deep(400, 3, 2500) and not rule.deep(444, 3, 2500)
+    assert rule.deep(592, 2, 2500)                                    # 72.0 and 64.6
+    assert rule.deep(800, 3, 6000) and not rule.deep(840, 3, 6000)    # two rounds of 444: 185 and 181, 191 and 201
+    assert not rule.deep(1776, 3, 2375)                               # 74 sequences of 9500 keys, 8 KV heads, three splits: 221.6 and 230.6

@@ -1,4 +1,4 @@
-"""Decode: 64-wide rows on both sides of the deeper ring (sixteen tiles of 16 keys a warp)."""
+"""Decode: 64-wide rows on both sides of the deeper ring (thirty-two tiles of 16 keys a warp in one round of CTAs, sixteen in several)."""
 
 import pytest
 import torch
@@ -9,7 +9,7 @@ from oracle import eager
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("keys", [1008, 1024, 1025, 1500])  # 63, 64, 65, 94 tiles for four warps
+@pytest.mark.parametrize("keys", [1025, 2032, 2048, 2049, 2500])  # 65, 127, 128, 129, 157 tiles for four warps
 @pytest.mark.parametrize("kind", ["dense", "sparse", "gated"])
 def test_deep_ring(keys, kind):
     import flash_sparse_attn as fsa
@@ -28,3 +28,15 @@ def test_deep_ring(keys, kind):
     torch.cuda.synchronize()
     fsa.check_status()
     assert_close("out", out, ref)
+
+
+# CTAs on 148 SMs, two KV heads: 370 take the deeper ring, 400, nearly three to an SM, do not; 460 do in rounds of two to an SM, 456 keys are too few
+@pytest.mark.parametrize("batch, keys", [(185, 2100), (200, 2100), (230, 1040), (230, 456)])
+def test_many_sequences(batch, keys):
+    import flash_sparse_attn as fsa
+
+    g = torch.Generator().manual_seed(batch)
+    q, k, v = (torch.randn(*s, 64, generator=g).to(torch.bfloat16) for s in ((batch, 4), (batch, keys, 2), (batch, keys, 2)))
+    out = fsa.flash_dense_attn_with_kvcache_func(*(t.cuda() for t in (q, k, v)), num_splits=1)
+    assert_close("out", out, eager.decode(q, k, v))
+    fsa.check_status()
