@@ -906,12 +906,62 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
                        __int_as_float(0x7fffffff)};
         const float2 al2 = make_float2(alpha, alpha);  // times log2(e) for the logsigmoid gate, whose exponential is 2^x
         const bool logsig = p.flags & F_LOGSIGMOID;
-        // rolled up: unrolled over the row, the gate's code alone is larger than the instruction caches hold beside the
-        // other roles', and its 128 columns took 6700 cycles
+        // logits = (q.k + g(alpha * delta_j)) * scale, g = logsigmoid or identity (flash_sparse_attn/ops/triton/flash_gated_fwd.py:104-122,
+        // activations.py:245-262). Two threads a row work the first 32 gates out before the scores are waited for. One thread a row (head sizes
+        // above 128) takes gate and score together: with the gates first head size 192, S = 4096, 16 / 4 heads takes 245 us, so 233; with
+        // an identity gate 205 and 189. Both loops are rolled up: unrolled over
+        // the row, the gate's code alone is larger than the instruction caches hold beside the other roles', and its 128 columns took 6700 cycles.
+        if constexpr (RO::HALVES == 1) {
+          ok = mbar_wait(&bars->s_full[q], par, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+#pragma unroll 1
+          for (int ch = 0; ch < TN / 32; ++ch) {
+            uint32_t r[32];
+            tmem_ld32(tS + ch * 32, r);
+            tmem_ld_wait();
+            const float4* d4 = reinterpret_cast<const float4*>(&bars->dl[ds][ch * 32]);
+            if (logsig) {
+#pragma unroll
+              for (int i = 0; i < 32; i += 4) {
+                const float4 dd = d4[i >> 2];
+                const float2 a = add_log_sigmoid2(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])),
+                                                  mul2(al2, make_float2(dd.x, dd.y)));
+                const float2 b = add_log_sigmoid2(make_float2(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])),
+                                                  mul2(al2, make_float2(dd.z, dd.w)));
+                r[i] = __float_as_uint(a.x);
+                r[i + 1] = __float_as_uint(a.y);
+                r[i + 2] = __float_as_uint(b.x);
+                r[i + 3] = __float_as_uint(b.y);
+              }
+            } else {
+#pragma unroll
+              for (int i = 0; i < 32; i += 4) {
+                const float4 dd = d4[i >> 2];
+                r[i] = __float_as_uint(fmaf(alpha, dd.x, __uint_as_float(r[i])));
+                r[i + 1] = __float_as_uint(fmaf(alpha, dd.y, __uint_as_float(r[i + 1])));
+                r[i + 2] = __float_as_uint(fmaf(alpha, dd.z, __uint_as_float(r[i + 2])));
+                r[i + 3] = __float_as_uint(fmaf(alpha, dd.w, __uint_as_float(r[i + 3])));
+              }
+            }
+            if (mode != FSA_MASK_NONE) {
+              mask_cols32(r, tile_bits(tm, ch * 32));
+            } else if (!rm.row_ok) {
+              // rows past the query length read as zero scores in fully visible tiles
+#pragma unroll
+              for (int i = 0; i < 32; ++i) r[i] = 0u;
+            }
+            tmem_st32(tS + ch * 32, r);
+#pragma unroll
+            for (int i = 0; i < 32; i += 8) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                mx[j] = max3(mx[j], __uint_as_float(r[i + 2 * j]), __uint_as_float(r[i + 2 * j + 1]));
+            }
+          }
+        } else {
 #pragma unroll 1
         for (int ch = 0; ch < NC / 32; ++ch) {
-          // g(alpha * delta_j), g = logsigmoid or identity (flash_sparse_attn/ops/triton/flash_gated_fwd.py:104-122,
-          // activations.py:245-262): the first 32 columns before the scores are waited for
           float2 g[16];
           {
             float4 dd[8];
@@ -962,6 +1012,7 @@ __global__ void __launch_bounds__(FwdRoles<HD, KIND>::NTHREADS, 1) fwd_kernel(co
                 mx[j] = max3(mx[j], __uint_as_float(r[i + 2 * j]), __uint_as_float(r[i + 2 * j + 1]));
             }
           }
+        }
         }
         if (!ok) break;
         __syncwarp();
