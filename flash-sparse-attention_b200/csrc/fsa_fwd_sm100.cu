@@ -1412,7 +1412,13 @@ cudaError_t launch_one(FwdKernelParams& p, cudaStream_t stream) {
     if (p.cluster == 1) return launch_one<HD, T, KIND>(p, stream);
     return launch_early(kern, (unsigned)grid * p.cluster, threads, smem, stream, p.cluster, p);
   }
-  return launch_early(kern, (unsigned)grid, threads, smem, stream, 1, p);
+  // Set up while the kernel in front still runs, except one round of equally long CTAs on more than half of the SMs: behind a call that leaves
+  // the other half free, more of them come to share a pair of SMs than when all are spread at once. Full attention, 8 heads of 128, 96 CTAs:
+  // S = 3000 56.8 us early, 55.4 not, over 6000 keys 101.1 and 98.3, sparse 105.3 and 101.8. Short calls (700 tokens, 32 heads 21.6 and 21.7), head
+  // size 64 (5000 tokens, 4 heads 75.4 and 76.7) and the gated kind gain as much as they lose.
+  const bool even = KIND != KIND_GATED && HD > 64 && !(p.flags & (F_CAUSAL | F_LOCAL | F_VARLEN_Q | F_VARLEN_K | F_USED_Q | F_USED_K));
+  const int sms = device_sm_count();
+  return launch_early_if(!(even && 2 * grid > sms && grid <= sms && p.n_tiles_k >= 12), kern, (unsigned)grid, threads, smem, stream, 1, p);
 }
 
 }  // namespace
