@@ -1072,7 +1072,8 @@ cudaError_t launch_variant(DecKernelParams& p, cudaStream_t stream) {
       return cudaSuccess;
     }
   }
-  const FsaDecLaunch how = fsa_dec_launch(grid, HD > 128 ? 1 : OCC, CL ? p.cluster : 1, room, p.n_tiles / (DWARPS * p.num_splits), device_sm_count());
+  const FsaDecLaunch how = fsa_dec_launch(grid, HD > 128 ? 1 : OCC, CL ? p.cluster : 1, room, p.num_splits, p.n_tiles / (DWARPS * p.num_splits),
+                                           device_sm_count());
   const int share = how.per_sm == 1 ? LONE_SMEM : how.per_sm == 2 ? PAIR_SMEM : 0;
   if (KIND == KIND_GATED && p.gate_ws) {
     const long long items = (long long)p.B * p.Hkv * p.n_tiles;

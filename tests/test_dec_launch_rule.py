@@ -18,19 +18,19 @@ LONE = {2: 74, 3: 46, 4: 33, 5: 27, 6: 20, 7: 18, 8: 15}   # and with one
 def rule(tmp_path_factory):
     d = tmp_path_factory.mktemp("rule")
     (d / "rule.cpp").write_text(f'#include "{os.path.abspath(HEADER)}"\n'
-                                'extern "C" int rule(long long c, int occ, int cluster, int room, long long tiles, int sms) {\n'
-                                '  const FsaDecLaunch r = fsa_dec_launch(c, occ, cluster, room, tiles, sms); return r.early ? r.per_sm : -1; }\n'
+                                'extern "C" int rule(long long c, int occ, int cluster, int room, int splits, long long tiles, int sms) {\n'
+                                '  const FsaDecLaunch r = fsa_dec_launch(c, occ, cluster, room, splits, tiles, sms); return r.early ? r.per_sm : -1; }\n'
                                 'extern "C" int deep(long long c, int occ, long long tiles, int sms) {\n'
                                 '  return fsa_dec_deep_ring(c, occ, tiles, sms); }\n')
     subprocess.run(["g++", "-O1", "-shared", "-fPIC", "-std=c++17", "-o", str(d / "rule.so"), str(d / "rule.cpp")], check=True)
     lib = ctypes.CDLL(str(d / "rule.so"))
     fn = lib.rule
-    fn.argtypes = [ctypes.c_longlong, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_longlong, ctypes.c_int]
+    fn.argtypes = [ctypes.c_longlong, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_longlong, ctypes.c_int]
 
-    def call(ctas, occ=3, cluster=1, keys=1000):
+    def call(ctas, occ=3, cluster=1, keys=1000, splits=1):
         """-1: behind the kernel in front, otherwise the CTAs an SM may hold (0: as many as find room)."""
         room = (LONE if ctas <= SMS else ROOM).get(cluster, 0)
-        return fn(ctas, occ, cluster, room, -(-keys // 16) // 4, SMS)
+        return fn(ctas, occ, cluster, room, splits, -(-keys // 16) // (4 * splits), SMS)
 
     call.deep = lambda ctas, occ, keys: bool(lib.deep(ctypes.c_longlong(ctas), occ, ctypes.c_longlong(-(-keys // 16) // 4), SMS))
     return call
@@ -49,8 +49,10 @@ def test_an_even_share(rule):
 
 def test_what_waits(rule):
     assert rule(280, occ=2, cluster=5) == -1 and rule(240, occ=2, cluster=5) == 0   # 15.8 us early, 12.6 not; 12.3 and 12.7
-    assert rule(296, occ=2, cluster=2) == 0 and rule(256, occ=2, cluster=4) == 0
+    assert rule(279, occ=2, cluster=3) == rule(259, occ=2, cluster=7) == -1         # 93 of three 15.3 us early, 12.3 not; 37 of seven 14.3 and 12.9
+    assert rule(296, occ=2, cluster=2) == rule(284, occ=2, cluster=4) == rule(264, occ=2, cluster=8) == 0
     assert rule(340, keys=300) == 0 and rule(340, keys=1000) == -1    # 10.2 us early, 10.6 not; 32.1 and 31.5
+    assert rule(360, keys=7540, splits=3) == 0    # 52.2 us early, 53.6 not
     assert rule(444, keys=768) == -1 and rule(296, occ=2, keys=2500) == -1
 
 
