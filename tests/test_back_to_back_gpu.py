@@ -76,6 +76,46 @@ def test_chain_equals_its_calls():
     fsa.check_status()
 
 
+def test_two_streams_that_join():
+    """Chains on two streams at a time, and a call that reads what both wrote: eagerly and from one captured graph."""
+    import flash_sparse_attn as fsa
+
+    state = _state()
+    other = {n: t.flip(0).contiguous() for n, t in state.items()}
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+
+    def both(sync):
+        here = torch.cuda.current_stream()
+        got = []
+        for s, x in zip(streams, (state, other)):
+            s.wait_stream(here)
+            with torch.cuda.stream(s):
+                got.append(_chain(x, sync))
+        for s in streams:
+            here.wait_stream(s)
+        out = fsa.flash_dense_attn_func(got[0][-2], got[1][-1], got[0][-1], is_causal=True)
+        return got[0] + got[1] + [fsa.flash_dense_attn_with_kvcache_func(out[:, -1], got[1][-2], got[0][-2], num_splits=3)]
+
+    state["k"] = state["k"].repeat_interleave(2, 2)  # as many KV heads as query heads: results serve as keys and values
+    state["v"], other["k"], other["v"] = (t.repeat_interleave(2, 2) for t in (state["v"], other["k"], other["v"]))
+    want = both(True)
+    torch.cuda.synchronize()
+    for _ in range(3):
+        got = both(False)
+        torch.cuda.synchronize()
+        for a, b in zip(got, want):
+            assert torch.equal(a, b)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = both(False)
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    fsa.check_status()
+
+
 def test_backward_passes_in_a_row():
     import flash_sparse_attn as fsa
 

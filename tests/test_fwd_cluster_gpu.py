@@ -1,5 +1,6 @@
 """Dense calls of few CTAs, whose key tiles are shared by the CTAs of a cluster: at the sizes where the cluster grows (none, two, four,
-eight CTAs on 148 SMs), with tiles that are not full, shares without a tile, and what keeps a call out of it."""
+eight CTAs on 148 SMs), with tiles that are not full, shares without a tile, and what keeps a call out of it. test_fwd_cluster_rule.py
+says which size a form takes."""
 
 import pytest
 import torch
@@ -21,6 +22,25 @@ def test_shares_of_the_keys(seqlen, hq, head_dim, causal):
     q = q * 3  # maxima that differ between the shares
     ref, lse_ref = eager.forward(q, k, v, None, causal, return_lse=True)
     out, lse = fsa.flash_dense_attn_func(*(t.cuda() for t in (q, k, v)), is_causal=causal, return_lse=True)
+    torch.cuda.synchronize()
+    fsa.check_status()
+    assert_close("out", out, ref)
+    assert torch.allclose(lse.cpu(), lse_ref, rtol=0, atol=2e-3)
+
+
+# by the rule: eight CTAs (9 and 12 pairs of query tiles over 17 and 24 key tiles), four where the batch is two, two at 16 heads
+@pytest.mark.parametrize("batch, seqlen, hq, hkv, pack", [(1, 2050, 1, 1, False), (1, 3000, 1, 1, False), (2, 2050, 1, 1, False),
+                                                          (2, 1000, 8, 2, False), (1, 1000, 4, 1, True), (1, 1300, 2, 1, True)])
+@pytest.mark.parametrize("head_dim", [64, 128])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_clusters_of_eight_batches_and_packed_heads(batch, seqlen, hq, hkv, pack, head_dim, causal, dtype):
+    import flash_sparse_attn as fsa
+
+    q, k, v = seeded_qkv(seqlen + hq, batch, seqlen, seqlen, hq, hkv, head_dim, dtype)
+    q = q * 3
+    ref, lse_ref = eager.forward(q, k, v, None, causal, return_lse=True)
+    out, lse = fsa.flash_dense_attn_func(*(t.cuda() for t in (q, k, v)), is_causal=causal, pack_gqa=pack, return_lse=True)
     torch.cuda.synchronize()
     fsa.check_status()
     assert_close("out", out, ref)

@@ -360,16 +360,36 @@ def test_gil_is_free_during_the_launch():
 
 
 @pytest.mark.gpu
-def test_scales_of_a_declined_call_are_packed_once(monkeypatch):
-    import flash_sparse_attn as fsa
-    from flash_sparse_attn.ops.triton import quant
+def test_scales_are_packed_once(monkeypatch):
+    """By the native launcher where it takes the call, by the Python one where it declines: both reach the library's entry point, whose
+    calls are counted on either way."""
+    import ctypes
 
-    count, pack = [], quant.scales_f32
-    monkeypatch.setattr(quant, "scales_f32", lambda *a: count.append(1) or pack(*a))
-    x = lambda *s: torch.randn(*s, 64, device=DEV).to(torch.float8_e4m3fn)  # noqa: E731  (native FP8 has 128 columns)
+    import flash_sparse_attn as fsa
+    from flash_sparse_attn import _lib
+
+    lib, count = _lib.load(), []
+    real = lib.fsa_pack_scales
+    address = lambda f: ctypes.cast(f, ctypes.c_void_p).value  # noqa: E731
+    stub = ctypes.CFUNCTYPE(ctypes.c_int, *real.argtypes)(lambda *a: count.append("native") or real(*a))
+    monkeypatch.setattr(lib, "fsa_pack_scales", lambda *a: count.append("python") or real(*a))
     one = torch.ones(1, device=DEV)
     kw = dict(is_quant=True, query_scale=one, key_scale=one, value_scale=one)
-    fsa.flash_dense_attn_with_kvcache_func(x(2, 4), x(2, 50, 2), x(2, 50, 2), **kw)
-    assert len(count) == 1
-    fsa.flash_dense_attn_func(x(2, 50, 4), x(2, 50, 2), x(2, 50, 2), **kw)
-    assert len(count) == 2
+
+    def packed(d, prompt):
+        x = lambda *s: torch.randn(*s, d, device=DEV).to(torch.float8_e4m3fn)  # noqa: E731
+        count.clear()
+        if prompt:
+            fsa.flash_dense_attn_func(x(2, 50, 4), x(2, 50, 2), x(2, 50, 2), **kw)
+        else:
+            fsa.flash_dense_attn_with_kvcache_func(x(2, 4), x(2, 50, 2), x(2, 50, 2), **kw)
+        return list(count)
+
+    _lib._host.init(address(lib.fsa_decode), address(lib.fsa_fwd), address(lib.fsa_topk_indices), address(stub))
+    try:
+        for prompt in (False, True):
+            assert packed(128, prompt) == ["native"]
+            assert packed(64, prompt) == ["python"]  # native FP8 has 128 columns
+    finally:
+        _lib._host.init(address(lib.fsa_decode), address(lib.fsa_fwd), address(lib.fsa_topk_indices), address(real))
+    fsa.check_status()

@@ -48,7 +48,6 @@ def test_every_tensor_that_asks_for_a_gradient_is_recorded(asked, monkeypatch):
 @pytest.mark.gpu
 def test_same_results_and_refusals():
     import flash_sparse_attn as fsa
-    from flash_sparse_attn.ops.triton import interface
     from fixtures import seeded_qkv
 
     q, k, v = (t.to(DEV) for t in seeded_qkv(1, 2, 300, 300, 4, 2, 64))
@@ -63,11 +62,10 @@ def test_same_results_and_refusals():
     alpha, delta = torch.randn(2, 300, 4, device=DEV, dtype=q.dtype), torch.randn(2, 300, 2, device=DEV, dtype=q.dtype)
     gated = fsa.flash_gated_attn_func(q, k, v, alpha, delta, is_causal=True)
     assert torch.equal(gated, fsa.flash_gated_attn_func(leaf, k, v, alpha, delta, is_causal=True))
-    with pytest.raises(Exception):
+    with pytest.raises(RuntimeError, match="vmap"):
         torch.func.vmap(lambda a: fsa.flash_sparse_attn_func(a, k, v))(q[None])
-    with torch.autograd.forward_ad.dual_level(), pytest.raises(Exception):
+    with torch.autograd.forward_ad.dual_level(), pytest.raises(NotImplementedError, match="jvp"):
         fsa.flash_sparse_attn_func(torch.autograd.forward_ad.make_dual(q, torch.ones_like(q)), k, v)
-    assert interface._AttnFunc is not None
 
 
 @pytest.mark.gpu
@@ -88,7 +86,7 @@ def test_native_topk_equals_the_python_launcher(dtype, monkeypatch):
     for bad in (0, 1001):
         with pytest.raises(AssertionError):
             topk_indices(x, bad)
-    with pytest.raises(Exception):
+    with pytest.raises((KeyError, AssertionError, RuntimeError, TypeError), match="int32"):
         topk_indices(torch.zeros(4, 10, dtype=torch.int32, device=DEV), 2)
     stored = torch.randn(2, 1000, device=DEV, requires_grad=True)
     assert not topk_indices(stored, 5).requires_grad
