@@ -248,7 +248,7 @@ __device__ __forceinline__ uint32_t elect_one() {
 // carries the single-lane predicate, instead of a divergent branch around a block of MMAs. `lead` has to come from
 // elect_one(): with "lane == 0" in its place the issue of a 128 x 128 x 16 MMA takes 68 to 80 cycles, the more the busier the
 // other warps of the scheduler are, with the elected lane 64, as long as the MMA itself
-// (benchmarks/tcgen05_issue_probe.cu).
+// (148 CTAs, 2000 steps of 40 MMAs and five commits each, ten warps beside the issuer copying, loading or calculating).
 #define FSA_UMMA_LEAD(NAME, KIND, AFMT, ATYPE, ACONS)                                                        \
   __device__ __forceinline__ void NAME(uint32_t lead, uint32_t d_tmem, ATYPE a, uint64_t bdesc, uint32_t idesc, \
                                        uint32_t accumulate) {                                                \
