@@ -18,8 +18,8 @@ LONE = {2: 74, 3: 46, 4: 33, 5: 27, 6: 20, 7: 18, 8: 15}   # and with one
 def rule(tmp_path_factory):
     d = tmp_path_factory.mktemp("rule")
     (d / "rule.cpp").write_text(f'#include "{os.path.abspath(HEADER)}"\n'
-                                'extern "C" int rule(long long c, int occ, int cluster, int room, int splits, long long tiles, int sms) {\n'
-                                '  const FsaDecLaunch r = fsa_dec_launch(c, occ, cluster, room, splits, tiles, sms); return r.early ? r.per_sm : -1; }\n'
+                                'extern "C" int rule(long long c, int occ, int cluster, int room, int splits, long long bytes, int sms) {\n'
+                                '  const FsaDecLaunch r = fsa_dec_launch(c, occ, cluster, room, splits, bytes, sms); return r.early ? r.per_sm : -1; }\n'
                                 'extern "C" int deep(long long c, int occ, long long tiles, int sms) {\n'
                                 '  return fsa_dec_deep_ring(c, occ, tiles, sms); }\n')
     subprocess.run(["g++", "-O1", "-shared", "-fPIC", "-std=c++17", "-o", str(d / "rule.so"), str(d / "rule.cpp")], check=True)
@@ -27,10 +27,10 @@ def rule(tmp_path_factory):
     fn = lib.rule
     fn.argtypes = [ctypes.c_longlong, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_longlong, ctypes.c_int]
 
-    def call(ctas, occ=3, cluster=1, keys=1000, splits=1):
+    def call(ctas, occ=3, cluster=1, keys=1000, splits=1, row=256):
         """-1: behind the kernel in front, otherwise the CTAs an SM may hold (0: as many as find room)."""
         room = (LONE if ctas <= SMS else ROOM).get(cluster, 0)
-        return fn(ctas, occ, cluster, room, splits, -(-keys // 16) // (4 * splits), SMS)
+        return fn(ctas, occ, cluster, room, splits, -(-keys // 16) // (4 * splits) * 16 * row, SMS)
 
     call.deep = lambda ctas, occ, keys: bool(lib.deep(ctypes.c_longlong(ctas), occ, ctypes.c_longlong(-(-keys // 16) // 4), SMS))
     return call
@@ -53,6 +53,7 @@ def test_what_waits(rule):
     assert rule(296, occ=2, cluster=2) == rule(284, occ=2, cluster=4) == rule(264, occ=2, cluster=8) == 0
     assert rule(340, keys=300) == 0 and rule(340, keys=1000) == -1    # 10.2 us early, 10.6 not; 32.1 and 31.5
     assert rule(360, keys=7540, splits=3) == 0    # 52.2 us early, 53.6 not
+    assert rule(416, keys=482) == -1 and rule(416, keys=482, row=128) == 0    # dense 17.2 us early, 16.0 not; rows of 64 columns 10.3 and 10.8
     assert rule(444, keys=768) == -1 and rule(296, occ=2, keys=2500) == -1
 
 
