@@ -81,14 +81,15 @@ inline int fsa_fwd_cluster_size(long long ctas, int tiles, int sms, Room room) {
 
 // Decode: whether a call is set up while the kernel in front of it still runs, and how many of its CTAs an SM may hold then (0: as many
 // as find room). `occ`: CTAs that find room on an SM; `cluster`: CTAs of a cluster (1: none), `room`: clusters that are resident at a
-// time; `splits`: of the keys, merged by a kernel behind this one unless in the cluster; `bytes`: of the key rows that a warp walks. Setting it up early saves 0.3 to 1 us, but the SMs that the kernel in front leaves first would take
-// as many CTAs as fit, and others none. Of calls of one round, us, over and over, one split, 4 KV heads of 128:
+// time; `splits`: of the keys, merged by a kernel behind this one unless in the cluster; `bytes`: of the key rows that a warp walks.
+// Setting it up early saves 0.3 to 1 us, but the SMs that the kernel in front leaves first would take as many CTAs as fit, and others
+// none. Of calls of one round, us, over and over, one split, 4 KV heads of 128:
 // - fewer to an SM than fit: the share is kept to what an even spread is. 280 CTAs of 300 keys 9.8 early, 9.0 behind one another, 8.9
-//   so; 260 of 2500 keys 54.1, 53.6 and 53.3; 128 in clusters of four 13.6, 13.4 and 13.0; gated, behind the pass over delta, 100 of 1000 keys
-//   36.5, 32.0 and 31.5.
-// - as many as fit: it pays where a call is short (340 CTAs of 300 keys 10.2 early, 10.6 not; of 1000 keys 32.1 and 31.5;
-//   416 of 482 keys 17.2 and 16.0, of 64 columns 10.3 and 10.8) and where the kernel
-//   in front is a merge of splits (15 sequences of 471 to 7540 keys, 8 KV heads, three splits: 52.2 early, 53.6 not).
+//   so; 260 of 2500 keys 54.1, 53.6 and 53.3; 128 in clusters of four 13.6, 13.4 and 13.0; gated, behind the pass over delta, 100 of 1000
+//   keys 36.5, 32.0 and 31.5.
+// - as many as fit: it pays where a call is short (340 CTAs of 300 keys 10.2 early, 10.6 not; of 1000 keys 32.1 and 31.5; 416 of 482 keys
+//   17.2 and 16.0, of 64 columns 10.3 and 10.8) and where the kernel in front is a merge of splits (15 sequences of 471 to 7540 keys,
+//   8 KV heads, three splits: 52.2 early, 53.6 not).
 // - nearly all clusters that are resident: the last ones find no room until the call in front has left (56 clusters of five 15.8 early, 12.6
 //   not; 48 12.3 and 12.7). Not so with two, four or eight, which a GPC's even number of SMs holds without a rest (32 of eight 13.0 and 13.2).
 struct FsaDecLaunch {
